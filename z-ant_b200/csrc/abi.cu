@@ -24,6 +24,7 @@
 #include "dwconv_q8.cuh"
 #include "smallc_conv_q8.cuh"
 #include "tc_conv_nhwc.cuh"
+#include "small_gemm_q8.cuh"
 #include "status.hpp"
 
 using namespace zb;
@@ -856,6 +857,19 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
 }
 
 int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, const size_t* a_shape, size_t a_rank,
+    if (host_consts && small_gemm_eligible(g, wz_zero)) {
+        // few output positions: warp-level MMAs, K split over the warps of many small CTAs
+        SmallGemmPrep prep;
+        const size_t taps = (size_t)g.KH * g.KW;
+        small_gemm_prepare(g, w, (size_t)g.Cg * taps, taps, 1, mult.data(), bias, x_zp, ctx->sm_count, prep);
+        Stager s(ctx);
+        const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
+        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(prep.bias.data(), prep.bias.size() * 4);
+        ZB_TRY(s.commit());
+        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+        return s.finish();
+    }
                                 float a_scale, int32_t a_zp, const int8_t* b, const size_t* b_shape, size_t b_rank,
                                 const float* b_scale, const int32_t* b_zp, size_t n_b_scale, float y_scale, int32_t y_zp,
                                 const int32_t* bias, size_t bias_len, int32_t y_dtype, void* y, const size_t* y_shape, size_t y_rank,
@@ -915,6 +929,20 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
 }
 
 int32_t zant_b200_qlinearadd(zant_ctx* ctx, int32_t dtype, const void* a, float a_scale, int32_t a_zp,
+    if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && y_dtype != ZANT_I32 && bz_zero && !is_device_ptr(b) && !(bias && is_device_ptr(bias))) {
+        ConvGeom g{};
+        g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
+        g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
+        SmallGemmPrep prep;
+        small_gemm_prepare(g, b, 1, N, 0, mult.data(), bias, a_zp, ctx->sm_count, prep);
+        Stager s(ctx);
+        const int ix = s.in(a, M * K), iy = s.out(y, M * N);
+        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ibb = s.in(prep.bias.data(), prep.bias.size() * 4);
+        ZB_TRY(s.commit());
+        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+        return s.finish();
+    }
                              const void* b, float b_scale, int32_t b_zp, float y_scale, int32_t y_zp, void* y, size_t n,
                              int32_t activation) {
     if (!q8_dtype(dtype)) return fail(ZANT_E_INPUT_ARRAY_WRONG_TYPE, "QLinearAdd tensors must be int8 or uint8");

@@ -26,6 +26,7 @@
 #include "smallc_conv_q8.cuh"
 #include "tc_conv_nhwc.cuh"
 #include "tc_gemm_tf32.cuh"
+#include "small_gemm_q8.cuh"
 #include "status.hpp"
 
 using namespace zb;
@@ -641,6 +642,19 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
     push("QLinearConv" + tail, [=]() {
         QConvArgs q{};
         q.x = pl->ptr(x); q.w = pl->p<int8_t>(w); q.y = pl->ptr(y);
+    if (const_bias && small_gemm_eligible(g, wz_zero)) {
+        // few output positions: warp-level MMAs, K split over the warps of many small CTAs
+        auto prep = std::make_shared<SmallGemmPrep>();
+        const size_t taps = (size_t)g.KH * g.KW;
+        small_gemm_prepare(g, (const int8_t*)T(w).host.data(), (size_t)g.Cg * taps, taps, 1, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, ctx->sm_count, *prep);
+        const int aw = pl->add_aux(prep->wfrag.data(), prep->wfrag.size() * 4), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4), ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
+        prep->wfrag.clear(); prep->wfrag.shrink_to_fit();
+        push("QLinearConv" + tail, [=]() {
+            return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
+                                  pl->ptr(y), yd == ZANT_U8, rq_of());
+        });
+        return ZANT_OK;
+    }
         q.mult = (const float*)pl->aux(am); q.w_zp = (const int32_t*)pl->aux(az); q.bias = pl->p<int32_t>(b);
         q.x_zp = xzp; q.rq = rq_of(); q.g = g;
         return run_qconv_generic(ctx, q, xd, yd);
@@ -1015,6 +1029,23 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
             push("QLinearMatMul", [=]() {
                 QMatArgs q{};
                 q.a = pl->ptr(x); q.b = pl->p<int8_t>(w); q.y = pl->ptr(y);
+            if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && yd != ZANT_I32 && (b < 0 || T(b).is_const)) {
+                ConvGeom g{};
+                g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
+                g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
+                if (small_gemm_eligible(g, bz_zero)) {
+                    auto prep = std::make_shared<SmallGemmPrep>();
+                    small_gemm_prepare(g, (const int8_t*)T(w).host.data(), 1, N, 0, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, ctx->sm_count, *prep);
+                    const int aw = pl->add_aux(prep->wfrag.data(), prep->wfrag.size() * 4), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4);
+                    const int ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
+                    prep->wfrag.clear(); prep->wfrag.shrink_to_fit();
+                    push("QLinearMatMul", [=]() {
+                        return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
+                                              pl->ptr(y), yd == ZANT_U8, rq);
+                    });
+                    return ZANT_OK;
+                }
+            }
                 q.mult = (const float*)pl->aux(am); q.b_zp = (const int32_t*)pl->aux(az); q.bias = pl->p<int32_t>(b);
                 q.a_zp = xzp; q.rq = rq; q.M = (int)M; q.N = (int)N; q.K = (int)K; q.y_i32 = yd == ZANT_I32;
                 return run_qmatmul_generic(ctx, q, xd, yd);
