@@ -156,7 +156,8 @@ int32_t zant_b200_ctx_set_arena_limit(zant_ctx* ctx, size_t max_bytes);
 /* The stream kernels are launched on (a cudaStream_t as void*). */
 void* zant_b200_ctx_stream(zant_ctx* ctx);
 int32_t zant_b200_ctx_synchronize(zant_ctx* ctx);
-/* Kernels launched by this context since creation (or since the last reset). */
+/* Operator kernels launched by this context since creation (or since the last reset); the launch that re-orders the
+ * weights a single-operator call brought along is part of staging them and is not counted. */
 uint64_t zant_b200_ctx_launch_count(zant_ctx* ctx);
 void zant_b200_ctx_reset_launch_count(zant_ctx* ctx);
 

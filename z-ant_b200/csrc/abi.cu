@@ -25,6 +25,7 @@
 #include "smallc_conv_q8.cuh"
 #include "tc_conv_nhwc.cuh"
 #include "small_gemm_q8.cuh"
+#include "weight_blocks.cuh"
 #include "status.hpp"
 
 using namespace zb;
@@ -92,6 +93,7 @@ int32_t zant_b200_ctx_destroy(zant_ctx* ctx) {
     if (!ctx) return ZANT_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    delete ctx->stage;
     if (ctx->arena) cudaFree(ctx->arena);
     if (ctx->status_word) cudaFree(ctx->status_word);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -733,14 +735,16 @@ int32_t zant_b200_qlinearconv_nhwc(zant_ctx* ctx, int32_t x_dtype, const void* x
     if (w_zp) for (size_t i = 0; i < n_w_scale; ++i) wz_zero = wz_zero && w_zp[i] == 0;
     TcConvPlan tcp;
     if (!tc_conv_nhwc_plan(g, wz_zero, x_zp, tcp)) return fail(ZANT_E_UNSUPPORTED, "shape not taken by the channels-last QLinearConv kernel");
-    std::vector<int8_t> w_blk; std::vector<float> mp; std::vector<int32_t> bp;
-    tc_conv_nhwc_prepare(tcp, w, mult.data(), bias, x_zp, w_blk, mp, bp);
+    mult.resize(tcp.a.m_pad, 1.0f);
+    const WBlockArgs wb = weight_blocks_of(tcp, x_zp, true);
     Stager s(ctx);
     const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-    const int iw = s.in(w_blk.data(), w_blk.size()), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bp.data(), bp.size() * 4);
+    const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+    const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
     ZB_TRY(s.commit());
-    ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
-                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, tc_conv_max_product(mp, bp, (long long)g.Cg * g.KH * g.KW)));
+    ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+    ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, weight_blocks_max_product(mult, bias, true, (long long)g.Cg * g.KH * g.KW)));
     return s.finish();
 }
 
@@ -769,22 +773,23 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
     for (int32_t v : wz) wz_zero = wz_zero && v == 0;
     const bool host_consts = !is_device_ptr(w) && !(bias && is_device_ptr(bias));
     PwConvPlan pwp;
-    if (host_consts && (!is_device_ptr(x) || pw_conv_ptr_ok(x, nullptr)) && (!is_device_ptr(y) || pw_conv_ptr_ok(nullptr, y)) &&
+    if ((!is_device_ptr(x) || pw_conv_ptr_ok(x, nullptr)) && (!is_device_ptr(y) || pw_conv_ptr_ok(nullptr, y)) &&
         (pw_stem_plan(g, wz_zero, x_zp, ctx->sm_count, pwp) || pw_conv_plan(g, wz_zero, ctx->sm_count, pwp))) {
         // 1x1: filters on the accumulator lanes, activations straight from NCHW as the MN-major operand; 3x3 stems: the same
         // kernel on patches written in shared memory
-        std::vector<int8_t> w_blk; std::vector<int32_t> bf;
-        pw_conv_prepare(pwp, w, bias, x_zp, w_blk, bf);
         bool finite = true;
         for (float f : mult) finite = finite && std::isfinite(f);
         std::vector<int32_t> caps;
         const bool capped = finite && y_dtype == ZANT_I8 && y_zp == 0 && requant_relu_caps(mult.data(), mult.size(), activation, lean_six(y_scale), caps);
+        const WBlockArgs wb = weight_blocks_of(pwp, x_zp);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(w_blk.data(), w_blk.size()), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bf.data(), bf.size() * 4);
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int ic = capped ? s.in(caps.data(), caps.size() * 4) : -1;
+        const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
         ZB_TRY(s.commit());
-        ZB_TRY(pw_conv_run(ctx, pwp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+        ZB_TRY(pw_conv_run(ctx, pwp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, finite, capped ? s.ptr<int32_t>(ic) : nullptr));
         return s.finish();
     }
@@ -801,16 +806,21 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         return s.finish();
     }
     TcConvPlan tcp;
-    if (host_consts && (long long)g.N * g.OH * g.OW >= 256 && (!is_device_ptr(x) || tc_conv_ptr_ok(x)) && tc_conv_plan(g, wz_zero, tcp)) {
+    if ((long long)g.N * g.OH * g.OW >= 256 && (!is_device_ptr(x) || tc_conv_ptr_ok(x)) && tc_conv_plan(g, wz_zero, tcp)) {
         // implicit GEMM straight from NCHW (stride 1): no im2col matrix
-        std::vector<int8_t> w_blk; std::vector<float> mp; std::vector<int32_t> bp;
-        tc_conv_prepare(tcp, w, mult.data(), bias, x_zp, w_blk, mp, bp);
+        std::vector<float> mp(mult);
+        mp.resize(tcp.a.m_pad, 1.0f);
+        const WBlockArgs wb = weight_blocks_of(tcp, x_zp, false);
+        const bool bias_dev = bias && is_device_ptr(bias);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(w_blk.data(), w_blk.size()), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bp.data(), bp.size() * 4);
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+        const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
         ZB_TRY(s.commit());
-        ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
-                           s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, tc_conv_max_product(mp, bp, (long long)g.Cg * g.KH * g.KW)));
+        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+        ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                           s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation},
+                           weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, (long long)g.Cg * g.KH * g.KW)));
         return s.finish();
     }
     if (host_consts && qdwconv_eligible(g, wz_zero) && (!is_device_ptr(x) || qdwconv_ptr_ok(x)) && (!is_device_ptr(y) || qdwconv_ptr_ok(y))) {
@@ -830,18 +840,34 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, finite, capped ? s.ptr<int32_t>(ic) : nullptr));
         return s.finish();
     }
-    if (qconv_tc_eligible(g, wz_zero) && host_consts) {
+    if (qconv_tc_eligible(g, wz_zero)) {
         // tensor-core path: im2col into the GEMM-blocked layout, tcgen05 GEMM, NCHW requantised store
         QGemmPrep prep;
-        qconv_gemm_prepare(g, w, mult.data(), bias, x_zp, prep);
+        qgemm_sizes(g.M, g.Cg * g.KH * g.KW, mult.data(), prep, (long long)g.N * g.OH * g.OW);
+        prep.tap_major = qconv_tap_major(g);
+        const WBlockArgs wb = weight_blocks_of(prep, g.M, g.Cg, g.KH * g.KW, x_zp);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(prep.w_blk.data(), prep.w_blk.size()), im = s.in(prep.mult.data(), prep.mult.size() * 4);
-        const int ib = s.in(prep.bias.data(), prep.bias.size() * 4);
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int ia = s.scratch(qgemm_a_bytes((size_t)g.N * g.OH * g.OW, prep));
+        const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
         ZB_TRY(s.commit());
-        ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, prep, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+        ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                             s.ptr<uint8_t>(ia), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+        return s.finish();
+    }
+    if (host_consts && small_gemm_eligible(g, wz_zero)) {
+        // few output positions: warp-level MMAs, K split over the warps of many small CTAs
+        SmallGemmPrep prep;
+        const size_t taps = (size_t)g.KH * g.KW;
+        small_gemm_prepare(g, w, (size_t)g.Cg * taps, taps, 1, mult.data(), bias, x_zp, ctx->sm_count, prep);
+        Stager s(ctx);
+        const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
+        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(prep.bias.data(), prep.bias.size() * 4);
+        ZB_TRY(s.commit());
+        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
         return s.finish();
     }
     Stager s(ctx);
@@ -857,19 +883,6 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
 }
 
 int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, const size_t* a_shape, size_t a_rank,
-    if (host_consts && small_gemm_eligible(g, wz_zero)) {
-        // few output positions: warp-level MMAs, K split over the warps of many small CTAs
-        SmallGemmPrep prep;
-        const size_t taps = (size_t)g.KH * g.KW;
-        small_gemm_prepare(g, w, (size_t)g.Cg * taps, taps, 1, mult.data(), bias, x_zp, ctx->sm_count, prep);
-        Stager s(ctx);
-        const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(prep.bias.data(), prep.bias.size() * 4);
-        ZB_TRY(s.commit());
-        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
-                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-        return s.finish();
-    }
                                 float a_scale, int32_t a_zp, const int8_t* b, const size_t* b_shape, size_t b_rank,
                                 const float* b_scale, const int32_t* b_zp, size_t n_b_scale, float y_scale, int32_t y_zp,
                                 const int32_t* bias, size_t bias_len, int32_t y_dtype, void* y, const size_t* y_shape, size_t y_rank,
@@ -899,21 +912,36 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
         ConvGeom g{};   // a matrix product is a 1x1 convolution over M "images" of one pixel
         g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
         g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
-        if (y_dtype != ZANT_I32 && qconv_tc_eligible(g, bz_zero) && !is_device_ptr(b) && !(bias && is_device_ptr(bias))) {
-            std::vector<int8_t> bt(K * N);
-            for (size_t k = 0; k < K; ++k) for (size_t j = 0; j < N; ++j) bt[j * K + k] = b[k * N + j];
+        if (y_dtype != ZANT_I32 && qconv_tc_eligible(g, bz_zero)) {
             QGemmPrep prep;
-            qgemm_prepare(bt.data(), (int)N, (int)K, mult.data(), bias, a_zp, prep);
+            qgemm_sizes((int)N, (int)K, mult.data(), prep);
+            WBlockArgs wb = weight_blocks_of(prep, (int)N, (int)K, 1, a_zp);
+            wb.sm = 1; wb.sc = N;                                       // [K][N]
             Stager s(ctx);
             const int ix = s.in(a, M * K), iy = s.out(y, M * N);
-            const int iw = s.in(prep.w_blk.data(), prep.w_blk.size()), im = s.in(prep.mult.data(), prep.mult.size() * 4);
-            const int ibb = s.in(prep.bias.data(), prep.bias.size() * 4);
+            const int iw = s.in(b, K * N), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, N * 4);
             const int isc = s.scratch(qgemm_a_bytes(M, prep));
+            const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
             ZB_TRY(s.commit());
-            ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, prep, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                                 s.ptr<uint8_t>(isc), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
             return s.finish();
         }
+    }
+    if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && y_dtype != ZANT_I32 && bz_zero && !is_device_ptr(b) && !(bias && is_device_ptr(bias))) {
+        ConvGeom g{};
+        g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
+        g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
+        SmallGemmPrep prep;
+        small_gemm_prepare(g, b, 1, N, 0, mult.data(), bias, a_zp, ctx->sm_count, prep);
+        Stager s(ctx);
+        const int ix = s.in(a, M * K), iy = s.out(y, M * N);
+        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ibb = s.in(prep.bias.data(), prep.bias.size() * 4);
+        ZB_TRY(s.commit());
+        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+        return s.finish();
     }
     Stager s(ctx);
     const int ia = s.in(a, M * K), ib = s.in(b, K * N), iy = s.out(y, M * N * dtype_size(y_dtype));
@@ -929,20 +957,6 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
 }
 
 int32_t zant_b200_qlinearadd(zant_ctx* ctx, int32_t dtype, const void* a, float a_scale, int32_t a_zp,
-    if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && y_dtype != ZANT_I32 && bz_zero && !is_device_ptr(b) && !(bias && is_device_ptr(bias))) {
-        ConvGeom g{};
-        g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
-        g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
-        SmallGemmPrep prep;
-        small_gemm_prepare(g, b, 1, N, 0, mult.data(), bias, a_zp, ctx->sm_count, prep);
-        Stager s(ctx);
-        const int ix = s.in(a, M * K), iy = s.out(y, M * N);
-        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ibb = s.in(prep.bias.data(), prep.bias.size() * 4);
-        ZB_TRY(s.commit());
-        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-        return s.finish();
-    }
                              const void* b, float b_scale, int32_t b_zp, float y_scale, int32_t y_zp, void* y, size_t n,
                              int32_t activation) {
     if (!q8_dtype(dtype)) return fail(ZANT_E_INPUT_ARRAY_WRONG_TYPE, "QLinearAdd tensors must be int8 or uint8");

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "host_stage.cuh"
 #include "status.hpp"
 
 struct zant_ctx {
@@ -19,6 +20,7 @@ struct zant_ctx {
     uint64_t launches = 0;
     int sm_count = 148;
     int* status_word = nullptr;   // device int: kernels with bounded waits report here
+    zb::HostStage* stage = nullptr;   // page-locked ring for pageable host buffers, created on first use
     int tf32 = 0;                 // float contractions: 0 = the exact FP32 kernels, 1 = tensor cores (kind::tf32, single pass), 2 = tensor cores, split operands (3 x TF32)
 };
 
@@ -62,12 +64,36 @@ inline int32_t check_launch(zant_ctx* ctx, const char* what) {
     return ZANT_OK;
 }
 
+// Where a host-visible copy of the status word lands: the context's page-locked ring where there is one.
+inline HostStage* host_stage(zant_ctx* ctx) {
+    if (!ctx->stage) ctx->stage = HostStage::create();
+    return ctx->stage;
+}
+
+// Host buffer -> device, ordered on the context's stream; `src` may be changed as soon as this returns.
+inline cudaError_t copy_to_device(zant_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return cudaSuccess;
+    if (HostStage* st = host_stage(ctx)) return st->to_device(dst, src, bytes, ctx->stream);
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);      // no page-locked memory to be had
+}
+
 // Drains the stream and reads the device status word that kernels with bounded waits write when
-// they give up; a non-zero value is reported once and cleared.
-inline int32_t drain_and_check_status(zant_ctx* ctx) {
+// they give up; a non-zero value is reported once and cleared.  With `host_dst` the same wait also brings a result back
+// (`bytes` from device memory): one synchronisation for both.
+inline int32_t drain_and_check_status(zant_ctx* ctx, void* host_dst = nullptr, const void* dev_src = nullptr, size_t bytes = 0) {
     int h = 0;
-    ZB_CUDA(cudaMemcpyAsync(&h, ctx->status_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    char* slot = nullptr;
+    if (ctx->stage || (host_dst && bytes && bytes + 256 <= HostStage::kSlot)) {
+        const size_t want = 256 + ((bytes + 256 <= HostStage::kSlot) ? bytes : 0);
+        if (HostStage* st = host_stage(ctx)) slot = (char*)st->result_slot(want, ctx->stream);
+    }
+    const bool via_slot = slot && bytes && bytes + 256 <= HostStage::kSlot;
+    if (host_dst && bytes) ZB_CUDA(cudaMemcpyAsync(via_slot ? (void*)(slot + 256) : host_dst, dev_src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    ZB_CUDA(cudaMemcpyAsync(slot ? (void*)slot : (void*)&h, ctx->status_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (ctx->stage) ctx->stage->drained();
+    if (slot) h = *reinterpret_cast<volatile int*>(slot);
+    if (via_slot) std::memcpy(host_dst, slot + 256, bytes);
     if (h != 0) {
         ZB_CUDA(cudaMemsetAsync(ctx->status_word, 0, sizeof(int), ctx->stream));
         return fail(ZANT_E_DEVICE_TIMEOUT, "a kernel gave up a bounded wait (device error %d)", h);
@@ -75,28 +101,27 @@ inline int32_t drain_and_check_status(zant_ctx* ctx) {
     return ZANT_OK;
 }
 
-inline bool is_device_ptr(const void* p) {
-    if (!p) return false;
+// What a caller's pointer is: one driver query per buffer.
+struct PtrKind { bool device = false, foreign = false, pinned = false; };
+inline PtrKind ptr_kind(const void* p, int device) {
+    PtrKind k;
+    if (!p) return k;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return k;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    k.device = a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    // Device memory that belongs to another GPU than `device`: a kernel of this context must not be handed such a pointer
+    // (without peer access it would take an illegal-address fault, which is sticky for the whole CUDA context).  Managed
+    // memory migrates and is accepted on every device.
+    k.foreign = a.type == cudaMemoryTypeDevice && a.device != device;
+    // Page-locked host memory (cudaHostAlloc / cudaHostRegister): copies to and from it are truly asynchronous, so calls
+    // that are handed such buffers need not wait for the stream.
+    k.pinned = a.type == cudaMemoryTypeHost;
+    return k;
 }
-
-// Device memory that belongs to another GPU than `device`: a kernel of this context must not be
-// handed such a pointer (without peer access it would take an illegal-address fault, which is sticky
-// for the whole CUDA context).  Managed memory migrates and is accepted on every device.
-inline bool is_foreign_device_ptr(const void* p, int device) {
-    if (!p) return false;
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeDevice && a.device != device;
-}
+inline bool is_device_ptr(const void* p) { return ptr_kind(p, 0).device; }
 
 // Every device allocation of the library goes through here.  `alloc_failures_armed()` is the test
 // hook behind zant_b200_debug_fail_alloc: while it is positive it counts allocations down and the
@@ -114,18 +139,6 @@ inline cudaError_t dev_malloc(void** p, size_t bytes) {
         }
     }
     return cudaMalloc(p, bytes);
-}
-
-// Page-locked host memory (cudaHostAlloc / cudaHostRegister): copies to and from it are truly
-// asynchronous, so calls that are handed such buffers do not wait for the stream.
-inline bool is_pinned_host_ptr(const void* p) {
-    if (!p) return false;
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
 }
 
 constexpr size_t kArenaAlign = 256;
@@ -152,9 +165,12 @@ inline int32_t arena_reserve(zant_ctx* ctx, size_t need_total) {
 class Stager {
   public:
     explicit Stager(zant_ctx* c) : ctx_(c) {}
-    ~Stager() { if (ctx_) ctx_->arena_used = 0; }
+    ~Stager() {
+        if (!ctx_) return;
+        ctx_->arena_used = 0;
+    }
 
-    struct Slot { const void* host_in; void* host_out; size_t bytes; size_t off; void* dev; bool staged; };
+    struct Slot { const void* host_in; void* host_out; size_t bytes; size_t off; void* dev; bool staged; bool pinned = false; };
 
     int in(const void* p, size_t bytes) { return add(p, nullptr, bytes, true); }
     int out(void* p, size_t bytes) { return add(nullptr, p, bytes, false); }
@@ -177,31 +193,29 @@ class Stager {
         for (auto& s : slots_) {
             if (!s.staged) continue;
             s.dev = ctx_->arena + s.off;
-            if (s.host_in && s.bytes)
-                ZB_CUDA(cudaMemcpyAsync(s.dev, s.host_in, s.bytes, cudaMemcpyHostToDevice, ctx_->stream));
+            if (!s.host_in || !s.bytes) continue;
+            if (s.pinned) { ZB_CUDA(cudaMemcpyAsync(s.dev, s.host_in, s.bytes, cudaMemcpyHostToDevice, ctx_->stream)); wait_ = true; }
+            else ZB_CUDA(copy_to_device(ctx_, s.dev, s.host_in, s.bytes));
         }
         return ZANT_OK;
     }
 
     template <typename T> T* ptr(int i) { return reinterpret_cast<T*>(slots_[i].dev); }
 
-    // Copies staged outputs back and, if anything was staged, waits for the stream.
+    // Copies staged outputs back and waits for the stream when there is one, or when the device still reads the caller's
+    // page-locked input.  (Pageable inputs left through the context's ring: nothing to wait for.)
     int32_t finish() {
-        bool any = false;
+        Slot* last = nullptr;
         for (auto& s : slots_) {
-            if (!s.staged) continue;
-            any = true;
-            if (s.host_out && s.bytes)
-                ZB_CUDA(cudaMemcpyAsync(s.host_out, s.dev, s.bytes, cudaMemcpyDeviceToHost, ctx_->stream));
+            if (!s.staged || !s.host_out || !s.bytes) continue;
+            if (last) ZB_CUDA(cudaMemcpyAsync(last->host_out, last->dev, last->bytes, cudaMemcpyDeviceToHost, ctx_->stream));
+            last = &s;
         }
-        if (any) {
-            // the call waits anyway: also pick up the status word that a bounded device-side wait writes
-            // when it gives up, so that the time-out is reported by the call that suffered it
-            const int32_t st = drain_and_check_status(ctx_);
-            ctx_->arena_used = 0;
-            return st;
-        }
-        return ZANT_OK;
+        ctx_->arena_used = 0;
+        if (!last && !wait_) return ZANT_OK;
+        // the call waits anyway: also pick up the status word that a bounded device-side wait writes
+        // when it gives up, so that the time-out is reported by the call that suffered it
+        return last ? drain_and_check_status(ctx_, last->host_out, last->dev, last->bytes) : drain_and_check_status(ctx_);
     }
 
   private:
@@ -209,14 +223,17 @@ class Stager {
         const void* p = is_in ? pin : pout;
         Slot s{nullptr, nullptr, bytes, 0, nullptr, false};
         if (p == nullptr) { s.dev = nullptr; }
-        else if (is_device_ptr(p)) { s.dev = const_cast<void*>(p); foreign_ = foreign_ || is_foreign_device_ptr(p, ctx_->device); }
-        else { s.staged = true; s.host_in = pin; s.host_out = pout; }
+        else {
+            const PtrKind k = ptr_kind(p, ctx_->device);
+            if (k.device) { s.dev = const_cast<void*>(p); foreign_ = foreign_ || k.foreign; }
+            else { s.staged = true; s.pinned = k.pinned; s.host_in = pin; s.host_out = pout; }
+        }
         slots_.push_back(s);
         return (int)slots_.size() - 1;
     }
     zant_ctx* ctx_;
     std::vector<Slot> slots_;
-    bool foreign_ = false;
+    bool foreign_ = false, wait_ = false;
 };
 
 inline int grid_for(size_t work_items, int block, int sm_count, int waves = 8) {

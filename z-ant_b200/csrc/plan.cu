@@ -313,11 +313,11 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     for (auto& t : plan->t) {
         if (t.alias >= 0 || t.elided) continue;
         t.arena_ptr = plan->arena + t.offset;
-        if (t.is_const && t.bytes) ZB_CUDA(cudaMemcpyAsync(t.arena_ptr, t.host.data(), t.bytes, cudaMemcpyHostToDevice, ctx->stream));
+        if (t.is_const && t.bytes) ZB_CUDA(copy_to_device(ctx, t.arena_ptr, t.host.data(), t.bytes));
     }
     for (size_t a = 0; a < plan->aux_host.size(); ++a)
         if (!plan->aux_host[a].empty())
-            ZB_CUDA(cudaMemcpyAsync(plan->arena + plan->aux_off[a], plan->aux_host[a].data(), plan->aux_host[a].size(), cudaMemcpyHostToDevice, ctx->stream));
+            ZB_CUDA(copy_to_device(ctx, plan->arena + plan->aux_off[a], plan->aux_host[a].data(), plan->aux_host[a].size()));
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
     for (auto& t : plan->t) { t.host.clear(); t.host.shrink_to_fit(); }
 
@@ -342,21 +342,34 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
     int out_root = plan->output;
     while (plan->t[out_root].alias >= 0) out_root = plan->t[out_root].alias;
     PlanTensor& tor = plan->t[out_root];
-    const bool in_dev = is_device_ptr(input), out_dev = is_device_ptr(output);
-    if (is_foreign_device_ptr(input, ctx->device) || is_foreign_device_ptr(output, ctx->device))
+    const PtrKind ki = ptr_kind(input, ctx->device), ko = ptr_kind(output, ctx->device);
+    const bool in_dev = ki.device, out_dev = ko.device;
+    // Pinned host buffers on both sides: the whole run stays asynchronous on the stream (the caller overlaps it with other
+    // contexts and calls zant_b200_ctx_synchronize).  Pageable buffers: wait, so that the result is in place when the call
+    // returns.
+    const bool async = out_dev || (ko.pinned && (in_dev || ki.pinned));
+    auto copy_in = [&]() -> cudaError_t {
+        if (in_dev || ki.pinned) return cudaMemcpyAsync(ti.arena_ptr, input, ti.bytes, in_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream);
+        return copy_to_device(ctx, ti.arena_ptr, input, ti.bytes);
+    };
+    // copies the result out; a call that has to wait reads the status word with the same synchronisation
+    auto copy_out = [&]() -> int32_t {
+        if (!async) return drain_and_check_status(ctx, output, tor.arena_ptr, to.bytes);
+        ZB_CUDA(cudaMemcpyAsync(output, tor.arena_ptr, to.bytes, out_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
+        return ZANT_OK;
+    };
+    if (ki.foreign || ko.foreign)
         return fail(ZANT_E_INVALID_INPUT, "input/output is device memory of another GPU than the plan's device %d", ctx->device);
     if (plan->graph_exec && !plan->profiling) {
         // replay: everything runs on the arena's own buffers
-        ZB_CUDA(cudaMemcpyAsync(ti.arena_ptr, input, ti.bytes, in_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
+        ZB_CUDA(copy_in());
         ZB_CUDA(cudaGraphLaunch(plan->graph_exec, ctx->stream));
         ctx->launches += (uint64_t)plan->launches_per_run;
-        ZB_CUDA(cudaMemcpyAsync(output, tor.arena_ptr, to.bytes, out_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
-        if (out_dev || (is_pinned_host_ptr(output) && (in_dev || is_pinned_host_ptr(input)))) return ZANT_OK;
-        return drain_and_check_status(ctx);
+        return copy_out();
     }
     ti.bound = in_dev ? const_cast<void*>(input) : nullptr;
     tor.bound = out_dev ? output : nullptr;
-    if (!in_dev) ZB_CUDA(cudaMemcpyAsync(ti.arena_ptr, input, ti.bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (!in_dev) ZB_CUDA(copy_in());
     auto mark = [&]() -> int32_t {
         if (plan->prof_used == plan->prof_events.size()) {
             cudaEvent_t e;
@@ -372,17 +385,8 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
         if (st != ZANT_OK) { ti.bound = nullptr; tor.bound = nullptr; return st; }
     }
     if (plan->profiling) { int32_t st = mark(); if (st != ZANT_OK) return st; }
-    if (!out_dev) {
-        ZB_CUDA(cudaMemcpyAsync(output, tor.arena_ptr, to.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        ti.bound = nullptr; tor.bound = nullptr;
-        // Pinned host buffers on both sides: the whole run stays asynchronous on the stream (the
-        // caller overlaps it with other contexts and calls zant_b200_ctx_synchronize).  Pageable
-        // buffers: wait, so that the result is in place when the call returns.
-        if (is_pinned_host_ptr(output) && (in_dev || is_pinned_host_ptr(input))) return ZANT_OK;
-        return drain_and_check_status(ctx);
-    }
     ti.bound = nullptr; tor.bound = nullptr;
-    return ZANT_OK;
+    return out_dev ? ZANT_OK : copy_out();
 }
 
 int32_t zant_b200_plan_use_graph(zant_plan* plan, int32_t enable) {
@@ -638,10 +642,6 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         });
         return ZANT_OK;
     }
-    const int am = pl->add_aux(mult.data(), mult.size() * 4), az = pl->add_aux(wzv.data(), wzv.size() * 4);
-    push("QLinearConv" + tail, [=]() {
-        QConvArgs q{};
-        q.x = pl->ptr(x); q.w = pl->p<int8_t>(w); q.y = pl->ptr(y);
     if (const_bias && small_gemm_eligible(g, wz_zero)) {
         // few output positions: warp-level MMAs, K split over the warps of many small CTAs
         auto prep = std::make_shared<SmallGemmPrep>();
@@ -655,6 +655,10 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         });
         return ZANT_OK;
     }
+    const int am = pl->add_aux(mult.data(), mult.size() * 4), az = pl->add_aux(wzv.data(), wzv.size() * 4);
+    push("QLinearConv" + tail, [=]() {
+        QConvArgs q{};
+        q.x = pl->ptr(x); q.w = pl->p<int8_t>(w); q.y = pl->ptr(y);
         q.mult = (const float*)pl->aux(am); q.w_zp = (const int32_t*)pl->aux(az); q.bias = pl->p<int32_t>(b);
         q.x_zp = xzp; q.rq = rq_of(); q.g = g;
         return run_qconv_generic(ctx, q, xd, yd);
@@ -1025,10 +1029,6 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                     return ZANT_OK;
                 }
             }
-            const int am = pl->add_aux(mult.data(), mult.size() * 4), az = pl->add_aux(bz.data(), bz.size() * 4);
-            push("QLinearMatMul", [=]() {
-                QMatArgs q{};
-                q.a = pl->ptr(x); q.b = pl->p<int8_t>(w); q.y = pl->ptr(y);
             if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && yd != ZANT_I32 && (b < 0 || T(b).is_const)) {
                 ConvGeom g{};
                 g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
@@ -1046,6 +1046,10 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                     return ZANT_OK;
                 }
             }
+            const int am = pl->add_aux(mult.data(), mult.size() * 4), az = pl->add_aux(bz.data(), bz.size() * 4);
+            push("QLinearMatMul", [=]() {
+                QMatArgs q{};
+                q.a = pl->ptr(x); q.b = pl->p<int8_t>(w); q.y = pl->ptr(y);
                 q.mult = (const float*)pl->aux(am); q.b_zp = (const int32_t*)pl->aux(az); q.bias = pl->p<int32_t>(b);
                 q.a_zp = xzp; q.rq = rq; q.M = (int)M; q.N = (int)N; q.K = (int)K; q.y_i32 = yd == ZANT_I32;
                 return run_qmatmul_generic(ctx, q, xd, yd);

@@ -181,7 +181,7 @@ struct QGemmPrep {
 // w: [n_out][K] int8 row-major (a convolution's [M][C][KH][KW] weight is exactly that).
 // `rows` (when known) lets wide outputs pick the tile width that wastes the least of the last wave of
 // 148 persistent CTAs: 256-wide tiles halve the number of tiles but a partly filled wave costs a full one.
-inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p, long long rows = 0) {
+inline void qgemm_sizes(int n_out, int K, const float* mult, QGemmPrep& p, long long rows = 0) {
     p.NT = n_out <= 64 ? 64 : (n_out <= 128 ? 128 : 256);
     if (p.NT == 256 && rows > 0) {
         const long long mt = (rows + 127) / 128;
@@ -192,8 +192,16 @@ inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, 
     p.N_pad = (n_out + p.NT - 1) / p.NT * p.NT;
     p.K = K;
     p.K16 = K <= 32 ? 2 : (K + 63) / 64 * 4;      // a stage holds 4 chunks of K (2 when K fits 32: first layers with 3 channels)
-    p.w_blk.assign((size_t)p.N_pad * p.K16 * 16, 0);
     p.mult.assign(p.N_pad, 1.0f);
+    for (int n = 0; n < n_out; ++n) {
+        p.mult[n] = mult[n];
+        p.mult_finite = p.mult_finite && std::isfinite(mult[n]);
+    }
+}
+
+inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p, long long rows = 0) {
+    qgemm_sizes(n_out, K, mult, p, rows);
+    p.w_blk.assign((size_t)p.N_pad * p.K16 * 16, 0);
     p.bias.assign(p.N_pad, 0);
     for (int n = 0; n < n_out; ++n) {
         int sum = 0;
@@ -203,8 +211,6 @@ inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, 
             dst_tile[(size_t)(k >> 4) * p.NT * 16 + (k & 15)] = wr[k];
             sum += wr[k];
         }
-        p.mult[n] = mult[n];
-        p.mult_finite = p.mult_finite && std::isfinite(mult[n]);
         p.bias[n] = (bias ? bias[n] : 0) - x_zp * sum;
     }
 }
@@ -212,10 +218,12 @@ inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, 
 // Convolution weights [M][C][KH][KW]: channel counts that are multiples of 16 (and more than one tap)
 // get the (tap, channel) K order that im2col_tapmajor_kernel produces; everything else keeps the
 // tensor's own order.
+inline bool qconv_tap_major(const ConvGeom& g) { return g.KH * g.KW > 1 && g.Cg % 16 == 0; }
+
 inline void qconv_gemm_prepare(const ConvGeom& g, const int8_t* w, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p) {
     const int taps = g.KH * g.KW, C = g.Cg, K = C * taps;
     const long long rows = (long long)g.N * g.OH * g.OW;
-    if (taps == 1 || C % 16 != 0) { qgemm_prepare(w, g.M, K, mult, bias, x_zp, p, rows); return; }
+    if (!qconv_tap_major(g)) { qgemm_prepare(w, g.M, K, mult, bias, x_zp, p, rows); return; }
     std::vector<int8_t> wt((size_t)g.M * K);
     for (int m = 0; m < g.M; ++m)
         for (int c = 0; c < C; ++c)
