@@ -1,6 +1,5 @@
-// FP32 kernels with the reference's arithmetic: every dot product is accumulated by ONE
-// thread in ascending k with a separate multiply and add (__fmul_rn/__fadd_rn are never
-// contracted into an FMA), so results are bit-identical to the reference's CPU loops.
+// FP32 kernels with the reference's arithmetic (the contractions are in contract_f32.cuh): multiplies and adds are
+// rounded separately (__fmul_rn/__fadd_rn are never contracted into an FMA), sums run in the reference's order.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -9,155 +8,6 @@
 #include "geometry.hpp"
 
 namespace zb {
-
-// ------------------------------------------------------------------------------------------
-// Tiled contraction  D[m,j] = sum_k A(m,k) * B(k,j)
-//   CONV = true : A is gathered on the fly from an NCHW input (implicit im2col, k = (c,kh,kw)
-//                 exactly as lean_im2col orders it), B(k,j) = W[j*K + k], D scattered to NCHW
-//                 with the bias added after the sum (op_convolution.zig:316-328).
-//   CONV = false: A(m,k) = a[m*sam + k*sak], B(k,j) = b[k*sbk + j*sbj] (covers MatMul and the
-//                 transposed operands of Gemm), then  v*alpha  and  + c*beta  as two separately
-//                 rounded steps (op_gemm.zig:128-178).
-// 64x64 output tile per CTA, 16-wide k slabs in shared memory, 4x4 outputs per thread.
-// ------------------------------------------------------------------------------------------
-struct ContractArgs {
-    const float* a; const float* b; float* d;
-    int M, N, K;
-    // plain-matrix strides (elements)
-    long long sam, sak, sbk, sbj;
-    // conv gather
-    ConvGeom g;
-    const float* bias;
-    // gemm epilogue
-    int epilogue;            // 0 plain store, 1 gemm (alpha, optional C)
-    float alpha, beta;
-    const float* c; int c_mode; long long c_rs, c_cs;   // c index = m*c_rs + j*c_cs
-};
-
-constexpr int CT_BM = 64, CT_BN = 64, CT_BK = 16, CT_PAD = 4;
-
-template <bool CONV>
-__global__ void __launch_bounds__(256) contract_f32_exact(const ContractArgs p) {
-    __shared__ float As[CT_BK][CT_BM + CT_PAD];
-    __shared__ float Bs[CT_BK][CT_BN + CT_PAD];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4x4 outputs each
-    const int m0 = blockIdx.x * CT_BM, j0 = blockIdx.y * CT_BN;
-
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-    // ---- A loader mapping
-    // conv / column-contiguous A: consecutive threads walk m (coalesced along ow);
-    // row-contiguous A (sak == 1): consecutive threads walk k.
-    const bool a_kfast = !CONV && p.sak == 1;
-    const int a_m = a_kfast ? (tid >> 4) : (tid & 63);     // + 16*i (k-fast)  |  fixed (m-fast)
-    const int a_k = a_kfast ? (tid & 15) : (tid >> 6);     // fixed (k-fast)    |  + 4*i (m-fast)
-    // conv: decode this thread's row once
-    int cn = 0, ih0 = 0, iw0 = 0;
-    bool row_ok = false;
-    if (CONV) {
-        const int m = m0 + a_m;
-        row_ok = m < p.M;
-        if (row_ok) {
-            const int ow = m % p.g.OW; const int t = m / p.g.OW;
-            const int oh = t % p.g.OH; cn = t / p.g.OH;
-            ih0 = oh * p.g.sh - p.g.pt; iw0 = ow * p.g.sw - p.g.pl;
-        }
-    }
-    const int khw = p.g.KH * p.g.KW;
-    // ---- B loader mapping: k-fast when B is k-contiguous (conv weights), else j-fast
-    const bool b_kfast = CONV || p.sbk == 1;
-    const int b_j = b_kfast ? (tid >> 4) : (tid & 63);
-    const int b_k = b_kfast ? (tid & 15) : (tid >> 6);
-
-    for (int k0 = 0; k0 < p.K; k0 += CT_BK) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float v = 0.0f;
-            if (CONV) {
-                const int k = k0 + a_k + 4 * i;
-                if (row_ok && k < p.K) {
-                    const int c = k / khw; const int r = k - c * khw;
-                    const int kh = r / p.g.KW; const int kw = r - kh * p.g.KW;
-                    const int ih = ih0 + kh * p.g.dh, iw = iw0 + kw * p.g.dw;
-                    if (ih >= 0 && ih < p.g.H && iw >= 0 && iw < p.g.W)
-                        v = __ldg(p.a + (((long long)cn * p.g.C + c) * p.g.H + ih) * p.g.W + iw);
-                }
-                As[a_k + 4 * i][a_m] = v;
-            } else if (a_kfast) {
-                const int m = m0 + a_m + 16 * i, k = k0 + a_k;
-                if (m < p.M && k < p.K) v = __ldg(p.a + (long long)m * p.sam + (long long)k * p.sak);
-                As[a_k][a_m + 16 * i] = v;
-            } else {
-                const int m = m0 + a_m, k = k0 + a_k + 4 * i;
-                if (m < p.M && k < p.K) v = __ldg(p.a + (long long)m * p.sam + (long long)k * p.sak);
-                As[a_k + 4 * i][a_m] = v;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float v = 0.0f;
-            if (b_kfast) {
-                const int j = j0 + b_j + 16 * i, k = k0 + b_k;
-                if (j < p.N && k < p.K)
-                    v = CONV ? __ldg(p.b + (long long)j * p.K + k)
-                             : __ldg(p.b + (long long)k * p.sbk + (long long)j * p.sbj);
-                Bs[b_k][b_j + 16 * i] = v;
-            } else {
-                const int j = j0 + b_j, k = k0 + b_k + 4 * i;
-                if (j < p.N && k < p.K) v = __ldg(p.b + (long long)k * p.sbk + (long long)j * p.sbj);
-                Bs[b_k + 4 * i][b_j] = v;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < CT_BK; ++kk) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(av[i], bv[j]));
-        }
-        __syncthreads();
-    }
-
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= p.M) continue;
-        if (CONV) {
-            const int ow = m % p.g.OW; const int t = m / p.g.OW;
-            const int oh = t % p.g.OH; const int n = t / p.g.OH;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int f = j0 + tx * 4 + j;
-                if (f >= p.N) continue;
-                const float bv = p.bias ? __ldg(p.bias + f) : 0.0f;
-                p.d[(((long long)n * p.g.M + f) * p.g.OH + oh) * p.g.OW + ow] = __fadd_rn(acc[i][j], bv);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int col = j0 + tx * 4 + j;
-                if (col >= p.N) continue;
-                float v = acc[i][j];
-                if (p.epilogue == 1) {
-                    v = __fmul_rn(v, p.alpha);
-                    if (p.c_mode) v = __fadd_rn(v, __fmul_rn(__ldg(p.c + (long long)m * p.c_rs + (long long)col * p.c_cs), p.beta));
-                }
-                p.d[(long long)m * p.N + col] = v;
-            }
-        }
-    }
-}
 
 // Element-wise pass over the part of a Gemm result that lies beyond the first matrix of a
 // batched tensor: the reference scales the WHOLE result tensor by alpha and adds beta*C to all

@@ -1,9 +1,12 @@
 // Device-level operator launchers: resolved geometry + device pointers -> kernel launches on
 // the context's stream.  Shared by the single-operator C entry points and by the plan.
 #pragma once
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include "context.cuh"
 #include "geometry.hpp"
+#include "contract_f32.cuh"
 #include "kernels_f32.cuh"
 #include "kernels_q8.cuh"
 
@@ -12,30 +15,76 @@ namespace zb {
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---------------------------------------------------------------------------- fp32
-inline int32_t run_conv_f32(zant_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
+// What a fused step applies to a contraction's finished sums.
+struct ContractFusion { int act = CT_ACT_NONE; float slope = 0.0f; const float* bias = nullptr; bool pool = false; };
+
+template <bool CONV, bool POOL, int BM, int BN, int TM, int TN>
+inline int32_t launch_contract_tile(zant_ctx* ctx, const ContractArgs& p) {
+    constexpr int smem = contract_smem<BM, BN>();
+    ZB_SMEM_ATTR(ctx, (contract_f32_tile<CONV, POOL, BM, BN, TM, TN>), smem);
+    const dim3 grid((unsigned)((p.M + BM - 1) / BM), (unsigned)((p.N + BN - 1) / BN));
+    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
+    contract_f32_tile<CONV, POOL, BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), smem, ctx->stream>>>(p);
+    return check_launch(ctx, "contract_f32_tile");
+}
+
+// Tile by cost: waves of tiles over the SMs times the tile's outputs over the share of the FP32 rate a tile of that shape
+// reaches (8 x 8 sums per thread keep the pipe busy; fewer spend more of their slots on operands).
+template <bool CONV, bool POOL>
+inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
+    p.neg_zero = 0x8000000080000000ull;
+    struct Shape { int bm, bn; double rate; };
+    static const Shape shapes[] = {{128, 128, 1.0}, {128, 64, 0.85}, {128, 32, 0.75}, {128, 16, 0.5}, {32, 32, 0.4}, {CF_BM, CF_BN, 0.12}};
+    int best = 0; double cost = 1e300;
+    for (int i = 0; i < 6; ++i) {
+        const double tiles = std::ceil((double)p.M / shapes[i].bm) * std::ceil((double)p.N / shapes[i].bn);
+        const double c = std::ceil(tiles / ctx->sm_count) * shapes[i].bm * shapes[i].bn / shapes[i].rate;
+        if (c < cost) { cost = c; best = i; }
+    }
+    switch (best) {
+        case 0: return launch_contract_tile<CONV, POOL, 128, 128, 8, 8>(ctx, p);
+        case 1: return launch_contract_tile<CONV, POOL, 128, 64, 8, 4>(ctx, p);
+        case 2: return launch_contract_tile<CONV, POOL, 128, 32, 8, 4>(ctx, p);
+        case 3: return launch_contract_tile<CONV, POOL, 128, 16, 4, 4>(ctx, p);
+        case 4: return launch_contract_tile<CONV, POOL, 32, 32, 4, 2>(ctx, p);
+        default: break;
+    }
+    constexpr int smem = contract_few_smem();
+    ZB_SMEM_ATTR(ctx, (contract_f32_few<CONV, POOL>), smem);
+    const dim3 grid((unsigned)((p.M + CF_BM - 1) / CF_BM), (unsigned)((p.N + CF_BN - 1) / CF_BN));
+    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
+    contract_f32_few<CONV, POOL><<<grid, 256, smem, ctx->stream>>>(p);
+    return check_launch(ctx, "contract_f32_few");
+}
+
+// `w_kn`: the weights as [K][N rounded up to 4] (a plan transposes them once), else null and `w` is [M][C][KH][KW].
+inline int32_t run_conv_f32(zant_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y,
+                            const ContractFusion& fu = ContractFusion{}, const float* w_kn = nullptr) {
     ContractArgs p{};
-    p.a = x; p.b = w; p.d = y; p.bias = bias; p.g = g;
-    const long long M = (long long)g.N * g.OH * g.OW;
+    p.a = x; p.b = w; p.d = y; p.bias = bias; p.g = g; p.act = fu.act; p.slope = fu.slope;
+    p.PH = g.OH / 2; p.PW = g.OW / 2;
+    const long long M = (long long)g.N * (fu.pool ? 4LL * p.PH * p.PW : (long long)g.OH * g.OW);
     if (M > 0x7fffffffLL) return fail(ZANT_E_TOO_LARGE, "Conv output pixels exceed int range");
     p.M = (int)M; p.N = g.M; p.K = g.C * g.KH * g.KW;
-    dim3 grid((p.M + CT_BM - 1) / CT_BM, (p.N + CT_BN - 1) / CT_BN);
-    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output channels");
-    contract_f32_exact<true><<<grid, 256, 0, ctx->stream>>>(p);
-    return check_launch(ctx, "contract_f32_exact<conv>");
+    p.padded = g.pt > 0 || g.pl > 0 || (g.OH - 1) * g.sh - g.pt + (g.KH - 1) * g.dh >= g.H || (g.OW - 1) * g.sw - g.pl + (g.KW - 1) * g.dw >= g.W;
+    p.y_vec = (g.OH * g.OW) % 4 == 0 && aligned16(y);
+    if (w_kn) { p.b = w_kn; p.sbk = (g.M + 3) / 4 * 4; p.sbj = 1; p.b_vec = 1; }
+    else { p.sbk = 1; p.sbj = p.K; }
+    return fu.pool ? launch_contract<true, true>(ctx, p) : launch_contract<true, false>(ctx, p);
 }
 
 inline int32_t run_contract_f32(zant_ctx* ctx, ContractArgs& p) {
-    dim3 grid((p.M + CT_BM - 1) / CT_BM, (p.N + CT_BN - 1) / CT_BN);
-    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
-    contract_f32_exact<false><<<grid, 256, 0, ctx->stream>>>(p);
-    return check_launch(ctx, "contract_f32_exact<matrix>");
+    p.a_vec = p.sak == 1 && p.sam % 4 == 0 && p.K % 4 == 0 && aligned16(p.a);
+    p.b_vec = p.sbj == 1 && p.sbk % 4 == 0 && p.N % 4 == 0 && aligned16(p.b);
+    return launch_contract<false, false>(ctx, p);
 }
 
-inline int32_t run_matmul_f32(zant_ctx* ctx, const MatGeom& g, const float* a, const float* b, float* y) {
+inline int32_t run_matmul_f32(zant_ctx* ctx, const MatGeom& g, const float* a, const float* b, float* y, const ContractFusion& fu = ContractFusion{}) {
     if (g.M > 0x7fffffffULL || g.N > 0x7fffffffULL || g.K > 0x7fffffffULL) return fail(ZANT_E_TOO_LARGE, "MatMul dims exceed int range");
     ContractArgs p{};
     p.a = a; p.b = b; p.d = y; p.M = (int)g.M; p.N = (int)g.N; p.K = (int)g.K;
     p.sam = (long long)g.K; p.sak = 1; p.sbk = (long long)g.N; p.sbj = 1;
+    p.bias = fu.bias; p.act = fu.act; p.slope = fu.slope;
     return run_contract_f32(ctx, p);
 }
 
@@ -47,7 +96,7 @@ inline int32_t run_gemm_f32(zant_ctx* ctx, const GemmGeom& g, const float* a, co
     // A' = A^T when transA: A is [K, rows] row-major; B' = B^T when transB: B is [cols, K].
     p.sam = ta ? 1 : (long long)g.K; p.sak = ta ? (long long)g.rows : 1;
     p.sbk = tb ? 1 : (long long)g.cols; p.sbj = tb ? (long long)g.K : 1;
-    p.epilogue = 1; p.alpha = alpha; p.beta = beta; p.c = c; p.c_mode = g.c_mode;
+    p.gemm = 1; p.alpha = alpha; p.beta = beta; p.c = c; p.c_mode = g.c_mode;
     if (g.c_mode == 1) { p.c_rs = (long long)g.cols; p.c_cs = 1; }
     else if (g.c_mode == 2) { p.c_rs = g.c_rows == 1 ? 0 : (long long)g.c_cols; p.c_cs = g.c_cols == 1 ? 0 : 1; }
     int32_t st = run_contract_f32(ctx, p);

@@ -84,6 +84,7 @@ struct zant_plan {
     // one stream, so they can share it; it is as large as the largest request.
     // float activation that the fusion pass asks the next Conv step to apply, and the tensor that step writes instead of its own
     int pending_fact = 0; float pending_slope = 0.0f; int pending_y = -1; bool pending_used = false;
+    int pending_pool = -1;      // exact path: the 2x2 / 2 MaxPool behind that activation, as the tensor it writes
     int im2col_scratch = -1;
     int shared_im2col_scratch(size_t bytes) {
         if (im2col_scratch < 0) im2col_scratch = add_scratch(bytes);
@@ -714,7 +715,25 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                 pl->pending_used = true;
                 return ZANT_OK;
             }
-            push("Conv", [=]() { return run_conv_f32(ctx, g, pl->p<float>(x), pl->p<float>(w), pl->p<float>(b), pl->p<float>(y)); });
+            // exact path; constant weights are transposed once to [K][filters], the order the kernel's slabs have
+            const int K = g.C * g.KH * g.KW, N4 = (g.M + 3) / 4 * 4;
+            int at = -1;
+            if (T(w).is_const && (long long)K * N4 <= (1LL << 28)) {
+                std::vector<float> wt((size_t)K * N4, 0.0f);
+                const float* ws = (const float*)T(w).host.data();
+                for (int m = 0; m < g.M; ++m) for (int k = 0; k < K; ++k) wt[(size_t)k * N4 + m] = ws[(size_t)m * K + k];
+                at = pl->add_aux(wt.data(), wt.size() * 4);
+            }
+            const int fact = pl->pending_fact; const float fslope = pl->pending_slope;
+            const bool pool = pl->pending_pool >= 0;
+            const int yw = pool ? pl->pending_pool : (pl->pending_y >= 0 ? pl->pending_y : y);
+            pl->pending_used = pool || pl->pending_y >= 0;
+            const std::string name = std::string("Conv") + (fact == FACT_RELU ? "+Relu" : (fact == FACT_LEAKY ? "+LeakyRelu" : "")) + (pool ? "+MaxPool" : "");
+            push(name.c_str(), [=]() {
+                ContractFusion fu;
+                fu.act = fact == FACT_RELU ? CT_ACT_RELU : (fact == FACT_LEAKY ? CT_ACT_LEAKY : CT_ACT_NONE); fu.slope = fslope; fu.pool = pool;
+                return run_conv_f32(ctx, g, pl->p<float>(x), pl->p<float>(w), pl->p<float>(b), pl->p<float>(yw), fu, at >= 0 ? (const float*)pl->aux(at) : nullptr);
+            });
             return ZANT_OK;
         }
         case ZANT_OP_MATMUL: {
@@ -1162,30 +1181,83 @@ static int32_t try_fuse(zant_plan* pl, size_t i0, size_t& consumed) {
     return try_fuse_fconv_group(pl, i0, consumed);
 }
 
-// Float Conv -> Relu | LeakyRelu on the tensor-core path (context in TF32 mode): the activation runs in the GEMM's
-// epilogue.  The exact FP32 path is left node by node: it mirrors the reference's call sequence.
+// Float Conv -> [Relu | LeakyRelu] -> [MaxPool 2x2 / 2] and MatMul -> Add(row vector) -> [Relu | LeakyRelu] as one step: what
+// lies behind the contraction runs on its finished sums, in the nodes' own order and with their own roundings, so the exact
+// path stays bit-identical to the node-by-node plan.  (Tensor-core path: the activation behind a Conv only.)
 static int32_t try_fuse_fconv_group(zant_plan* pl, size_t i0, size_t& consumed) {
     consumed = 0;
-    if (!pl->ctx->tf32 || i0 + 1 >= pl->nodes.size()) return ZANT_OK;
-    const PlanNode& conv = pl->nodes[i0];
-    const PlanNode& act = pl->nodes[i0 + 1];
-    if (conv.op != ZANT_OP_CONV || conv.out.size() != 1) return ZANT_OK;
-    if ((act.op != ZANT_OP_RELU && act.op != ZANT_OP_LEAKY_RELU) || act.in.size() != 1 || act.out.size() != 1 || act.in[0] != conv.out[0]) return ZANT_OK;
-    if (pl->t[act.out[0]].dtype != ZANT_F32 || pl->t[act.out[0]].bytes != pl->t[conv.out[0]].bytes) return ZANT_OK;
+    const PlanNode& head = pl->nodes[i0];
+    const bool conv = head.op == ZANT_OP_CONV, mat = head.op == ZANT_OP_MATMUL && !pl->ctx->tf32;
+    if ((!conv && !mat) || head.out.size() != 1 || head.in.size() < 2 || i0 + 1 >= pl->nodes.size()) return ZANT_OK;
     ChainCtx c{pl, std::vector<int>(pl->t.size(), 0)};
     for (const PlanNode& n : pl->nodes) for (int id : n.in) if (id >= 0) c.consumers[id]++;
-    if (!only_feeds_next(c, conv.out[0])) return ZANT_OK;
-    pl->pending_fact = act.op == ZANT_OP_RELU ? FACT_RELU : FACT_LEAKY;
-    pl->pending_slope = act.a.alpha;
-    pl->pending_y = act.out[0];
-    pl->pending_used = false;
+    auto T = [&](int id) -> const PlanTensor& { return pl->t[id]; };
+    size_t j = i0 + 1;
+    int cur = head.out[0], bias = -1;
+    std::vector<int> interior;
+    if (mat) {
+        const PlanNode& add = pl->nodes[j];
+        if (add.op != ZANT_OP_ADD || add.in.size() != 2 || add.out.size() != 1 || add.in[0] != cur || !only_feeds_next(c, cur)) return ZANT_OK;
+        bias = add.in[1];
+        const auto& ys = T(cur).shape;
+        if (bias < 0 || T(bias).dtype != ZANT_F32 || T(cur).dtype != ZANT_F32 || T(add.out[0]).shape != ys || ys.empty()) return ZANT_OK;
+        // a row vector of the product's columns: the last dimension and nothing else
+        if (T(bias).shape.empty() || T(bias).shape.back() != ys.back() || numel(T(bias).shape.data(), T(bias).shape.size()) != ys.back() || T(bias).shape.size() > ys.size()) return ZANT_OK;
+        interior.push_back(cur);
+        cur = add.out[0];
+        ++j;
+    }
+    int fact = FACT_NONE; float slope = 0.0f;
+    if (j < pl->nodes.size() && only_feeds_next(c, cur)) {
+        const PlanNode& act = pl->nodes[j];
+        if ((act.op == ZANT_OP_RELU || act.op == ZANT_OP_LEAKY_RELU) && act.in.size() == 1 && act.out.size() == 1 && act.in[0] == cur &&
+            T(act.out[0]).dtype == ZANT_F32 && T(cur).dtype == ZANT_F32 && T(act.out[0]).bytes == T(cur).bytes) {
+            fact = act.op == ZANT_OP_RELU ? FACT_RELU : FACT_LEAKY; slope = act.a.alpha;
+            interior.push_back(cur);
+            cur = act.out[0];
+            ++j;
+        }
+    }
     const size_t first_step = pl->steps.size();
-    const int32_t st = build_node_impl(pl, i0, 1);
-    const bool used = pl->pending_used;
-    pl->pending_fact = FACT_NONE; pl->pending_slope = 0.0f; pl->pending_y = -1; pl->pending_used = false;
-    if (st != ZANT_OK) return st;
-    if (used) { pl->t[conv.out[0]].elided = true; consumed = 2; }
-    else consumed = 1;
+    if (mat) {
+        const int x = head.in[0], w = head.in[1];
+        ZB_TRY(need_inputs(head, 2, 2, "MatMul"));
+        MatGeom g;
+        ZB_TRY(matmul_check(T(x).shape.data(), T(x).shape.size(), T(w).shape.data(), T(w).shape.size(), T(head.out[0]).shape.data(), T(head.out[0]).shape.size(), g));
+        if (numel(T(head.out[0]).shape.data(), T(head.out[0]).shape.size()) != g.M * g.N) return ZANT_OK;      // (a batched product: only its first matrix is computed)
+        zant_ctx* ctx = pl->ctx;
+        const int yw = cur;
+        pl->steps.push_back([=]() {
+            ContractFusion fu;
+            fu.bias = pl->p<float>(bias); fu.act = fact == FACT_RELU ? CT_ACT_RELU : (fact == FACT_LEAKY ? CT_ACT_LEAKY : CT_ACT_NONE); fu.slope = slope;
+            return run_matmul_f32(ctx, g, pl->p<float>(x), pl->p<float>(w), pl->p<float>(yw), fu);
+        });
+        pl->step_names.push_back(std::string("MatMul+Add") + (fact == FACT_RELU ? "+Relu" : (fact == FACT_LEAKY ? "+LeakyRelu" : "")));
+    } else {
+        int pool_y = -1;
+        if (!pl->ctx->tf32 && j < pl->nodes.size() && only_feeds_next(c, cur)) {
+            const PlanNode& pool = pl->nodes[j];
+            if (pool.op == ZANT_OP_MAXPOOL && pool.in.size() == 1 && pool.out.size() == 1 && pool.in[0] == cur && pool2x2(pool.a) &&
+                T(pool.out[0]).dtype == ZANT_F32 && T(cur).dtype == ZANT_F32 && T(cur).shape.size() == 4 && T(pool.out[0]).shape.size() == 4) {
+                const auto& si = T(cur).shape; const auto& so = T(pool.out[0]).shape;
+                if (so[0] == si[0] && so[1] == si[1] && so[2] == si[2] / 2 && so[3] == si[3] / 2 && so[2] > 0 && so[3] > 0) {
+                    pool_y = pool.out[0];
+                    interior.push_back(cur);
+                    ++j;
+                }
+            }
+        }
+        if (interior.empty()) return ZANT_OK;
+        pl->pending_fact = fact; pl->pending_slope = slope; pl->pending_y = fact == FACT_NONE ? -1 : cur; pl->pending_pool = pool_y;
+        pl->pending_used = false;
+        const int32_t st = build_node_impl(pl, i0, 1);
+        const bool used = pl->pending_used;
+        pl->pending_fact = FACT_NONE; pl->pending_slope = 0.0f; pl->pending_y = -1; pl->pending_pool = -1; pl->pending_used = false;
+        if (st != ZANT_OK) return st;
+        if (!used) { interior.clear(); j = i0 + 1; }
+    }
+    for (int id : interior) pl->t[id].elided = true;
+    consumed = j - i0;
     record_step_cost(pl, first_step, i0, consumed);
     return ZANT_OK;
 }
