@@ -38,3 +38,16 @@ def test_pageable_transfers(ctx, n):
     x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
     for _ in range(2):
         assert np.array_equal(ctx.ReLU(x), np.maximum(x, 0))
+
+
+@pytest.mark.parametrize("N,C,H,W,M,k", [(1, 192, 18, 18, 160, 3),      # a 256-filter tile's weights leave no room for two stages
+                                         (2, 64, 3, 3, 16, 3), (1, 64, 5, 100, 48, 1)])   # mostly empty row blocks
+def test_channels_last_shapes_that_fill_tiles_badly(ctx, oracle, N, C, H, W, M, k):
+    rng = np.random.default_rng(C)
+    x = codes(rng, (N, C, H, W), I8)
+    w = rng.integers(-127, 128, (M, C, k, k), dtype=np.int8)
+    args = (np.array([0.01], np.float32), None, float(np.float32(0.02 * np.sqrt(C * k * k))), 0)
+    kw = dict(pads=(k // 2,) * 4)
+    want = oracle.qlinearconv(x, 0.02, 0, w, *args, **kw)
+    got = ctx.qlinearconv_nhwc(np.ascontiguousarray(x.transpose(0, 2, 3, 1)), 0.02, 0, w, *args, **kw)
+    assert np.array_equal(got.transpose(0, 3, 1, 2), want)

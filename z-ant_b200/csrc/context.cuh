@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "host_stage.cuh"
@@ -21,6 +22,7 @@ struct zant_ctx {
     int sm_count = 148;
     int* status_word = nullptr;   // device int: kernels with bounded waits report here
     zb::HostStage* stage = nullptr;   // page-locked ring for pageable host buffers, created on first use
+    bool in_plan = false;         // the launches are a plan's: weights and constants were written before the run
     int tf32 = 0;                 // float contractions: 0 = the exact FP32 kernels, 1 = tensor cores (kind::tf32, single pass), 2 = tensor cores, split operands (3 x TF32)
 };
 
@@ -56,6 +58,28 @@ namespace zb {
 #ifndef ZB_TRY
 #define ZB_TRY(expr) do { int32_t _s = (expr); if (_s != ZANT_OK) return _s; } while (0)
 #endif
+
+// Launches behind the stream's previous kernel with programmatic dependent launch: a network is a chain of launches of a few
+// microseconds each, and the next kernel's scheduling, barrier and TMEM set-up then overlap the previous one's tail.  Every
+// kernel launched this way calls ptx::grid_wait before it touches what another kernel wrote (ptx_sm100.cuh).
+template <typename... P, typename... A>
+inline void launch(zant_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // an error is picked up by check_launch
+}
+
+// The same for kernels that read their weights and per-filter constants before grid_wait: in a plan these were written long ago;
+// in a single-operator call the launch before may have written them, so the kernel starts when everything before it is done.
+template <typename... P, typename... A>
+inline void launch_const(zant_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    if (ctx->in_plan) launch(ctx, kernel, grid, block, smem, std::forward<A>(args)...);
+    else kernel<<<grid, block, smem, ctx->stream>>>(std::forward<A>(args)...);
+}
 
 inline int32_t check_launch(zant_ctx* ctx, const char* what) {
     cudaError_t e = cudaGetLastError();

@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "geometry.hpp"
+#include "ptx_sm100.cuh"
 
 namespace zb {
 
@@ -115,6 +116,7 @@ constexpr int contract_smem() { return CT_NS * CT_BK * (BM + 4 + BN + 4) * 4 + 3
 
 template <bool CONV, bool POOL, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) contract_f32_tile(const __grid_constant__ ContractArgs p) {
+    ptx::grid_start();
     constexpr int THREADS = (BM / TM) * (BN / TN), TX = BN / TN, LDA = BM + 4, LDB = BN + 4;
     extern __shared__ __align__(16) float ct_smem[];
     float* As = ct_smem;                                   // [stage][k][row]
@@ -307,6 +309,7 @@ constexpr int contract_few_smem() { return CF_NS * (CF_BM * (CF_BK + 4) + CF_BK 
 
 template <bool CONV, bool POOL>
 __global__ void __launch_bounds__(256) contract_f32_few(const __grid_constant__ ContractArgs p) {
+    ptx::grid_start();
     constexpr int LDA = CF_BK + 4;
     extern __shared__ __align__(16) float ct_smem[];
     float* As = ct_smem;                                   // [stage][row][k]

@@ -108,6 +108,7 @@ __device__ __forceinline__ uint32_t dw_load_unaligned(const QDwArgs& p, long lon
 // straight from global memory) whose OUTPUT rows are not (stride 2 from 28 x 28 to 14 x 14): only the output is staged.
 template <int STRIDE, bool XU8, bool LEAN, bool ALIGNED, bool SMEM = false, bool SIN = SMEM>
 __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
+    ptx::grid_start();
     extern __shared__ __align__(16) uint8_t dw_smem[];
     const int lane = threadIdx.x & 31;
     const int LW = 1 << p.log2LW;
@@ -298,6 +299,7 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
 // rows and the first output row are peeled off so that the row loop carries no range checks.
 template <bool XU8, bool LEAN>
 __global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwArgs p) {
+    ptx::grid_start();
     const int lane = threadIdx.x & 31;
     const int LW = 1 << p.log2LW;                            // lanes per plane, each 8 columns
     const int ppw = 32 >> p.log2LW;
@@ -395,6 +397,7 @@ struct QDwRowsArgs {
 
 template <bool XU8, bool LEAN, int W, int S>
 __global__ void __launch_bounds__(256) qdwconv3x3_rows_kernel(const QDwRowsArgs a) {
+    ptx::grid_start();
     constexpr int NA = (W + 2 + 3) / 4;                             // words that hold the bytes col -1 .. col W
     constexpr int OW = S == 1 ? W : W / 2;
     extern __shared__ __align__(128) uint8_t dw_rows_smem[];
@@ -538,6 +541,7 @@ __global__ void __launch_bounds__(256) qdwconv3x3_rows_kernel(const QDwRowsArgs 
 // TWO: a word may span two planes (H*W is not a multiple of 4), i.e. two channels with their own weights and constants.
 template <bool XU8, bool LEAN, bool TWO>
 __global__ void __launch_bounds__(256) qdwconv3x3_flat_kernel(const QDwArgs p, int Lw, int Lp, int kgroups) {
+    ptx::grid_start();
     const int t = threadIdx.x;
     if (t >= Lw * kgroups) return;
     const int P = p.H * p.W;
@@ -674,8 +678,8 @@ inline void qdwconv_prepare(const ConvGeom& g, const int8_t* w, const int32_t* b
 
 template <int STRIDE, bool ALIGNED>
 inline int32_t qdwconv_launch_s(zant_ctx* ctx, const QDwArgs& a, int grid, bool x_u8, bool lean) {
-    if (x_u8) { if (lean) qdwconv3x3_kernel<STRIDE, true, true, ALIGNED><<<grid, 256, 0, ctx->stream>>>(a); else qdwconv3x3_kernel<STRIDE, true, false, ALIGNED><<<grid, 256, 0, ctx->stream>>>(a); }
-    else { if (lean) qdwconv3x3_kernel<STRIDE, false, true, ALIGNED><<<grid, 256, 0, ctx->stream>>>(a); else qdwconv3x3_kernel<STRIDE, false, false, ALIGNED><<<grid, 256, 0, ctx->stream>>>(a); }
+    if (x_u8) { if (lean) launch(ctx, qdwconv3x3_kernel<STRIDE, true, true, ALIGNED>, grid, 256, 0, a); else launch(ctx, qdwconv3x3_kernel<STRIDE, true, false, ALIGNED>, grid, 256, 0, a); }
+    else { if (lean) launch(ctx, qdwconv3x3_kernel<STRIDE, false, true, ALIGNED>, grid, 256, 0, a); else launch(ctx, qdwconv3x3_kernel<STRIDE, false, false, ALIGNED>, grid, 256, 0, a); }
     return check_launch(ctx, "qdwconv3x3_kernel");
 }
 
@@ -683,10 +687,10 @@ template <int STRIDE, bool XU8, bool LEAN>
 inline int32_t qdwconv_launch_smem_t(zant_ctx* ctx, const QDwArgs& a, int grid, size_t smem, bool stage_in) {
     if (stage_in) {
         ZB_SMEM_ATTR(ctx, (qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, true>), 96 * 1024);
-        qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, true><<<grid, 256, smem, ctx->stream>>>(a);
+        launch(ctx, qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, true>, grid, 256, smem, a);
     } else {
         ZB_SMEM_ATTR(ctx, (qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, false>), 96 * 1024);
-        qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, false><<<grid, 256, smem, ctx->stream>>>(a);
+        launch(ctx, qdwconv3x3_kernel<STRIDE, XU8, LEAN, true, true, false>, grid, 256, smem, a);
     }
     return check_launch(ctx, "qdwconv3x3_kernel<smem>");
 }
@@ -729,8 +733,8 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
             const int ppw8 = 32 >> a.log2LW;
             const long long groups8 = ((long long)a.planes + ppw8 - 1) / ppw8;
             const int grid8 = (int)std::min<long long>((groups8 + 7) / 8, (long long)ctx->sm_count * 16);
-            if (x_u8) { if (lean) qdwconv3x3_s1w8_kernel<true, true><<<grid8, 256, 0, ctx->stream>>>(a); else qdwconv3x3_s1w8_kernel<true, false><<<grid8, 256, 0, ctx->stream>>>(a); }
-            else { if (lean) qdwconv3x3_s1w8_kernel<false, true><<<grid8, 256, 0, ctx->stream>>>(a); else qdwconv3x3_s1w8_kernel<false, false><<<grid8, 256, 0, ctx->stream>>>(a); }
+            if (x_u8) { if (lean) launch(ctx, qdwconv3x3_s1w8_kernel<true, true>, grid8, 256, 0, a); else launch(ctx, qdwconv3x3_s1w8_kernel<true, false>, grid8, 256, 0, a); }
+            else { if (lean) launch(ctx, qdwconv3x3_s1w8_kernel<false, true>, grid8, 256, 0, a); else launch(ctx, qdwconv3x3_s1w8_kernel<false, false>, grid8, 256, 0, a); }
             return check_launch(ctx, "qdwconv3x3_s1w8_kernel");
         }
     }
@@ -754,7 +758,7 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
             const size_t smem = (size_t)3 * in_stride + 2 * out_stride + 32;
             const int rgrid = (int)std::min<long long>(ra.batches, (long long)ctx->sm_count * 8);
             auto go = [&](auto kernel) -> int32_t {
-                kernel<<<rgrid, 256, smem, ctx->stream>>>(ra);
+                launch(ctx, kernel, rgrid, 256, smem, ra);
                 return check_launch(ctx, "qdwconv3x3_rows_kernel");
             };
             auto pick = [&](auto w_tag, auto s_tag) -> int32_t {
@@ -780,7 +784,7 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
             const long long periods = ((nb + 3) / 4 + Lw - 1) / Lw;
             const int fgrid = (int)std::min<long long>((periods + kg - 1) / kg, (long long)ctx->sm_count * 8);
             auto go = [&](auto kernel) -> int32_t {
-                kernel<<<fgrid, 256, 0, ctx->stream>>>(a, (int)Lw, Lp, kg);
+                launch(ctx, kernel, fgrid, 256, 0, a, (int)Lw, Lp, kg);
                 return check_launch(ctx, "qdwconv3x3_flat_kernel");
             };
             if (Lp == 1) {

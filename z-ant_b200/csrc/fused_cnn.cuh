@@ -92,6 +92,7 @@ constexpr int C1M_GROUP_BYTES = C1M_G * C1M_IMG_FLOATS * 4;   // 9408: a multipl
 // quantized bytes are double-buffered too, which leaves one __syncthreads per group.
 // Three CTAs per SM (80 registers per thread; a fourth would need 64 registers and spills).
 __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(const Conv1MmaArgs a) {
+    ptx::grid_start();
     __shared__ __align__(128) float stage[2][C1M_G * C1M_IMG_FLOATS];
     __shared__ uint32_t img2[2][C1M_G][28][8];   // quantized uint8 rows of 32 bytes (28 pixels + 4 pad)
     __shared__ __align__(8) uint64_t bars[2];
@@ -321,6 +322,8 @@ __global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_parity_kernel(const __
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    ptx::grid_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "geometry.hpp"
+#include "ptx_sm100.cuh"
 
 namespace zb {
 
@@ -15,6 +16,7 @@ namespace zb {
 __global__ void gemm_tail_f32(float* y, size_t begin, size_t total, float alpha,
                               const float* c, int c_mode, float beta,
                               size_t rows, size_t cols, size_t c_rows, size_t c_cols, size_t y_ch, size_t c_ch) {
+    ptx::grid_start();
     for (size_t i = begin + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float v = __fmul_rn(0.0f, alpha);   // untouched elements hold the zero the caller cleared them to
         (void)y_ch;
@@ -41,6 +43,7 @@ template <> __device__ __forceinline__ uint8_t pool_init<uint8_t>() { return 0; 
 
 template <typename T>
 __global__ void maxpool_nchw(const T* __restrict__ x, T* __restrict__ y, const PoolGeom g) {
+    ptx::grid_start();
     const size_t total = (size_t)g.NC * g.OH * g.OW;
     const bool small = total < 0xffffffffull;         // 32-bit index arithmetic: 64-bit division costs hundreds of instructions
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -74,6 +77,7 @@ __global__ void maxpool_nchw(const T* __restrict__ x, T* __restrict__ y, const P
 // the maximum of neighbouring bytes, and stores 4 outputs.  Same values as maxpool_nchw.
 template <bool SIGNED>
 __global__ void maxpool2x2s2_q8(const uint2* __restrict__ x, uint32_t* __restrict__ y, size_t planes_rows, int ow4, int w8) {
+    ptx::grid_start();
     // planes_rows = NC * OH output rows; an output row has ow4 words, its two input rows have w8 (= ow4) uint2 each
     const size_t total = planes_rows * (size_t)ow4;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -91,6 +95,7 @@ __global__ void maxpool2x2s2_q8(const uint2* __restrict__ x, uint32_t* __restric
 // reference's comparison chain (start at -inf, take a value only if it is greater), in the window's kh, kw order, so NaNs
 // are skipped exactly as there.
 __global__ void maxpool2x2s2_f32(const float4* __restrict__ x, float2* __restrict__ y, size_t planes_rows, int ow2, int w4) {
+    ptx::grid_start();
     const size_t total = planes_rows * (size_t)ow2;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / ow2;
@@ -118,6 +123,7 @@ struct CeilOp { __device__ float operator()(float v) const { return (isnan(v) ||
 // mul_lean / div_lean: equal sizes, one rounded operation per element.
 template <bool DIV>
 __global__ void binary_same_f32(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, size_t n) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         y[i] = DIV ? __fdiv_rn(a[i], b[i]) : __fmul_rn(a[i], b[i]);
 }
@@ -125,6 +131,7 @@ __global__ void binary_same_f32(const float* __restrict__ a, const float* __rest
 // lean_softmax: one thread per row walks it three times in index order (maximum; exp and running sum;
 // division), which reproduces the reference's summation order.
 __global__ void softmax_rows_f32(const float* __restrict__ x, float* __restrict__ y, size_t rows, size_t cols) {
+    ptx::grid_start();
     for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < rows; r += (size_t)gridDim.x * blockDim.x) {
         if (cols == 0) continue;
         const float* xr = x + r * cols;
@@ -139,6 +146,7 @@ __global__ void softmax_rows_f32(const float* __restrict__ x, float* __restrict_
 
 template <typename F>
 __global__ void unary_f32(const float* __restrict__ x, float* __restrict__ y, size_t n, bool vec, F f) {
+    ptx::grid_start();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     size_t done = 0;
@@ -158,6 +166,7 @@ __global__ void unary_f32(const float* __restrict__ x, float* __restrict__ y, si
 
 // Add of equal-sized tensors (lib_elementWise_math.zig:72-110).
 __global__ void add_same_f32(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, size_t n, bool vec) {
+    ptx::grid_start();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     size_t done = 0;
@@ -178,6 +187,7 @@ __global__ void add_same_f32(const float* __restrict__ a, const float* __restric
 // Broadcasting Add up to rank 4 (lib_elementWise_math.zig:112-209).
 struct BcastArgs { int rank; size_t out_shape[4]; size_t a_stride[4]; size_t b_stride[4]; size_t total; };
 __global__ void add_bcast_f32(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, const BcastArgs g) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < g.total; i += (size_t)gridDim.x * blockDim.x) {
         size_t rem = i, ia = 0, ib = 0;
         for (int d = g.rank - 1; d >= 0; --d) {
@@ -192,6 +202,7 @@ __global__ void add_bcast_f32(const float* __restrict__ a, const float* __restri
 // Sum of a tensor list in list order (lib_elementWise_math.zig:243-257).
 struct SumListArgs { const float* t[8]; int n; };
 __global__ void sum_list_f32(const SumListArgs l, float* __restrict__ y, size_t n, bool accumulate) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float s = accumulate ? y[i] : l.t[0][i];
         for (int k = accumulate ? 0 : 1; k < l.n; ++k) s = __fadd_rn(s, l.t[k][i]);
@@ -206,6 +217,7 @@ __global__ void sum_list_f32(const SumListArgs l, float* __restrict__ y, size_t 
 template <typename Word>
 __global__ void copy2d(const char* __restrict__ src, size_t sp, char* __restrict__ dst, size_t dp,
                        size_t row_words, size_t rows) {
+    ptx::grid_start();
     const size_t total = row_words * rows;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / row_words, w = i - r * row_words;
@@ -222,6 +234,7 @@ struct ResizeArgs { int rank; size_t out_shape[8]; size_t in_stride[8]; int axis
 // modulo cost hundreds of instructions per element; with them a 2.8 M-element nearest-neighbour upsampling took 33 us).
 template <typename T, typename IDX>
 __global__ void resize_gather(const T* __restrict__ x, T* __restrict__ y, const int32_t* __restrict__ table, const ResizeArgs g) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < g.total; i += (size_t)gridDim.x * blockDim.x) {
         IDX rem = (IDX)i, src = 0;
         for (int d = g.rank - 1; d >= 0; --d) {
@@ -243,6 +256,7 @@ struct ReduceArgs {
     size_t keep_ostride[8], keep_istride[8], red_size[8], red_istride[8];
 };
 __global__ void reduce_mean_f32(const float* __restrict__ x, float* __restrict__ y, const ReduceArgs g) {
+    ptx::grid_start();
     for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < g.out_total; o += (size_t)gridDim.x * blockDim.x) {
         size_t rem = o, base = 0;
         for (int i = 0; i < g.n_keep; ++i) { base += (rem / g.keep_ostride[i]) * g.keep_istride[i]; rem %= g.keep_ostride[i]; }
@@ -265,6 +279,7 @@ __global__ void reduce_mean_f32(const float* __restrict__ x, float* __restrict__
 // Mean of ALL elements into y[0] with the reference's strictly sequential sum
 // (lib_reduction_math.zig:120-128).  One thread: the order of additions is the contract.
 __global__ void reduce_all_mean_f32(const float* __restrict__ x, float* __restrict__ y, size_t n) {
+    ptx::grid_start();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         float s = 0.0f;
         for (size_t i = 0; i < n; ++i) s = __fadd_rn(s, x[i]);
@@ -281,6 +296,7 @@ struct StridedMapDev { int rank; long long out_dims[8]; long long in_stride[8]; 
 
 template <typename T>
 __global__ void strided_copy_k(const T* __restrict__ x, T* __restrict__ y, const StridedMapDev m) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m.total; i += (size_t)gridDim.x * blockDim.x) {
         size_t t = i;
         long long src = m.base;
@@ -296,6 +312,7 @@ __global__ void strided_copy_k(const T* __restrict__ x, T* __restrict__ y, const
 template <typename T>
 __global__ void gather_axis_k(const T* __restrict__ x, const int32_t* __restrict__ idx, T* __restrict__ y,
                               size_t outer, size_t n_idx, size_t inner, size_t axis_dim) {
+    ptx::grid_start();
     const size_t total = outer * n_idx * inner;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t j = i % inner, t = i / inner;

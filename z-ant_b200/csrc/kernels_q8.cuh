@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "geometry.hpp"
+#include "ptx_sm100.cuh"
 
 namespace zb {
 
@@ -161,6 +162,7 @@ template <bool U8> __device__ __forceinline__ void store_q(void* p, size_t i, in
 // ---------------------------------------------------------------------------- Quantize / Dequantize
 template <bool YU8>
 __global__ void quantize_linear_k(const float* __restrict__ x, void* __restrict__ y, size_t n, float scale, int zp, bool vec) {
+    ptx::grid_start();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     size_t done = 0;
@@ -188,6 +190,7 @@ __global__ void quantize_linear_k(const float* __restrict__ x, void* __restrict_
 
 template <typename Q>
 __global__ void dequantize_linear_k(const Q* __restrict__ q, float* __restrict__ y, size_t n, float scale, int zp) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         y[i] = __fmul_rn(__int2float_rn((int)q[i] - zp), scale);
 }
@@ -206,6 +209,7 @@ struct QConvArgs {
 
 template <bool XU8, bool YU8>
 __global__ void qconv_nchw_generic(const QConvArgs p) {
+    ptx::grid_start();
     const ConvGeom& g = p.g;
     const size_t total = (size_t)g.N * g.M * g.OH * g.OW;
     const int Mg = g.M / g.G;
@@ -247,6 +251,7 @@ struct QMatArgs {
 
 template <bool AU8, bool YU8>
 __global__ void qmatmul_generic(const QMatArgs p) {
+    ptx::grid_start();
     const size_t total = (size_t)p.M * p.N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int j = (int)(i % p.N); const size_t row = i / p.N;
@@ -264,6 +269,7 @@ __global__ void qmatmul_generic(const QMatArgs p) {
 template <bool U8>
 __global__ void qadd_k(const void* __restrict__ a, float a_s, int a_zp, const void* __restrict__ b, float b_s, int b_zp,
                        float y_s, int y_zp, int act, void* __restrict__ y, size_t n) {
+    ptx::grid_start();
     const int lo = sat_q<U8>(y_zp);
     const int six = sat_q<U8>(rne_clamped(__fdiv_rn(6.0f, y_s)) + y_zp);
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -283,6 +289,7 @@ __global__ void qadd_k(const void* __restrict__ a, float a_s, int a_zp, const vo
 template <bool U8>
 __global__ void __launch_bounds__(256) qadd_vec_k(const uint4* __restrict__ a, float a_s, int a_zp, const uint4* __restrict__ b, float b_s, int b_zp,
                                                   float y_s, int y_zp, int act, uint4* __restrict__ y, size_t n16) {
+    ptx::grid_start();
     const int t_lo = U8 ? 0 : -128, t_hi = U8 ? 255 : 127;
     const QuantFast qf = quant_fast(y_s, (float)(t_lo - y_zp), (float)(t_hi - y_zp));
     const int lo = sat_q<U8>(y_zp);
@@ -317,6 +324,7 @@ __global__ void __launch_bounds__(256) qadd_vec_k(const uint4* __restrict__ a, f
 template <bool U8>
 __global__ void qgap_k(const void* __restrict__ x, void* __restrict__ y, size_t planes, int hw,
                        float x_s, int x_zp, float y_s, int y_zp) {
+    ptx::grid_start();
     const int lane = threadIdx.x & 31;
     const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -341,6 +349,7 @@ __global__ void qgap_k(const void* __restrict__ x, void* __restrict__ y, size_t 
 template <bool U8>
 __global__ void qgap_small_k(const uint8_t* __restrict__ x, void* __restrict__ y, size_t planes, int hw,
                              float x_s, int x_zp, float y_s, int y_zp) {
+    ptx::grid_start();
     const size_t total = planes * (size_t)hw;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t pidx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pidx < planes; pidx += stride) {
@@ -367,6 +376,7 @@ __global__ void qgap_small_k(const uint8_t* __restrict__ x, void* __restrict__ y
 
 // ---------------------------------------------------------------------------- 256-entry table lookup
 __global__ void lut_q8_k(const uint8_t* __restrict__ x, uint8_t* __restrict__ y, size_t n, const uint8_t* __restrict__ lut_g, bool vec) {
+    ptx::grid_start();
     __shared__ uint8_t lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = lut_g[i];
     __syncthreads();

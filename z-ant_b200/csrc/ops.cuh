@@ -20,11 +20,14 @@ struct ContractFusion { int act = CT_ACT_NONE; float slope = 0.0f; const float* 
 
 template <bool CONV, bool POOL, int BM, int BN, int TM, int TN>
 inline int32_t launch_contract_tile(zant_ctx* ctx, const ContractArgs& p) {
-    constexpr int smem = contract_smem<BM, BN>();
-    ZB_SMEM_ATTR(ctx, (contract_f32_tile<CONV, POOL, BM, BN, TM, TN>), smem);
+    ZB_SMEM_ATTR(ctx, (contract_f32_tile<CONV, POOL, BM, BN, TM, TN>), 122880);
     const dim3 grid((unsigned)((p.M + BM - 1) / BM), (unsigned)((p.N + BN - 1) / BN));
+    // Up to three tiles per SM: ask for so much shared memory that no SM takes more than its share.  A grid that starts while
+    // its predecessor drains would otherwise pile up on the SMs that are free first (128 tiles, two to an SM: 290 -> 540 us).
+    const long long share = ((long long)grid.x * grid.y + ctx->sm_count - 1) / ctx->sm_count;
+    const size_t smem = std::max<size_t>(contract_smem<BM, BN>(), share == 1 ? 122880 : (share == 2 ? 81920 : (share == 3 ? 61440 : 0)));
     if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
-    contract_f32_tile<CONV, POOL, BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), smem, ctx->stream>>>(p);
+    launch(ctx, contract_f32_tile<CONV, POOL, BM, BN, TM, TN>, grid, (BM / TM) * (BN / TN), smem, p);
     return check_launch(ctx, "contract_f32_tile");
 }
 
@@ -53,7 +56,7 @@ inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     ZB_SMEM_ATTR(ctx, (contract_f32_few<CONV, POOL>), smem);
     const dim3 grid((unsigned)((p.M + CF_BM - 1) / CF_BM), (unsigned)((p.N + CF_BN - 1) / CF_BN));
     if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
-    contract_f32_few<CONV, POOL><<<grid, 256, smem, ctx->stream>>>(p);
+    launch(ctx, contract_f32_few<CONV, POOL>, grid, 256, smem, p);
     return check_launch(ctx, "contract_f32_few");
 }
 
@@ -103,7 +106,7 @@ inline int32_t run_gemm_f32(zant_ctx* ctx, const GemmGeom& g, const float* a, co
     if (st != ZANT_OK) return st;
     const size_t first = g.rows * g.cols, total = g.batch * first;
     if (total > first) {
-        gemm_tail_f32<<<grid_for(total - first, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
+        launch(ctx, gemm_tail_f32, grid_for(total - first, 256, ctx->sm_count), 256, 0, 
             y, first, total, alpha, c, g.c_mode, beta, g.rows, g.cols, g.c_rows, g.c_cols, 0, g.c_ch);
         st = check_launch(ctx, "gemm_tail_f32");
     }
@@ -122,9 +125,9 @@ inline int32_t run_maxpool(zant_ctx* ctx, const PoolGeom& g, const T* x, T* y) {
             const size_t words = total / 4;
             const int grid = grid_for(words, 256, ctx->sm_count, 16);
             if (std::is_signed<T>::value)
-                maxpool2x2s2_q8<true><<<grid, 256, 0, ctx->stream>>>((const uint2*)x, (uint32_t*)y, (size_t)g.NC * g.OH, g.OW / 4, g.W / 8);
+                launch(ctx, maxpool2x2s2_q8<true>, grid, 256, 0, (const uint2*)x, (uint32_t*)y, (size_t)g.NC * g.OH, g.OW / 4, g.W / 8);
             else
-                maxpool2x2s2_q8<false><<<grid, 256, 0, ctx->stream>>>((const uint2*)x, (uint32_t*)y, (size_t)g.NC * g.OH, g.OW / 4, g.W / 8);
+                launch(ctx, maxpool2x2s2_q8<false>, grid, 256, 0, (const uint2*)x, (uint32_t*)y, (size_t)g.NC * g.OH, g.OW / 4, g.W / 8);
             return check_launch(ctx, "maxpool2x2s2_q8");
         }
     }
@@ -134,11 +137,11 @@ inline int32_t run_maxpool(zant_ctx* ctx, const PoolGeom& g, const T* x, T* y) {
                           (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(y) & 7u) == 0;
         if (fast) {
             const size_t pairs = total / 2;
-            maxpool2x2s2_f32<<<grid_for(pairs, 256, ctx->sm_count, 16), 256, 0, ctx->stream>>>((const float4*)x, (float2*)y, (size_t)g.NC * g.OH, g.OW / 2, g.W / 4);
+            launch(ctx, maxpool2x2s2_f32, grid_for(pairs, 256, ctx->sm_count, 16), 256, 0, (const float4*)x, (float2*)y, (size_t)g.NC * g.OH, g.OW / 2, g.W / 4);
             return check_launch(ctx, "maxpool2x2s2_f32");
         }
     }
-    maxpool_nchw<T><<<grid_for(total, 256, ctx->sm_count), 256, 0, ctx->stream>>>(x, y, g);
+    launch(ctx, maxpool_nchw<T>, grid_for(total, 256, ctx->sm_count), 256, 0, x, y, g);
     return check_launch(ctx, "maxpool_nchw");
 }
 
@@ -146,21 +149,21 @@ template <typename F>
 inline int32_t run_unary_f32(zant_ctx* ctx, const float* x, float* y, size_t n, F f, const char* name) {
     if (n == 0) return ZANT_OK;
     const bool vec = aligned16(x) && aligned16(y);
-    unary_f32<F><<<grid_for(vec ? (n + 3) / 4 : n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(x, y, n, vec, f);
+    launch(ctx, unary_f32<F>, grid_for(vec ? (n + 3) / 4 : n, 256, ctx->sm_count), 256, 0, x, y, n, vec, f);
     return check_launch(ctx, name);
 }
 
 inline int32_t run_binary_same_f32(zant_ctx* ctx, const float* a, const float* b, float* y, size_t n, bool divide) {
     if (n == 0) return ZANT_OK;
     const int grid = grid_for(n, 256, ctx->sm_count);
-    if (divide) binary_same_f32<true><<<grid, 256, 0, ctx->stream>>>(a, b, y, n);
-    else binary_same_f32<false><<<grid, 256, 0, ctx->stream>>>(a, b, y, n);
+    if (divide) launch(ctx, binary_same_f32<true>, grid, 256, 0, a, b, y, n);
+    else launch(ctx, binary_same_f32<false>, grid, 256, 0, a, b, y, n);
     return check_launch(ctx, divide ? "div_f32" : "mul_f32");
 }
 
 inline int32_t run_softmax_f32(zant_ctx* ctx, const float* x, float* y, size_t rows, size_t cols) {
     if (rows == 0 || cols == 0) return ZANT_OK;
-    softmax_rows_f32<<<grid_for(rows, 128, ctx->sm_count), 128, 0, ctx->stream>>>(x, y, rows, cols);
+    launch(ctx, softmax_rows_f32, grid_for(rows, 128, ctx->sm_count), 128, 0, x, y, rows, cols);
     return check_launch(ctx, "softmax_rows_f32");
 }
 
@@ -168,13 +171,13 @@ inline int32_t run_add_f32(zant_ctx* ctx, const BcastGeom& g, const float* a, co
     if (g.total == 0) return ZANT_OK;
     if (g.same_size) {
         const bool vec = aligned16(a) && aligned16(b) && aligned16(y);
-        add_same_f32<<<grid_for(vec ? (g.total + 3) / 4 : g.total, 256, ctx->sm_count), 256, 0, ctx->stream>>>(a, b, y, g.total, vec);
+        launch(ctx, add_same_f32, grid_for(vec ? (g.total + 3) / 4 : g.total, 256, ctx->sm_count), 256, 0, a, b, y, g.total, vec);
         return check_launch(ctx, "add_same_f32");
     }
     BcastArgs k{};
     k.rank = g.rank; k.total = g.total;
     for (int d = 0; d < g.rank; ++d) { k.out_shape[d] = g.out_shape[d]; k.a_stride[d] = g.a_stride[d]; k.b_stride[d] = g.b_stride[d]; }
-    add_bcast_f32<<<grid_for(g.total, 256, ctx->sm_count), 256, 0, ctx->stream>>>(a, b, y, k);
+    launch(ctx, add_bcast_f32, grid_for(g.total, 256, ctx->sm_count), 256, 0, a, b, y, k);
     return check_launch(ctx, "add_bcast_f32");
 }
 
@@ -185,7 +188,7 @@ inline int32_t run_sum_list_f32(zant_ctx* ctx, const float* const* ts, size_t nt
         SumListArgs l{};
         l.n = (int)std::min<size_t>(8, nt - done);
         for (int i = 0; i < l.n; ++i) l.t[i] = ts[done + i];
-        sum_list_f32<<<grid_for(n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(l, y, n, done != 0);
+        launch(ctx, sum_list_f32, grid_for(n, 256, ctx->sm_count), 256, 0, l, y, n, done != 0);
         int32_t st = check_launch(ctx, "sum_list_f32");
         if (st != ZANT_OK) return st;
         done += l.n;
@@ -199,11 +202,11 @@ inline int32_t run_copy2d(zant_ctx* ctx, const void* src, size_t sp, void* dst, 
     const char* s = static_cast<const char*>(src);
     char* d = static_cast<char*>(dst);
     if ((bits & 15) == 0) {
-        copy2d<uint4><<<grid_for(row_bytes / 16 * rows, 256, ctx->sm_count), 256, 0, ctx->stream>>>(s, sp, d, dp, row_bytes / 16, rows);
+        launch(ctx, copy2d<uint4>, grid_for(row_bytes / 16 * rows, 256, ctx->sm_count), 256, 0, s, sp, d, dp, row_bytes / 16, rows);
     } else if ((bits & 3) == 0) {
-        copy2d<uint32_t><<<grid_for(row_bytes / 4 * rows, 256, ctx->sm_count), 256, 0, ctx->stream>>>(s, sp, d, dp, row_bytes / 4, rows);
+        launch(ctx, copy2d<uint32_t>, grid_for(row_bytes / 4 * rows, 256, ctx->sm_count), 256, 0, s, sp, d, dp, row_bytes / 4, rows);
     } else {
-        copy2d<uint8_t><<<grid_for(row_bytes * rows, 256, ctx->sm_count), 256, 0, ctx->stream>>>(s, sp, d, dp, row_bytes, rows);
+        launch(ctx, copy2d<uint8_t>, grid_for(row_bytes * rows, 256, ctx->sm_count), 256, 0, s, sp, d, dp, row_bytes, rows);
     }
     return check_launch(ctx, "copy2d");
 }
@@ -231,11 +234,11 @@ inline int32_t run_resize(zant_ctx* ctx, size_t esz, const void* x, void* y, con
     const int grid = grid_for(k.total, 256, ctx->sm_count);
     const bool small = k.total < 0x7fffffffull && s < 0x7fffffffull;      // s: elements of the input
     if (esz == 4) {
-        if (small) resize_gather<uint32_t, uint32_t><<<grid, 256, 0, ctx->stream>>>((const uint32_t*)x, (uint32_t*)y, table_dev, k);
-        else resize_gather<uint32_t, size_t><<<grid, 256, 0, ctx->stream>>>((const uint32_t*)x, (uint32_t*)y, table_dev, k);
+        if (small) launch(ctx, resize_gather<uint32_t, uint32_t>, grid, 256, 0, (const uint32_t*)x, (uint32_t*)y, table_dev, k);
+        else launch(ctx, resize_gather<uint32_t, size_t>, grid, 256, 0, (const uint32_t*)x, (uint32_t*)y, table_dev, k);
     } else {
-        if (small) resize_gather<uint8_t, uint32_t><<<grid, 256, 0, ctx->stream>>>((const uint8_t*)x, (uint8_t*)y, table_dev, k);
-        else resize_gather<uint8_t, size_t><<<grid, 256, 0, ctx->stream>>>((const uint8_t*)x, (uint8_t*)y, table_dev, k);
+        if (small) launch(ctx, resize_gather<uint8_t, uint32_t>, grid, 256, 0, (const uint8_t*)x, (uint8_t*)y, table_dev, k);
+        else launch(ctx, resize_gather<uint8_t, size_t>, grid, 256, 0, (const uint8_t*)x, (uint8_t*)y, table_dev, k);
     }
     return check_launch(ctx, "resize_gather");
 }
@@ -246,14 +249,14 @@ inline int32_t run_reduce_mean_f32(zant_ctx* ctx, const ReduceGeom& g, const flo
         return ZANT_OK;
     }
     if (g.mode == 1) {
-        reduce_all_mean_f32<<<1, 32, 0, ctx->stream>>>(x, y, g.total);
+        launch(ctx, reduce_all_mean_f32, 1, 32, 0, x, y, g.total);
         return check_launch(ctx, "reduce_all_mean_f32");
     }
     ReduceArgs k{};
     k.out_total = g.out_total; k.count = g.count; k.n_keep = g.n_keep; k.n_red = g.n_red;
     for (int i = 0; i < 8; ++i) { k.keep_ostride[i] = g.keep_ostride[i]; k.keep_istride[i] = g.keep_istride[i]; k.red_size[i] = g.red_size[i]; k.red_istride[i] = g.red_istride[i]; }
     if (g.out_total == 0) return ZANT_OK;
-    reduce_mean_f32<<<grid_for(g.out_total, 128, ctx->sm_count), 128, 0, ctx->stream>>>(x, y, k);
+    launch(ctx, reduce_mean_f32, grid_for(g.out_total, 128, ctx->sm_count), 128, 0, x, y, k);
     return check_launch(ctx, "reduce_mean_f32");
 }
 
@@ -262,17 +265,17 @@ inline int32_t run_quantize(zant_ctx* ctx, const float* x, void* y, size_t n, fl
     if (n == 0) return ZANT_OK;
     const bool vec = aligned16(x) && ((reinterpret_cast<uintptr_t>(y) & 3) == 0);
     const int grid = grid_for(vec ? (n + 3) / 4 : n, 256, ctx->sm_count);
-    if (out_dtype == ZANT_U8) quantize_linear_k<true><<<grid, 256, 0, ctx->stream>>>(x, y, n, scale, zp, vec);
-    else quantize_linear_k<false><<<grid, 256, 0, ctx->stream>>>(x, y, n, scale, zp, vec);
+    if (out_dtype == ZANT_U8) launch(ctx, quantize_linear_k<true>, grid, 256, 0, x, y, n, scale, zp, vec);
+    else launch(ctx, quantize_linear_k<false>, grid, 256, 0, x, y, n, scale, zp, vec);
     return check_launch(ctx, "quantize_linear_k");
 }
 
 inline int32_t run_dequantize(zant_ctx* ctx, int32_t in_dtype, const void* q, float* y, size_t n, float scale, int zp) {
     if (n == 0) return ZANT_OK;
     const int grid = grid_for(n, 256, ctx->sm_count);
-    if (in_dtype == ZANT_U8) dequantize_linear_k<uint8_t><<<grid, 256, 0, ctx->stream>>>((const uint8_t*)q, y, n, scale, zp);
-    else if (in_dtype == ZANT_I8) dequantize_linear_k<int8_t><<<grid, 256, 0, ctx->stream>>>((const int8_t*)q, y, n, scale, zp);
-    else dequantize_linear_k<int32_t><<<grid, 256, 0, ctx->stream>>>((const int32_t*)q, y, n, scale, zp);
+    if (in_dtype == ZANT_U8) launch(ctx, dequantize_linear_k<uint8_t>, grid, 256, 0, (const uint8_t*)q, y, n, scale, zp);
+    else if (in_dtype == ZANT_I8) launch(ctx, dequantize_linear_k<int8_t>, grid, 256, 0, (const int8_t*)q, y, n, scale, zp);
+    else launch(ctx, dequantize_linear_k<int32_t>, grid, 256, 0, (const int32_t*)q, y, n, scale, zp);
     return check_launch(ctx, "dequantize_linear_k");
 }
 
@@ -281,10 +284,10 @@ inline int32_t run_qconv_generic(zant_ctx* ctx, const QConvArgs& p, int32_t x_dt
     if (total == 0) return ZANT_OK;
     const int grid = grid_for(total, 128, ctx->sm_count, 32);
     const bool xu = x_dtype == ZANT_U8, yu = y_dtype == ZANT_U8;
-    if (xu && yu) qconv_nchw_generic<true, true><<<grid, 128, 0, ctx->stream>>>(p);
-    else if (xu) qconv_nchw_generic<true, false><<<grid, 128, 0, ctx->stream>>>(p);
-    else if (yu) qconv_nchw_generic<false, true><<<grid, 128, 0, ctx->stream>>>(p);
-    else qconv_nchw_generic<false, false><<<grid, 128, 0, ctx->stream>>>(p);
+    if (xu && yu) launch(ctx, qconv_nchw_generic<true, true>, grid, 128, 0, p);
+    else if (xu) launch(ctx, qconv_nchw_generic<true, false>, grid, 128, 0, p);
+    else if (yu) launch(ctx, qconv_nchw_generic<false, true>, grid, 128, 0, p);
+    else launch(ctx, qconv_nchw_generic<false, false>, grid, 128, 0, p);
     return check_launch(ctx, "qconv_nchw_generic");
 }
 
@@ -293,10 +296,10 @@ inline int32_t run_qmatmul_generic(zant_ctx* ctx, const QMatArgs& p, int32_t a_d
     if (total == 0) return ZANT_OK;
     const int grid = grid_for(total, 128, ctx->sm_count, 32);
     const bool au = a_dtype == ZANT_U8, yu = y_dtype == ZANT_U8;
-    if (au && yu) qmatmul_generic<true, true><<<grid, 128, 0, ctx->stream>>>(p);
-    else if (au) qmatmul_generic<true, false><<<grid, 128, 0, ctx->stream>>>(p);
-    else if (yu) qmatmul_generic<false, true><<<grid, 128, 0, ctx->stream>>>(p);
-    else qmatmul_generic<false, false><<<grid, 128, 0, ctx->stream>>>(p);
+    if (au && yu) launch(ctx, qmatmul_generic<true, true>, grid, 128, 0, p);
+    else if (au) launch(ctx, qmatmul_generic<true, false>, grid, 128, 0, p);
+    else if (yu) launch(ctx, qmatmul_generic<false, true>, grid, 128, 0, p);
+    else launch(ctx, qmatmul_generic<false, false>, grid, 128, 0, p);
     return check_launch(ctx, "qmatmul_generic");
 }
 
@@ -309,8 +312,8 @@ inline int32_t run_qadd(zant_ctx* ctx, int32_t dtype, const void* a, float a_s, 
     if (zp_ok && n >= 16 && aligned16(a) && aligned16(b) && aligned16(y)) {
         const size_t n16 = n / 16;
         const int grid = grid_for(n16, 256, ctx->sm_count);
-        if (u8) qadd_vec_k<true><<<grid, 256, 0, ctx->stream>>>((const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
-        else qadd_vec_k<false><<<grid, 256, 0, ctx->stream>>>((const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
+        if (u8) launch(ctx, qadd_vec_k<true>, grid, 256, 0, (const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
+        else launch(ctx, qadd_vec_k<false>, grid, 256, 0, (const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
         ZB_TRY(check_launch(ctx, "qadd_vec_k"));
         done = n16 * 16;
         if (done == n) return ZANT_OK;
@@ -318,8 +321,8 @@ inline int32_t run_qadd(zant_ctx* ctx, int32_t dtype, const void* a, float a_s, 
     const char* pa = (const char*)a + done; const char* pb = (const char*)b + done; char* py = (char*)y + done;
     const size_t rest = n - done;
     const int grid = grid_for(rest, 256, ctx->sm_count);
-    if (u8) qadd_k<true><<<grid, 256, 0, ctx->stream>>>(pa, a_s, a_zp, pb, b_s, b_zp, y_s, y_zp, act, py, rest);
-    else qadd_k<false><<<grid, 256, 0, ctx->stream>>>(pa, a_s, a_zp, pb, b_s, b_zp, y_s, y_zp, act, py, rest);
+    if (u8) launch(ctx, qadd_k<true>, grid, 256, 0, pa, a_s, a_zp, pb, b_s, b_zp, y_s, y_zp, act, py, rest);
+    else launch(ctx, qadd_k<false>, grid, 256, 0, pa, a_s, a_zp, pb, b_s, b_zp, y_s, y_zp, act, py, rest);
     return check_launch(ctx, "qadd_k");
 }
 
@@ -329,20 +332,20 @@ inline int32_t run_qgap(zant_ctx* ctx, int32_t dtype, const void* x, void* y, si
     if (hw <= 256 && planes >= 4096 && (reinterpret_cast<uintptr_t>(x) & 3u) == 0) {
         // many small planes: a thread per plane
         const int grid = grid_for(planes, 128, ctx->sm_count);
-        if (dtype == ZANT_U8) qgap_small_k<true><<<grid, 128, 0, ctx->stream>>>((const uint8_t*)x, y, planes, hw, x_s, x_zp, y_s, y_zp);
-        else qgap_small_k<false><<<grid, 128, 0, ctx->stream>>>((const uint8_t*)x, y, planes, hw, x_s, x_zp, y_s, y_zp);
+        if (dtype == ZANT_U8) launch(ctx, qgap_small_k<true>, grid, 128, 0, (const uint8_t*)x, y, planes, hw, x_s, x_zp, y_s, y_zp);
+        else launch(ctx, qgap_small_k<false>, grid, 128, 0, (const uint8_t*)x, y, planes, hw, x_s, x_zp, y_s, y_zp);
         return check_launch(ctx, "qgap_small_k");
     }
     const int grid = grid_for(planes * 32, 256, ctx->sm_count);
-    if (dtype == ZANT_U8) qgap_k<true><<<grid, 256, 0, ctx->stream>>>(x, y, planes, hw, x_s, x_zp, y_s, y_zp);
-    else qgap_k<false><<<grid, 256, 0, ctx->stream>>>(x, y, planes, hw, x_s, x_zp, y_s, y_zp);
+    if (dtype == ZANT_U8) launch(ctx, qgap_k<true>, grid, 256, 0, x, y, planes, hw, x_s, x_zp, y_s, y_zp);
+    else launch(ctx, qgap_k<false>, grid, 256, 0, x, y, planes, hw, x_s, x_zp, y_s, y_zp);
     return check_launch(ctx, "qgap_k");
 }
 
 inline int32_t run_lut(zant_ctx* ctx, const void* x, void* y, size_t n, const uint8_t* lut_dev) {
     if (n == 0) return ZANT_OK;
     const bool vec = aligned16(x) && aligned16(y);
-    lut_q8_k<<<grid_for(vec ? (n + 15) / 16 : n, 256, ctx->sm_count), 256, 0, ctx->stream>>>((const uint8_t*)x, (uint8_t*)y, n, lut_dev, vec);
+    launch(ctx, lut_q8_k, grid_for(vec ? (n + 15) / 16 : n, 256, ctx->sm_count), 256, 0, (const uint8_t*)x, (uint8_t*)y, n, lut_dev, vec);
     return check_launch(ctx, "lut_q8_k");
 }
 
@@ -362,8 +365,8 @@ inline int32_t run_strided_copy(zant_ctx* ctx, size_t esz, const void* x, void* 
     d.rank = m.rank; d.base = m.base; d.total = m.total;
     for (int i = 0; i < 8; ++i) { d.out_dims[i] = m.out_dims[i]; d.in_stride[i] = m.in_stride[i]; }
     const int grid = grid_for(m.total, 256, ctx->sm_count);
-    if (esz == 4) strided_copy_k<uint32_t><<<grid, 256, 0, ctx->stream>>>((const uint32_t*)x, (uint32_t*)y, d);
-    else strided_copy_k<uint8_t><<<grid, 256, 0, ctx->stream>>>((const uint8_t*)x, (uint8_t*)y, d);
+    if (esz == 4) launch(ctx, strided_copy_k<uint32_t>, grid, 256, 0, (const uint32_t*)x, (uint32_t*)y, d);
+    else launch(ctx, strided_copy_k<uint8_t>, grid, 256, 0, (const uint8_t*)x, (uint8_t*)y, d);
     return check_launch(ctx, "strided_copy_k");
 }
 
@@ -371,8 +374,8 @@ inline int32_t run_gather(zant_ctx* ctx, size_t esz, const void* x, const int32_
     const size_t total = g.outer * g.n_idx * g.inner;
     if (total == 0) return ZANT_OK;
     const int grid = grid_for(total, 256, ctx->sm_count);
-    if (esz == 4) gather_axis_k<uint32_t><<<grid, 256, 0, ctx->stream>>>((const uint32_t*)x, idx_dev, (uint32_t*)y, g.outer, g.n_idx, g.inner, g.axis_dim);
-    else gather_axis_k<uint8_t><<<grid, 256, 0, ctx->stream>>>((const uint8_t*)x, idx_dev, (uint8_t*)y, g.outer, g.n_idx, g.inner, g.axis_dim);
+    if (esz == 4) launch(ctx, gather_axis_k<uint32_t>, grid, 256, 0, (const uint32_t*)x, idx_dev, (uint32_t*)y, g.outer, g.n_idx, g.inner, g.axis_dim);
+    else launch(ctx, gather_axis_k<uint8_t>, grid, 256, 0, (const uint8_t*)x, idx_dev, (uint8_t*)y, g.outer, g.n_idx, g.inner, g.axis_dim);
     return check_launch(ctx, "gather_axis_k");
 }
 

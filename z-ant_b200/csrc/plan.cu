@@ -99,6 +99,12 @@ struct zant_plan {
 
 namespace {
 
+struct InPlan {
+    explicit InPlan(zant_ctx* c) : ctx(c) { ctx->in_plan = true; }
+    ~InPlan() { ctx->in_plan = false; }
+    zant_ctx* ctx;
+};
+
 const char* kAutoPadNames[] = {"NOTSET", "SAME_UPPER", "SAME_LOWER", "VALID"};
 
 int32_t need_inputs(const PlanNode& n, size_t lo, size_t hi, const char* name) {
@@ -314,17 +320,18 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     for (auto& t : plan->t) {
         if (t.alias >= 0 || t.elided) continue;
         t.arena_ptr = plan->arena + t.offset;
-        if (t.is_const && t.bytes) ZB_CUDA(copy_to_device(ctx, t.arena_ptr, t.host.data(), t.bytes));
+        if (t.is_const && t.bytes) ZB_CUDA(cudaMemcpyAsync(t.arena_ptr, t.host.data(), t.bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
     for (size_t a = 0; a < plan->aux_host.size(); ++a)
         if (!plan->aux_host[a].empty())
-            ZB_CUDA(copy_to_device(ctx, plan->arena + plan->aux_off[a], plan->aux_host[a].data(), plan->aux_host[a].size()));
+            ZB_CUDA(cudaMemcpyAsync(plan->arena + plan->aux_off[a], plan->aux_host[a].data(), plan->aux_host[a].size(), cudaMemcpyHostToDevice, ctx->stream));
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
     for (auto& t : plan->t) { t.host.clear(); t.host.shrink_to_fit(); }
 
     // 3. one dry count of launches
     plan->finalized = true;
     const uint64_t before = ctx->launches;
+    InPlan scope(ctx);
     for (auto& s : plan->steps) { int32_t st = s(); if (st != ZANT_OK) { plan->finalized = false; return st; } }
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
     plan->launches_per_run = (int)(ctx->launches - before);
@@ -380,6 +387,7 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
         ZB_CUDA(cudaEventRecord(plan->prof_events[plan->prof_used++], ctx->stream));
         return ZANT_OK;
     };
+    InPlan scope(ctx);
     for (size_t s = 0; s < plan->steps.size(); ++s) {
         if (plan->profiling) { int32_t st = mark(); if (st != ZANT_OK) return st; }
         int32_t st = plan->steps[s]();
@@ -405,6 +413,7 @@ int32_t zant_b200_plan_use_graph(zant_plan* plan, int32_t enable) {
         plan->t[r].bound = nullptr;
     }
     const uint64_t before = ctx->launches;
+    InPlan scope(ctx);
     ZB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int32_t st = ZANT_OK;
     for (auto& step : plan->steps) { st = step(); if (st != ZANT_OK) break; }
@@ -1534,7 +1543,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         k.x_scale = a1.x_scale; k.x_zp = a1.x_zp;
         k.wfrag = (const uint32_t*)pl->aux(a_wf); k.biasfrag = (const int32_t*)pl->aux(a_bf); k.multfrag = (const float*)pl->aux(a_mf); k.status = ctx->status_word; k.plane_bytes = plane_bytes;
         const int blocks = std::min<int>((int)((B + C1M_G - 1) / C1M_G), ctx->sm_count * 8);
-        conv1_mma_relu_pool_kernel<<<blocks, C1M_THREADS, 0, ctx->stream>>>(k);
+        launch(ctx, conv1_mma_relu_pool_kernel, blocks, C1M_THREADS, 0, k);
         return check_launch(ctx, "conv1_mma_relu_pool_kernel");
     });
     push("Fused[QLinearConv+Relu+MaxPool] tcgen05", [=]() {
@@ -1545,7 +1554,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         for (int m = 0; m < 64; ++m) { k.mult[m] = m2[m]; k.bias[m] = b2[m]; }
         k.y = (int8_t*)pl->scratch(s_pool2); k.n_images = (int)B; k.n_tiles = (int)c2_tiles; k.status = ctx->status_word;
         const int blocks = std::min<int>((int)c2_tiles, ctx->sm_count);
-        tc_conv3x3_pool_parity_kernel<<<blocks, Cfg::THREADS, Cfg::SMEM_BYTES, ctx->stream>>>(k);
+        launch_const(ctx, tc_conv3x3_pool_parity_kernel, blocks, Cfg::THREADS, Cfg::SMEM_BYTES, k);
         return check_launch(ctx, "tc_conv3x3_pool_parity_kernel");
     });
     const zant_node_attrs f1a = f1.a, f2a = f2.a, dqa = N[11].a;
@@ -1559,7 +1568,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         k.y_scale = f1a.y_scale; k.y_zp = f1a.y_zp; k.act = ZANT_QACT_RELU; k.status = ctx->status_word;
         const int tiles = (int)((B + 127) / 128) * (512 / FC_NT);
         const int blocks = std::min(tiles, ctx->sm_count);
-        tc_gemm_i8_kernel<FC_NT, FC_KC, FC_STAGES><<<blocks, Cfg::THREADS, Cfg::SMEM_BYTES, ctx->stream>>>(k);
+        launch_const(ctx, tc_gemm_i8_kernel<FC_NT, FC_KC, FC_STAGES>, blocks, Cfg::THREADS, Cfg::SMEM_BYTES, k);
         return check_launch(ctx, "tc_gemm_i8_kernel");
     });
     push("Fused[QLinearMatMul+DequantizeLinear]", [=]() {
@@ -1569,15 +1578,15 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         k.y = pl->p<float>(y); k.M = (int)B; k.K = 512; k.NCLS = (int)NCLS;
         k.y_scale = f2a.y_scale; k.y_zp = f2a.y_zp; k.dq_scale = dqa.x_scale; k.dq_zp = dqa.x_zp;
         // one or two column blocks of 8 classes
-        auto launch = [&](auto nc) -> int32_t {
+        auto with = [&](auto nc) -> int32_t {
             constexpr int NC = decltype(nc)::value;
             constexpr int smem = fcout_smem_bytes<NC, 512>();
             ZB_SMEM_ATTR(ctx, (fc_out_dequant_kernel<NC, 512>), smem);
             const int blocks = std::min<int>((int)((B + 127) / 128), ctx->sm_count * 3);
-            fc_out_dequant_kernel<NC, 512><<<blocks, FCOUT_THREADS, smem, ctx->stream>>>(k);
+            launch(ctx, fc_out_dequant_kernel<NC, 512>, blocks, FCOUT_THREADS, smem, k);
             return check_launch(ctx, "fc_out_dequant_kernel");
         };
-        return NCLS <= 8 ? launch(std::integral_constant<int, 8>{}) : launch(std::integral_constant<int, 16>{});
+        return NCLS <= 8 ? with(std::integral_constant<int, 8>{}) : with(std::integral_constant<int, 16>{});
     });
     for (int k = 0; k < 11; ++k) pl->t[N[k].out[0]].elided = true;   // interior tensors live only inside the fused kernels
     consumed = 12;

@@ -24,6 +24,16 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// ---------------------------------------------------------------------------- programmatic dependent launch
+// A kernel launched behind another one on its stream may start while that one drains.  grid_trigger: the next kernel may be
+// scheduled as soon as every CTA of this one has come here; grid_wait: returns when the kernels before this one are complete
+// and their writes visible (at once when the launch was an ordinary one).  Before grid_wait a kernel touches constants only:
+// nothing that an earlier kernel writes, and nothing that an earlier kernel may still read is written.  A kernel that allocates
+// TMEM triggers after the allocation: a successor's CTA on the same SM could otherwise take the columns and wait for this one.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_start() { grid_trigger(); grid_wait(); }
+
 // ---------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -27,6 +27,7 @@
 #include "context.cuh"
 #include "geometry.hpp"
 #include "kernels_q8.cuh"
+#include "ptx_sm100.cuh"
 
 namespace zb {
 
@@ -66,6 +67,7 @@ template <bool XU8, bool YU8, int PATH, int MT>
 __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const SmallGemmArgs a) {
     constexpr int LD = 36;                                     // row pitch of the partial sums: 16-byte rows, banks spread
     extern __shared__ int red[];                               // [warps][MT * 16][LD]
+    ptx::grid_start();
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gq = lane >> 2, tq = lane & 3;
     const int m0 = blockIdx.x * (MT * 16), p0 = blockIdx.y * 32;
@@ -295,10 +297,10 @@ inline int32_t run_small_gemm(zant_ctx* ctx, const ConvGeom& g, const SmallGemmP
         constexpr int PATH = decltype(path_c)::value, MT = decltype(mt_c)::value;
         const size_t smem = (size_t)p.warps * MT * 16 * 36 * 4;          // 36 KB at most
         const int threads = p.warps * 32;
-        if (x_u8 && y_u8) small_gemm_q8_kernel<true, true, PATH, MT><<<grid, threads, smem, ctx->stream>>>(a);
-        else if (x_u8) small_gemm_q8_kernel<true, false, PATH, MT><<<grid, threads, smem, ctx->stream>>>(a);
-        else if (y_u8) small_gemm_q8_kernel<false, true, PATH, MT><<<grid, threads, smem, ctx->stream>>>(a);
-        else small_gemm_q8_kernel<false, false, PATH, MT><<<grid, threads, smem, ctx->stream>>>(a);
+        if (x_u8 && y_u8) launch(ctx, small_gemm_q8_kernel<true, true, PATH, MT>, grid, threads, smem, a);
+        else if (x_u8) launch(ctx, small_gemm_q8_kernel<true, false, PATH, MT>, grid, threads, smem, a);
+        else if (y_u8) launch(ctx, small_gemm_q8_kernel<false, true, PATH, MT>, grid, threads, smem, a);
+        else launch(ctx, small_gemm_q8_kernel<false, false, PATH, MT>, grid, threads, smem, a);
         return check_launch(ctx, "small_gemm_q8_kernel");
     };
     auto with_mt = [&](auto path_c) -> int32_t {

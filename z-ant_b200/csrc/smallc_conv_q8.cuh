@@ -29,6 +29,7 @@
 
 #include "context.cuh"
 #include "geometry.hpp"
+#include "ptx_sm100.cuh"
 #include "kernels_q8.cuh"
 #include "tc_conv_nchw.cuh"
 
@@ -68,6 +69,7 @@ __device__ __forceinline__ void mma_m16n8k16_s8(int (&d)[4], uint32_t a0, uint32
 // compile-time count so that the unrolled MMA loops carry no tests.
 template <int MT, int NTL, int KSC, bool XU8, bool LEAN>
 __global__ void __launch_bounds__(kSmallcThreads) qconv3x3_smallc_kernel(const SmallcArgs a) {
+    ptx::grid_start();
     extern __shared__ __align__(16) uint8_t s_in[];      // [C][RIN][P]
     __shared__ uint8_t s_lut[256];                       // copy of the optional activation table
     if (a.lut) for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = __ldg(a.lut + i);
@@ -226,7 +228,7 @@ template <int MT, int NTL>
 inline int32_t smallc_launch(zant_ctx* ctx, const SmallcArgs& a, int grid, size_t smem, bool x_u8, bool lean) {
     auto go = [&](auto kernel) -> int32_t {
         if (smem > 48 * 1024) ZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, kSmallcThreads, smem, ctx->stream>>>(a);
+        launch(ctx, kernel, grid, kSmallcThreads, smem, a);
         return check_launch(ctx, "qconv3x3_smallc_kernel");
     };
     if (a.KS == 1) {

@@ -14,6 +14,7 @@
 
 #include "context.cuh"
 #include "geometry.hpp"
+#include "ptx_sm100.cuh"
 #include "tc_gemm.cuh"
 
 namespace zb {
@@ -26,6 +27,7 @@ struct Im2colArgs {
 };
 
 __global__ void im2col_blocked_kernel(const Im2colArgs p) {
+    ptx::grid_start();
     const ConvGeom& g = p.g;
     const size_t total = (size_t)((p.M + 127) / 128) * p.K16 * 128;
     const int khw = g.KH * g.KW, ohw = g.OH * g.OW;
@@ -69,6 +71,7 @@ struct PwBlockArgs {
 };
 
 __global__ void __launch_bounds__(256) pointwise_blocked_kernel(const PwBlockArgs p) {
+    ptx::grid_start();
     __shared__ uint32_t tile[64][33];                 // [channel][32 words of 4 pixels], padded against bank conflicts
     const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5;
     const int mt = blockIdx.x, kg = blockIdx.y;       // row tile, group of 4 K chunks (64 channels)
@@ -119,6 +122,7 @@ struct TapMajorArgs {
 };
 
 __global__ void __launch_bounds__(256) im2col_tapmajor_kernel(const TapMajorArgs p) {
+    ptx::grid_start();
     __shared__ uint32_t tile[64][33];
     uint8_t (*tile8)[132] = reinterpret_cast<uint8_t (*)[132]>(&tile[0][0]);   // the same rows, byte view (33 words = 132 bytes)
     const ConvGeom& g = p.g;
@@ -238,7 +242,7 @@ template <int NT, int KC, int MODE>
 inline int32_t launch_tc_gemm_kc(zant_ctx* ctx, const TcGemmArgs& k, int tiles) {
     using Cfg = TcGemmCfg<NT, KC, 8, MODE>;
     ZB_SMEM_ATTR(ctx, (tc_gemm_i8_kernel<NT, KC, 8, MODE>), Cfg::SMEM_BYTES);
-    tc_gemm_i8_kernel<NT, KC, 8, MODE><<<std::min(tiles, ctx->sm_count), Cfg::THREADS, Cfg::SMEM_BYTES, ctx->stream>>>(k);
+    launch_const(ctx, tc_gemm_i8_kernel<NT, KC, 8, MODE>, std::min(tiles, ctx->sm_count), Cfg::THREADS, Cfg::SMEM_BYTES, k);
     return check_launch(ctx, "tc_gemm_i8_kernel");
 }
 
@@ -261,18 +265,18 @@ inline int32_t run_qconv_tc(zant_ctx* ctx, const ConvGeom& g, const void* x, boo
     if (pointwise && (g.H * g.W) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 3u) == 0 && m_tiles <= 0x7fffffff / 128 && (p.K16 + 3) / 4 <= 65535) {
         PwBlockArgs pa{};
         pa.x = (const uint8_t*)x; pa.a = a_blk; pa.C = g.C; pa.HW = g.H * g.W; pa.M = (int)M; pa.K16 = p.K16;
-        pointwise_blocked_kernel<<<dim3((unsigned)m_tiles, (unsigned)((p.K16 + 3) / 4)), 256, 0, ctx->stream>>>(pa);
+        launch(ctx, pointwise_blocked_kernel, dim3((unsigned)m_tiles, (unsigned)((p.K16 + 3) / 4)), 256, 0, pa);
         ZB_TRY(check_launch(ctx, "pointwise_blocked_kernel"));
     } else if ((p.tap_major || (g.KH * g.KW == 1 && g.C % 16 == 0)) && (long long)g.KH * g.KW * ((g.C + 63) / 64) <= 65535) {
         // (with a single tap the two K orders are the same: 1x1 filters on planes that are not whole words come here)
         TapMajorArgs ta{};
         ta.x = (const uint8_t*)x; ta.a = a_blk; ta.g = g; ta.M = (int)M; ta.K16 = p.K16; ta.cgroups = (g.C + 63) / 64; ta.pad_value = x_zp;
-        im2col_tapmajor_kernel<<<dim3((unsigned)m_tiles, (unsigned)(g.KH * g.KW * ta.cgroups)), 256, 0, ctx->stream>>>(ta);
+        launch(ctx, im2col_tapmajor_kernel, dim3((unsigned)m_tiles, (unsigned)(g.KH * g.KW * ta.cgroups)), 256, 0, ta);
         ZB_TRY(check_launch(ctx, "im2col_tapmajor_kernel"));
     } else {
         if (p.tap_major) return fail(ZANT_E_TOO_LARGE, "too many taps x channel groups for the tap-major gather");
         const size_t chunks = (size_t)m_tiles * p.K16 * 128;
-        im2col_blocked_kernel<<<grid_for(chunks, 256, ctx->sm_count, 16), 256, 0, ctx->stream>>>(ia);
+        launch(ctx, im2col_blocked_kernel, grid_for(chunks, 256, ctx->sm_count, 16), 256, 0, ia);
         ZB_TRY(check_launch(ctx, "im2col_blocked_kernel"));
     }
     TcGemmArgs k{};

@@ -212,6 +212,8 @@ __global__ void __launch_bounds__(kTcConvThreads, 1) tc_conv_nchw_kernel(const _
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    if (warp != 0) ptx::grid_wait();                     // (the loader: behind the weights)
 
     if (warp == 0) {
         // ------------------------------------------------------------------ loader: bulk copies of activations (and weights)
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(kTcConvThreads, 1) tc_conv_nchw_kernel(const _
             for (int cs = 0; cs < a.c_stages; ++cs)
                 ptx::bulk_g2s(ptx::smem_u32(smem + a.off_wres) + (uint32_t)cs * w_stage_bytes, a.w + (size_t)cs * w_stage_bytes, w_stage_bytes, wfull);
         }
+        ptx::grid_wait();
         // One tiled TMA load per stage: the box holds CB*16 channels x the bytes of the patch rows.  With
         // full-width tiles the image plane is addressed as one row of H*W bytes (4-byte elements) and the
         // box starts at the 16-byte boundary below the first wanted byte; otherwise the map is (W, H, C, N)
@@ -848,7 +851,7 @@ inline void tc_conv_prepare(const TcConvPlan& p, const int8_t* w, const float* m
 template <int NT, bool XU8, bool LEAN>
 inline int32_t tc_conv_launch_t(zant_ctx* ctx, const TcConvPlan& p, const TcConvArgs& a, const CUtensorMap& x_map, int grid) {
     ZB_SMEM_ATTR(ctx, (tc_conv_nchw_kernel<NT, XU8, LEAN>), 232448);
-    tc_conv_nchw_kernel<NT, XU8, LEAN><<<grid, kTcConvThreads, p.smem_bytes, ctx->stream>>>(a, x_map);
+    launch_const(ctx, tc_conv_nchw_kernel<NT, XU8, LEAN>, grid, kTcConvThreads, p.smem_bytes, a, x_map);
     return check_launch(ctx, "tc_conv_nchw_kernel");
 }
 

@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(kTcConvThreads, 1) tc_conv_nhwc_kernel(const _
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    if (warp != 0) ptx::grid_wait();                     // (the loader: behind the weights)
 
     if (warp == 0) {
         // ------------------------------------------------------------------ loader
@@ -102,6 +104,7 @@ __global__ void __launch_bounds__(kTcConvThreads, 1) tc_conv_nhwc_kernel(const _
             for (int cs = 0; cs < a.c_stages; ++cs)
                 ptx::bulk_g2s(ptx::smem_u32(smem + a.off_wres) + (uint32_t)cs * w_stage_bytes, a.w + (size_t)cs * w_stage_bytes, w_stage_bytes, wfull);
         }
+        ptx::grid_wait();
         const uint32_t box_bytes = (uint32_t)(KC * a.PW * a.PH);
         TcConvCursor cur;
         tc_conv_cursor_init(a, (int)blockIdx.x, (int)gridDim.x, cur);
@@ -306,22 +309,23 @@ inline bool tc_conv_nhwc_plan(const ConvGeom& g, bool w_zp_all_zero, int x_zp, T
     a.BH = std::max(1, std::min(a.OH, 128 / a.PW));
     a.wseg = (a.OW + a.BW - 1) / a.BW;
     a.full_width = 0;
-    p.NT = g.M <= 64 ? 64 : (g.M <= 128 ? 128 : 256);
-    a.m_pad = (g.M + p.NT - 1) / p.NT * p.NT;
-    a.n_tiles = a.m_pad / p.NT;
     const int taps = a.KH * a.KW;
     const int budget = 232448 - kTcConvTail - 2048;
     const int blocks_in_image = (a.OH + a.BH - 1) / a.BH;
     const TcConvArgs base = a;
     bool placed = false;
     int w_stage = 0;
-    // 128 channels per stage when C allows and the stage's weights leave room for two stages, else 64
+    // the filter tile that covers M when a stage's weights leave room for two stages, else a narrower one (3x3 over 64 channels
+    // and 256 filters are 147 KB); 128 channels per stage when C allows and there is room, else 64
+    for (p.NT = g.M <= 64 ? 64 : (g.M <= 128 ? 128 : 256); p.NT >= 64 && !placed; p.NT /= 2)
     for (int KC = g.C % 128 == 0 ? 128 : 64; KC >= 64 && !placed; KC -= 64)
     for (int rb = 4; rb >= 1 && !placed; rb /= 2) {
         w_stage = taps * p.NT * KC;
         const long long w_all = (long long)(g.C / KC) * w_stage;
         if (2 * rb * p.NT > 512 || (rb > 1 && rb > blocks_in_image)) continue;
         a = base;
+        a.m_pad = (g.M + p.NT - 1) / p.NT * p.NT;
+        a.n_tiles = a.m_pad / p.NT;
         a.CB = KC / 16; a.c_stages = g.C / KC;
         a.RB = rb; a.BHT = rb * a.BH;
         a.PH = a.BHT + halo_h;
@@ -343,11 +347,12 @@ inline bool tc_conv_nhwc_plan(const ConvGeom& g, bool w_zp_all_zero, int x_zp, T
         }
     }
     if (!placed) return false;
+    p.NT *= 2;                                                   // (the loop has halved it once more)
     p.smem_bytes = (size_t)a.off_out + kTcConvTail;
     p.w_bytes = (size_t)a.n_tiles * a.c_stages * w_stage;
     p.row_efficiency = (double)a.OH * a.OW / ((double)a.hseg * a.RB * a.wseg * 128.0);
     const long long tiles = (long long)a.N * a.hseg * a.wseg * a.n_tiles;
-    return tiles <= 0x7fffffffLL && p.row_efficiency >= 0.5;
+    return tiles <= 0x7fffffffLL;
 }
 
 // Blocks `w` ([M][C][KH][KW] int8) as [filter tile][channel stage][tap][NT rows of KC bytes], every row
@@ -408,7 +413,7 @@ template <int NT>
 inline int32_t tc_conv_nhwc_launch_nt(zant_ctx* ctx, const TcConvPlan& p, const TcConvArgs& a, const CUtensorMap& m, int grid, bool x_u8, bool lean) {
     auto go = [&](auto kernel) -> int32_t {
         ZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-        kernel<<<grid, kTcConvThreads, p.smem_bytes, ctx->stream>>>(a, m);
+        launch_const(ctx, kernel, grid, kTcConvThreads, p.smem_bytes, a, m);
         return check_launch(ctx, "tc_conv_nhwc_kernel");
     };
     if (x_u8) return lean ? go(tc_conv_nhwc_kernel<NT, true, true>) : go(tc_conv_nhwc_kernel<NT, true, false>);

@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(TcGemmCfg<NT, KC, STAGES, MODE>::THREADS, 1) t
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    ptx::grid_wait();
 
     if (warp == 0) {
         if (ptx::elect_one()) {
@@ -300,6 +302,7 @@ template <int NC, int K> constexpr int fcout_smem_bytes() { return NC * K + (FCO
 // instead of 40 dp4a per row and 16 bytes.
 template <int NC, int K>   // NC: compile-time bound on the number of classes, a multiple of 8
 __global__ void __launch_bounds__(FCOUT_THREADS) fc_out_dequant_kernel(const FcOutArgs p) {
+    ptx::grid_start();
     extern __shared__ __align__(16) uint8_t fc_smem[];
     uint32_t* sw = reinterpret_cast<uint32_t*>(fc_smem);   // [NC][K/4]: word (n, k4) = weights of class n for k = 4*k4 .. 4*k4+3
     constexpr int kw = K / 4, K16 = K / 16, KS = K / 32, NB = NC / 8, PITCH = fcout_pitch<K>();

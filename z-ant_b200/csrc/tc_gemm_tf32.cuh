@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_tf32_kernel(const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    ptx::grid_wait();
 
     if (warp == 0) {
         if (ptx::elect_one()) {
@@ -292,6 +294,7 @@ __device__ __forceinline__ void tf_store_chunk(float* a, long long tile, int kc,
 // K chunks; where each k reads is a table built on the host (no division in the loop).  A warp's 32 lanes read 32
 // consecutive pixels of one tap and write 512 contiguous bytes.
 __global__ void __launch_bounds__(256) im2col_f32_blocked_kernel(const TfIm2colArgs p) {
+    ptx::grid_start();
     const ConvGeom& g = p.g;
     const int tid = threadIdx.x, r = tid & 127;
     const long long n_tiles = (p.rows + 127) / 128;
@@ -325,6 +328,7 @@ __global__ void __launch_bounds__(256) im2col_f32_blocked_kernel(const TfIm2colA
 // A row-major (or transposed) matrix [M][K] with element strides (sm, sk) -> blocked, rounded to TF32.
 __global__ void __launch_bounds__(256) block_matrix_f32_kernel(const float* __restrict__ x, float* __restrict__ a, long long M, int K, int K4,
                                                                long long sm, long long sk, int KC, int parts) {
+    ptx::grid_start();
     const long long rows_pad = (M + 127) / 128 * 128;
     const long long total = rows_pad * K4;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -414,7 +418,7 @@ inline int32_t launch_tf_gemm(zant_ctx* ctx, const TfGemmArgs& k, int tiles) {
     constexpr int KC = SPLIT ? 4 : 8;          // the same bytes per stage in both forms
     using Cfg = TfGemmCfg<NT, KC, STAGES, SPLIT>;
     ZB_SMEM_ATTR(ctx, (tc_gemm_tf32_kernel<NT, KC, STAGES, SPLIT>), Cfg::SMEM_BYTES);
-    tc_gemm_tf32_kernel<NT, KC, STAGES, SPLIT><<<std::min(tiles, ctx->sm_count), Cfg::THREADS, Cfg::SMEM_BYTES, ctx->stream>>>(k);
+    launch_const(ctx, tc_gemm_tf32_kernel<NT, KC, STAGES, SPLIT>, std::min(tiles, ctx->sm_count), Cfg::THREADS, Cfg::SMEM_BYTES, k);
     return check_launch(ctx, SPLIT ? "tc_gemm_tf32_kernel<split>" : "tc_gemm_tf32_kernel");
 }
 
@@ -448,7 +452,7 @@ inline int32_t run_conv_tf32(zant_ctx* ctx, const ConvGeom& g, const float* x, c
     ia.ktab = reinterpret_cast<const int2*>(ktab_dev);
     if ((long long)g.C * g.H * g.W > 0x7fffffffLL || g.KH * g.dh > 0x7fff || g.KW * g.dw > 0x7fff) return fail(ZANT_E_TOO_LARGE, "convolution geometry exceeds the gather table's range");
     const long long n_tiles = (ia.rows + 127) / 128;
-    im2col_f32_blocked_kernel<<<(unsigned)std::min<long long>(n_tiles, (long long)ctx->sm_count * 16), 256, 0, ctx->stream>>>(ia);
+    launch(ctx, im2col_f32_blocked_kernel, (unsigned)std::min<long long>(n_tiles, (long long)ctx->sm_count * 16), 256, 0, ia);
     ZB_TRY(check_launch(ctx, "im2col_f32_blocked_kernel"));
     return run_tf_gemm(ctx, p, a_blk, w_blk_dev, bias_dev, ia.rows, g.OH * g.OW, act, slope, y);
 }
@@ -458,7 +462,7 @@ inline int32_t run_matmul_tf32(zant_ctx* ctx, const float* a, long long M, int K
                                const float* w_blk_dev, const float* bias_dev, float* a_blk, int act, float slope, float* y) {
     if (M <= 0) return ZANT_OK;
     const long long chunks = (M + 127) / 128 * 128 * (long long)p.K4;
-    block_matrix_f32_kernel<<<grid_for((size_t)chunks, 256, ctx->sm_count, 16), 256, 0, ctx->stream>>>(a, a_blk, M, K, p.K4, sm, sk, p.KC, p.parts);
+    launch(ctx, block_matrix_f32_kernel, grid_for((size_t)chunks, 256, ctx->sm_count, 16), 256, 0, a, a_blk, M, K, p.K4, sm, sk, p.KC, p.parts);
     ZB_TRY(check_launch(ctx, "block_matrix_f32_kernel"));
     return run_tf_gemm(ctx, p, a_blk, w_blk_dev, bias_dev, M, 0, act, slope, y);
 }

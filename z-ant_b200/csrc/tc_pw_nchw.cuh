@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    if (warp != 0) ptx::grid_wait();                     // (the loader: behind the weights)
 
     if (warp == 0) {
         // ------------------------------------------------------------------ loader: the filter tile's weights once, then (mode 0) one box per stage and block
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
             const uint32_t w_bytes = (uint32_t)a.a_steps * 4096u;
             ptx::mbar_arrive_expect_tx(wfull, w_bytes);
             ptx::bulk_g2s(ptx::smem_u32(sA), a.w + (size_t)mt * w_bytes, w_bytes, wfull);
+            ptx::grid_wait();
             if (a.mode == 0) {
                 int s = 0; uint32_t ph = 0;
                 bool alive = true;
@@ -731,7 +734,7 @@ inline void pw_conv_prepare(const PwConvPlan& p, const int8_t* w, const int32_t*
 template <bool XU8, bool LEAN>
 inline int32_t pw_conv_launch_t(zant_ctx* ctx, const PwConvPlan& p, const PwConvArgs& a, const CUtensorMap& x_map, int grid) {
     ZB_SMEM_ATTR(ctx, (tc_pw_nchw_kernel<XU8, LEAN>), 232448);
-    tc_pw_nchw_kernel<XU8, LEAN><<<grid, kPwThreads, p.smem_bytes, ctx->stream>>>(a, x_map);
+    launch_const(ctx, tc_pw_nchw_kernel<XU8, LEAN>, grid, kPwThreads, p.smem_bytes, a, x_map);
     return check_launch(ctx, "tc_pw_nchw_kernel");
 }
 
