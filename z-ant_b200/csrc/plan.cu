@@ -27,6 +27,7 @@
 #include "tc_conv_nhwc.cuh"
 #include "tc_gemm_tf32.cuh"
 #include "small_gemm_q8.cuh"
+#include "tc_nhwc_net.cuh"
 #include "status.hpp"
 
 using namespace zb;
@@ -42,12 +43,31 @@ struct PlanTensor {
     void* bound = nullptr;      // caller's device buffer bound for the current run (input/output)
     int alias = -1;             // Reshape output: shares the buffer of this tensor
     bool elided = false;        // interior of a fused chain: never materialised, no arena space
+    // Kept channels-last between convolutions (tc_nhwc_net.cuh): pixels `nh_pix` bytes apart, channel 0 of pixel (0,0) `nh_off` bytes
+    // into the buffer of tensor `nh_root` (a Concat's operands live in its result; else the tensor itself).
+    bool nh = false;
+    int nh_root = -1;
+    size_t nh_off = 0, nh_pix = 0;
+    int nh_lo = 0;              // split TF32: channels from a hi half to its lo half
 };
 
 struct PlanNode {
     int32_t op = 0;
     std::vector<int> in, out;
     zant_node_attrs a{};
+};
+
+// A convolution with what follows it, as one channels-last step.
+struct NhGroup {
+    size_t first = 0, count = 0;
+    int x = -1, y = -1;                  // tensors read and written
+    std::vector<int> interior;
+    int qact = -1;                       // int8: activation flag that a Relu node became (-1: the node's own)
+    int lut_node = -1;                   // int8: activation node that becomes a table
+    int fact = 0; float slope = 0.0f;    // TF32
+    bool pool = false, up2 = false;
+    int dequant = -1;                    // DequantizeLinear node
+    bool on = false;                     // the layout pass took it
 };
 
 struct zant_plan {
@@ -71,6 +91,7 @@ struct zant_plan {
     std::vector<cudaEvent_t> prof_events;   // pool, reused between reads
     size_t prof_used = 0;                   // events recorded since the last read
 
+    std::vector<NhGroup> nh_groups;   // channels-last convolution groups found by the layout pass, by first node
     void* ptr(int id) const {
         int r = id;
         while (t[r].alias >= 0) r = t[r].alias;
@@ -216,9 +237,11 @@ int32_t zant_b200_plan_node(zant_plan* plan, int32_t op, const int32_t* inputs, 
 static int32_t build_node(zant_plan* pl, size_t node_index, int32_t fuse);
 static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t fuse);
 static int32_t try_fuse(zant_plan* pl, size_t node_index, size_t& consumed);
-static int32_t try_fuse_small_cnn(zant_plan* pl, size_t node_index, size_t& consumed);
+static int32_t try_fuse_small_cnn(zant_plan* pl, size_t node_index, size_t& consumed, bool probe = false);
 static int32_t try_fuse_qconv_group(zant_plan* pl, size_t node_index, size_t& consumed);
 static int32_t try_fuse_fconv_group(zant_plan* pl, size_t node_index, size_t& consumed);
+static void nh_layout(zant_plan* pl);
+static int32_t build_nh(zant_plan* pl, size_t node_index, size_t& consumed);
 
 // Multiply-accumulates of one node (contractions only; everything else counts as 0).
 static double node_macs(const zant_plan* pl, const PlanNode& n) {
@@ -284,9 +307,14 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     // 1. validate nodes, derive constants, record launch closures
     plan->steps.clear(); plan->step_names.clear(); plan->step_macs.clear(); plan->step_bytes.clear();
     size_t i = 0;
+    if (fuse) nh_layout(plan);
     while (i < plan->nodes.size()) {
         size_t consumed = 0;
         if (fuse) {
+            int32_t st = build_nh(plan, i, consumed);
+            if (st != ZANT_OK) return st;
+        }
+        if (fuse && consumed == 0) {
             int32_t st = try_fuse(plan, i, consumed);
             if (st != ZANT_OK) return st;
         }
@@ -300,10 +328,12 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
 
     // 2. arena layout: every non-aliased tensor and every derived constant at a fixed offset
     size_t off = 0;
-    for (auto& t : plan->t) {
-        if (t.alias >= 0 || t.elided) continue;
+    for (size_t id = 0; id < plan->t.size(); ++id) {
+        PlanTensor& t = plan->t[id];
+        if (t.alias >= 0 || t.elided || (t.nh && t.nh_root != (int)id)) continue;
         t.offset = off;
-        off += align_up(t.bytes ? t.bytes : 1, kArenaAlign);
+        const size_t bytes = t.nh ? t.shape[0] * t.shape[2] * t.shape[3] * t.nh_pix : t.bytes;
+        off += align_up(bytes ? bytes : 1, kArenaAlign);
     }
     plan->aux_off.resize(plan->aux_host.size());
     for (size_t a = 0; a < plan->aux_host.size(); ++a) {
@@ -319,7 +349,7 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     ZB_ALLOC(plan->arena, off);
     for (auto& t : plan->t) {
         if (t.alias >= 0 || t.elided) continue;
-        t.arena_ptr = plan->arena + t.offset;
+        t.arena_ptr = t.nh ? plan->arena + plan->t[t.nh_root].offset + t.nh_off : plan->arena + t.offset;
         if (t.is_const && t.bytes) ZB_CUDA(cudaMemcpyAsync(t.arena_ptr, t.host.data(), t.bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
     for (size_t a = 0; a < plan->aux_host.size(); ++a)
@@ -432,6 +462,9 @@ size_t zant_b200_plan_arena_bytes(zant_plan* plan) { return plan ? plan->arena_b
 int32_t zant_b200_plan_launches_per_run(zant_plan* plan) { return plan ? plan->launches_per_run : 0; }
 void* zant_b200_plan_tensor_ptr(zant_plan* plan, int32_t id) {
     if (!plan || !plan->finalized || id < 0 || id >= (int)plan->t.size()) return nullptr;
+    int r = id;
+    while (plan->t[r].alias >= 0) r = plan->t[r].alias;
+    if (plan->t[r].nh) return nullptr;        // kept in another layout: zant_b200_plan_read_tensor converts
     return plan->ptr(id);
 }
 
@@ -485,6 +518,29 @@ int32_t zant_b200_plan_read_tensor(zant_plan* plan, int32_t id, void* host_dst) 
     }
     ZB_CUDA(cudaSetDevice(plan->ctx->device));
     ZB_CUDA(cudaStreamSynchronize(plan->ctx->stream));
+    int r = id;
+    while (plan->t[r].alias >= 0) r = plan->t[r].alias;
+    const PlanTensor& t = plan->t[r];
+    if (t.nh) {
+        const size_t N = t.shape[0], C = t.shape[1], hw = t.shape[2] * t.shape[3], esz = dtype_size(t.dtype);
+        const PlanTensor& root = plan->t[t.nh_root];
+        std::vector<char> raw(N * hw * t.nh_pix);
+        ZB_CUDA(cudaMemcpy(raw.data(), root.arena_ptr, raw.size(), cudaMemcpyDeviceToHost));
+        for (size_t n = 0; n < N; ++n)
+            for (size_t c = 0; c < C; ++c)
+                for (size_t p = 0; p < hw; ++p) {
+                    const char* src = raw.data() + (n * hw + p) * t.nh_pix + t.nh_off + c * esz;
+                    char* dst = (char*)host_dst + ((n * C + c) * hw + p) * esz;
+                    std::memcpy(dst, src, esz);
+                    if (t.nh_lo) {
+                        float hi, lo;
+                        std::memcpy(&hi, src, 4); std::memcpy(&lo, src + (size_t)t.nh_lo * 4, 4);
+                        hi += lo;
+                        std::memcpy(dst, &hi, 4);
+                    }
+                }
+        return ZANT_OK;
+    }
     ZB_CUDA(cudaMemcpy(host_dst, plan->ptr(id), plan->t[id].bytes, cudaMemcpyDeviceToHost));
     return ZANT_OK;
 }
@@ -1343,7 +1399,7 @@ static int32_t try_fuse_qconv_group(zant_plan* pl, size_t i0, size_t& consumed) 
     return ZANT_OK;
 }
 
-static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
+static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bool probe) {
     consumed = 0;
     if (i0 + 12 > pl->nodes.size()) return ZANT_OK;
     const int kOps[12] = {ZANT_OP_QUANTIZE_LINEAR, ZANT_OP_QLINEAR_CONV, ZANT_OP_RELU, ZANT_OP_MAXPOOL, ZANT_OP_QLINEAR_CONV, ZANT_OP_RELU,
@@ -1398,6 +1454,8 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         for (size_t k = 1; k < q->in.size(); ++k)
             if (q->in[k] >= 0 && !T(q->in[k]).is_const) return ZANT_OK;
 
+    if (NCLS > 16 || B > (1u << 20)) return ZANT_OK;         // two column blocks of classes; 32-bit plane offsets in stage 1
+    if (probe) { consumed = 12; return ZANT_OK; }
     zant_ctx* ctx = pl->ctx;
     auto push = [&](const char* name, std::function<int32_t()> fn) { pl->steps.push_back(std::move(fn)); pl->step_names.push_back(name); };
     auto scales_of = [&](const PlanNode& q, size_t M, std::vector<float>& mult) {
@@ -1483,7 +1541,6 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
     }
     std::vector<float> m4; std::vector<int32_t> b4;
     if (!scales_of(f2, NCLS, m4) || !bias_of(f2, NCLS, b4)) return ZANT_OK;
-    if (NCLS > 16) return ZANT_OK;
     {
         const int8_t* w = (const int8_t*)T(f2.in[1]).host.data();   // [512][NCLS]
         for (size_t n = 0; n < NCLS; ++n) {
@@ -1494,7 +1551,6 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
     }
 
     // stage 1 -> stage 2 hand-over: parity planes (TcConvParityCfg), every tile of stage 2 copies 136 rows of each plane
-    if (B > (1u << 20)) return ZANT_OK;                     // 32-bit plane offsets in stage 1
     const long long c2_tiles = ((long long)B * 36 + 127) / 128;
     const long long plane_bytes = (TcConvParityCfg::plane_rows(c2_tiles) * 16 + 255) / 256 * 256;
     const int s_pool1 = pl->add_scratch((size_t)(8 * plane_bytes));
@@ -1600,5 +1656,337 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed) {
         pl->step_macs.resize(pl->steps.size(), 0.0); pl->step_bytes.resize(pl->steps.size(), 0.0);
         for (int k = 0; k < 4; ++k) { pl->step_macs[pl->steps.size() - 4 + k] = macs[k]; pl->step_bytes[pl->steps.size() - 4 + k] = bytes[k]; }
     }
+    return ZANT_OK;
+}
+
+// --------------------------------------------------------------------------------------------
+// Layout pass: activations between convolutions stay channels-last (tc_nhwc_net.cuh) where their producer can write and every
+// reader can read that form.  Producers: convolution groups, MaxPool, Concat over channels (its operands are written in place),
+// and, for at most four channels, QuantizeLinear; readers: convolution groups, MaxPool, Concat.  Everything else - graph
+// input and output, and whatever this pass does not know - keeps NCHW.  int8 contexts and, in TF32 mode, float ones alike.
+// --------------------------------------------------------------------------------------------
+static int nh_kind(const zant_plan* pl, int32_t dtype) {
+    if (dtype == ZANT_I8) return NH_I8;
+    if (dtype == ZANT_U8) return NH_U8;
+    if (dtype == ZANT_F32 && pl->ctx->tf32) return pl->ctx->tf32 == 2 ? NH_TF32X3 : NH_TF32;
+    return -1;
+}
+
+static bool nh_conv_geom(const zant_plan* pl, const PlanNode& n, ConvGeom& g) {
+    const PlanTensor &x = pl->t[n.in[0]], &w = pl->t[n.in[1]], &y = pl->t[n.out[0]];
+    const zant_node_attrs& a = n.a;
+    if (n.op == ZANT_OP_QLINEAR_CONV)
+        return conv_resolve_onnx(x.shape.data(), x.shape.size(), w.shape.data(), w.shape.size(), y.shape.data(), y.shape.size(), a.strides, a.n_strides, a.pads, a.n_pads,
+                                 a.dilations, a.n_dilations, a.group, a.auto_pad < 0 ? 0 : a.auto_pad, g) == ZANT_OK;
+    const char* ap = (a.auto_pad >= 0 && a.auto_pad <= 3) ? kAutoPadNames[a.auto_pad] : nullptr;
+    return conv_resolve_ref(x.shape.data(), x.shape.size(), w.shape.data(), w.shape.size(), y.shape.data(), y.shape.size(), a.strides, a.n_strides, a.n_pads ? a.pads : nullptr,
+                            a.n_pads, a.n_dilations ? a.dilations : nullptr, a.n_dilations, a.group, ap, ap ? std::strlen(ap) : 0, g) == ZANT_OK;
+}
+
+// Reads the convolution at node `i` with the activation, pool, upsampling and dequantisation behind it; false when the
+// channels-last kernel cannot run it.
+static bool nh_parse(const zant_plan* pl, const ChainCtx& c, size_t i, NhGroup& q) {
+    const PlanNode& n = pl->nodes[i];
+    auto T = [&](int id) -> const PlanTensor& { return pl->t[id]; };
+    const bool i8 = n.op == ZANT_OP_QLINEAR_CONV;
+    if ((!i8 && n.op != ZANT_OP_CONV) || n.a.channels_last || n.out.size() != 1 || n.in.size() < (i8 ? 3u : 2u) || n.in.size() > (i8 ? 5u : 3u)) return false;
+    for (size_t k = 1; k < n.in.size(); ++k) if (n.in[k] >= 0 && !T(n.in[k]).is_const) return false;
+    const int x = n.in[0], w = n.in[1];
+    if (x < 0 || w < 0 || T(x).is_const || T(x).shape.size() != 4 || T(w).shape.size() != 4 || T(n.out[0]).shape.size() != 4 || (i8 && n.in[2] < 0)) return false;
+    const int kind = nh_kind(pl, T(x).dtype);
+    if (kind < 0 || (kind <= NH_U8) != i8 || (!i8 && T(x).dtype != ZANT_F32)) return false;
+    ConvGeom g;
+    if (!nh_conv_geom(pl, n, g)) return false;
+    bool monotone = true;
+    if (i8) {
+        if (T(n.out[0]).dtype != ZANT_I8 || n.a.y_zp != 0 || T(w).dtype != ZANT_I8 || T(n.in[2]).dtype != ZANT_F32) return false;
+        if (check_zero_point(T(x).dtype, n.a.x_zp, "QLinearConv x") != ZANT_OK) return false;
+        if ((g.pt || g.pl || g.pb || g.pr) && n.a.x_zp != 0) return false;            // the halo is zero fill
+        const int wz = opt_in(n, 3), b = opt_in(n, 4);
+        if (wz >= 0 && (T(wz).dtype != ZANT_I32 || !all_zero_i32(T(wz)))) return false;
+        if (b >= 0 && (T(b).dtype != ZANT_I32 || T(b).bytes != (size_t)g.M * 4)) return false;
+        const size_t nws = T(n.in[2]).bytes / 4;
+        if (nws != 1 && nws != (size_t)g.M) return false;
+        std::vector<float> mult;
+        requant_multipliers(n.a.x_scale, (const float*)T(n.in[2]).host.data(), nws, n.a.y_scale, (size_t)g.M, mult);
+        if (!positive_finite(mult)) return false;
+    } else {
+        // (fewer than 128 positions stay with the exact kernels, as without this pass)
+        if (T(w).dtype != ZANT_F32 || T(n.out[0]).dtype != ZANT_F32 || g.M > 2048 || (long long)g.N * g.OH * g.OW < 128) return false;
+        const int b = opt_in(n, 2);
+        if (b >= 0 && (T(b).dtype != ZANT_F32 || T(b).bytes != (size_t)g.M * 4)) return false;
+    }
+    q = NhGroup{};
+    q.first = i; q.x = x;
+    size_t j = i + 1;
+    int cur = n.out[0];
+    auto next = [&](int32_t op) { return j < pl->nodes.size() && only_feeds_next(c, cur) && pl->nodes[j].op == op && !pl->nodes[j].in.empty() && pl->nodes[j].in[0] == cur && pl->nodes[j].out.size() == 1; };
+    auto take = [&]() { q.interior.push_back(cur); cur = pl->nodes[j].out[0]; ++j; };
+    if (i8 && (next(ZANT_OP_RELU) || next(ZANT_OP_LEAKY_RELU) || next(ZANT_OP_CLIP))) {
+        const PlanNode& act = pl->nodes[j];
+        if (act.in.size() == 1 && T(act.out[0]).dtype == ZANT_I8 && T(act.out[0]).shape == T(cur).shape && act.a.x_scale == n.a.y_scale && act.a.x_zp == n.a.y_zp) {
+            if (identity_scale_relu(act)) q.qact = n.a.activation == ZANT_QACT_NONE ? ZANT_QACT_RELU : n.a.activation;
+            else {
+                q.lut_node = (int)j;
+                uint8_t lut[256];
+                activation_lut(act, ZANT_I8, lut);
+                for (int v = -127; v < 128; ++v) monotone = monotone && (int8_t)lut[v & 255] >= (int8_t)lut[(v - 1) & 255];
+            }
+            take();
+        }
+    } else if (!i8 && (next(ZANT_OP_RELU) || next(ZANT_OP_LEAKY_RELU))) {
+        const PlanNode& act = pl->nodes[j];
+        if (act.in.size() == 1 && T(act.out[0]).dtype == ZANT_F32 && T(act.out[0]).shape == T(cur).shape) {
+            q.fact = act.op == ZANT_OP_RELU ? FACT_RELU : FACT_LEAKY; q.slope = act.a.alpha;
+            take();
+        }
+    }
+    NhConvPlan np;
+    if (monotone && next(ZANT_OP_MAXPOOL)) {
+        const PlanNode& pool = pl->nodes[j];
+        const auto& so = T(pool.out[0]).shape;
+        if (pool.in.size() == 1 && pool2x2(pool.a) && T(pool.out[0]).dtype == T(cur).dtype && so.size() == 4 && so[0] == (size_t)g.N && so[1] == (size_t)g.M &&
+            so[2] == (size_t)g.OH / 2 && so[3] == (size_t)g.OW / 2 && nh_conv_plan(g, kind, true, pl->ctx->sm_count, np)) {
+            q.pool = true;
+            take();
+        }
+    }
+    if (!q.pool && !nh_conv_plan(g, kind, false, pl->ctx->sm_count, np)) return false;
+    if (next(ZANT_OP_RESIZE)) {
+        // nearest neighbour by two, as the index table says: every pixel goes to a 2 x 2 block
+        const PlanNode& rs = pl->nodes[j];
+        const auto &si = T(cur).shape, &so = T(rs.out[0]).shape;
+        if (rs.in.size() == 1 && T(rs.out[0]).dtype == T(cur).dtype && rs.a.n_scales == 4 && so.size() == 4 && so[0] == si[0] && so[1] == si[1] && so[2] == 2 * si[2] && so[3] == 2 * si[3]) {
+            std::vector<int32_t> table, off;
+            resize_index_table(si.data(), so.data(), 4, rs.a.coord_mode, table, off);
+            bool ok = true;
+            for (int d = 0; d < 4; ++d) for (size_t o = 0; o < so[d]; ++o) ok = ok && table[off[d] + o] == (int32_t)(d < 2 ? o : o / 2);
+            if (ok) { q.up2 = true; take(); }
+        }
+    } else if (i8 && next(ZANT_OP_DEQUANTIZE_LINEAR) && T(pl->nodes[j].out[0]).dtype == ZANT_F32 && T(pl->nodes[j].out[0]).shape == T(cur).shape) {
+        q.dequant = (int)j;
+        take();
+    }
+    q.y = cur;
+    q.count = j - i;
+    return true;
+}
+
+static void nh_layout(zant_plan* pl) {
+    pl->nh_groups.clear();
+    ChainCtx c{pl, std::vector<int>(pl->t.size(), 0)};
+    for (const PlanNode& n : pl->nodes) for (int id : n.in) if (id >= 0) c.consumers[id]++;
+    auto T = [&](int id) -> PlanTensor& { return pl->t[id]; };
+    const size_t nn = pl->nodes.size();
+    std::vector<int> group_of(nn, -1);
+    std::vector<char> own(nn, 0);                            // nodes of the small CNN's own chain
+    for (size_t i = 0; i < nn; ++i) {
+        size_t took = 0;
+        if (pl->nodes[i].op == ZANT_OP_QUANTIZE_LINEAR) try_fuse_small_cnn(pl, i, took, true);
+        for (size_t k = i; k < i + took; ++k) own[k] = 1;
+    }
+    for (size_t i = 0; i < nn; ++i) {
+        NhGroup q;
+        if (own[i] || group_of[i] >= 0 || !nh_parse(pl, c, i, q)) continue;
+        q.on = true;
+        for (size_t k = i; k < i + q.count; ++k) group_of[k] = (int)pl->nh_groups.size();
+        pl->nh_groups.push_back(q);
+    }
+    if (pl->nh_groups.empty()) return;
+    std::vector<char> lay(pl->t.size(), 0);
+    for (size_t id = 0; id < pl->t.size(); ++id) {
+        const PlanTensor& t = T((int)id);
+        lay[id] = !t.is_const && t.shape.size() == 4 && (int)id != pl->input && (int)id != pl->output && nh_kind(pl, t.dtype) >= 0 && t.bytes != 0;
+    }
+    std::vector<int> concat_of(pl->t.size(), -1);            // Concat node that a tensor is an operand of
+    std::vector<char> operand_twice(pl->t.size(), 0);
+    for (size_t i = 0; i < nn; ++i)
+        if (pl->nodes[i].op == ZANT_OP_CONCAT) for (int id : pl->nodes[i].in) if (id >= 0) { operand_twice[id] = operand_twice[id] || concat_of[id] >= 0; concat_of[id] = (int)i; }
+    auto first_layer = [&](int id) { return T(id).shape.size() == 4 && T(id).shape[1] <= 4; };
+    bool changed = true;
+    while (changed) {
+        changed = false;
+        auto off = [&](int id) { if (id >= 0 && lay[id]) { lay[id] = 0; changed = true; } };
+        for (size_t i = 0; i < nn; ++i) {
+            const PlanNode& n = pl->nodes[i];
+            const int gi = group_of[i];
+            if (gi >= 0 && pl->nh_groups[gi].on) {
+                NhGroup& q = pl->nh_groups[gi];
+                if (i != q.first) continue;
+                for (int id : q.interior) lay[id] = 0;                             // interior: no layout of its own
+                if (lay[q.y] && T(q.y).shape[1] % 16 != 0) off(q.y);               // the epilogue stores 16 channels at a time
+                const bool in_ok = lay[q.x] || (first_layer(q.x) && lay[q.y]);
+                // an NCHW result cannot be upsampled in place, and a first layer pays for its conversion only in front of more such layers
+                if (!in_ok || (!lay[q.y] && q.up2)) { q.on = false; changed = true; off(q.x); off(q.y); }
+                continue;
+            }
+            switch (n.op) {
+                case ZANT_OP_MAXPOOL:
+                    if (n.in.size() == 1 && n.out.size() == 1 && lay[n.in[0]] && lay[n.out[0]] && T(n.in[0]).shape[1] % 16 == 0) break;
+                    for (int id : n.in) off(id);
+                    for (int id : n.out) off(id);
+                    break;
+                case ZANT_OP_CONCAT: {
+                    const int64_t ax = n.a.axis < 0 ? n.a.axis + 4 : n.a.axis;
+                    bool ok = ax == 1 && n.out.size() == 1 && lay[n.out[0]] && concat_of[n.out[0]] < 0;
+                    for (int id : n.in) ok = ok && id >= 0 && lay[id] && T(id).shape[1] % 16 == 0 && !operand_twice[id];
+                    if (ok) break;
+                    for (int id : n.in) off(id);
+                    for (int id : n.out) off(id);
+                    break;
+                }
+                case ZANT_OP_QUANTIZE_LINEAR:
+                    for (int id : n.in) off(id);
+                    for (int id : n.out)
+                        if (own[i] || n.out.size() != 1 || !lay[id] || !first_layer(id) || check_zero_point(T(id).dtype, n.a.y_zp, "QuantizeLinear y") != ZANT_OK) off(id);
+                    break;
+                default:
+                    for (int id : n.in) off(id);
+                    for (int id : n.out) off(id);
+            }
+        }
+    }
+    // storage
+    const int parts = pl->ctx->tf32 == 2 ? 2 : 1;
+    for (size_t id = 0; id < pl->t.size(); ++id) {
+        PlanTensor& t = T((int)id);
+        if (!lay[id]) continue;
+        const size_t esz = dtype_size(t.dtype), chans = t.shape[1] <= 4 ? (esz == 1 ? 16 : (parts == 2 ? 8 : 4)) : t.shape[1];
+        t.nh = true;
+        t.nh_root = concat_of[id] >= 0 ? pl->nodes[concat_of[id]].out[0] : (int)id;
+        if (t.nh_root == (int)id) { t.nh_pix = chans * esz * (esz == 4 ? parts : 1); t.nh_lo = esz == 4 && parts == 2 ? (int)chans : 0; }
+    }
+    for (size_t i = 0; i < nn; ++i) {
+        const PlanNode& n = pl->nodes[i];
+        if (n.op != ZANT_OP_CONCAT || !T(n.out[0]).nh) continue;
+        size_t o = 0;
+        for (int id : n.in) {
+            PlanTensor& t = T(id);
+            t.nh_off = o; t.nh_pix = T(n.out[0]).nh_pix; t.nh_lo = T(n.out[0]).nh_lo;
+            o += t.shape[1] * dtype_size(t.dtype);
+        }
+    }
+    for (NhGroup& q : pl->nh_groups) if (q.on) for (int id : q.interior) T(id).elided = true;
+}
+
+static NhView nh_view(zant_plan* pl, int id) {
+    const PlanTensor& t = pl->t[id];
+    return NhView{t.arena_ptr, (long long)t.nh_pix, (int)t.shape[2], (int)t.shape[3], t.nh_lo};
+}
+
+static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
+    consumed = 0;
+    const PlanNode& n = pl->nodes[i];
+    zant_ctx* ctx = pl->ctx;
+    auto T = [&](int id) -> const PlanTensor& { return pl->t[id]; };
+    auto push = [&](const std::string& name, std::function<int32_t()> fn) { pl->steps.push_back(std::move(fn)); pl->step_names.push_back(name); };
+    const size_t first_step = pl->steps.size();
+    if (n.op == ZANT_OP_CONCAT && n.out.size() == 1 && T(n.out[0]).nh) {      // its operands are in place
+        std::vector<const size_t*> shapes; std::vector<size_t> ranks;
+        for (int id : n.in) { shapes.push_back(T(id).shape.data()); ranks.push_back(T(id).shape.size()); }
+        ConcatGeom g; size_t os[8];
+        ZB_TRY(concat_resolve(shapes.data(), ranks.data(), n.in.size(), n.a.axis, os, g));
+        for (int id : n.in) if (T(id).dtype != T(n.out[0]).dtype) return fail(ZANT_E_INPUT_ARRAY_WRONG_TYPE, "Concat dtype mismatch");
+        for (size_t d = 0; d < 4; ++d) if (T(n.out[0]).shape[d] != os[d]) return fail(ZANT_E_MISMATCHED_SHAPE, "Concat output dim %zu", d);
+        consumed = 1;
+        return ZANT_OK;
+    }
+    if (n.op == ZANT_OP_QUANTIZE_LINEAR && n.out.size() == 1 && T(n.out[0]).nh) {
+        ZB_TRY(need_inputs(n, 1, 1, "QuantizeLinear"));
+        const int x = n.in[0], y = n.out[0];
+        ZB_TRY(want_dtype(pl, x, ZANT_F32, "QuantizeLinear"));
+        if (T(x).bytes != T(y).bytes * 4) return fail(ZANT_E_OUTPUT_TENSOR_DIFFERENT_SIZE, "QuantizeLinear sizes differ");
+        const int N = (int)T(y).shape[0], C = (int)T(y).shape[1];
+        const long long hw = (long long)(T(y).shape[2] * T(y).shape[3]);
+        const float sc = n.a.y_scale; const int zp = n.a.y_zp; const bool u8 = T(y).dtype == ZANT_U8;
+        push("QuantizeLinear", [=]() { return run_to_nhwc(ctx, 0, pl->ptr(x), pl->t[y].arena_ptr, N, C, hw, sc, zp, u8); });
+        record_step_cost(pl, first_step, i, 1);
+        consumed = 1;
+        return ZANT_OK;
+    }
+    if (n.op == ZANT_OP_MAXPOOL && n.out.size() == 1 && T(n.out[0]).nh) {
+        const zant_node_attrs& a = n.a;
+        const int x = n.in[0], y = n.out[0];
+        PoolGeom g;
+        const size_t ones[2] = {1, 1};
+        ZB_TRY(pool_resolve(T(x).shape.data(), T(x).shape.size(), T(y).shape.data(), T(y).shape.size(), a.kernel_shape, 2, a.n_strides ? a.strides : ones, 2,
+                            a.n_dilations ? a.dilations : ones, 2, a.pads, a.n_pads, a.auto_pad < 0 ? 0 : a.auto_pad, g));
+        if (T(x).dtype != T(y).dtype) return fail(ZANT_E_INPUT_ARRAY_WRONG_TYPE, "MaxPool dtype mismatch");
+        const int kind = nh_kind(pl, T(x).dtype), N = (int)T(x).shape[0], C = (int)T(x).shape[1];
+        push("MaxPool", [=]() { return run_nh_maxpool(ctx, kind, g, N, C, nh_view(pl, x), nh_view(pl, y)); });
+        record_step_cost(pl, first_step, i, 1);
+        consumed = 1;
+        return ZANT_OK;
+    }
+    const NhGroup* found = nullptr;
+    for (const NhGroup& q : pl->nh_groups) if (q.on && q.first == i) found = &q;
+    if (!found) return ZANT_OK;
+    const NhGroup q = *found;
+    ConvGeom g;
+    if (!nh_conv_geom(pl, n, g)) return fail(ZANT_E_INVALID_DIMENSIONS, "convolution geometry");
+    const int kind = nh_kind(pl, T(q.x).dtype);
+    auto np = std::make_shared<NhConvPlan>();
+    if (!nh_conv_plan(g, kind, q.pool, ctx->sm_count, *np)) return fail(ZANT_E_UNSUPPORTED, "shape not taken by the channels-last kernel");
+    const bool i8 = kind <= NH_U8, split = kind == NH_TF32X3;
+    const int x = q.x, y = q.y;
+    int xbuf = -1;                                            // scratch of a first layer's converted input
+    if (!T(x).nh) {
+        const size_t px = (size_t)g.N * g.H * g.W;
+        xbuf = pl->add_scratch(px * (split ? 64 : 16));
+        const int mode = i8 ? 1 : (split ? 3 : 2), C = g.C; const long long hw = (long long)g.H * g.W;
+        push(i8 ? "ToChannelsLast" : "ToChannelsLast(tf32)", [=]() { return run_to_nhwc(ctx, mode, pl->ptr(x), pl->scratch(xbuf), g.N, C, hw, 1.0f, 0, false); });
+    }
+    NhConvArgs base = np->a;
+    std::vector<uint8_t> wb;
+    int am = -1, ab = -1, alut = -1;
+    std::string name;
+    if (i8) {
+        std::vector<float> mult, mp; std::vector<int32_t> bp;
+        const PlanTensor& ws = T(n.in[2]);
+        const int b = opt_in(n, 4);
+        requant_multipliers(n.a.x_scale, (const float*)ws.host.data(), ws.bytes / 4, n.a.y_scale, (size_t)g.M, mult);
+        nh_prepare_i8(*np, (const int8_t*)T(n.in[1]).host.data(), mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, n.a.x_zp, wb, mp, bp);
+        am = pl->add_aux(mp.data(), mp.size() * 4); ab = pl->add_aux(bp.data(), bp.size() * 4);
+        base.act = q.qact >= 0 ? q.qact : n.a.activation;
+        base.six = lean_six(n.a.y_scale);
+        name = "QLinearConv(tc-implicit)";
+        if (q.qact >= 0) name += "+Relu";
+        if (q.lut_node >= 0) {
+            uint8_t lut[256];
+            activation_lut(pl->nodes[q.lut_node], ZANT_I8, lut);
+            alut = pl->add_aux(lut, 256);
+            name += "+ActivationLut";
+        }
+        if (q.pool) name += "+MaxPool";
+        if (q.dequant >= 0) { base.dq_scale = pl->nodes[q.dequant].a.x_scale; base.dq_zp = pl->nodes[q.dequant].a.x_zp; }
+    } else {
+        std::vector<float> bp;
+        const int b = opt_in(n, 2);
+        nh_prepare_tf32(*np, (const float*)T(n.in[1]).host.data(), b >= 0 ? (const float*)T(b).host.data() : nullptr, wb, bp);
+        ab = pl->add_aux(bp.data(), bp.size() * 4);
+        base.act = q.fact; base.slope = q.slope;
+        name = std::string("Conv(tf32)") + (q.fact == FACT_RELU ? "+Relu" : (q.fact == FACT_LEAKY ? "+LeakyRelu" : ""));
+    }
+    if (q.up2) name += "+Resize";
+    if (q.dequant >= 0) name += "+DequantizeLinear";
+    const int aw = pl->add_aux(wb.data(), wb.size());
+    base.up2 = q.up2 ? 1 : 0;
+    push(name, [=]() {
+        NhConvArgs a = base;
+        const PlanTensor& yt = pl->t[y];
+        a.w = (const uint8_t*)pl->aux(aw);
+        if (i8) { a.mult = (const float*)pl->aux(am); a.bias = (const int32_t*)pl->aux(ab); a.lut = alut >= 0 ? (const uint8_t*)pl->aux(alut) : nullptr; }
+        else a.fbias = (const float*)pl->aux(ab);
+        if (yt.nh) {
+            const NhView v = nh_view(pl, y);
+            a.y = (uint8_t*)v.ptr; a.y_pix = v.pix; a.y_row = v.pix * v.W; a.y_img = a.y_row * v.H; a.lo_out = v.lo; a.round_out = 1;
+        } else {
+            a.y = (uint8_t*)pl->ptr(y); a.nchw = q.dequant >= 0 ? 2 : 1;
+        }
+        const NhView xv = xbuf >= 0 ? NhView{pl->scratch(xbuf), split ? 64 : 16, g.H, g.W, split ? 8 : 0} : nh_view(pl, x);
+        return nh_conv_run(ctx, *np, a, xv);
+    });
+    record_step_cost(pl, first_step, i, q.count);
+    consumed = q.count;
     return ZANT_OK;
 }
