@@ -60,6 +60,13 @@ inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     return check_launch(ctx, "contract_f32_few");
 }
 
+inline int32_t run_transpose_pad_f32(zant_ctx* ctx, const float* w, float* wt, int M, int K, int N4) {
+    const dim3 grid((unsigned)((K + 31) / 32), (unsigned)((N4 + 31) / 32));
+    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output channels");
+    launch(ctx, transpose_pad_f32, grid, 256, 0, w, wt, M, K, N4);
+    return check_launch(ctx, "transpose_pad_f32");
+}
+
 // `w_kn`: the weights as [K][N rounded up to 4] (a plan transposes them once), else null and `w` is [M][C][KH][KW].
 inline int32_t run_conv_f32(zant_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y,
                             const ContractFusion& fu = ContractFusion{}, const float* w_kn = nullptr) {

@@ -83,6 +83,7 @@ struct zant_plan {
     char* arena = nullptr;
     size_t arena_bytes = 0;
     std::vector<std::function<int32_t()>> steps;
+    std::vector<std::function<int32_t()>> init_steps;   // run once when the constants are in the arena: weights into a kernel's layout
     std::vector<std::string> step_names;
     std::vector<double> step_macs, step_bytes;   // algorithmic work of each step: multiply-accumulates, bytes crossing the step's boundary
     int launches_per_run = 0;
@@ -355,6 +356,10 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     for (size_t a = 0; a < plan->aux_host.size(); ++a)
         if (!plan->aux_host[a].empty())
             ZB_CUDA(cudaMemcpyAsync(plan->arena + plan->aux_off[a], plan->aux_host[a].data(), plan->aux_host[a].size(), cudaMemcpyHostToDevice, ctx->stream));
+    const uint64_t launched = ctx->launches;
+    for (auto& s : plan->init_steps) { int32_t st = s(); if (st != ZANT_OK) return st; }
+    plan->init_steps.clear();
+    ctx->launches = launched;
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
     for (auto& t : plan->t) { t.host.clear(); t.host.shrink_to_fit(); }
 
@@ -784,10 +789,8 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
             const int K = g.C * g.KH * g.KW, N4 = (g.M + 3) / 4 * 4;
             int at = -1;
             if (T(w).is_const && (long long)K * N4 <= (1LL << 28)) {
-                std::vector<float> wt((size_t)K * N4, 0.0f);
-                const float* ws = (const float*)T(w).host.data();
-                for (int m = 0; m < g.M; ++m) for (int k = 0; k < K; ++k) wt[(size_t)k * N4 + m] = ws[(size_t)m * K + k];
-                at = pl->add_aux(wt.data(), wt.size() * 4);
+                at = pl->add_scratch((size_t)K * N4 * 4);
+                pl->init_steps.push_back([=]() { return run_transpose_pad_f32(ctx, pl->p<float>(w), (float*)pl->scratch(at), g.M, K, N4); });
             }
             const int fact = pl->pending_fact; const float fslope = pl->pending_slope;
             const bool pool = pl->pending_pool >= 0;
@@ -797,7 +800,7 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
             push(name.c_str(), [=]() {
                 ContractFusion fu;
                 fu.act = fact == FACT_RELU ? CT_ACT_RELU : (fact == FACT_LEAKY ? CT_ACT_LEAKY : CT_ACT_NONE); fu.slope = fslope; fu.pool = pool;
-                return run_conv_f32(ctx, g, pl->p<float>(x), pl->p<float>(w), pl->p<float>(b), pl->p<float>(yw), fu, at >= 0 ? (const float*)pl->aux(at) : nullptr);
+                return run_conv_f32(ctx, g, pl->p<float>(x), pl->p<float>(w), pl->p<float>(b), pl->p<float>(yw), fu, at >= 0 ? (const float*)pl->scratch(at) : nullptr);
             });
             return ZANT_OK;
         }
@@ -1937,15 +1940,20 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
         push(i8 ? "ToChannelsLast" : "ToChannelsLast(tf32)", [=]() { return run_to_nhwc(ctx, mode, pl->ptr(x), pl->scratch(xbuf), g.N, C, hw, 1.0f, 0, false); });
     }
     NhConvArgs base = np->a;
-    std::vector<uint8_t> wb;
     int am = -1, ab = -1, alut = -1;
     std::string name;
     if (i8) {
-        std::vector<float> mult, mp; std::vector<int32_t> bp;
+        std::vector<float> mp; std::vector<int32_t> bp((size_t)base.const_n, 0);
         const PlanTensor& ws = T(n.in[2]);
         const int b = opt_in(n, 4);
-        requant_multipliers(n.a.x_scale, (const float*)ws.host.data(), ws.bytes / 4, n.a.y_scale, (size_t)g.M, mult);
-        nh_prepare_i8(*np, (const int8_t*)T(n.in[1]).host.data(), mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, n.a.x_zp, wb, mp, bp);
+        requant_multipliers(n.a.x_scale, (const float*)ws.host.data(), ws.bytes / 4, n.a.y_scale, (size_t)g.M, mp);
+        mp.resize((size_t)base.const_n, 1.0f);
+        const int K = g.Cg * g.KH * g.KW;
+        for (int m = 0; m < g.M; ++m) {
+            int sum = 0;
+            if (n.a.x_zp != 0) for (int k = 0; k < K; ++k) sum += ((const int8_t*)T(n.in[1]).host.data())[(size_t)m * K + k];
+            bp[m] = (b >= 0 ? ((const int32_t*)T(b).host.data())[m] : 0) - n.a.x_zp * sum;
+        }
         am = pl->add_aux(mp.data(), mp.size() * 4); ab = pl->add_aux(bp.data(), bp.size() * 4);
         base.act = q.qact >= 0 ? q.qact : n.a.activation;
         base.six = lean_six(n.a.y_scale);
@@ -1960,21 +1968,22 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
         if (q.pool) name += "+MaxPool";
         if (q.dequant >= 0) { base.dq_scale = pl->nodes[q.dequant].a.x_scale; base.dq_zp = pl->nodes[q.dequant].a.x_zp; }
     } else {
-        std::vector<float> bp;
+        std::vector<float> bp((size_t)base.const_n, 0.0f);
         const int b = opt_in(n, 2);
-        nh_prepare_tf32(*np, (const float*)T(n.in[1]).host.data(), b >= 0 ? (const float*)T(b).host.data() : nullptr, wb, bp);
+        if (b >= 0) std::memcpy(bp.data(), T(b).host.data(), (size_t)g.M * 4);
         ab = pl->add_aux(bp.data(), bp.size() * 4);
         base.act = q.fact; base.slope = q.slope;
         name = std::string("Conv(tf32)") + (q.fact == FACT_RELU ? "+Relu" : (q.fact == FACT_LEAKY ? "+LeakyRelu" : ""));
     }
     if (q.up2) name += "+Resize";
     if (q.dequant >= 0) name += "+DequantizeLinear";
-    const int aw = pl->add_aux(wb.data(), wb.size());
+    const int aw = pl->add_scratch(np->w_bytes), w = n.in[1];
+    pl->init_steps.push_back([=]() { return run_nh_weights(ctx, *np, pl->ptr(w), pl->scratch(aw)); });
     base.up2 = q.up2 ? 1 : 0;
     push(name, [=]() {
         NhConvArgs a = base;
         const PlanTensor& yt = pl->t[y];
-        a.w = (const uint8_t*)pl->aux(aw);
+        a.w = (const uint8_t*)pl->scratch(aw);
         if (i8) { a.mult = (const float*)pl->aux(am); a.bias = (const int32_t*)pl->aux(ab); a.lut = alut >= 0 ? (const uint8_t*)pl->aux(alut) : nullptr; }
         else a.fbias = (const float*)pl->aux(ab);
         if (yt.nh) {

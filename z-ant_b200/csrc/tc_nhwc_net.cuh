@@ -100,22 +100,16 @@ __device__ __forceinline__ uint64_t nh_desc(uint32_t addr, uint32_t row_bytes) {
 // One lane's (`leader`) MMA of a converged warp.
 template <int KIND>
 __device__ __forceinline__ void nh_mma(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0u;
-    if (KIND <= NH_U8)
-        asm volatile(
-            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %8, 0;\n\t"
-            "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, p;\n\t}\n"
-            ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(zero), "r"(leader) : "memory");
-    else
+    if (KIND <= NH_U8) {
+        ptx::mma_i8_if(leader, d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
+    } else {
+        const uint32_t zero = 0u;
         asm volatile(
             "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %8, 0;\n\t"
             "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
             "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %5, {%7, %7, %7, %7}, p;\n\t}\n"
             ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(zero), "r"(leader) : "memory");
-}
-__device__ __forceinline__ void nh_commit(uint32_t leader, uint32_t bar) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar), "r"(leader) : "memory");
+    }
 }
 
 // The tiles of a CTA, grid-size apart, as a mixed-radix counter: divisions at the start only (a tile's four cost its 19 warps
@@ -338,16 +332,16 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                         else group(std::integral_constant<int, 1>{}, it0, bl);
                     }
                     if (!a.w_resident) {
-                        nh_commit(leader, wempty(ws));
+                        ptx::mma_commit_if(leader, wempty(ws));
                         if (++ws == a.w_stages) { ws = 0; wph ^= 1u; }
                     }
                 }
                 if (!alive) break;
-                nh_commit(leader, empty(s));
+                ptx::mma_commit_if(leader, empty(s));
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
             if (!alive) break;
-            nh_commit(leader, tfull(b));
+            ptx::mma_commit_if(leader, tfull(b));
         }
         __syncwarp();
     } else {
@@ -496,12 +490,12 @@ struct NhConvPlan {
 };
 
 // Taps of pair `it` (KC = 16) without a pool; the second one lies behind the first in shared memory.  -1: none (zero weights).
-inline int nh_pair(int it, int which, int taps) {
+__host__ __device__ inline int nh_pair(int it, int which, int taps) {
     const int t = 2 * it + which;
     return t < taps ? t : -1;
 }
 // NH_POOL_VIEWS: view of pair `it`: two rows apart, i.e. in the same parity plane.
-inline int nh_view_pair(int it, int which) { return (it >> 2) * 4 + (it & 3) + which * 8; }
+__host__ __device__ inline int nh_view_pair(int it, int which) { return (it >> 2) * 4 + (it & 3) + which * 8; }
 
 // Operand offsets, in 16-byte units.
 inline void nh_offsets(NhConvArgs& a, int mode) {
@@ -619,74 +613,61 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
     return best < 1e300;
 }
 
-// Weights [M][C][KH][KW] as [filter tile][channel stage][iteration][part][NB rows of KC bytes], rows swizzled as the tensor core reads
+// Weights [M][C][KH][KW] -> [filter tile][channel stage][iteration][part][NB rows of KC bytes], rows swizzled as the tensor core reads
 // them (16-byte chunk c of row j at c ^ (j % 8), c ^ (j / 2 % 4), c ^ (j / 4 % 2) for rows of 128, 64, 32 bytes); KC = 16: [filter
 // tile][pair][2][NB rows of 16 bytes].  Rows of an iteration: the tile's filters (no pool), those of the four members for the
 // iteration's view (NH_POOL_VIEWS), those of two members for a middle view, or of one member for each outer view (NH_POOL_PAIRS).
-template <typename T, typename F>
-inline void nh_block_weights(const NhConvPlan& p, const T* w, int part, std::vector<uint8_t>& out, F f) {
-    const NhConvArgs& a = p.a;
-    const int taps = a.KH * a.KW, NT = p.NT, KC = a.KC, chans = KC / (int)sizeof(T);
-    const int NB = NT * (p.pool == NH_POOL_VIEWS ? 4 : (p.pool == NH_POOL_PAIRS ? 2 : 1));
-    struct Put { int it, half, row, tap; };                   // tap `tap` of filter j goes to row `row` + j of iteration `it` (half: of a pair)
-    std::vector<Put> puts;
-    if (p.pool == NH_POOL_VIEWS) {
-        for (int it = 0; it < a.T; ++it)
-            for (int half = 0; half < (KC == 16 ? 2 : 1); ++half) {
-                const int view = KC == 16 ? nh_view_pair(it, half) : it;
-                for (int m = 0; m < 4; ++m) {
-                    const int kh = view / 4 - (m >> 1), kw = view % 4 - (m & 1);
-                    if (kh >= 0 && kh < 3 && kw >= 0 && kw < 3) puts.push_back({it, half, m * NT, kh * 3 + kw});
-                }
-            }
-    } else if (p.pool == NH_POOL_PAIRS) {
-        for (int kh = 0; kh < 3; ++kh) {
-            puts.push_back({kh * 3, 0, 0, kh * 3 + 1}); puts.push_back({kh * 3, 0, NT, kh * 3});                  // rx = 1: dx = 0 has kw = 1, dx = 1 has kw = 0
-            puts.push_back({kh * 3 + 1, 0, 0, kh * 3 + 2}); puts.push_back({kh * 3 + 1, 0, NT, kh * 3 + 1});      // rx = 2
-            puts.push_back({kh * 3 + 2, 0, 0, kh * 3}); puts.push_back({kh * 3 + 2, 0, NT, kh * 3 + 2});          // rx = 0: dx = 0; rx = 3: dx = 1
+// Done on the device when a plan is finalized, a thread per 16-byte chunk (the byte shuffle of a 1024 x 512 x 3 x 3 tensor took the
+// host 30 ms).  T: int8_t, or float (rounded to TF32, part 1 the remainder).
+struct NhWeightArgs { const void* w; uint8_t* out; int M, C, taps, NT, NB, KC, T, c_stages, parts, pool; long long chunks; };
+template <typename T>
+__global__ void __launch_bounds__(256) nh_weights_k(const __grid_constant__ NhWeightArgs a) {
+    ptx::grid_start();
+    constexpr int PER = 16 / (int)sizeof(T);
+    const int per_row = a.KC / 16;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.chunks; i += (long long)gridDim.x * blockDim.x) {
+        long long t = i;
+        int slot = (int)(t % per_row); t /= per_row;
+        const int row = (int)(t % a.NB); t /= a.NB;
+        int half = 0, part = 0;
+        if (a.KC == 16) { half = (int)(t & 1); t >>= 1; } else { part = (int)(t % a.parts); t /= a.parts; }
+        const int it = (int)(t % a.T); t /= a.T;
+        const int cs = (int)(t % a.c_stages), nt = (int)(t / a.c_stages);
+        slot ^= a.KC == 128 ? (row & 7) : (a.KC == 64 ? (row >> 1) & 3 : (a.KC == 32 ? (row >> 2) & 1 : 0));      // the chunk that is stored here
+        const int blk = row / a.NT, m = nt * a.NT + row - blk * a.NT, c0 = (cs * per_row + slot) * PER;
+        int tap = -1;
+        if (a.pool == NH_POOL_VIEWS) {
+            const int view = a.KC == 16 ? nh_view_pair(it, half) : it, kh = view / 4 - (blk >> 1), kw = view % 4 - (blk & 1);
+            if (kh >= 0 && kh < 3 && kw >= 0 && kw < 3) tap = kh * 3 + kw;
+        } else if (a.pool == NH_POOL_PAIRS) {
+            const int kh = it / 3, j = it - 3 * kh;            // rx = 1: kw = 1, 0; rx = 2: kw = 2, 1; rx = 0: kw = 0 and rx = 3: kw = 2
+            tap = kh * 3 + (j == 2 ? 2 * blk : j + 1 - blk);
+        } else {
+            tap = a.KC == 16 ? nh_pair(it, half, a.taps) : it;
         }
-    } else {
-        for (int it = 0; it < a.T; ++it)
-            for (int half = 0; half < (KC == 16 ? 2 : 1); ++half) {
-                const int tap = KC == 16 ? nh_pair(it, half, taps) : it;
-                if (tap >= 0) puts.push_back({it, half, 0, tap});
-            }
-    }
-    for (int m = 0; m < a.M; ++m) {
-        const int nt = m / NT, j = m % NT;
-        for (int c = 0; c < p.w_cin; ++c) {
-            const int cs = c / chans, cb = c % chans * (int)sizeof(T);
-            const T* src = w + ((size_t)m * p.w_cin + c) * taps;
-            uint8_t* stage = out.data() + ((size_t)nt * a.c_stages + cs) * a.T * a.w_chunk;
-            for (const Put& u : puts) {
-                const T v = f(src[u.tap]);
-                const int row = u.row + j, x = KC == 128 ? (row & 7) : (KC == 64 ? (row >> 1) & 3 : (KC == 32 ? (row >> 2) & 1 : 0));
-                uint8_t* dst = stage + (size_t)u.it * a.w_chunk;
-                if (KC == 16) dst += (size_t)(u.half * NB + row) * 16 + cb;
-                else dst += ((size_t)part * NB + row) * KC + ((((cb >> 4) ^ x) << 4) | (cb & 15));
-                std::memcpy(dst, &v, sizeof(T));
+        union { T v[PER]; uint4 q; } u;
+        u.q = make_uint4(0u, 0u, 0u, 0u);
+        if (m < a.M && tap >= 0) {
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                if (c0 + k >= a.C) break;
+                const T v = __ldg((const T*)a.w + ((size_t)m * a.C + c0 + k) * a.taps + tap);
+                if constexpr (sizeof(T) == 4) { const float hi = round_tf32(v); u.v[k] = part == 0 ? hi : round_tf32(__fadd_rn(v, -hi)); }
+                else u.v[k] = v;
             }
         }
+        reinterpret_cast<uint4*>(a.out)[i] = u.q;
     }
 }
-
-inline void nh_prepare_i8(const NhConvPlan& p, const int8_t* w, const float* mult, const int32_t* bias, int x_zp, std::vector<uint8_t>& wb, std::vector<float>& mp, std::vector<int32_t>& bp) {
-    const int K = p.w_cin * p.a.KH * p.a.KW;
-    wb.assign(p.w_bytes, 0); mp.assign(p.a.const_n, 1.0f); bp.assign(p.a.const_n, 0);
-    nh_block_weights<int8_t>(p, w, 0, wb, [](int8_t v) { return v; });
-    for (int m = 0; m < p.a.M; ++m) {
-        int sum = 0;
-        for (int k = 0; k < K; ++k) sum += w[(size_t)m * K + k];
-        mp[m] = mult[m];
-        bp[m] = (bias ? bias[m] : 0) - x_zp * sum;
-    }
-}
-
-inline void nh_prepare_tf32(const NhConvPlan& p, const float* w, const float* bias, std::vector<uint8_t>& wb, std::vector<float>& bp) {
-    wb.assign(p.w_bytes, 0); bp.assign(p.a.const_n, 0.0f);
-    nh_block_weights<float>(p, w, 0, wb, [](float v) { return host_round_tf32(v); });
-    if (p.a.parts == 2) nh_block_weights<float>(p, w, 1, wb, [](float v) { const float hi = host_round_tf32(v); return host_round_tf32(v - hi); });
-    for (int m = 0; m < p.a.M; ++m) bp[m] = bias ? bias[m] : 0.0f;
+inline int32_t run_nh_weights(zant_ctx* ctx, const NhConvPlan& p, const void* w, void* out) {
+    NhWeightArgs a{};
+    a.w = w; a.out = (uint8_t*)out; a.M = p.a.M; a.C = p.w_cin; a.taps = p.a.KH * p.a.KW; a.NT = p.a.NT; a.KC = p.a.KC; a.T = p.a.T; a.c_stages = p.a.c_stages;
+    a.NB = p.a.NT * (p.pool == NH_POOL_VIEWS ? 4 : (p.pool == NH_POOL_PAIRS ? 2 : 1));
+    a.parts = p.a.parts; a.pool = p.pool; a.chunks = (long long)p.w_bytes / 16;
+    const int grid = grid_for((size_t)a.chunks, 256, ctx->sm_count);
+    if (p.kind <= NH_U8) launch(ctx, nh_weights_k<int8_t>, grid, 256, 0, a);
+    else launch(ctx, nh_weights_k<float>, grid, 256, 0, a);
+    return check_launch(ctx, "nh_weights_k");
 }
 
 // A channels-last buffer: `ptr` = channel 0 of pixel (0, 0), pixels `pix` bytes apart; lo: split form, channel offset of the lo half.
