@@ -13,6 +13,7 @@ calls raise.  The directory name contains a hyphen, so the package is loaded by 
 `__graft_entry__.load_package`) and registers itself as `zant_b200`.
 """
 import ctypes as C
+import functools
 import os
 
 import numpy as np
@@ -27,6 +28,7 @@ AUTO_PAD = {"NOTSET": 0, "SAME_UPPER": 1, "SAME_LOWER": 2, "VALID": 3}
 QACT = {None: 0, "none": 0, "relu": 1, "relu6": 2}
 COORD_MODE = {"half_pixel": 0, "align_corners": 1, "asymmetric": 2}
 SIZE_MAX = (1 << 64) - 1
+_TORCH_DTYPE = {}       # torch dtype -> code, filled when the first tensor is seen
 
 OP = dict(Conv=1, MatMul=2, Gemm=3, MaxPool=4, Relu=5, LeakyRelu=6, Add=7, Concat=8, Resize=9, ReduceMean=10,
           Reshape=11, Clip=12, Sigmoid=13, Softmax=14, Tanh=15, Ceil=16, Mul=17, Div=18, Transpose=19, Slice=27, Gather=28,
@@ -75,6 +77,19 @@ class NodeAttrs(C.Structure):
     ]
 
 
+# Argument types of the entry points that are called per operator or per pass: with them ctypes converts Python integers and
+# addresses itself (a conv call spent half of its 9 us on the host wrapping 22 arguments one by one).
+# p pointer, z size_t, i int32, f float.
+_SIGNATURES = {
+    "conv_f32": "p ppz ppz pz ppz pz pz pz z pz", "mat_mul_f32": "p ppz ppz ppz", "gemm_lean_f32": "p ppz ppz ppz ffii ppz", "gemm_f32": "p ppz ppz ppz ffii ppz",
+    "maxpool_f32": "p ppz ppz pz pz pz pz i", "maxpool_q8": "p i ppz ppz pz pz pz pz i", "relu_f32": "p pp z", "leaky_relu_f32": "p p f p z",
+    "clip_f32": "p p ff p z", "sigmoid_f32": "p pp z", "tanh_f32": "p pp z", "ceil_f32": "p pp z", "mul_f32": "p pz pz p", "div_f32": "p pz pz p",
+    "sum_tensors_f32": "p ppz ppz ppz", "quantize_linear": "p p z f i i p", "dequantize_linear": "p i p z f i p",
+    "qlinearconv": "p i ppz f i ppz pp z f i p z i ppz pz pz pz z i i", "qlinearconv_nhwc": "p i ppz f i ppz pp z f i p z i ppz pz pz pz z i i",
+    "qlinearmatmul": "p i ppz f i ppz pp z f i p z i ppz i", "qlinearadd": "p i p f i p f i f i p z i", "plan_run": "p pp",
+}
+_CTYPE = {"p": C.c_void_p, "z": C.c_size_t, "i": C.c_int32, "f": C.c_float}
+
 _lib = None
 
 
@@ -94,6 +109,8 @@ def lib():
         _lib.zant_b200_plan_arena_bytes.restype = C.c_size_t
         _lib.zant_b200_plan_tensor_ptr.restype = C.c_void_p
         _lib.zant_b200_plan_step_name.restype = C.c_char_p
+        for name, sig in _SIGNATURES.items():
+            getattr(_lib, "zant_b200_" + name).argtypes = [_CTYPE[ch] for ch in sig.replace(" ", "")]
     return _lib
 
 
@@ -120,13 +137,18 @@ def check(status):
 
 
 # ----------------------------------------------------------------------------------------- helpers
-def _sz(seq):
-    if seq is None:
-        return None, 0
-    vals = [SIZE_MAX if v == "SIZE_MAX" else int(v) for v in seq]
+@functools.lru_cache(maxsize=8192)
+def _dims(vals):
+    """(size_t array, length) of a tuple of sizes.  The library only reads the array, so equal tuples share one."""
+    vals = [SIZE_MAX if v == "SIZE_MAX" else int(v) for v in vals]
     return (C.c_size_t * max(len(vals), 1))(*vals), len(vals)
 
 
+def _sz(seq):
+    return (None, 0) if seq is None else _dims(tuple(seq))
+
+
+@functools.lru_cache(maxsize=64)
 def _bytes(s):
     if s is None:
         return None, 0
@@ -142,6 +164,15 @@ def _ptr(a):
     return a.ctypes.data_as(C.c_void_p)
 
 
+def _addr(a):
+    """The same as a plain integer, for the entry points of _SIGNATURES."""
+    if a is None:
+        return None
+    if hasattr(a, "data_ptr"):
+        return a.data_ptr()
+    return a.__array_interface__["data"][0]
+
+
 def _host(a, dt=None):
     """numpy arrays are made contiguous (and cast when dt is given); device tensors pass through."""
     if a is None or hasattr(a, "data_ptr"):
@@ -155,8 +186,10 @@ def _shape(a):
 
 def _dtype_code(a):
     if hasattr(a, "data_ptr"):
-        import torch
-        return {torch.float32: F32, torch.int8: I8, torch.uint8: U8, torch.int32: I32}[a.dtype]
+        if not _TORCH_DTYPE:
+            import torch
+            _TORCH_DTYPE.update({torch.float32: F32, torch.int8: I8, torch.uint8: U8, torch.int32: I32})
+        return _TORCH_DTYPE[a.dtype]
     return DTYPE_OF[a.dtype]
 
 
@@ -168,11 +201,16 @@ def _shape_list(shapes):
     return ptrs, ranks, keep
 
 
-def _numel(shape):
+@functools.lru_cache(maxsize=8192)
+def _product(shape):
     n = 1
     for d in shape:
         n *= int(d)
     return n
+
+
+def _numel(shape):
+    return _product(tuple(shape))
 
 
 # ----------------------------------------------------------------------------------------- shape helpers (no GPU needed)
@@ -312,10 +350,10 @@ class Context:
         y = self._out(out, y_shape, F32)
         xs, xr = _sz(_shape(x)); ws, wr = _sz(_shape(w)); ys, yr = _sz(y_shape)
         st, ns = _sz(stride); pd, npd = _sz(pads); dl, nd = _sz(dilations); ap, apl = _bytes(auto_pad)
-        check(lib().zant_b200_conv_f32(self._h, _ptr(x), xs, C.c_size_t(xr), _ptr(w), ws, C.c_size_t(wr), _ptr(bias),
-                                       C.c_size_t(0 if bias is None else _numel(_shape(bias))), _ptr(y), ys, C.c_size_t(yr),
-                                       st, C.c_size_t(ns), pd, C.c_size_t(npd), dl, C.c_size_t(nd),
-                                       C.c_size_t(0 if group is None else group), ap, C.c_size_t(apl)))
+        check(lib().zant_b200_conv_f32(self._h, _addr(x), xs, xr, _addr(w), ws, wr, _addr(bias),
+                                       (0 if bias is None else _numel(_shape(bias))), _addr(y), ys, yr,
+                                       st, ns, pd, npd, dl, nd,
+                                       (0 if group is None else group), ap, apl))
         return y
 
     def Conv(self, x, w, bias=None, stride=(1,), pads=None, dilations=None, group=None, auto_pad=None):
@@ -328,7 +366,7 @@ class Context:
         yshape = tuple(sa[:-2]) + (sa[-2], sb[-1]) if len(sa) >= 2 and len(sb) >= 2 else (1, 1)
         y = self._out(out, yshape, F32)
         as_, ar = _sz(sa); bs, br = _sz(sb); ys, yr = _sz(yshape)
-        check(lib().zant_b200_mat_mul_f32(self._h, _ptr(a), as_, C.c_size_t(ar), _ptr(b), bs, C.c_size_t(br), _ptr(y), ys, C.c_size_t(yr)))
+        check(lib().zant_b200_mat_mul_f32(self._h, _addr(a), as_, ar, _addr(b), bs, br, _addr(y), ys, yr))
         return y
 
     def gemm(self, a, b, c=None, alpha=1.0, beta=1.0, transA=False, transB=False, out=None):
@@ -341,9 +379,9 @@ class Context:
         y = self._out(out, yshape, F32)
         as_, ar = _sz(sa); bs, br = _sz(sb); ys, yr = _sz(yshape)
         cs, cr = _sz(None if c is None else _shape(c))
-        check(lib().zant_b200_gemm_f32(self._h, _ptr(a), as_, C.c_size_t(ar), _ptr(b), bs, C.c_size_t(br), _ptr(c), cs, C.c_size_t(cr),
-                                       C.c_float(alpha), C.c_float(beta), C.c_int32(int(transA)), C.c_int32(int(transB)),
-                                       _ptr(y), ys, C.c_size_t(yr)))
+        check(lib().zant_b200_gemm_f32(self._h, _addr(a), as_, ar, _addr(b), bs, br, _addr(c), cs, cr,
+                                       alpha, beta, int(transA), int(transB),
+                                       _addr(y), ys, yr))
         return y
 
     def gemm_lean(self, a, b, c=None, alpha=1.0, beta=1.0, transA=False, transB=False, out=None):
@@ -354,9 +392,9 @@ class Context:
         y = self._out(out, yshape, F32)
         as_, ar = _sz(sa); bs, br = _sz(sb); ys, yr = _sz(yshape)
         cs, cr = _sz(None if c is None else _shape(c))
-        check(lib().zant_b200_gemm_lean_f32(self._h, _ptr(a), as_, C.c_size_t(ar), _ptr(b), bs, C.c_size_t(br), _ptr(c), cs, C.c_size_t(cr),
-                                            C.c_float(alpha), C.c_float(beta), C.c_int32(int(transA)), C.c_int32(int(transB)),
-                                            _ptr(y), ys, C.c_size_t(yr)))
+        check(lib().zant_b200_gemm_lean_f32(self._h, _addr(a), as_, ar, _addr(b), bs, br, _addr(c), cs, cr,
+                                            alpha, beta, int(transA), int(transB),
+                                            _addr(y), ys, yr))
         return y
 
     def onnx_maxpool_lean(self, x, y_shape, kernel, strides, dilations, pads, auto_pad="NOTSET", out=None):
@@ -365,12 +403,12 @@ class Context:
         y = self._out(out, y_shape, dt)
         xs, xr = _sz(_shape(x)); ys, yr = _sz(y_shape)
         k, nk = _sz(kernel); s, ns = _sz(strides); d, nd = _sz(dilations); p, npd = _sz(pads)
-        tail = (xs, C.c_size_t(xr), _ptr(y), ys, C.c_size_t(yr), k, C.c_size_t(nk), s, C.c_size_t(ns), d, C.c_size_t(nd),
-                p, C.c_size_t(npd), C.c_int32(AUTO_PAD[auto_pad]))
+        tail = (xs, xr, _addr(y), ys, yr, k, nk, s, ns, d, nd,
+                p, npd, AUTO_PAD[auto_pad])
         if dt == F32:
-            check(lib().zant_b200_maxpool_f32(self._h, _ptr(x), *tail))
+            check(lib().zant_b200_maxpool_f32(self._h, _addr(x), *tail))
         else:
-            check(lib().zant_b200_maxpool_q8(self._h, C.c_int32(dt), _ptr(x), *tail))
+            check(lib().zant_b200_maxpool_q8(self._h, dt, _addr(x), *tail))
         return y
 
     def onnx_maxpool(self, x, kernel, strides, dilations, pads, auto_pad="NOTSET", ceil_mode=False):
@@ -380,25 +418,25 @@ class Context:
     def ReLU(self, x, out=None):
         x = _host(x, np.float32)
         y = self._out(out, _shape(x), F32)
-        check(lib().zant_b200_relu_f32(self._h, _ptr(x), _ptr(y), C.c_size_t(_numel(_shape(x)))))
+        check(lib().zant_b200_relu_f32(self._h, _addr(x), _addr(y), _numel(_shape(x))))
         return y
 
     def leakyReLU(self, x, slope, out=None):
         x = _host(x, np.float32)
         y = self._out(out, _shape(x), F32)
-        check(lib().zant_b200_leaky_relu_f32(self._h, _ptr(x), C.c_float(slope), _ptr(y), C.c_size_t(_numel(_shape(x)))))
+        check(lib().zant_b200_leaky_relu_f32(self._h, _addr(x), slope, _addr(y), _numel(_shape(x))))
         return y
 
     def clip(self, x, lo, hi, out=None):
         x = _host(x, np.float32)
         y = self._out(out, _shape(x), F32)
-        check(lib().zant_b200_clip_f32(self._h, _ptr(x), C.c_float(lo), C.c_float(hi), _ptr(y), C.c_size_t(_numel(_shape(x)))))
+        check(lib().zant_b200_clip_f32(self._h, _addr(x), lo, hi, _addr(y), _numel(_shape(x))))
         return y
 
     def _unary(self, fn, x, out=None):
         x = _host(x, np.float32)
         y = self._out(out, _shape(x), F32)
-        check(fn(self._h, _ptr(x), _ptr(y), C.c_size_t(_numel(_shape(x)))))
+        check(fn(self._h, _addr(x), _addr(y), _numel(_shape(x))))
         return y
 
     def sigmoid(self, x, out=None):
@@ -422,7 +460,7 @@ class Context:
     def _binary(self, fn, a, b, out=None):
         a = _host(a, np.float32); b = _host(b, np.float32)
         y = self._out(out, _shape(a), F32)
-        check(fn(self._h, _ptr(a), C.c_size_t(_numel(_shape(a))), _ptr(b), C.c_size_t(_numel(_shape(b))), _ptr(y)))
+        check(fn(self._h, _addr(a), _numel(_shape(a)), _addr(b), _numel(_shape(b)), _addr(y)))
         return y
 
     def mul(self, a, b, out=None):
@@ -443,7 +481,7 @@ class Context:
                 yshape = sa
         y = self._out(out, yshape, F32)
         as_, ar = _sz(sa); bs, br = _sz(sb); ys, yr = _sz(yshape)
-        check(lib().zant_b200_sum_tensors_f32(self._h, _ptr(a), as_, C.c_size_t(ar), _ptr(b), bs, C.c_size_t(br), _ptr(y), ys, C.c_size_t(yr)))
+        check(lib().zant_b200_sum_tensors_f32(self._h, _addr(a), as_, ar, _addr(b), bs, br, _addr(y), ys, yr))
         return y
 
     def add_bias(self, t, bias):
@@ -598,15 +636,15 @@ class Context:
     def quantize_linear(self, x, scale, zp, out_dtype=U8, out=None):
         x = _host(x, np.float32)
         y = self._out(out, _shape(x), out_dtype)
-        check(lib().zant_b200_quantize_linear(self._h, _ptr(x), C.c_size_t(_numel(_shape(x))), C.c_float(scale), C.c_int32(zp),
-                                              C.c_int32(out_dtype), _ptr(y)))
+        check(lib().zant_b200_quantize_linear(self._h, _addr(x), _numel(_shape(x)), scale, zp,
+                                              out_dtype, _addr(y)))
         return y
 
     def dequantize_linear(self, q, scale, zp, out=None):
         q = _host(q)
         y = self._out(out, _shape(q), F32)
-        check(lib().zant_b200_dequantize_linear(self._h, C.c_int32(_dtype_code(q)), _ptr(q), C.c_size_t(_numel(_shape(q))),
-                                                C.c_float(scale), C.c_int32(zp), _ptr(y)))
+        check(lib().zant_b200_dequantize_linear(self._h, _dtype_code(q), _addr(q), _numel(_shape(q)),
+                                                scale, zp, _addr(y)))
         return y
 
     def qlinearconv(self, x, x_scale, x_zp, w, w_scale, w_zp, y_scale, y_zp, bias=None, y_dtype=I8, stride=(1, 1),
@@ -620,12 +658,12 @@ class Context:
         y = self._out(out, y_shape, y_dtype)
         xs, xr = _sz(_shape(x)); ws, wr = _sz(_shape(w)); ys, yr = _sz(y_shape)
         st, ns = _sz(stride); pd, npd = _sz(pads); dl, nd = _sz(dilations)
-        check(lib().zant_b200_qlinearconv(self._h, C.c_int32(_dtype_code(x)), _ptr(x), xs, C.c_size_t(xr), C.c_float(x_scale),
-                                          C.c_int32(x_zp), _ptr(w), ws, C.c_size_t(wr), _ptr(w_scale), _ptr(w_zp),
-                                          C.c_size_t(w_scale.size), C.c_float(y_scale), C.c_int32(y_zp), _ptr(bias),
-                                          C.c_size_t(0 if bias is None else bias.size), C.c_int32(y_dtype), _ptr(y), ys,
-                                          C.c_size_t(yr), st, C.c_size_t(ns), pd, C.c_size_t(npd), dl, C.c_size_t(nd),
-                                          C.c_size_t(group), C.c_int32(AUTO_PAD[auto_pad]), C.c_int32(QACT[activation])))
+        check(lib().zant_b200_qlinearconv(self._h, _dtype_code(x), _addr(x), xs, xr, x_scale,
+                                          x_zp, _addr(w), ws, wr, _addr(w_scale), _addr(w_zp),
+                                          w_scale.size, y_scale, y_zp, _addr(bias),
+                                          (0 if bias is None else bias.size), y_dtype, _addr(y), ys,
+                                          yr, st, ns, pd, npd, dl, nd,
+                                          group, AUTO_PAD[auto_pad], QACT[activation]))
         return y
 
     def qlinearconv_nhwc(self, x, x_scale, x_zp, w, w_scale, w_zp, y_scale, y_zp, bias=None, y_dtype=I8, stride=(1, 1),
@@ -642,12 +680,12 @@ class Context:
         y = self._out(out, y_shape, y_dtype)
         xs, xr = _sz(_shape(x)); ws, wr = _sz(_shape(w)); ys, yr = _sz(y_shape)
         st, ns = _sz(stride); pd, npd = _sz(pads); dl, nd = _sz(dilations)
-        check(lib().zant_b200_qlinearconv_nhwc(self._h, C.c_int32(_dtype_code(x)), _ptr(x), xs, C.c_size_t(xr), C.c_float(x_scale),
-                                               C.c_int32(x_zp), _ptr(w), ws, C.c_size_t(wr), _ptr(w_scale), _ptr(w_zp),
-                                               C.c_size_t(w_scale.size), C.c_float(y_scale), C.c_int32(y_zp), _ptr(bias),
-                                               C.c_size_t(0 if bias is None else bias.size), C.c_int32(y_dtype), _ptr(y), ys,
-                                               C.c_size_t(yr), st, C.c_size_t(ns), pd, C.c_size_t(npd), dl, C.c_size_t(nd),
-                                               C.c_size_t(group), C.c_int32(AUTO_PAD[auto_pad]), C.c_int32(QACT[activation])))
+        check(lib().zant_b200_qlinearconv_nhwc(self._h, _dtype_code(x), _addr(x), xs, xr, x_scale,
+                                               x_zp, _addr(w), ws, wr, _addr(w_scale), _addr(w_zp),
+                                               w_scale.size, y_scale, y_zp, _addr(bias),
+                                               (0 if bias is None else bias.size), y_dtype, _addr(y), ys,
+                                               yr, st, ns, pd, npd, dl, nd,
+                                               group, AUTO_PAD[auto_pad], QACT[activation]))
         return y
 
     def qlinearmatmul(self, a, a_scale, a_zp, b, b_scale, b_zp, y_scale, y_zp, bias=None, y_dtype=I8, activation=None, out=None):
@@ -658,20 +696,20 @@ class Context:
         yshape = (_shape(a)[0], _shape(b)[1])
         y = self._out(out, yshape, y_dtype)
         as_, ar = _sz(_shape(a)); bs, br = _sz(_shape(b)); ys, yr = _sz(yshape)
-        check(lib().zant_b200_qlinearmatmul(self._h, C.c_int32(_dtype_code(a)), _ptr(a), as_, C.c_size_t(ar), C.c_float(a_scale),
-                                            C.c_int32(a_zp), _ptr(b), bs, C.c_size_t(br), _ptr(b_scale), _ptr(b_zp),
-                                            C.c_size_t(b_scale.size), C.c_float(y_scale), C.c_int32(y_zp), _ptr(bias),
-                                            C.c_size_t(0 if bias is None else bias.size), C.c_int32(y_dtype), _ptr(y), ys,
-                                            C.c_size_t(yr), C.c_int32(QACT[activation])))
+        check(lib().zant_b200_qlinearmatmul(self._h, _dtype_code(a), _addr(a), as_, ar, a_scale,
+                                            a_zp, _addr(b), bs, br, _addr(b_scale), _addr(b_zp),
+                                            b_scale.size, y_scale, y_zp, _addr(bias),
+                                            (0 if bias is None else bias.size), y_dtype, _addr(y), ys,
+                                            yr, QACT[activation]))
         return y
 
     def qlinearadd(self, a, a_scale, a_zp, b, b_scale, b_zp, y_scale, y_zp, activation=None, out=None):
         a = _host(a); b = _host(b)
         dt = _dtype_code(a)
         y = self._out(out, _shape(a), dt)
-        check(lib().zant_b200_qlinearadd(self._h, C.c_int32(dt), _ptr(a), C.c_float(a_scale), C.c_int32(a_zp), _ptr(b),
-                                         C.c_float(b_scale), C.c_int32(b_zp), C.c_float(y_scale), C.c_int32(y_zp), _ptr(y),
-                                         C.c_size_t(_numel(_shape(a))), C.c_int32(QACT[activation])))
+        check(lib().zant_b200_qlinearadd(self._h, dt, _addr(a), a_scale, a_zp, _addr(b),
+                                         b_scale, b_zp, y_scale, y_zp, _addr(y),
+                                         _numel(_shape(a)), QACT[activation]))
         return y
 
     def qlinear_global_avgpool(self, x, x_scale, x_zp, y_scale, y_zp, out=None):
@@ -845,7 +883,7 @@ class Plan:
         """predict(): numpy in -> numpy out, or device tensors in place (asynchronous)."""
         x = _host(x, NP_DTYPE[self.in_dtype]) if not hasattr(x, "data_ptr") else x
         y = np.zeros(self.out_shape, NP_DTYPE[self.out_dtype]) if out is None else out
-        check(lib().zant_b200_plan_run(self._h, _ptr(x), _ptr(y)))
+        check(lib().zant_b200_plan_run(self._h, _addr(x), _addr(y)))
         return y
 
     def read_tensor(self, tid):
