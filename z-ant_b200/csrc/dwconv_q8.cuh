@@ -7,7 +7,9 @@
 // feeds them to dp4a against the three filter rows (the fourth dp4a weight is 0), accumulating into
 // the output rows the input row belongs to; an output row is requantised, packed and stored as one
 // 4-byte word once its last input row has been seen.  Several narrow planes share a warp (LW lanes per
-// plane).  Pixels outside the image hold the input zero point, which is folded into the bias
+// plane).  The walk is serial: where there are too few planes to fill the chip, the rows are cut into bands that different warps
+// take, each reading one input row above and below its own (dw_bands; 32 planes of 112 x 112 as 16 warps of 112 rows each
+// took 23 us).  Pixels outside the image hold the input zero point, which is folded into the bias
 // (bias - x_zp * sum(w)) exactly as in the tensor-core paths.
 // ALIGNED: rows are whole 4-byte words (W % 4 == 0 and OW % 4 == 0).  Otherwise the four bytes of a lane
 // are cut out of the two aligned words that hold them and the outputs are stored bytewise, which covers
@@ -41,6 +43,10 @@ struct QDwArgs {
     const int32_t* cap;       // lean epilogue, act_mode 1: per-channel accumulator bound of the activation (requant_relu_caps)
     int act_mode;             // lean epilogue: 0 no activation, 1 clamp of the accumulator to [0, cap], 2 clamp of the packed codes
 };
+// With a plane's output rows cut into `bands` bands of band_rows that different warps take.  A struct of its own: two more words in the
+// parameters of the whole-plane kernels (128 bytes without) made the 8-column one 10 % slower (186 -> 206 us).
+struct QDwBands : QDwArgs { int bands, band_rows; };
+template <bool BANDS> using QDwParam = std::conditional_t<BANDS, QDwBands, QDwArgs>;
 
 template <bool XU8>
 __device__ __forceinline__ int dw_dp4a(uint32_t x, uint32_t w, int acc) {
@@ -106,8 +112,9 @@ __device__ __forceinline__ uint32_t dw_load_unaligned(const QDwArgs& p, long lon
 // memory is touched by row-wise byte copies of consecutive rows only; the arithmetic is that of the aligned form.
 // SIN: the input planes are staged too; false with SMEM = true is the form for input rows of whole words (aligned loads
 // straight from global memory) whose OUTPUT rows are not (stride 2 from 28 x 28 to 14 x 14): only the output is staged.
-template <int STRIDE, bool XU8, bool LEAN, bool ALIGNED, bool SMEM = false, bool SIN = SMEM>
-__global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
+// BANDS: rows cut into bands (an instantiation of its own: the band's bounds in registers cost whole planes 10 to 25 %).
+template <int STRIDE, bool XU8, bool LEAN, bool ALIGNED, bool SMEM = false, bool SIN = SMEM, bool BANDS = false>
+__global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwParam<BANDS> p) {
     ptx::grid_start();
     extern __shared__ __align__(16) uint8_t dw_smem[];
     const int lane = threadIdx.x & 31;
@@ -127,7 +134,12 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
     uint8_t* const s_out = dw_smem + (SIN ? (size_t)P * p.H * Wp : 0);
     const int g_first = SMEM ? (int)blockIdx.x * 8 + wib : (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int g_step = SMEM ? (int)gridDim.x * 8 : warps;
-    for (int g = g_first; SMEM ? (g - wib < groups) : (g < groups); g += g_step) {
+    int bands = 1, band_rows = p.OH;
+    if constexpr (BANDS) { bands = p.bands; band_rows = p.band_rows; }
+    const int items = BANDS ? groups * bands : groups;
+    for (int it = g_first; SMEM ? (it - wib < items) : (it < items); it += g_step) {
+        const int g = BANDS ? it / bands : it;
+        const int row0 = BANDS ? (it - g * bands) * band_rows : 0, row1 = BANDS ? min(p.OH, row0 + band_rows) : p.OH;     // output rows
         const int plane = g * ppw + sub;
         const bool live = plane < p.planes && col_ok;
         if (SMEM && !SIN) __syncthreads();                       // the previous pass's copy-out has left the output image
@@ -186,7 +198,7 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
             for (int r = 0; r < 3; ++r)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[r][i] = b;
-            // input rows -1 .. H (the first and last are padding), three per trip; the loads of the next trip
+            // input rows row0 - 1 .. row1 (-1 and H are padding), three per trip; the loads of the next trip
             // are issued before this trip's arithmetic so that their latency is covered
             auto load_row = [&](int ih) -> uint32_t {
                 if (!(live && ih >= 0 && ih < p.H)) return p.pad_word;
@@ -194,20 +206,20 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
                 if (ALIGNED) return __ldg(xin + (size_t)ih * in_words + col);
                 return dw_load_unaligned(p, xplane + (long long)ih * p.W + col * 4, p.W - col * 4);
             };
-            uint32_t nx0 = load_row(-1), nx1 = load_row(0), nx2 = load_row(1);
-            for (int base = -1; base <= p.H; base += 3) {
+            uint32_t nx0 = load_row(row0 - 1), nx1 = load_row(row0), nx2 = load_row(row0 + 1);
+            for (int base = row0 - 1; base <= row1; base += 3) {
                 const uint32_t cur_rows[3] = {nx0, nx1, nx2};
                 nx0 = load_row(base + 3); nx1 = load_row(base + 4); nx2 = load_row(base + 5);
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
                     const int ih = base + r;
-                    if (ih > p.H) break;
+                    if (ih > row1) break;
                     const uint32_t M = cur_rows[r];
                     uint32_t L = __shfl_up_sync(0xffffffffu, M, 1), R = __shfl_down_sync(0xffffffffu, M, 1);
                     if (col == 0) L = p.pad_word;
                     if (col * 4 + 4 >= p.W) R = p.pad_word;
                     const uint32_t w0 = __byte_perm(L, M, 0x6543), w1 = M, w2 = __byte_perm(M, R, 0x4321), w3 = __byte_perm(M, R, 0x5432);
-                    // base is -1 mod 3, so r is (ih + 1) % 3 at compile time and names the slots of the three output rows
+                    // r is (ih - row0 + 1) % 3 at compile time and names the slots of the three output rows
                     int* a_prev = acc[(r + 2) % 3];   // output row ih - 1: this input row is its filter row 2
                     int* a_cur = acc[r % 3];          // output row ih: filter row 1
                     int* a_next = acc[(r + 1) % 3];   // output row ih + 1: filter row 0
@@ -219,7 +231,7 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
                     a_next[2] = dw_dp4a<XU8>(w2, k0, a_next[2]); a_next[3] = dw_dp4a<XU8>(w3, k0, a_next[3]);
                     // output row ih - 1 has now seen its three input rows
                     const int oh = ih - 1;
-                    if (oh >= 0 && oh < p.OH) {
+                    if (oh >= row0 && oh < row1) {
                         store_row(oh, dw_requant4<LEAN>(a_prev, m, cp, p));
                     }
                     a_prev[0] = a_prev[1] = a_prev[2] = a_prev[3] = b;   // the slot becomes output row ih + 2
@@ -236,8 +248,15 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
                 return dw_load_unaligned(p, xplane + (long long)ih * p.W + col * 8 + k * 4, p.W - col * 8 - k * 4);
             };
             // the four words of the next output row are loaded while this one is computed
-            uint32_t n00 = load_w(0, 0, c0), n01 = load_w(0, 1, c1), n10 = load_w(1, 0, c0), n11 = load_w(1, 1, c1);
-            for (int oh = 0; oh < p.OH; ++oh) {
+            if (BANDS && row0 > 0) {        // the row above the band is filter row 0 of its first output row
+                const uint32_t M0 = load_w(2 * row0 - 1, 0, c0), M1 = load_w(2 * row0 - 1, 1, c1);
+                uint32_t L = __shfl_up_sync(0xffffffffu, M1, 1);
+                if (col == 0) L = p.pad_word;
+                nxt[0] = dw_dp4a<XU8>(__byte_perm(L, M0, 0x6543), k0, b); nxt[1] = dw_dp4a<XU8>(__byte_perm(M0, M0, 0x0321), k0, b);
+                nxt[2] = dw_dp4a<XU8>(__byte_perm(M0, M1, 0x6543), k0, b); nxt[3] = dw_dp4a<XU8>(__byte_perm(M1, M1, 0x0321), k0, b);
+            }
+            uint32_t n00 = load_w(2 * row0, 0, c0), n01 = load_w(2 * row0, 1, c1), n10 = load_w(2 * row0 + 1, 0, c0), n11 = load_w(2 * row0 + 1, 1, c1);
+            for (int oh = row0; oh < row1; ++oh) {
                 int cur[4] = {nxt[0], nxt[1], nxt[2], nxt[3]};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) nxt[i] = b;
@@ -297,8 +316,8 @@ __global__ void __launch_bounds__(256) qdwconv3x3_kernel(const QDwArgs p) {
 // Stride 1 on planes whose rows are whole 8-byte groups (W % 8 == 0): a lane owns 8 columns (one 8-byte
 // load per row), which halves the per-output share of loads, shuffles and address arithmetic; the padding
 // rows and the first output row are peeled off so that the row loop carries no range checks.
-template <bool XU8, bool LEAN>
-__global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwArgs p) {
+template <bool XU8, bool LEAN, bool BANDS>
+__global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwParam<BANDS> p) {
     ptx::grid_start();
     const int lane = threadIdx.x & 31;
     const int LW = 1 << p.log2LW;                            // lanes per plane, each 8 columns
@@ -310,15 +329,20 @@ __global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwArgs p) {
     const bool col_ok = col < wu2;
     const bool first_col = col == 0, last_col = col == wu2 - 1;
     const uint2 padrow = make_uint2(p.pad_word, p.pad_word);
-    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
+    int bands = 1, band_rows = p.OH;
+    if constexpr (BANDS) { bands = p.bands; band_rows = p.band_rows; }
+    const int items = BANDS ? groups * bands : groups;
+    for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += warps) {
+        const int g = BANDS ? it / bands : it;
+        const int row0 = BANDS ? (it - g * bands) * band_rows : 0, row1 = BANDS ? min(p.H, row0 + band_rows) : p.H;
         const int plane = g * ppw + sub;
         const bool live = plane < p.planes && col_ok;
         const int c = live ? plane % p.C : 0;
         const uint32_t k0 = __ldg(p.wrow + c * 3), k1 = __ldg(p.wrow + c * 3 + 1), k2 = __ldg(p.wrow + c * 3 + 2);
         const float m = __ldg(p.mult + c);
         const int b = __ldg(p.bias + c);
-        const uint2* xr = reinterpret_cast<const uint2*>(p.x + (size_t)(live ? plane : 0) * p.H * p.W) + (live ? col : 0);
-        uint2* yr = reinterpret_cast<uint2*>(p.y + (size_t)(live ? plane : 0) * p.H * p.W) + (live ? col : 0);
+        const uint2* xr = reinterpret_cast<const uint2*>(p.x + ((size_t)(live ? plane : 0) * p.H + row0) * p.W) + (live ? col : 0);
+        uint2* yr = reinterpret_cast<uint2*>(p.y + ((size_t)(live ? plane : 0) * p.H + row0) * p.W) + (live ? col : 0);
         int A[8], B[8], C[8];                                // three output rows in flight
 #pragma unroll
         for (int i = 0; i < 8; ++i) A[i] = B[i] = C[i] = b;
@@ -344,34 +368,35 @@ __global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwArgs p) {
             for (int i = 0; i < 8; ++i) row[i] = b;
         };
         auto load = [&]() -> uint2 { const uint2 v = live ? __ldg(xr) : padrow; xr += wu2; return v; };
-        // rows -1 (padding) and 0: nothing to emit yet.  A = output row 0, B = row 1, C = row 2.
-        step(padrow, nullptr, nullptr, A);
+        // the row above the band (padding above row 0) and its first: nothing to emit yet.  A = output row row0, B, C the next two.
+        step(BANDS && live && row0 > 0 ? __ldg(xr - wu2) : padrow, nullptr, nullptr, A);
         step(load(), nullptr, A, B);
-        int ih = 1;
+        int ih = row0 + 1;
         // three input rows per trip (the slots return to their roles); the next trip's rows are requested before this
         // trip's arithmetic, so that their latency is covered by it
         uint2 n0 = padrow, n1 = padrow, n2 = padrow;
-        if (ih + 2 < p.H) { n0 = load(); n1 = load(); n2 = load(); }
-        for (; ih + 2 < p.H; ih += 3) {
+        if (ih + 2 < row1) { n0 = load(); n1 = load(); n2 = load(); }
+        for (; ih + 2 < row1; ih += 3) {
             const uint2 r0 = n0, r1 = n1, r2 = n2;
-            if (ih + 5 < p.H) { n0 = load(); n1 = load(); n2 = load(); }
+            if (ih + 5 < row1) { n0 = load(); n1 = load(); n2 = load(); }
             step(r0, A, B, C); emit(A);                      // A becomes output row ih + 2
             step(r1, B, C, A); emit(B);
             step(r2, C, A, B); emit(C);
         }
-        // up to two more input rows, then the padding row below the image
-        int left = p.H - ih;                                 // 0, 1 or 2 rows (H >= 1)
+        // up to two more input rows, then the row below the band (padding below the image)
+        int left = row1 - ih;                                // 0, 1 or 2 rows
+        const bool below = BANDS && live && row1 < p.H;
         if (left == 2) {
-            const uint2 r0 = load(), r1 = load();
+            const uint2 r0 = load(), r1 = load(), r2 = below ? __ldg(xr) : padrow;
             step(r0, A, B, C); emit(A);
             step(r1, B, C, nullptr); emit(B);
-            step(padrow, C, nullptr, nullptr); emit(C);
+            step(r2, C, nullptr, nullptr); emit(C);
         } else if (left == 1) {
-            const uint2 r0 = load();
+            const uint2 r0 = load(), r1 = below ? __ldg(xr) : padrow;
             step(r0, A, B, nullptr); emit(A);
-            step(padrow, B, nullptr, nullptr); emit(B);
-        } else if (p.H >= 1) {
-            step(padrow, A, nullptr, nullptr); emit(A);
+            step(r1, B, nullptr, nullptr); emit(B);
+        } else {
+            step(below ? __ldg(xr) : padrow, A, nullptr, nullptr); emit(A);
         }
     }
 }
@@ -677,10 +702,15 @@ inline void qdwconv_prepare(const ConvGeom& g, const int8_t* w, const int32_t* b
 }
 
 template <int STRIDE, bool ALIGNED>
-inline int32_t qdwconv_launch_s(zant_ctx* ctx, const QDwArgs& a, int grid, bool x_u8, bool lean) {
-    if (x_u8) { if (lean) launch(ctx, qdwconv3x3_kernel<STRIDE, true, true, ALIGNED>, grid, 256, 0, a); else launch(ctx, qdwconv3x3_kernel<STRIDE, true, false, ALIGNED>, grid, 256, 0, a); }
-    else { if (lean) launch(ctx, qdwconv3x3_kernel<STRIDE, false, true, ALIGNED>, grid, 256, 0, a); else launch(ctx, qdwconv3x3_kernel<STRIDE, false, false, ALIGNED>, grid, 256, 0, a); }
-    return check_launch(ctx, "qdwconv3x3_kernel");
+inline int32_t qdwconv_launch_s(zant_ctx* ctx, const QDwBands& a, int grid, bool x_u8, bool lean) {
+    auto go = [&](auto whole, auto banded) -> int32_t {
+        if (a.bands > 1) launch(ctx, banded, grid, 256, 0, a); else launch(ctx, whole, grid, 256, 0, static_cast<const QDwArgs&>(a));
+        return check_launch(ctx, "qdwconv3x3_kernel");
+    };
+    if (x_u8) return lean ? go(qdwconv3x3_kernel<STRIDE, true, true, ALIGNED>, qdwconv3x3_kernel<STRIDE, true, true, ALIGNED, false, false, true>)
+                          : go(qdwconv3x3_kernel<STRIDE, true, false, ALIGNED>, qdwconv3x3_kernel<STRIDE, true, false, ALIGNED, false, false, true>);
+    return lean ? go(qdwconv3x3_kernel<STRIDE, false, true, ALIGNED>, qdwconv3x3_kernel<STRIDE, false, true, ALIGNED, false, false, true>)
+                : go(qdwconv3x3_kernel<STRIDE, false, false, ALIGNED>, qdwconv3x3_kernel<STRIDE, false, false, ALIGNED, false, false, true>);
 }
 
 template <int STRIDE, bool XU8, bool LEAN>
@@ -704,12 +734,24 @@ inline int32_t qdwconv_launch_smem(zant_ctx* ctx, const QDwArgs& a, int grid, si
     return lean ? qdwconv_launch_smem_t<2, false, true>(ctx, a, grid, smem, stage_in) : qdwconv_launch_smem_t<2, false, false>(ctx, a, grid, smem, stage_in);
 }
 
+// Bands of a plane's OH output rows when its planes fill only `groups` warps: as many as bring the launch to four CTAs of eight
+// warps per SM (what the registers allow), of at least four rows - two where even those leave the chip half empty - because a band reads
+// two rows that are not its own.  Measured, whole planes -> bands: 32 x 112 x 112 at batch 1 5.2 -> 2.6 us, at batch 8 23 -> 5;
+// 144 x 40 x 40 at batch 37 18.7 -> 9.9; half and twice as many warps are 5 to 40 % slower there.
+inline void dw_bands(const zant_ctx* ctx, long long groups, QDwBands& a) {
+    const long long want = ((long long)ctx->sm_count * 32 + groups - 1) / std::max<long long>(1, groups);
+    const int rows = groups * (a.OH / 4) < (long long)ctx->sm_count * 16 ? 2 : 4;
+    const int n = (int)std::max<long long>(1, std::min<long long>(want, a.OH / rows));
+    a.band_rows = (a.OH + n - 1) / n;
+    a.bands = (a.OH + a.band_rows - 1) / a.band_rows;
+}
+
 // x and y must be 4-byte aligned (the caller checks with qdwconv_ptr_ok).
 inline bool qdwconv_ptr_ok(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
 
 inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool x_u8, int x_zp, const uint32_t* wrow_dev, const float* mult_dev,
                            const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq, bool mult_finite, const int32_t* cap_dev = nullptr) {
-    QDwArgs a{};
+    QDwBands a{};
     a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.wrow = wrow_dev; a.mult = mult_dev; a.bias = bias_dev;
     a.planes = g.N * g.C; a.C = g.C; a.H = g.H; a.W = g.W; a.OH = g.OH; a.OW = g.OW;
     a.x_bytes = (long long)g.N * g.C * g.H * g.W;
@@ -723,8 +765,8 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
     a.act_mode = rq.act == ZANT_QACT_NONE ? 0 : (cap_dev ? 1 : 2);
     const int ppw = 32 >> a.log2LW;
     const long long groups = ((long long)a.planes + ppw - 1) / ppw;
-    const int grid = (int)std::min<long long>((groups + 7) / 8, (long long)ctx->sm_count * 16);
-    if (grid == 0) return ZANT_OK;
+    a.bands = 1; a.band_rows = g.OH;
+    if (groups == 0) return ZANT_OK;
     if (g.sh == 1 && g.W % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 7u) == 0 && (reinterpret_cast<uintptr_t>(y) & 7u) == 0) {
         // 8 columns per lane
         const int cols8 = g.W / 8;
@@ -732,10 +774,14 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
         if (a.log2LW <= 5) {
             const int ppw8 = 32 >> a.log2LW;
             const long long groups8 = ((long long)a.planes + ppw8 - 1) / ppw8;
-            const int grid8 = (int)std::min<long long>((groups8 + 7) / 8, (long long)ctx->sm_count * 16);
-            if (x_u8) { if (lean) launch(ctx, qdwconv3x3_s1w8_kernel<true, true>, grid8, 256, 0, a); else launch(ctx, qdwconv3x3_s1w8_kernel<true, false>, grid8, 256, 0, a); }
-            else { if (lean) launch(ctx, qdwconv3x3_s1w8_kernel<false, true>, grid8, 256, 0, a); else launch(ctx, qdwconv3x3_s1w8_kernel<false, false>, grid8, 256, 0, a); }
-            return check_launch(ctx, "qdwconv3x3_s1w8_kernel");
+            dw_bands(ctx, groups8, a);
+            const int grid8 = (int)std::min<long long>((groups8 * a.bands + 7) / 8, (long long)ctx->sm_count * 16);
+            auto go = [&](auto whole, auto banded) -> int32_t {
+                if (a.bands > 1) launch(ctx, banded, grid8, 256, 0, a); else launch(ctx, whole, grid8, 256, 0, static_cast<const QDwArgs&>(a));
+                return check_launch(ctx, "qdwconv3x3_s1w8_kernel");
+            };
+            if (x_u8) return lean ? go(qdwconv3x3_s1w8_kernel<true, true, false>, qdwconv3x3_s1w8_kernel<true, true, true>) : go(qdwconv3x3_s1w8_kernel<true, false, false>, qdwconv3x3_s1w8_kernel<true, false, true>);
+            return lean ? go(qdwconv3x3_s1w8_kernel<false, true, false>, qdwconv3x3_s1w8_kernel<false, true, true>) : go(qdwconv3x3_s1w8_kernel<false, false, false>, qdwconv3x3_s1w8_kernel<false, false, true>);
         }
     }
     const bool aligned = g.W % 4 == 0 && g.OW % 4 == 0;
@@ -805,6 +851,8 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
             return qdwconv_launch_smem(ctx, a, sgrid, smem, g.sh, x_u8, lean, stage_in);
         }
     }
+    dw_bands(ctx, groups, a);
+    const int grid = (int)std::min<long long>((groups * a.bands + 7) / 8, (long long)ctx->sm_count * 16);
     if (g.sh == 1) return aligned ? qdwconv_launch_s<1, true>(ctx, a, grid, x_u8, lean) : qdwconv_launch_s<1, false>(ctx, a, grid, x_u8, lean);
     return aligned ? qdwconv_launch_s<2, true>(ctx, a, grid, x_u8, lean) : qdwconv_launch_s<2, false>(ctx, a, grid, x_u8, lean);
 }
