@@ -283,38 +283,77 @@ __global__ void qadd_k(const void* __restrict__ a, float a_s, int a_zp, const vo
     }
 }
 
-// The same, sixteen values per thread (16-byte loads and stores); the division by y_s goes through quantize_fast, which
-// proves the rounding from a multiply and a residual and divides only where it cannot.  Requires 16-byte aligned buffers
-// and a y_zp inside the type's range; the tail (n % 16 values) is left to qadd_k.
+// A QLinearAdd in words of four codes.  The reference form, round((fl(a) + fl(b)) / y_s) with every step rounded, costs a division per
+// value; u = a' * (a_s / y_s) + b' * (b_s / y_s) in one multiply and one FMA differs from that quotient by less than
+//     eps = 8 * 2^-24 * 255 * (a_s + b_s) / y_s
+// (three roundings of terms of at most 255 a_s and 255 b_s there, one of each ratio, one product and one sum here), so both round to
+// the same integer unless u lies within eps of a tie.  A word with such a value takes the reference form (qadd_word_exact, out of
+// line: 32 inlined divisions in a convolution's epilogue cost 4 us of instruction fetches a launch).
+struct QAddTail {
+    const uint8_t* res;            // fused into a convolution: the other operand (a), laid out like the output; b are the convolution's codes
+    float ra, rb;                  // a_s / y_s, b_s / y_s
+    float ca, cb;                  // 2^23 + zero points (int8: + 128), what a code placed in a float's low byte is too large by
+    float lim;                     // 0.5 - eps; negative: always the reference form
+    int y_off;                     // y_zp minus the bits of the rounding constant
+    int lo, hi;                    // activation bounds on the codes (the type's range without one)
+    float a_s, b_s, y_s; int a_zp, b_zp, y_zp;
+};
 template <bool U8>
-__global__ void __launch_bounds__(256) qadd_vec_k(const uint4* __restrict__ a, float a_s, int a_zp, const uint4* __restrict__ b, float b_s, int b_zp,
-                                                  float y_s, int y_zp, int act, uint4* __restrict__ y, size_t n16) {
-    ptx::grid_start();
+inline QAddTail qadd_tail(float a_s, int a_zp, float b_s, int b_zp, float y_s, int y_zp, int act) {
+    QAddTail t{};
+    t.ra = a_s / y_s; t.rb = b_s / y_s;
+    t.ca = 8388608.0f + (float)(a_zp + (U8 ? 0 : 128)); t.cb = 8388608.0f + (float)(b_zp + (U8 ? 0 : 128));
+    const double eps = 8.0 / 16777216.0 * 255.0 * ((double)std::fabs(t.ra) + (double)std::fabs(t.rb));
+    const bool usable = a_s > 1e-30f && b_s > 1e-30f && y_s > 1e-30f && a_s < 1e30f && b_s < 1e30f && y_s < 1e30f && eps < 0.01 && t.ra > 1e-30f && t.rb > 1e-30f;
+    t.lim = usable ? (float)(0.4999999 - eps) : -1.0f;
+    t.y_off = y_zp - 0x4b400000;
     const int t_lo = U8 ? 0 : -128, t_hi = U8 ? 255 : 127;
-    const QuantFast qf = quant_fast(y_s, (float)(t_lo - y_zp), (float)(t_hi - y_zp));
-    const int lo = sat_q<U8>(y_zp);
-    const int six = sat_q<U8>(rne_clamped(__fdiv_rn(6.0f, y_s)) + y_zp);
+    auto sat = [&](int v) { return v < t_lo ? t_lo : (v > t_hi ? t_hi : v); };
+    t.lo = act != ZANT_QACT_NONE ? sat(y_zp) : t_lo;
+    float six = 6.0f / y_s;
+    six = six != six || six < -512.0f ? -512.0f : (six > 511.0f ? 511.0f : six);
+    t.hi = act == ZANT_QACT_RELU6 ? sat((int)std::nearbyintf(six) + y_zp) : t_hi;
+    t.a_s = a_s; t.b_s = b_s; t.y_s = y_s; t.a_zp = a_zp; t.b_zp = b_zp; t.y_zp = y_zp;
+    return t;
+}
+template <bool U8>
+__device__ __noinline__ uint32_t qadd_word_exact(uint32_t a, uint32_t b, float a_s, float b_s, float y_s, int a_zp, int b_zp, int y_zp, int lo, int hi) {
+    uint32_t pk = 0;
+#pragma unroll 1
+    for (int j = 0; j < 32; j += 8) {
+        const int qa = U8 ? (int)((a >> j) & 255u) : (int)(int8_t)(a >> j), qb = U8 ? (int)((b >> j) & 255u) : (int)(int8_t)(b >> j);
+        const float fa = __fmul_rn(__int2float_rn(qa - a_zp), a_s), fb = __fmul_rn(__int2float_rn(qb - b_zp), b_s);
+        const int t = sat_q<U8>(rne_clamped(__fdiv_rn(__fadd_rn(fa, fb), y_s)) + y_zp);
+        pk |= (uint32_t)(min(max(t, lo), hi) & 255) << j;
+    }
+    return pk;
+}
+template <bool U8>
+__device__ __forceinline__ uint32_t qadd_word(uint32_t a, uint32_t b, const QAddTail& t) {
+    const uint32_t xa = U8 ? a : a ^ 0x80808080u, xb = U8 ? b : b ^ 0x80808080u;
+    int k[4];
+    float far = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float fa = __fadd_rn(__uint_as_float(__byte_perm(xa, 0x4b000000u, 0x7440u + j)), -t.ca);
+        const float fb = __fadd_rn(__uint_as_float(__byte_perm(xb, 0x4b000000u, 0x7440u + j)), -t.cb);
+        const float u = __fmaf_rn(fa, t.ra, __fmul_rn(fb, t.rb));
+        const float m = __fadd_rn(u, 12582912.0f);                 // rounds to an integer in the low bits (|u| < 2^21)
+        far = fmaxf(far, fabsf(__fadd_rn(u, -__fadd_rn(m, -12582912.0f))));
+        k[j] = min(max(__float_as_int(m) + t.y_off, t.lo), t.hi);
+    }
+    if (far > t.lim) return qadd_word_exact<U8>(a, b, t.a_s, t.b_s, t.y_s, t.a_zp, t.b_zp, t.y_zp, t.lo, t.hi);
+    return U8 ? pack_sat_u8x4(k[0], k[1], k[2], k[3]) : pack_sat_s8x4(k[0], k[1], k[2], k[3]);
+}
+
+// Sixteen values per thread (16-byte loads and stores).  Requires 16-byte aligned buffers and a y_zp inside the type's range; the tail
+// (n % 16 values) is left to qadd_k.
+template <bool U8>
+__global__ void __launch_bounds__(256) qadd_vec_k(const uint4* __restrict__ a, const uint4* __restrict__ b, uint4* __restrict__ y, size_t n16, const __grid_constant__ QAddTail t) {
+    ptx::grid_start();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += (size_t)gridDim.x * blockDim.x) {
         const uint4 va = __ldg(a + i), vb = __ldg(b + i);
-        const uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
-        uint32_t out[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            uint32_t pk = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int qa = U8 ? (int)((wa[w] >> (8 * j)) & 255u) : (int)(int8_t)(wa[w] >> (8 * j));
-                const int qb = U8 ? (int)((wb[w] >> (8 * j)) & 255u) : (int)(int8_t)(wb[w] >> (8 * j));
-                const float fa = __fmul_rn(__int2float_rn(qa - a_zp), a_s);
-                const float fb = __fmul_rn(__int2float_rn(qb - b_zp), b_s);
-                int t = quantize_fast(__fadd_rn(fa, fb), qf) + y_zp;
-                if (act != ZANT_QACT_NONE) t = max(t, lo);
-                if (act == ZANT_QACT_RELU6) t = min(t, six);
-                pk |= (uint32_t)(t & 255) << (8 * j);
-            }
-            out[w] = pk;
-        }
-        y[i] = make_uint4(out[0], out[1], out[2], out[3]);
+        y[i] = make_uint4(qadd_word<U8>(va.x, vb.x, t), qadd_word<U8>(va.y, vb.y, t), qadd_word<U8>(va.z, vb.z, t), qadd_word<U8>(va.w, vb.w, t));
     }
 }
 

@@ -319,8 +319,8 @@ inline int32_t run_qadd(zant_ctx* ctx, int32_t dtype, const void* a, float a_s, 
     if (zp_ok && n >= 16 && aligned16(a) && aligned16(b) && aligned16(y)) {
         const size_t n16 = n / 16;
         const int grid = grid_for(n16, 256, ctx->sm_count);
-        if (u8) launch(ctx, qadd_vec_k<true>, grid, 256, 0, (const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
-        else launch(ctx, qadd_vec_k<false>, grid, 256, 0, (const uint4*)a, a_s, a_zp, (const uint4*)b, b_s, b_zp, y_s, y_zp, act, (uint4*)y, n16);
+        if (u8) launch(ctx, qadd_vec_k<true>, grid, 256, 0, (const uint4*)a, (const uint4*)b, (uint4*)y, n16, qadd_tail<true>(a_s, a_zp, b_s, b_zp, y_s, y_zp, act));
+        else launch(ctx, qadd_vec_k<false>, grid, 256, 0, (const uint4*)a, (const uint4*)b, (uint4*)y, n16, qadd_tail<false>(a_s, a_zp, b_s, b_zp, y_s, y_zp, act));
         ZB_TRY(check_launch(ctx, "qadd_vec_k"));
         done = n16 * 16;
         if (done == n) return ZANT_OK;

@@ -564,6 +564,9 @@ struct QConvFusion {
     int y_act = -1;          // tensor written when the pool is not fused (-1: the node's output)
     int y_pool = -1;         // pooled tensor; >= 0 asks for the fused pool
     bool pool_done = false;  // out: the step writes y_pool
+    int add_node = -1;       // QLinearAdd behind the convolution (and its activation); its other operand
+    int add_res = -1;
+    bool add_done = false;   // out: the step writes the sum
 };
 
 static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
@@ -613,6 +616,15 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
     const std::string tail = std::string(fz.activation >= 0 ? "+Relu" : "") + (lut_aux >= 0 ? "+ActivationLut" : "");
     auto push = [&](const std::string& name, std::function<int32_t()> fn) { pl->steps.push_back(std::move(fn)); pl->step_names.push_back(name); };
     fz.pool_done = false;
+    // a QLinearAdd behind the convolution, for the kernels that take it: the sum's tensor, and the operation with its operand's address
+    const int add_res = fz.add_res, y_sum = fz.add_node >= 0 ? pl->nodes[fz.add_node].out[0] : -1;
+    QAddTail add0{};
+    if (fz.add_node >= 0) {
+        const PlanNode& an = pl->nodes[fz.add_node];
+        const bool first = an.in[0] == add_res;
+        add0 = qadd_tail<false>(first ? an.a.x_scale : an.a.b_scale, first ? an.a.x_zp : an.a.b_zp, first ? an.a.b_scale : an.a.x_scale, first ? an.a.b_zp : an.a.x_zp, an.a.y_scale, an.a.y_zp, an.a.activation);
+    }
+    auto add_of = [pl, add0, add_res]() { QAddTail t = add0; t.res = (const uint8_t*)pl->ptr(add_res); return t; };
 
     if (a.channels_last) {
         TcConvPlan ncp;
@@ -641,6 +653,18 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         std::vector<int32_t> caps;
         const bool capped = finite && yd == ZANT_I8 && rq0.y_zp == 0 && requant_relu_caps(mult.data(), mult.size(), rq0.act, lean_six(rq0.y_scale), caps);
         const int ac = capped ? pl->add_aux(caps.data(), caps.size() * 4) : -1;
+        // from 8 MB of output on (below, a CTA has a tile or two, whose epilogue the addition makes longer by more than the launch it
+        // saves: 37 images of 160 x 160 took 512 us with it, 484 without; 1024 of 224 x 224 go from 114 + 80 to 165 us in the largest)
+        if (!stem && fz.add_node >= 0 && (long long)g.N * g.M * g.OH * g.OW >= (8LL << 20) && xd == ZANT_I8 && yd == ZANT_I8 && rq0.y_zp == 0 && finite) {
+            fz.add_done = true;
+            push("QLinearConv(tc-pointwise)" + tail + "+QLinearAdd", [=]() {
+                if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y_sum))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");
+                const QAddTail add = add_of();
+                return pw_conv_run(ctx, pwp, pl->ptr(x), false, (const int8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y_sum), false, rq_of(), true,
+                                   ac >= 0 ? (const int32_t*)pl->aux(ac) : nullptr, &add);
+            });
+            return ZANT_OK;
+        }
         push(std::string(stem ? "QLinearConv(tc-stem)" : "QLinearConv(tc-pointwise)") + tail, [=]() {
             if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");
             return pw_conv_run(ctx, pwp, pl->ptr(x), xd == ZANT_U8, (const int8_t*)pl->aux(aw), (const float*)pl->aux(am),
@@ -720,6 +744,15 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         small_gemm_prepare(g, (const int8_t*)T(w).host.data(), (size_t)g.Cg * taps, taps, 1, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, ctx->sm_count, *prep);
         const int aw = pl->add_aux(prep->wfrag.data(), prep->wfrag.size() * 4), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4), ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
         prep->wfrag.clear(); prep->wfrag.shrink_to_fit();
+        if (fz.add_node >= 0 && yd == ZANT_I8) {
+            fz.add_done = true;
+            push("QLinearConv" + tail + "+QLinearAdd", [=]() {
+                const QAddTail add = add_of();
+                return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
+                                      pl->ptr(y_sum), false, rq_of(), &add);
+            });
+            return ZANT_OK;
+        }
         push("QLinearConv" + tail, [=]() {
             return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
                                   pl->ptr(y), yd == ZANT_U8, rq_of());
@@ -1385,13 +1418,27 @@ static int32_t try_fuse_qconv_group(zant_plan* pl, size_t i0, size_t& consumed) 
             }
         }
     }
-    if (interior.empty() && !want_pool) return ZANT_OK;        // nothing behind the node: the plain path builds it
+    // residual addition behind that: the other operand is a tensor that an earlier node left in the arena
+    if (!want_pool && !conv.a.channels_last && j < pl->nodes.size() && only_feeds_next(c, cur)) {
+        const PlanNode& add = pl->nodes[j];
+        if (add.op == ZANT_OP_QLINEAR_ADD && add.in.size() == 2 && add.out.size() == 1 && (add.in[0] == cur) != (add.in[1] == cur)) {
+            const int r = add.in[0] == cur ? add.in[1] : add.in[0], y = add.out[0];
+            bool there = false;
+            for (size_t k = 0; k < i0; ++k) for (int id : pl->nodes[k].out) there = there || id == r;
+            if (r >= 0 && there && !T(r).elided && !T(r).nh && T(r).alias < 0 && r != pl->input && r != pl->output && y != pl->output && T(cur).dtype == ZANT_I8 &&
+                T(r).dtype == ZANT_I8 && T(y).dtype == ZANT_I8 && T(r).bytes == T(cur).bytes && T(y).bytes == T(cur).bytes && check_zero_point(ZANT_I8, add.a.y_zp, "QLinearAdd y") == ZANT_OK) {
+                fz.add_node = (int)j;
+                fz.add_res = r;
+            }
+        }
+    }
+    if (interior.empty() && !want_pool && fz.add_node < 0) return ZANT_OK;        // nothing behind the node: the plain path builds it
     fz.y_act = cur;
     const size_t first_step = pl->steps.size();
     ZB_TRY(build_qconv(pl, conv, fz));
-    if (fz.pool_done) { interior.push_back(cur); ++j; }
+    if (fz.pool_done || fz.add_done) { interior.push_back(cur); ++j; }
     if (interior.empty()) {
-        // the pool was asked for but the chosen kernel cannot take it: nothing was fused after all
+        // the pool or the addition was asked for but the chosen kernel cannot take it: nothing was fused after all
         record_step_cost(pl, first_step, i0, 1);
         consumed = 1;
         return ZANT_OK;

@@ -41,6 +41,7 @@ struct SmallGemmArgs {
     int vec;               // PATH 0: rows are whole 16-byte units; PATH 1, 2: output planes are whole words
     uint32_t pad;          // input zero point as a byte
     Requant rq;
+    QAddTail add;          // res != nullptr: a QLinearAdd behind it (int8)
 };
 
 constexpr int kSmallWarps = 8;
@@ -203,7 +204,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const S
                 if (m >= g.M) break;
                 int s = __ldg(a.bias + m);
                 for (int w = 0; w < warps; ++w) s += red[w * (MT * 16 * LD) + (r0 + j) * LD + col];
-                store_q<YU8>(a.y, (size_t)p * g.M + m, requant_one<YU8>(s, __ldg(a.mult + m), a.rq));
+                int q = requant_one<YU8>(s, __ldg(a.mult + m), a.rq);
+                if (!YU8 && a.add.res) q = (int)(int8_t)qadd_word<false>((uint32_t)__ldg(a.add.res + (size_t)p * g.M + m), (uint32_t)(q & 255), a.add);
+                store_q<YU8>(a.y, (size_t)p * g.M + m, q);
             }
         } else {
             // four positions of one filter
@@ -219,14 +222,19 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const S
             int n = p / a.OHW, pos = p - n * a.OHW;
             if (a.vec) {
                 uint32_t pk = 0;
+                const size_t at = ((size_t)n * g.M + m) * a.OHW + pos;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) pk |= (uint32_t)(requant_one<YU8>(s[j], mu, a.rq) & 255) << (8 * j);
-                *reinterpret_cast<uint32_t*>((uint8_t*)a.y + ((size_t)n * g.M + m) * a.OHW + pos) = pk;
+                if (!YU8 && a.add.res) pk = qadd_word<false>(__ldg(reinterpret_cast<const uint32_t*>(a.add.res + at)), pk, a.add);
+                *reinterpret_cast<uint32_t*>((uint8_t*)a.y + at) = pk;
             } else {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (p + j >= a.P) break;
-                    store_q<YU8>(a.y, ((size_t)n * g.M + m) * a.OHW + pos, requant_one<YU8>(s[j], mu, a.rq));
+                    const size_t at = ((size_t)n * g.M + m) * a.OHW + pos;
+                    int q = requant_one<YU8>(s[j], mu, a.rq);
+                    if (!YU8 && a.add.res) q = (int)(int8_t)qadd_word<false>((uint32_t)__ldg(a.add.res + at), (uint32_t)(q & 255), a.add);
+                    store_q<YU8>(a.y, at, q);
                     if (++pos == a.OHW) { pos = 0; ++n; }
                 }
             }
@@ -283,8 +291,9 @@ inline void small_gemm_prepare(const ConvGeom& g, const int8_t* w, size_t sm, si
 }
 
 inline int32_t run_small_gemm(zant_ctx* ctx, const ConvGeom& g, const SmallGemmPrep& p, const void* x, bool x_u8, int x_zp, const uint32_t* w_dev, const float* mult_dev,
-                              const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq) {
+                              const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq, const QAddTail* add = nullptr) {
     SmallGemmArgs a{};
+    if (add) a.add = *add;
     a.x = (const uint8_t*)x; a.w = (const uint4*)w_dev; a.y = y; a.mult = mult_dev; a.bias = bias_dev; a.g = g;
     a.OHW = g.OH * g.OW; a.P = g.N * a.OHW; a.c_steps = p.c_steps; a.k_steps = p.k_steps; a.pad = (uint32_t)(x_zp & 255); a.rq = rq;
     // a word path needs word-aligned rows on the side it vectorises; x that is not falls back to byte loads

@@ -44,6 +44,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "context.cuh"
@@ -223,8 +224,12 @@ __device__ __forceinline__ void pw_stem_builder(const PwConvArgs& a, uint32_t sm
     }
 }
 
-template <bool XU8, bool LEAN>
-__global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_constant__ PwConvArgs a, const __grid_constant__ CUtensorMap x_map) {
+// Tail: QAddTail when a QLinearAdd follows the convolution (its other operand is read while the accumulators are on their way out
+// of TMEM: a pass over three tensors less), else PwNoTail.
+struct PwNoTail {};
+template <bool XU8, bool LEAN, typename Tail>
+__global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_constant__ PwConvArgs a, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ Tail add) {
+    constexpr bool ADD = std::is_same<Tail, QAddTail>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sA = smem;                                  // [k16][128 filters][16]
     uint8_t* sStages = smem + a.off_stages;
@@ -510,7 +515,20 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
             bool has = ch * 32 < n_loop;
             if (has) ptx::tmem_ld16(taddr + (uint32_t)(ch * 32), va);
             while (has) {
-                uint32_t pk[8];
+                uint32_t pk[8], rr[ADD ? 8 : 1];
+                if constexpr (ADD) {
+                    const int c0 = ch * 32;
+                    const uint8_t* r = add.res + ((size_t)img * a.M + (size_t)m) * a.HW + p0 + c0;
+                    if (a.mode != 1) {
+                        uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
+                        if (live && c0 < n_valid) r0 = __ldg(reinterpret_cast<const uint4*>(r));
+                        if (live && c0 + 32 <= n_valid) r1 = __ldg(reinterpret_cast<const uint4*>(r + 16));
+                        rr[0] = r0.x; rr[1] = r0.y; rr[2] = r0.z; rr[3] = r0.w; rr[4] = r1.x; rr[5] = r1.y; rr[6] = r1.z; rr[7] = r1.w;
+                    } else {
+#pragma unroll
+                        for (int j4 = 0; j4 < 8; ++j4) rr[j4] = live && c0 + j4 * 4 < n_valid ? __ldg(reinterpret_cast<const uint32_t*>(r) + j4) : 0u;
+                    }
+                }
                 ptx::tmem_wait_ld();
                 ptx::tmem_ld16(taddr + (uint32_t)(ch * 32 + 16), vb);
                 requant16(va, pk);
@@ -522,6 +540,11 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
                 if (LEAN && a.lut) {
 #pragma unroll
                     for (int j4 = 0; j4 < 8; ++j4) pk[j4] = lut4_smem(sLut, pk[j4]);
+                }
+                if constexpr (ADD) {
+#pragma unroll
+                    for (int j4 = 0; j4 < 8; ++j4) pk[j4] = qadd_word<false>(rr[j4], pk[j4], add);
+                    __syncwarp();                              // (lanes that took the exact form)
                 }
                 const int c0 = ch * 32;
                 if (a.mode != 1) {
@@ -731,10 +754,10 @@ inline void pw_conv_prepare(const PwConvPlan& p, const int8_t* w, const int32_t*
     }
 }
 
-template <bool XU8, bool LEAN>
-inline int32_t pw_conv_launch_t(zant_ctx* ctx, const PwConvPlan& p, const PwConvArgs& a, const CUtensorMap& x_map, int grid) {
-    ZB_SMEM_ATTR(ctx, (tc_pw_nchw_kernel<XU8, LEAN>), 232448);
-    launch_const(ctx, tc_pw_nchw_kernel<XU8, LEAN>, grid, kPwThreads, p.smem_bytes, a, x_map);
+template <bool XU8, bool LEAN, typename Tail = PwNoTail>
+inline int32_t pw_conv_launch_t(zant_ctx* ctx, const PwConvPlan& p, const PwConvArgs& a, const CUtensorMap& x_map, int grid, const Tail& add = Tail{}) {
+    ZB_SMEM_ATTR(ctx, (tc_pw_nchw_kernel<XU8, LEAN, Tail>), 232448);
+    launch_const(ctx, tc_pw_nchw_kernel<XU8, LEAN, Tail>, grid, kPwThreads, p.smem_bytes, a, x_map, add);
     return check_launch(ctx, "tc_pw_nchw_kernel");
 }
 
@@ -768,9 +791,10 @@ inline bool pw_conv_ptr_ok(const void* x, const void* y) {
     return (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(y) & 31u) == 0;
 }
 
-// `cap_dev`: per-filter accumulator bounds from requant_relu_caps when that returned true, else null.
+// `cap_dev`: per-filter accumulator bounds from requant_relu_caps when that returned true, else null.  `add`: a QLinearAdd behind it
+// (int8 input and output, output zero point 0, finite multipliers).
 inline int32_t pw_conv_run(zant_ctx* ctx, const PwConvPlan& p, const void* x, bool x_u8, const int8_t* w_blk_dev, const float* mult_dev,
-                           const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq, bool mult_finite, const int32_t* cap_dev) {
+                           const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq, bool mult_finite, const int32_t* cap_dev, const QAddTail* add = nullptr) {
     PwConvArgs a = p.a;
     a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.w = w_blk_dev; a.mult = mult_dev; a.bias = bias_dev;
     a.y_scale = rq.y_scale; a.y_zp = rq.y_zp; a.act = rq.act; a.out_u8 = y_u8 ? 1 : 0; a.lut = rq.lut;
@@ -782,6 +806,10 @@ inline int32_t pw_conv_run(zant_ctx* ctx, const PwConvPlan& p, const void* x, bo
     const int grid = p.m_tiles * a.cpm;
     alignas(64) CUtensorMap x_map{};
     if (a.mode == 0) ZB_TRY(pw_conv_encode_map(a, x, &x_map));
+    if (add) {
+        if (x_u8 || !lean) return fail(ZANT_E_UNSUPPORTED, "pointwise QLinearConv with QLinearAdd takes int8 tensors");
+        return pw_conv_launch_t<false, true, QAddTail>(ctx, p, a, x_map, grid, *add);
+    }
     if (x_u8) return lean ? pw_conv_launch_t<true, true>(ctx, p, a, x_map, grid) : pw_conv_launch_t<true, false>(ctx, p, a, x_map, grid);
     return lean ? pw_conv_launch_t<false, true>(ctx, p, a, x_map, grid) : pw_conv_launch_t<false, false>(ctx, p, a, x_map, grid);
 }
