@@ -24,6 +24,7 @@
 #include "dwconv_q8.cuh"
 #include "smallc_conv_q8.cuh"
 #include "tc_conv_nhwc.cuh"
+#include "tc_nhwc_net.cuh"
 #include "small_gemm_q8.cuh"
 #include "weight_blocks.cuh"
 #include "status.hpp"
@@ -838,6 +839,38 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         ZB_TRY(s.commit());
         ZB_TRY(run_qdwconv(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, finite, capped ? s.ptr<int32_t>(ic) : nullptr));
+        return s.finish();
+    }
+    NhConvPlan nhp;
+    bool mult_ok = true;
+    for (float f : mult) mult_ok = mult_ok && f > 0.0f && std::isfinite(f);
+    const int nh_kind8 = x_dtype == ZANT_U8 ? NH_U8 : NH_I8;
+    if (wz_zero && y_dtype == ZANT_I8 && y_zp == 0 && (long long)g.N * g.OH * g.OW >= 256 && g.N <= 65535 && mult_ok &&
+        (x_zp == 0 || !(g.pt || g.pl || g.pb || g.pr)) && (!is_device_ptr(x) || (reinterpret_cast<uintptr_t>(x) & 3u) == 0) && nh_conv_plan_kept(g, nh_kind8, ctx->sm_count, nhp)) {
+        // pixels of all channels together, then the channels-last kernel, which needs no im2col matrix: the taps are boxes of the image
+        const int pix = (g.C + 15) / 16 * 16, hw = g.H * g.W, K = g.Cg * g.KH * g.KW;
+        std::vector<float> mp(mult);
+        mp.resize((size_t)nhp.a.const_n, 1.0f);
+        const bool bias_here = x_zp == 0 && !(bias && is_device_ptr(bias));        // nothing to fold in: padded on the host
+        std::vector<int32_t> bp((size_t)(bias_here ? nhp.a.const_n : 0), 0);
+        if (bias_here && bias) std::memcpy(bp.data(), bias, (size_t)g.M * 4);
+        Stager s(ctx);
+        const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = bias_here ? s.in(bp.data(), bp.size() * 4) : s.in(bias, (size_t)g.M * 4);
+        const int ixl = s.scratch((size_t)g.N * hw * pix), iwb = s.scratch(nhp.w_bytes), ibb = s.scratch((size_t)nhp.a.const_n * 4);
+        ZB_TRY(s.commit());
+        const uint64_t launched = ctx->launches;
+        ZB_TRY(run_nh_weights(ctx, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb)));
+        if (!bias_here) {
+            launch(ctx, nh_bias_k, (unsigned)((nhp.a.const_n + 7) / 8), 256, 0, (const int8_t*)s.ptr<int8_t>(iw), (const int32_t*)s.ptr<int32_t>(ib), s.ptr<int32_t>(ibb), g.M, K, nhp.a.const_n, x_zp);
+            ZB_TRY(check_launch(ctx, "nh_bias_k"));
+        }
+        ctx->launches = launched;                       // (not operator launches)
+        ZB_TRY(run_to_nhwc_bytes(ctx, s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix));
+        NhConvArgs a = nhp.a;
+        a.w = s.ptr<uint8_t>(iwb); a.mult = s.ptr<float>(im); a.bias = s.ptr<int32_t>(bias_here ? ib : ibb);
+        a.y = s.ptr<uint8_t>(iy); a.nchw = 1; a.act = activation; a.six = lean_six(y_scale);
+        ZB_TRY(nh_conv_run(ctx, nhp, a, NhView{s.ptr<char>(ixl), pix, g.H, g.W, 0}));
         return s.finish();
     }
     if (qconv_tc_eligible(g, wz_zero)) {

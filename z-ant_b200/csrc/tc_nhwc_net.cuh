@@ -16,6 +16,9 @@
 //   NH_POOL_PAIRS (64-filter tiles)   per filter row and member row: the two middle views with both members' filters (2 NT columns),
 //                                     the outer ones with one member's - 24 MMAs, no zeros
 //
+// Stride 2 reads the four parity planes as well, with one accumulator: tap (kh, kw) is plane ((kh - pt) & 1, (kw - pl) & 1) shifted by
+// ((kh - pt) >> 1, (kw - pl) >> 1).  (A 1x1 filter with stride 2 reads one plane, as an image of its own.)
+//
 // At most 16 channel bytes (KC = 16: first layers, 16-channel int8 layers) would leave half of every 32-byte K step empty: there a
 // pixel is one 16-byte row without swizzle, and a K step takes TWO views, whose distance in shared memory is the descriptor's
 // leading-dimension offset: 8 MMAs instead of 16.
@@ -53,7 +56,7 @@
 
 namespace zb {
 
-enum NhPool { NH_POOL_NONE = 0, NH_POOL_VIEWS = 1, NH_POOL_PAIRS = 2 };
+enum NhPool { NH_POOL_NONE = 0, NH_POOL_VIEWS = 1, NH_POOL_PAIRS = 2, NH_STRIDE2 = 3 };
 enum NhKind { NH_I8 = 0, NH_U8 = 1, NH_TF32 = 2, NH_TF32X3 = 3 };      // type of the activations read
 
 struct NhConvArgs {
@@ -112,6 +115,8 @@ __device__ __forceinline__ void nh_mma(uint32_t leader, uint32_t d_tmem, uint32_
     }
 }
 
+__host__ __device__ __forceinline__ int nh_shift(int d) { return d >= 0 ? d / 2 : -((1 - d) / 2); }
+
 // The tiles of a CTA, grid-size apart, as a mixed-radix counter: divisions at the start only (a tile's four cost its 19 warps
 // more issue slots than a first layer's epilogue has to spare).
 struct NhTile { int nt, ws, hs, img, d_nt, d_ws, d_hs, d_img; };
@@ -134,7 +139,8 @@ template <int KIND, int POOL>
 __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid_constant__ NhConvArgs a, const __grid_constant__ NhMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr bool I8 = KIND <= NH_U8;
-    constexpr int PLANES = POOL ? 4 : 1, SETS = POOL ? 4 : 1;      // accumulators per row block
+    constexpr bool POOLED = POOL == NH_POOL_VIEWS || POOL == NH_POOL_PAIRS;
+    constexpr int PLANES = POOL ? 4 : 1, SETS = POOLED ? 4 : 1;    // parity planes per stage, accumulators per row block
     float* sMult = reinterpret_cast<float*>(smem + a.off_const);
     int* sBias = reinterpret_cast<int*>(sMult + a.const_n);         // TF32: the float bias' bits
     uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + a.const_n);
@@ -195,11 +201,15 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                     uint32_t dst = stage0;
                     for (int part = 0; part < a.parts; ++part) {
                         const int c0 = cs * chans + part * a.lo_off;
-                        if (POOL) {
+                        if (POOLED) {
                             // parity plane (pr, pc) of the zero-bordered image: rows 2 * i + pr - 1; the odd image rows (pr = 0) start one higher
 #pragma unroll
                             for (int pp = 0; pp < 4; ++pp, dst += (uint32_t)a.plane_bytes)
                                 ptx::tma_load_4d(dst, &maps.m[pp], c0, w0 - ((pp & 1) ? 0 : 1), h0 - ((pp & 2) ? 0 : 1), T.img, full(s));
+                        } else if (POOL == NH_STRIDE2) {
+#pragma unroll
+                            for (int pp = 0; pp < 4; ++pp, dst += (uint32_t)a.plane_bytes)
+                                ptx::tma_load_4d(dst, &maps.m[pp], c0, w0 + nh_shift(-a.pl), h0 + nh_shift(-a.pt), T.img, full(s));
                         } else {
                             ptx::tma_load_4d(dst, &maps.m[0], c0, w0 - a.pl, h0 - a.pt, T.img, full(s));
                             dst += (uint32_t)a.plane_bytes;
@@ -391,7 +401,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
                                 s[j] = (int)v[0][j4 * 4 + j];
-                                if (POOL) s[j] = max(__vimax3_s32(s[j], (int)v[SETS > 1 ? 1 : 0][j4 * 4 + j], (int)v[SETS > 2 ? 2 : 0][j4 * 4 + j]), (int)v[SETS > 3 ? 3 : 0][j4 * 4 + j]);
+                                if (POOLED) s[j] = max(__vimax3_s32(s[j], (int)v[SETS > 1 ? 1 : 0][j4 * 4 + j], (int)v[SETS > 2 ? 2 : 0][j4 * 4 + j]), (int)v[SETS > 3 ? 3 : 0][j4 * 4 + j]);
                             }
                             uint32_t pk = pack_act_s8x4(rq_round(s[0] + b4.x, m4.x), rq_round(s[1] + b4.y, m4.y), rq_round(s[2] + b4.z, m4.z), rq_round(s[3] + b4.w, m4.w),
                                                         a.act != ZANT_QACT_NONE, hi4);
@@ -427,7 +437,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                                 float q = __fadd_rn(__uint_as_float(v[m][j]), bs);
                                 if (a.act == FACT_RELU) q = q > 0.0f ? q : 0.0f;
                                 else if (a.act == FACT_LEAKY) q = q <= 0.0f ? __fmul_rn(a.slope, q) : q;
-                                best = !POOL ? q : (q > best ? q : best);
+                                best = !POOLED ? q : (q > best ? q : best);
                             }
                             r[j] = best;
                         }
@@ -485,6 +495,7 @@ struct NhConvPlan {
     NhConvArgs a{};
     int kind = NH_I8, NT = 0;
     int pool = 0;                 // NhPool
+    bool half = false;            // 1x1, stride 2: every second row and column of the input is the image
     int cin = 0, w_cin = 0;       // channels a pixel of the input holds, channels of the weights (fewer: zero weights behind them)
     size_t smem_bytes = 0, w_bytes = 0;
 };
@@ -497,6 +508,7 @@ __host__ __device__ inline int nh_pair(int it, int which, int taps) {
 // NH_POOL_VIEWS: view of pair `it`: two rows apart, i.e. in the same parity plane.
 __host__ __device__ inline int nh_view_pair(int it, int which) { return (it >> 2) * 4 + (it & 3) + which * 8; }
 
+// Stride 2: row (or column) d of the image relative to 2 * i lies in parity plane d & 1, row i + nh_shift(d).
 // Operand offsets, in 16-byte units.
 inline void nh_offsets(NhConvArgs& a, int mode) {
     const int unit = a.KC / 16, taps = a.KH * a.KW;
@@ -514,6 +526,9 @@ inline void nh_offsets(NhConvArgs& a, int mode) {
             if (mode == NH_POOL_VIEWS) { const int v0 = nh_view_pair(it, 0), v1 = nh_view_pair(it, 1); o0 = view_at(v0 / 4, v0 % 4); o1 = view_at(v1 / 4, v1 % 4); }
             else { const int t1 = nh_pair(it, 1, taps); o0 = tap_at(nh_pair(it, 0, taps)); o1 = t1 >= 0 ? tap_at(t1) : o0; }
             a.aoff[it] = o0 | ((o1 - o0) << 16);
+        } else if (mode == NH_STRIDE2) {
+            const int dh = it / a.KW - a.pt, dw = it % a.KW - a.pl;
+            a.aoff[it] = (uint32_t)(((dh & 1) * 2 + (dw & 1)) * (a.plane_bytes / 16) + ((nh_shift(dh) - nh_shift(-a.pt)) * a.PW + nh_shift(dw) - nh_shift(-a.pl)) * unit);
         } else a.aoff[it] = mode == NH_POOL_VIEWS ? view_at(it / 4, it % 4) : tap_at(it);
     }
 }
@@ -528,7 +543,7 @@ inline double nh_cost(const NhConvArgs& a, int kind, int mode, long long tiles, 
     const double mma = iters * ksteps * per * a.RB * (mode == NH_POOL_PAIRS ? (4 * clocks(NB) + 4 * clocks(NT)) / 3.0 : clocks(NB));
     const double issue = iters * (40.0 + 20.0 * ksteps) + iters / a.w_group * 150.0 + a.c_stages * 150.0;
     const double bytes = (double)a.c_stages * planes * a.parts * a.PH * a.PW * a.KC + (resident ? 0.0 : (double)w_all);
-    const double epi = (double)a.RB * NT / 64.0 * (mode ? 700.0 : 450.0);
+    const double epi = (double)a.RB * NT / 64.0 * (mode == NH_POOL_VIEWS || mode == NH_POOL_PAIRS ? 700.0 : 450.0);
     const double tile = std::max(std::max(mma + issue, bytes / 40.0), epi) + 300.0;
     return std::ceil((double)tiles / sm_count) * tile + epi;
 }
@@ -537,10 +552,12 @@ inline double nh_cost(const NhConvArgs& a, int kind, int mode, long long tiles, 
 inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, NhConvPlan& p) {
     const bool i8 = kind <= NH_U8;
     const int esz = i8 ? 1 : 4, parts = kind == NH_TF32X3 ? 2 : 1;
-    if (g.G != 1 || g.sh != 1 || g.sw != 1 || g.N <= 0 || g.OH <= 0 || g.OW <= 0 || g.M > 4096) return false;
+    const bool s2 = g.sh == 2 && (g.KH > 1 || g.KW > 1), planed = pool || s2;
+    if (g.sh == 2 && !s2 && (g.pt || g.pl)) return false;
+    if (g.G != 1 || g.sh != g.sw || (g.sh != 1 && g.sh != 2) || (g.sh == 2 && (pool || !i8 || g.dh != 1 || g.dw != 1 || g.H < 2 || g.W < 2)) || g.N <= 0 || g.OH <= 0 || g.OW <= 0 || g.M > 4096) return false;
     if (pool && (g.KH != 3 || g.KW != 3 || g.dh != 1 || g.dw != 1 || g.pt != 1 || g.pl != 1 || g.pb != 1 || g.pr != 1 || g.H % 2 || g.W % 2)) return false;
-    const int halo_w = pool ? 1 : (g.KW - 1) * g.dw, halo_h = pool ? 1 : (g.KH - 1) * g.dh;
-    if (halo_w > 32 || halo_h > 32 || g.pt > halo_h + 1 || g.pl > halo_w + 1) return false;
+    const int halo_w = pool ? 1 : (s2 ? nh_shift(g.KW - 1 - g.pl) - nh_shift(-g.pl) : (g.KW - 1) * g.dw), halo_h = pool ? 1 : (s2 ? nh_shift(g.KH - 1 - g.pt) - nh_shift(-g.pt) : (g.KH - 1) * g.dh);
+    if (halo_w > 32 || halo_h > 32 || (s2 ? g.pt >= g.KH || g.pl >= g.KW : g.pt > halo_h + 1 || g.pl > halo_w + 1)) return false;
     NhConvArgs base{};
     base.N = g.N; base.M = g.M; base.KH = g.KH; base.KW = g.KW; base.dh = g.dh; base.dw = g.dw; base.pt = g.pt; base.pl = g.pl;
     base.GH = pool ? g.OH / 2 : g.OH; base.GW = pool ? g.OW / 2 : g.OW;
@@ -551,18 +568,18 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
     base.parts = parts;
     const int cin = parts > 1 ? (g.C + 7) / 8 * 8 : g.C;             // (a stage of the hi half must not run into the lo half)
     base.lo_off = cin;
-    const int cbytes = cin * esz, planes = pool ? 4 : 1, sets = pool ? 4 : 1, taps = g.KH * g.KW;
-    p.kind = kind; p.cin = cin; p.w_cin = g.C;
+    const int cbytes = cin * esz, planes = planed ? 4 : 1, sets = pool ? 4 : 1, taps = g.KH * g.KW;
+    p.kind = kind; p.cin = cin; p.w_cin = g.C; p.half = g.sh == 2 && !s2;
     if (taps > 64) return false;
     double best = 1e300;
     for (int NT = pool ? 16 : 32; NT <= (pool ? 64 : 256); NT *= 2)
         for (int KC = 16; KC <= 128; KC *= 2)
             for (int rb = 1; rb <= 4; ++rb) {
-                const int mode = !pool ? NH_POOL_NONE : (NT <= 32 ? NH_POOL_VIEWS : NH_POOL_PAIRS);
+                const int mode = s2 ? NH_STRIDE2 : !pool ? NH_POOL_NONE : (NT <= 32 ? NH_POOL_VIEWS : NH_POOL_PAIRS);
                 const int NB = NT * (mode == NH_POOL_VIEWS ? 4 : (mode == NH_POOL_PAIRS ? 2 : 1));
                 if (2 * sets * rb * NT > 512 || (NT > 32 && NT / 2 >= g.M) || (mode == NH_POOL_PAIRS && KC == 16)) continue;
-                if (KC > 16 && KC / 2 >= cbytes) continue;               // (channels past C arrive as zeros)
-                if (KC == 16 && (cbytes > 16 || parts > 1)) continue;
+                if (KC > (s2 ? 32 : 16) && KC / 2 >= cbytes) continue;               // (channels past C arrive as zeros)
+                if (KC == 16 && (cbytes > 16 || parts > 1 || s2)) continue;
                 NhConvArgs a = base;
                 a.n_tiles = (g.M + NT - 1) / NT;
                 a.KC = KC; a.c_stages = (cbytes + KC - 1) / KC;
@@ -670,6 +687,37 @@ inline int32_t run_nh_weights(zant_ctx* ctx, const NhConvPlan& p, const void* w,
     return check_launch(ctx, "nh_weights_k");
 }
 
+// bias - x_zp * (sum of the filter's weights), zeros behind the last filter: a warp per entry.
+__global__ void __launch_bounds__(256) nh_bias_k(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int32_t* __restrict__ out, int M, int K, int n, int x_zp) {
+    ptx::grid_start();
+    const int m = (int)((blockIdx.x * 256 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (m >= n) return;
+    int s = 0;
+    if (m < M && x_zp != 0) for (int k = lane; k < K; k += 32) s += __ldg(w + (size_t)m * K + k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[m] = m < M ? (bias ? __ldg(bias + m) : 0) - x_zp * s : 0;
+}
+
+// A single call's plan: the search below visits some hundred tilings (20 us, as long as a small convolution takes), so a thread keeps
+// the plans of the last shapes it used.
+inline bool nh_conv_plan_kept(const ConvGeom& g, int kind, int sm_count, NhConvPlan& p) {
+    struct Entry { ConvGeom g; int kind = -1, sm = 0; bool ok = false; NhConvPlan p; };
+    constexpr int kEntries = 16;
+    static thread_local std::vector<Entry> kept;
+    static thread_local int next = 0;
+    static_assert(std::is_trivially_copyable<ConvGeom>::value && sizeof(ConvGeom) % sizeof(int) == 0, "compared as bytes");
+    for (const Entry& e : kept) if (e.kind == kind && e.sm == sm_count && std::memcmp(&e.g, &g, sizeof(g)) == 0) { p = e.p; return e.ok; }
+    Entry e;
+    e.g = g; e.kind = kind; e.sm = sm_count;
+    e.ok = nh_conv_plan(g, kind, false, sm_count, e.p);
+    p = e.p;
+    const bool ok = e.ok;
+    if ((int)kept.size() < kEntries) kept.push_back(e);
+    else { kept[next] = e; next = (next + 1) % kEntries; }
+    return ok;
+}
+
 // A channels-last buffer: `ptr` = channel 0 of pixel (0, 0), pixels `pix` bytes apart; lo: split form, channel offset of the lo half.
 struct NhView { void* ptr; long long pix; int H, W; int lo; };
 
@@ -690,7 +738,7 @@ inline int32_t nh_encode_map(int N, const NhView& x, int chan_elems, int esz, in
     if (parity) {
         // plane (pr, pc) of the zero-bordered image: pr = 0 are the odd image rows, pr = 1 the even ones, columns likewise
         base += (pr ? 0 : (long long)row) + (pc ? 0 : x.pix);
-        dims[1] = x.W / 2; dims[2] = x.H / 2; strides[0] = 2 * (cuuint64_t)x.pix; strides[1] = 2 * row;
+        dims[1] = (x.W + pc) / 2; dims[2] = (x.H + pr) / 2; strides[0] = 2 * (cuuint64_t)x.pix; strides[1] = 2 * row;
     }
     const cuuint32_t box[4] = {(cuuint32_t)(KC / esz), (cuuint32_t)box_w, (cuuint32_t)box_h, 1}, estr[4] = {1, 1, 1, 1};
     const CUtensorMapSwizzle sw = KC == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (KC == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : (KC == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE));
@@ -711,6 +759,7 @@ template <int KIND>
 inline int32_t nh_launch_k(zant_ctx* ctx, const NhConvPlan& p, const NhConvArgs& a, const NhMaps& maps) {
     if (p.pool == NH_POOL_VIEWS) return nh_launch_t<KIND, NH_POOL_VIEWS>(ctx, p, a, maps);
     if (p.pool == NH_POOL_PAIRS) return nh_launch_t<KIND, NH_POOL_PAIRS>(ctx, p, a, maps);
+    if constexpr (KIND <= NH_U8) { if (p.pool == NH_STRIDE2) return nh_launch_t<KIND, NH_STRIDE2>(ctx, p, a, maps); }
     return nh_launch_t<KIND, NH_POOL_NONE>(ctx, p, a, maps);
 }
 
@@ -720,8 +769,11 @@ inline int32_t nh_conv_run(zant_ctx* ctx, const NhConvPlan& p, NhConvArgs a, con
     a.status = ctx->status_word;
     a.lo_off = x.lo;
     NhMaps maps;
-    for (int pp = 0; pp < (p.pool ? 4 : 1); ++pp)
-        ZB_TRY(nh_encode_map(a.N, x, a.parts > 1 ? x.lo + p.cin : p.cin, esz, a.KC, a.PW, a.PH, p.pool != 0, pp >> 1, pp & 1, &maps.m[pp]));
+    for (int pp = 0; pp < (p.pool ? 4 : 1); ++pp) {
+        // (the pooled form numbers the planes of the bordered image, whose odd rows are the image's even ones)
+        const int pr = p.pool == NH_STRIDE2 || p.half ? 1 - (pp >> 1) : pp >> 1, pc = p.pool == NH_STRIDE2 || p.half ? 1 - (pp & 1) : pp & 1;
+        ZB_TRY(nh_encode_map(a.N, x, a.parts > 1 ? x.lo + p.cin : p.cin, esz, a.KC, a.PW, a.PH, p.pool != 0 || p.half, pr, pc, &maps.m[pp]));
+    }
     switch (p.kind) {
         case NH_I8: return nh_launch_k<NH_I8>(ctx, p, a, maps);
         case NH_U8: return nh_launch_k<NH_U8>(ctx, p, a, maps);
@@ -798,6 +850,45 @@ inline int32_t run_to_nhwc(zant_ctx* ctx, int mode, const void* x, void* y, int 
         default: launch(ctx, to_nhwc_small_k<3>, grid, 256, 0, a); break;
     }
     return check_launch(ctx, "to_nhwc_small_k");
+}
+
+// Any 8-bit NCHW tensor -> pixels of `pix` bytes (channels rounded up to 16, zeros behind the last): 64 channels x 128 pixels of one
+// image through shared memory.  The rows of a channel plane start at any byte: a thread cuts its word out of two aligned ones.
+constexpr int kToNhwcPx = 128, kToNhwcCh = 64, kToNhwcPitch = kToNhwcPx + 4;
+__global__ void __launch_bounds__(256) to_nhwc_bytes_k(const uint8_t* __restrict__ x, uint8_t* __restrict__ y, int C, int HW, int pix, long long bytes) {
+    ptx::grid_start();
+    __shared__ __align__(16) uint8_t tile[kToNhwcCh * kToNhwcPitch];
+    const int p0 = (int)blockIdx.x * kToNhwcPx, c0 = (int)blockIdx.y * kToNhwcCh;
+    const long long n = blockIdx.z;
+    for (int i = threadIdx.x; i < kToNhwcCh * (kToNhwcPx / 4); i += 256) {
+        const int c = i / (kToNhwcPx / 4), w = i - c * (kToNhwcPx / 4);
+        uint32_t v = 0;
+        if (c0 + c < C && p0 + 4 * w < HW) {
+            const long long at = (n * C + c0 + c) * (long long)HW + p0 + 4 * w, al = at & ~3LL;
+            const uint32_t* s = reinterpret_cast<const uint32_t*>(x + al);
+            if (al + 8 <= bytes) {
+                const uint32_t lo = __ldg(s), sh = (uint32_t)(at & 3) * 8u;
+                v = sh ? __funnelshift_r(lo, __ldg(s + 1), sh) : lo;
+            } else {
+                for (int k = 0; k < 4; ++k) if (at + k < bytes) v |= (uint32_t)__ldg(x + at + k) << (8 * k);
+            }
+        }
+        *reinterpret_cast<uint32_t*>(tile + c * kToNhwcPitch + 4 * w) = v;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kToNhwcPx * (kToNhwcCh / 16); i += 256) {
+        const int p = i >> 2, c = (i & 3) * 16;
+        if (p0 + p >= HW || c0 + c >= pix) continue;
+        uint32_t q[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int k = 0; k < 16; ++k) q[k >> 2] |= (uint32_t)tile[(c + k) * kToNhwcPitch + p] << (8 * (k & 3));
+        *reinterpret_cast<uint4*>(y + (n * HW + p0 + p) * (long long)pix + c0 + c) = make_uint4(q[0], q[1], q[2], q[3]);
+    }
+}
+inline int32_t run_to_nhwc_bytes(zant_ctx* ctx, const void* x, void* y, int N, int C, int HW, int pix) {
+    const dim3 grid((unsigned)((HW + kToNhwcPx - 1) / kToNhwcPx), (unsigned)((pix + kToNhwcCh - 1) / kToNhwcCh), (unsigned)N);
+    launch(ctx, to_nhwc_bytes_k, grid, 256, 0, (const uint8_t*)x, (uint8_t*)y, C, HW, pix, (long long)N * C * HW);
+    return check_launch(ctx, "to_nhwc_bytes_k");
 }
 
 // MaxPool: a thread owns 16 bytes of one output pixel's channels.  KIND as above; split form: the larger hi + lo.
