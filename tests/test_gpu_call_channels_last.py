@@ -22,7 +22,9 @@ CASES = [
     (2, 16, 9, 200, 24, 3, 2, (1, 1, 1, 1), I8, 0, "relu6"),        # a row of 100 outputs
     (1, 130, 26, 300, 40, 3, 2, (1, 1, 1, 1), I8, 0, None),         # two column segments
     (40, 8, 3, 3, 9, 3, 1, (1, 1, 1, 1), I8, 0, "relu"),            # tiles of mostly dead rows
-    (3, 256, 14, 14, 512, 3, 2, (1, 1, 1, 1), I8, 0, "relu"),       # streamed weights
+    (7, 256, 14, 14, 512, 3, 2, (1, 1, 1, 1), I8, 0, "relu"),       # streamed weights, two images per tile, an odd one
+    (90, 40, 2, 5, 24, 3, 1, (1, 1, 1, 1), U8, 0, None),            # four images per tile
+    (300, 70, 3, 3, 33, 1, 2, (0, 0, 0, 0), I8, 3, "relu"),         # 1 x 1 with stride 2 onto 2 x 2: 32 images per tile
 ]
 
 

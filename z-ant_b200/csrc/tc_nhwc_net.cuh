@@ -61,6 +61,7 @@ enum NhKind { NH_I8 = 0, NH_U8 = 1, NH_TF32 = 2, NH_TF32X3 = 3 };      // type o
 
 struct NhConvArgs {
     int N, M, KH, KW, dh, dw, pt, pl;
+    int imgs, IB;                 // images; images per tile, where whole patches of them fit one row block (N: groups of IB)
     int GH, GW;                   // rows of the product: output pixels, or pooled ones
     int BW, PW, BH, RB, PH;       // a row block is BH x BW pixels at pitch PW; RB blocks per tile; patch rows
     int hseg, wseg, n_tiles;
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t box = (uint32_t)(a.KC * a.PW * a.PH), esz = I8 ? 1u : 4u;
+            const uint32_t box = (uint32_t)(a.KC * a.PW * a.PH * a.IB), esz = I8 ? 1u : 4u;
             const int chans = a.KC / (int)esz;
             int s = 0; uint32_t ph = 0;
             bool alive = true;
@@ -209,9 +210,9 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                         } else if (POOL == NH_STRIDE2) {
 #pragma unroll
                             for (int pp = 0; pp < 4; ++pp, dst += (uint32_t)a.plane_bytes)
-                                ptx::tma_load_4d(dst, &maps.m[pp], c0, w0 + nh_shift(-a.pl), h0 + nh_shift(-a.pt), T.img, full(s));
+                                ptx::tma_load_4d(dst, &maps.m[pp], c0, w0 + nh_shift(-a.pl), h0 + nh_shift(-a.pt), T.img * a.IB, full(s));
                         } else {
-                            ptx::tma_load_4d(dst, &maps.m[0], c0, w0 - a.pl, h0 - a.pt, T.img, full(s));
+                            ptx::tma_load_4d(dst, &maps.m[0], c0, w0 - a.pl, h0 - a.pt, T.img * a.IB, full(s));
                             dst += (uint32_t)a.plane_bytes;
                         }
                     }
@@ -360,8 +361,9 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
         const int quarter = warp & 3, part = (warp - 2) >> 2;      // (warp 18 is the weights')
         constexpr int CH = 16;
         const int row = quarter * 32 + lane;
-        const int oh_l = row / a.PW, ow_l = row - oh_l * a.PW;
-        const bool row_live = oh_l < a.BH && ow_l < a.BW;
+        const int img_l = a.IB > 1 ? row / (a.PH * a.PW) : 0, row_i = row - img_l * (a.PH * a.PW);
+        const int oh_l = row_i / a.PW, ow_l = row_i - oh_l * a.PW;
+        const bool row_live = oh_l < a.BH && ow_l < a.BW && img_l < a.IB;
         const uint32_t hi4 = a.act == ZANT_QACT_RELU6 ? 0x01010101u * (uint32_t)(a.six & 255) : 0x7f7f7f7fu;
         const int per_blk = NT / CH, chunks = a.RB * per_blk;
         int tile_it = 0;
@@ -379,7 +381,8 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
             int rb = rb0, h = hc0;
             for (int ch = part; ch < chunks; ch += 4) {
                 const int g0 = h0 + rb * a.BH, gh = g0 + oh_l;
-                const bool live = row_live && gh < a.GH && gw < a.GW;
+                const int img = POOLED ? T.img : T.img * a.IB + img_l;
+                const bool live = row_live && gh < a.GH && gw < a.GW && (POOLED || img < a.imgs);
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((b * a.RB + rb) * SETS * NT + h * CH);
                 const int c0 = T.nt * NT + h * CH;
                 h += 4;
@@ -390,7 +393,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
 #pragma unroll
                     for (int m = 0; m < SETS; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * NT), v[m]);
                     ptx::tmem_wait_ld();
-                    uint8_t* yp = a.nchw ? a.y : a.y + (long long)T.img * a.y_img + (long long)gh * (a.up2 ? 2 : 1) * a.y_row + (long long)gw * (a.up2 ? 2 : 1) * a.y_pix;
+                    uint8_t* yp = a.nchw ? a.y : a.y + (long long)img * a.y_img + (long long)gh * (a.up2 ? 2 : 1) * a.y_row + (long long)gw * (a.up2 ? 2 : 1) * a.y_pix;
                     if constexpr (I8) {
                         uint32_t wd[CH / 4];
 #pragma unroll
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                         }
                         if (!live) continue;
                         if (a.nchw) {
-                            const size_t plane = (size_t)a.GH * a.GW, at = ((size_t)T.img * a.M + c0) * plane + (size_t)gh * a.GW + gw;
+                            const size_t plane = (size_t)a.GH * a.GW, at = ((size_t)img * a.M + c0) * plane + (size_t)gh * a.GW + gw;
 #pragma unroll
                             for (int j = 0; j < CH; ++j) {
                                 if (c0 + j >= a.M) break;
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                         }
                         if (!live) continue;
                         if (a.nchw) {
-                            const size_t plane = (size_t)a.GH * a.GW, at = ((size_t)T.img * a.M + c0) * plane + (size_t)gh * a.GW + gw;
+                            const size_t plane = (size_t)a.GH * a.GW, at = ((size_t)img * a.M + c0) * plane + (size_t)gh * a.GW + gw;
 #pragma unroll
                             for (int j = 0; j < CH; ++j) {
                                 if (c0 + j >= a.M) break;
@@ -542,7 +545,7 @@ inline double nh_cost(const NhConvArgs& a, int kind, int mode, long long tiles, 
     const double iters = (double)a.c_stages * a.T;
     const double mma = iters * ksteps * per * a.RB * (mode == NH_POOL_PAIRS ? (4 * clocks(NB) + 4 * clocks(NT)) / 3.0 : clocks(NB));
     const double issue = iters * (40.0 + 20.0 * ksteps) + iters / a.w_group * 150.0 + a.c_stages * 150.0;
-    const double bytes = (double)a.c_stages * planes * a.parts * a.PH * a.PW * a.KC + (resident ? 0.0 : (double)w_all);
+    const double bytes = (double)a.c_stages * planes * a.parts * a.PH * a.PW * a.IB * a.KC + (resident ? 0.0 : (double)w_all);
     const double epi = (double)a.RB * NT / 64.0 * (mode == NH_POOL_VIEWS || mode == NH_POOL_PAIRS ? 700.0 : 450.0);
     const double tile = std::max(std::max(mma + issue, bytes / 40.0), epi) + 300.0;
     return std::ceil((double)tiles / sm_count) * tile + epi;
@@ -565,6 +568,10 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
     base.BW = (base.GW + base.wseg - 1) / base.wseg;
     base.PW = base.BW + halo_w;
     base.BH = std::max(1, std::min(base.GH, 128 / base.PW));
+    // images whose whole patch is at most half a row block share one (7 x 7 outputs with stride 2: two, of 64 rows each)
+    base.imgs = g.N; base.IB = 1;
+    if (!pool && base.wseg == 1 && base.BH == base.GH) base.IB = std::max(1, std::min(g.N, 128 / ((base.GH + halo_h) * base.PW)));
+    base.N = (g.N + base.IB - 1) / base.IB;
     base.parts = parts;
     const int cin = parts > 1 ? (g.C + 7) / 8 * 8 : g.C;             // (a stage of the hi half must not run into the lo half)
     base.lo_off = cin;
@@ -589,7 +596,7 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
                 if (a.PH > 256 || (rb > 1 && (rb - 1) * a.BH >= a.GH)) continue;
                 if (parts > 1 && cin % (KC / 4) != 0) continue;
                 a.hseg = (a.GH + rb * a.BH - 1) / (rb * a.BH);
-                const int rows = std::max(a.PH * a.PW, (rb - 1) * a.BH * a.PW + 128 + halo_h * a.PW + halo_w);
+                const int rows = std::max(a.PH * a.PW * a.IB, (rb - 1) * a.BH * a.PW + 128 + halo_h * a.PW + halo_w);
                 a.plane_bytes = (rows * KC + 1023) / 1024 * 1024;
                 a.const_n = (a.n_tiles * NT + 15) / 16 * 16;
                 const int tail = a.const_n * 8 + kNhTail;
@@ -721,7 +728,7 @@ inline bool nh_conv_plan_kept(const ConvGeom& g, int kind, int sm_count, NhConvP
 // A channels-last buffer: `ptr` = channel 0 of pixel (0, 0), pixels `pix` bytes apart; lo: split form, channel offset of the lo half.
 struct NhView { void* ptr; long long pix; int H, W; int lo; };
 
-inline int32_t nh_encode_map(int N, const NhView& x, int chan_elems, int esz, int KC, int box_w, int box_h, bool parity, int pr, int pc, CUtensorMap* map) {
+inline int32_t nh_encode_map(int N, int box_n, const NhView& x, int chan_elems, int esz, int KC, int box_w, int box_h, bool parity, int pr, int pc, CUtensorMap* map) {
     using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static std::atomic<EncodeFn> encode{nullptr};
@@ -740,7 +747,7 @@ inline int32_t nh_encode_map(int N, const NhView& x, int chan_elems, int esz, in
         base += (pr ? 0 : (long long)row) + (pc ? 0 : x.pix);
         dims[1] = (x.W + pc) / 2; dims[2] = (x.H + pr) / 2; strides[0] = 2 * (cuuint64_t)x.pix; strides[1] = 2 * row;
     }
-    const cuuint32_t box[4] = {(cuuint32_t)(KC / esz), (cuuint32_t)box_w, (cuuint32_t)box_h, 1}, estr[4] = {1, 1, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)(KC / esz), (cuuint32_t)box_w, (cuuint32_t)box_h, (cuuint32_t)box_n}, estr[4] = {1, 1, 1, 1};
     const CUtensorMapSwizzle sw = KC == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (KC == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : (KC == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE));
     const CUresult r = encode.load()(map, esz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr,
                                      CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -772,7 +779,7 @@ inline int32_t nh_conv_run(zant_ctx* ctx, const NhConvPlan& p, NhConvArgs a, con
     for (int pp = 0; pp < (p.pool ? 4 : 1); ++pp) {
         // (the pooled form numbers the planes of the bordered image, whose odd rows are the image's even ones)
         const int pr = p.pool == NH_STRIDE2 || p.half ? 1 - (pp >> 1) : pp >> 1, pc = p.pool == NH_STRIDE2 || p.half ? 1 - (pp & 1) : pp & 1;
-        ZB_TRY(nh_encode_map(a.N, x, a.parts > 1 ? x.lo + p.cin : p.cin, esz, a.KC, a.PW, a.PH, p.pool != 0 || p.half, pr, pc, &maps.m[pp]));
+        ZB_TRY(nh_encode_map(a.imgs, a.IB, x, a.parts > 1 ? x.lo + p.cin : p.cin, esz, a.KC, a.PW, a.PH, p.pool != 0 || p.half, pr, pc, &maps.m[pp]));
     }
     switch (p.kind) {
         case NH_I8: return nh_launch_k<NH_I8>(ctx, p, a, maps);
