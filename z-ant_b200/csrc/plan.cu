@@ -665,6 +665,27 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
             });
             return ZANT_OK;
         }
+        const std::vector<PwConvPlan> parts = stem ? std::vector<PwConvPlan>{} : pw_conv_parts(g, wz_zero, ctx->sm_count, pwp);
+        if (!parts.empty()) {
+            std::vector<int> aws, abs;
+            int m0 = 0;
+            for (const PwConvPlan& part : parts) {
+                pw_conv_prepare(part, (const int8_t*)T(w).host.data() + (size_t)m0 * g.C, b >= 0 ? (const int32_t*)T(b).host.data() + m0 : nullptr, xzp, w_blk, bf);
+                aws.push_back(pl->add_aux(w_blk.data(), w_blk.size())); abs.push_back(pl->add_aux(bf.data(), bf.size() * 4));
+                m0 += part.a.M;
+            }
+            push("QLinearConv(tc-pointwise)" + tail, [=]() {
+                if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");
+                int at = 0;
+                for (size_t i = 0; i < parts.size(); ++i) {
+                    ZB_TRY(pw_conv_run(ctx, parts[i], pl->ptr(x), xd == ZANT_U8, (const int8_t*)pl->aux(aws[i]), (const float*)pl->aux(am) + at, (const int32_t*)pl->aux(abs[i]),
+                                       (uint8_t*)pl->ptr(y) + (size_t)at * g.H * g.W, yd == ZANT_U8, rq_of(), finite, ac >= 0 ? (const int32_t*)pl->aux(ac) + at : nullptr));
+                    at += parts[i].a.M;
+                }
+                return (int32_t)ZANT_OK;
+            });
+            return ZANT_OK;
+        }
         push(std::string(stem ? "QLinearConv(tc-stem)" : "QLinearConv(tc-pointwise)") + tail, [=]() {
             if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");
             return pw_conv_run(ctx, pwp, pl->ptr(x), xd == ZANT_U8, (const int8_t*)pl->aux(aw), (const float*)pl->aux(am),

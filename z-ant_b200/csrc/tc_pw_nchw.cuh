@@ -58,6 +58,7 @@ namespace zb {
 struct PwConvArgs {
     const uint8_t* x; uint8_t* y; const int8_t* w; const float* mult; const int32_t* bias;
     int N, C, M, HW;
+    int y_planes;         // planes of an image in y (more than M when this launch writes a part of the filters)
     int k_steps;          // K steps of 32 channels (C rounded up)
     int KS;               // K steps per stage (a stage holds KS * 32 channels)
     int n_px;             // pixels per tile: a multiple of 16, at most 256
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
             ptx::tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 256);
             uint8_t* sOut = sOut0 + ((a.outs == 2 && (tile_it & 1)) ? a.out_stride : 0);
-            uint8_t* yrow = a.y + ((size_t)img * a.M + (size_t)m) * a.HW + p0;
+            uint8_t* yrow = a.y + ((size_t)img * a.y_planes + (size_t)m) * a.HW + p0;
             // 16 accumulators -> four packed words
             auto requant16 = [&](const uint32_t (&v)[16], uint32_t* pk) {
                 if constexpr (LEAN) {
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
                 uint32_t pk[8], rr[ADD ? 8 : 1];
                 if constexpr (ADD) {
                     const int c0 = ch * 32;
-                    const uint8_t* r = add.res + ((size_t)img * a.M + (size_t)m) * a.HW + p0 + c0;
+                    const uint8_t* r = add.res + ((size_t)img * a.y_planes + (size_t)m) * a.HW + p0 + c0;
                     if (a.mode != 1) {
                         uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
                         if (live && c0 < n_valid) r0 = __ldg(reinterpret_cast<const uint4*>(r));
@@ -575,7 +576,7 @@ __global__ void __launch_bounds__(kPwThreads, 1) tc_pw_nchw_kernel(const __grid_
                 // the staged block [rows_here][HW] is the image's contiguous run of these filters' planes
                 ptx::fence_proxy_async_smem();
                 ptx::named_barrier_sync(1, n_epi);
-                uint8_t* dst = a.y + ((size_t)img * a.M + (size_t)mt * 128) * a.HW;
+                uint8_t* dst = a.y + ((size_t)img * a.y_planes + (size_t)mt * 128) * a.HW;
                 const int bytes = rows_here * a.HW;
                 if (a.bulk_out) {
                     if (leader) bulk_s2g(dst, ptx::smem_u32(sOut), (uint32_t)bytes);
@@ -616,7 +617,7 @@ inline bool pw_conv_plan(const ConvGeom& g, bool w_zp_all_zero, int sm_count, Pw
     if ((long long)g.N * hw < 256) return false;
     PwConvArgs& a = p.a;
     a = PwConvArgs{};
-    a.N = g.N; a.C = g.C; a.M = g.M; a.HW = (int)hw;
+    a.N = g.N; a.C = g.C; a.M = a.y_planes = g.M; a.HW = (int)hw;
     a.k_steps = (g.C + 31) / 32;
     a.KS = a.k_steps >= 2 ? 2 : 1;
     a.G = 1; a.m_pad = 128; a.a_steps = a.k_steps;
@@ -671,6 +672,36 @@ inline bool pw_conv_plan(const ConvGeom& g, bool w_zp_all_zero, int sm_count, Pw
     return true;
 }
 
+// Filters that do not fill their last tile of 128 lanes (96, 144, 192: the expansions of mobile networks) in parts: the whole tiles, and
+// the rest in the group form, of 64 and of up to 64 filters, whose lanes all have work; each part reads the input again.  The epilogue
+// bounds the kernel at 3300 lane outputs per ns (16 -> 96 filters on 112 x 112, batch 1024: 1.64 G lane outputs, a quarter of them of
+// filters that do not exist, in 497 us), the input and output move at 6.4 KB per ns; a part costs a launch, about 4 us.  Returns the parts'
+// plans in order, empty when one launch is the better choice.
+inline std::vector<PwConvPlan> pw_conv_parts(const ConvGeom& g, bool w_zp_all_zero, int sm_count, const PwConvPlan& whole) {
+    std::vector<PwConvPlan> parts;
+    const int rest = g.M % 128;
+    if (whole.a.mode != 0 || whole.a.G != 1 || rest == 0) return parts;
+    std::vector<int> sizes;
+    if (g.M >= 128) sizes.push_back(g.M - rest);
+    if (rest > 64) sizes.push_back(64);
+    if (rest > 96) return parts;                             // a tile of more than 96 filters is full enough
+    sizes.push_back(rest > 64 ? rest - 64 : rest);
+    const double px = (double)g.N * g.H * g.W;
+    auto us = [&](double lanes, double m) { return std::max(px * lanes / 3.3e6, px * (g.C + m) / 6.4e6) + 4.0; };
+    double split = 0.0;
+    for (int m : sizes) {
+        ConvGeom part = g;
+        part.M = m;
+        PwConvPlan p;
+        if (!pw_conv_plan(part, w_zp_all_zero, sm_count, p) || p.a.mode != 0 || (m <= 64 && p.a.G == 1)) return {};
+        p.a.y_planes = g.M;
+        parts.push_back(p);
+        split += us(m <= 16 ? 16.0 : (m <= 32 ? 32.0 : (m <= 64 ? 64.0 : m)), m);
+    }
+    if (split > 0.95 * us((double)whole.m_tiles * 128, g.M)) parts.clear();
+    return parts;
+}
+
 // 3x3 stems (at most three input channels, stride 1 or 2, at most 64 filters) on the same kernel: the patches of the input are
 // written as the B operand in shared memory (mode 2).  False when the shape is not taken.  The weights ([M][cin][3][3]) go
 // through pw_conv_prepare as [M][9 * cin].
@@ -687,7 +718,7 @@ inline bool pw_stem_plan(const ConvGeom& g, bool w_zp_all_zero, int x_zp, int sm
     PwConvArgs& a = p.a;
     a = PwConvArgs{};
     a.mode = 2;
-    a.N = g.N; a.C = 9 * g.C; a.M = g.M; a.HW = (int)hw;
+    a.N = g.N; a.C = 9 * g.C; a.M = a.y_planes = g.M; a.HW = (int)hw;
     a.cin = g.C; a.ih = g.H; a.iw = g.W; a.oh = g.OH; a.ow = g.OW; a.cs = g.sh; a.pt = g.pt; a.pl = g.pl;
     a.pad_word = 0x01010101u * (uint32_t)(x_zp & 255);
     // p / ow by one multiplication: exact while p * ow < 2^32, p < oh * ow
