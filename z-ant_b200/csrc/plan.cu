@@ -1787,6 +1787,19 @@ static bool nh_parse(const zant_plan* pl, const ChainCtx& c, size_t i, NhGroup& 
         const int b = opt_in(n, 2);
         if (b >= 0 && (T(b).dtype != ZANT_F32 || T(b).bytes != (size_t)g.M * 4)) return false;
     }
+    // the input has to come channels-last from somewhere, or be a first layer's (the search for a tiling below takes 75 us a shape)
+    if (T(x).shape[1] > 4) {
+        bool from = false;
+        for (size_t k = 0; k < i; ++k) {
+            const PlanNode& p = pl->nodes[k];
+            bool makes = false;
+            for (int id : p.out) makes = makes || id == x;
+            if (!makes) continue;
+            const bool conv = p.op == ZANT_OP_QLINEAR_CONV || p.op == ZANT_OP_CONV;
+            from = (conv && p.a.group <= 1) || p.op == ZANT_OP_RELU || p.op == ZANT_OP_LEAKY_RELU || p.op == ZANT_OP_CLIP || p.op == ZANT_OP_MAXPOOL || p.op == ZANT_OP_RESIZE || p.op == ZANT_OP_CONCAT;
+        }
+        if (!from) return false;
+    }
     q = NhGroup{};
     q.first = i; q.x = x;
     size_t j = i + 1;
