@@ -745,7 +745,7 @@ int32_t zant_b200_qlinearconv_nhwc(zant_ctx* ctx, int32_t x_dtype, const void* x
     ZB_TRY(s.commit());
     ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
     ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, weight_blocks_max_product(mult, bias, true, (long long)g.Cg * g.KH * g.KW)));
+                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, weight_blocks_max_product(mult, bias, true, g.M, (long long)g.Cg * g.KH * g.KW)));
     return s.finish();
 }
 
@@ -821,7 +821,7 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
         ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation},
-                           weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, (long long)g.Cg * g.KH * g.KW)));
+                           weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, g.M, (long long)g.Cg * g.KH * g.KW)));
         return s.finish();
     }
     if (host_consts && qdwconv_eligible(g, wz_zero) && (!is_device_ptr(x) || qdwconv_ptr_ok(x)) && (!is_device_ptr(y) || qdwconv_ptr_ok(y))) {

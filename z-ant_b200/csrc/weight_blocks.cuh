@@ -116,11 +116,12 @@ inline int32_t run_weight_blocks(zant_ctx* ctx, WBlockArgs a, const int8_t* w, c
     return e == cudaSuccess ? ZANT_OK : fail(ZANT_E_CUDA, "launch of weight_blocks_kernel failed: %s", cudaGetErrorString(e));
 }
 
-// |accumulator * multiplier| <= this, for tc_conv_run / tc_conv_nhwc_run (tc_conv_max_product without the folded bias, which only
-// the device knows): |x - x_zp| <= 255 for every activation and |x_zp| <= 255 for the folded zero point.
-inline double weight_blocks_max_product(const std::vector<float>& mult, const int32_t* bias_host, bool bias_known, long long K) {
+// |accumulator * multiplier| <= this over the M filters, for tc_conv_run / tc_conv_nhwc_run (tc_conv_max_product without the folded
+// bias, which only the device knows): |x - x_zp| <= 255 for every activation and |x_zp| <= 255 for the folded zero point.  `mult` may
+// be padded behind the filters; `bias_host` is the caller's array of M values.
+inline double weight_blocks_max_product(const std::vector<float>& mult, const int32_t* bias_host, bool bias_known, int M, long long K) {
     double worst = 0.0;
-    for (size_t m = 0; m < mult.size(); ++m) {
+    for (int m = 0; m < M; ++m) {
         if (!std::isfinite(mult[m])) return INFINITY;
         const double b = bias_host ? std::fabs((double)bias_host[m]) : (bias_known ? 0.0 : 2147483648.0);
         worst = std::max(worst, (2.0 * 255.0 * 128.0 * (double)K + b) * std::fabs((double)mult[m]));
