@@ -1898,7 +1898,8 @@ static void nh_layout(zant_plan* pl) {
                 NhGroup& q = pl->nh_groups[gi];
                 if (i != q.first) continue;
                 for (int id : q.interior) lay[id] = 0;                             // interior: no layout of its own
-                if (lay[q.y] && T(q.y).shape[1] % 16 != 0) off(q.y);               // the epilogue stores 16 channels at a time
+                // the epilogue stores 16 channels at a time, and dequantised values as NCHW only
+                if (T(q.y).shape[1] % 16 != 0 || q.dequant >= 0) off(q.y);
                 const bool in_ok = lay[q.x] || (first_layer(q.x) && lay[q.y]);
                 // an NCHW result cannot be upsampled in place, and a first layer pays for its conversion only in front of more such layers
                 if (!in_ok || (!lay[q.y] && q.up2)) { q.on = false; changed = true; off(q.x); off(q.y); }
