@@ -94,9 +94,18 @@ inline HostStage* host_stage(zant_ctx* ctx) {
     return ctx->stage;
 }
 
-// Host buffer -> device, ordered on the context's stream; `src` may be changed as soon as this returns.
+// Work enqueued now becomes part of a CUDA graph that the caller is capturing on the context's stream.
+inline bool stream_capturing(zant_ctx* ctx) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &s) != cudaSuccess) { cudaGetLastError(); return true; }
+    return s != cudaStreamCaptureStatusNone;
+}
+
+// Host buffer -> device, ordered on the context's stream; `src` may be changed as soon as this returns.  (In a capture the copy
+// becomes a node that reads `src` at every replay; the ring's slots would hold something else by then.)
 inline cudaError_t copy_to_device(zant_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return cudaSuccess;
+    if (stream_capturing(ctx)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (HostStage* st = host_stage(ctx)) return st->to_device(dst, src, bytes, ctx->stream);
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);      // no page-locked memory to be had
 }
@@ -105,6 +114,7 @@ inline cudaError_t copy_to_device(zant_ctx* ctx, void* dst, const void* src, siz
 // they give up; a non-zero value is reported once and cleared.  With `host_dst` the same wait also brings a result back
 // (`bytes` from device memory): one synchronisation for both.
 inline int32_t drain_and_check_status(zant_ctx* ctx, void* host_dst = nullptr, const void* dev_src = nullptr, size_t bytes = 0) {
+    if (stream_capturing(ctx)) return fail(ZANT_E_CUDA, "the context's stream is being captured: it cannot be waited for");
     int h = 0;
     char* slot = nullptr;
     if (ctx->stage || (host_dst && bytes && bytes + 256 <= HostStage::kSlot)) {
@@ -210,6 +220,8 @@ class Stager {
         size_t total = 0;
         for (auto& s : slots_) if (s.staged) { s.off = total; total += align_up(s.bytes ? s.bytes : 1, kArenaAlign); }
         if (total) {
+            // the arena is the next call's as soon as this one returns: a replay would find that call's data there
+            if (stream_capturing(ctx_)) return fail(ZANT_E_CUDA, "a call with host buffers or a workspace cannot be captured into a CUDA graph");
             int32_t st = arena_reserve(ctx_, total);
             if (st != ZANT_OK) return st;
             ctx_->arena_used = total;
