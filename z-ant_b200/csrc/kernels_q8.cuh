@@ -302,9 +302,11 @@ template <bool U8>
 inline QAddTail qadd_tail(float a_s, int a_zp, float b_s, int b_zp, float y_s, int y_zp, int act) {
     QAddTail t{};
     t.ra = a_s / y_s; t.rb = b_s / y_s;
-    t.ca = 8388608.0f + (float)(a_zp + (U8 ? 0 : 128)); t.cb = 8388608.0f + (float)(b_zp + (U8 ? 0 : 128));
+    t.ca = 8388608.0f + (float)a_zp + (U8 ? 0.0f : 128.0f); t.cb = 8388608.0f + (float)b_zp + (U8 ? 0.0f : 128.0f);
     const double eps = 8.0 / 16777216.0 * 255.0 * ((double)std::fabs(t.ra) + (double)std::fabs(t.rb));
-    const bool usable = a_s > 1e-30f && b_s > 1e-30f && y_s > 1e-30f && a_s < 1e30f && b_s < 1e30f && y_s < 1e30f && eps < 0.01 && t.ra > 1e-30f && t.rb > 1e-30f;
+    // (the entry point takes any zero points: outside the type's range a difference exceeds 255)
+    const int z_lo = U8 ? 0 : -128, z_hi = U8 ? 255 : 127;
+    const bool usable = a_zp >= z_lo && a_zp <= z_hi && b_zp >= z_lo && b_zp <= z_hi && a_s > 1e-30f && b_s > 1e-30f && y_s > 1e-30f && a_s < 1e30f && b_s < 1e30f && y_s < 1e30f && eps < 0.01 && t.ra > 1e-30f && t.rb > 1e-30f;
     t.lim = usable ? (float)(0.4999999 - eps) : -1.0f;
     t.y_off = y_zp - 0x4b400000;
     const int t_lo = U8 ? 0 : -128, t_hi = U8 ? 255 : 127;
