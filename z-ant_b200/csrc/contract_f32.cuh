@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(256) contract_f32_few(const __grid_constant__ 
 __global__ void __launch_bounds__(256) transpose_pad_f32(const float* __restrict__ w, float* __restrict__ wt, int M, int K, int N4) {
     ptx::grid_start();
     __shared__ float tile[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, k0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, k0 = blockIdx.y * 32, m0 = blockIdx.x * 32;
     for (int r = ty; r < 32; r += 8) tile[r][tx] = (m0 + r < M && k0 + tx < K) ? __ldg(w + (size_t)(m0 + r) * K + k0 + tx) : 0.0f;
     __syncthreads();
     for (int r = ty; r < 32; r += 8)

@@ -21,12 +21,11 @@ struct ContractFusion { int act = CT_ACT_NONE; float slope = 0.0f; const float* 
 template <bool CONV, bool POOL, int BM, int BN, int TM, int TN>
 inline int32_t launch_contract_tile(zant_ctx* ctx, const ContractArgs& p) {
     ZB_SMEM_ATTR(ctx, (contract_f32_tile<CONV, POOL, BM, BN, TM, TN>), 122880);
-    const dim3 grid((unsigned)((p.M + BM - 1) / BM), (unsigned)((p.N + BN - 1) / BN));
+    const dim3 grid(((unsigned)p.M + BM - 1) / BM, ((unsigned)p.N + BN - 1) / BN);
     // Up to three tiles per SM: ask for so much shared memory that no SM takes more than its share.  A grid that starts while
     // its predecessor drains would otherwise pile up on the SMs that are free first (128 tiles, two to an SM: 290 -> 540 us).
     const long long share = ((long long)grid.x * grid.y + ctx->sm_count - 1) / ctx->sm_count;
     const size_t smem = std::max<size_t>(contract_smem<BM, BN>(), share == 1 ? 122880 : (share == 2 ? 81920 : (share == 3 ? 61440 : 0)));
-    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
     launch(ctx, contract_f32_tile<CONV, POOL, BM, BN, TM, TN>, grid, (BM / TM) * (BN / TN), smem, p);
     return check_launch(ctx, "contract_f32_tile");
 }
@@ -38,12 +37,14 @@ inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     p.neg_zero = 0x8000000080000000ull;
     struct Shape { int bm, bn; double rate; };
     static const Shape shapes[] = {{128, 128, 1.0}, {128, 64, 0.85}, {128, 32, 0.75}, {128, 16, 0.5}, {32, 32, 0.4}, {CF_BM, CF_BN, 0.12}};
-    int best = 0; double cost = 1e300;
+    int best = -1; double cost = 1e300;
     for (int i = 0; i < 6; ++i) {
-        const double tiles = std::ceil((double)p.M / shapes[i].bm) * std::ceil((double)p.N / shapes[i].bn);
-        const double c = std::ceil(tiles / ctx->sm_count) * shapes[i].bm * shapes[i].bn / shapes[i].rate;
+        const double row_tiles = std::ceil((double)p.M / shapes[i].bm), col_tiles = std::ceil((double)p.N / shapes[i].bn);
+        if (col_tiles > 65535.0 || row_tiles * shapes[i].bm > 2147483648.0) continue;        // (grid.y; a tile's rows are ints)
+        const double c = std::ceil(row_tiles * col_tiles / ctx->sm_count) * shapes[i].bm * shapes[i].bn / shapes[i].rate;
         if (c < cost) { cost = c; best = i; }
     }
+    if (best < 0) return fail(ZANT_E_TOO_LARGE, "too many output columns");
     switch (best) {
         case 0: return launch_contract_tile<CONV, POOL, 128, 128, 8, 8>(ctx, p);
         case 1: return launch_contract_tile<CONV, POOL, 128, 64, 8, 4>(ctx, p);
@@ -54,15 +55,14 @@ inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     }
     constexpr int smem = contract_few_smem();
     ZB_SMEM_ATTR(ctx, (contract_f32_few<CONV, POOL>), smem);
-    const dim3 grid((unsigned)((p.M + CF_BM - 1) / CF_BM), (unsigned)((p.N + CF_BN - 1) / CF_BN));
-    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output columns");
+    const dim3 grid(((unsigned)p.M + CF_BM - 1) / CF_BM, ((unsigned)p.N + CF_BN - 1) / CF_BN);
     launch(ctx, contract_f32_few<CONV, POOL>, grid, 256, smem, p);
     return check_launch(ctx, "contract_f32_few");
 }
 
 inline int32_t run_transpose_pad_f32(zant_ctx* ctx, const float* w, float* wt, int M, int K, int N4) {
-    const dim3 grid((unsigned)((K + 31) / 32), (unsigned)((N4 + 31) / 32));
-    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many output channels");
+    const dim3 grid((unsigned)((N4 + 31) / 32), (unsigned)((K + 31) / 32));
+    if (grid.y > 65535) return fail(ZANT_E_TOO_LARGE, "too many taps");
     launch(ctx, transpose_pad_f32, grid, 256, 0, w, wt, M, K, N4);
     return check_launch(ctx, "transpose_pad_f32");
 }

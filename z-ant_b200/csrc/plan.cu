@@ -842,7 +842,7 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
             // exact path; constant weights are transposed once to [K][filters], the order the kernel's slabs have
             const int K = g.C * g.KH * g.KW, N4 = (g.M + 3) / 4 * 4;
             int at = -1;
-            if (T(w).is_const && (long long)K * N4 <= (1LL << 28)) {
+            if (T(w).is_const && (long long)K * N4 <= (1LL << 28) && K <= 65535 * 32) {
                 at = pl->add_scratch((size_t)K * N4 * 4);
                 pl->init_steps.push_back([=]() { return run_transpose_pad_f32(ctx, pl->p<float>(w), (float*)pl->scratch(at), g.M, K, N4); });
             }
