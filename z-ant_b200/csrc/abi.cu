@@ -892,14 +892,16 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
     }
     if (host_consts && small_gemm_eligible(g, wz_zero)) {
         // few output positions: warp-level MMAs, K split over the warps of many small CTAs
-        SmallGemmPrep prep;
-        const size_t taps = (size_t)g.KH * g.KW;
-        small_gemm_prepare(g, w, (size_t)g.Cg * taps, taps, 1, mult.data(), bias, x_zp, ctx->sm_count, prep);
+        const SmallGemmPlan sg = small_gemm_plan(g, ctx->sm_count);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(prep.bias.data(), prep.bias.size() * 4);
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+        const int iwf = s.scratch(sg.w_bytes), ibf = s.scratch(x_zp != 0 ? (size_t)g.M * 4 : 0);
         ZB_TRY(s.commit());
-        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+        const uint64_t launched = ctx->launches;
+        ZB_TRY(run_small_gemm_weights(ctx, g, sg, false, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), x_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
+        ctx->launches = launched;                       // (not operator launches)
+        ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(x_zp != 0 ? ibf : ib),
                               s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
         return s.finish();
     }
@@ -966,13 +968,16 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
         ConvGeom g{};
         g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
         g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
-        SmallGemmPrep prep;
-        small_gemm_prepare(g, b, 1, N, 0, mult.data(), bias, a_zp, ctx->sm_count, prep);
+        const SmallGemmPlan sg = small_gemm_plan(g, ctx->sm_count);
         Stager s(ctx);
         const int ix = s.in(a, M * K), iy = s.out(y, M * N);
-        const int iw = s.in(prep.wfrag.data(), prep.wfrag.size() * 4), im = s.in(prep.mult.data(), prep.mult.size() * 4), ibb = s.in(prep.bias.data(), prep.bias.size() * 4);
+        const int iw = s.in(b, K * N), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, N * 4);
+        const int iwf = s.scratch(sg.w_bytes), ibf = s.scratch(a_zp != 0 ? N * 4 : 0);
         ZB_TRY(s.commit());
-        ZB_TRY(run_small_gemm(ctx, g, prep, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<uint32_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+        const uint64_t launched = ctx->launches;
+        ZB_TRY(run_small_gemm_weights(ctx, g, sg, true, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), a_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
+        ctx->launches = launched;                       // (not operator launches)
+        ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(a_zp != 0 ? ibf : ib),
                               s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
         return s.finish();
     }

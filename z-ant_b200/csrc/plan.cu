@@ -760,23 +760,20 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
     }
     if (const_bias && small_gemm_eligible(g, wz_zero)) {
         // few output positions: warp-level MMAs, K split over the warps of many small CTAs
-        auto prep = std::make_shared<SmallGemmPrep>();
-        const size_t taps = (size_t)g.KH * g.KW;
-        small_gemm_prepare(g, (const int8_t*)T(w).host.data(), (size_t)g.Cg * taps, taps, 1, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, ctx->sm_count, *prep);
-        const int aw = pl->add_aux(prep->wfrag.data(), prep->wfrag.size() * 4), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4), ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
-        prep->wfrag.clear(); prep->wfrag.shrink_to_fit();
+        const SmallGemmPlan sg = small_gemm_plan(g, ctx->sm_count);
+        const int aw = pl->add_scratch(sg.w_bytes), am = pl->add_aux(mult.data(), mult.size() * 4), ab = xzp != 0 ? pl->add_scratch((size_t)g.M * 4) : -1;
+        auto bias_of = [=]() { return ab >= 0 ? (int32_t*)pl->scratch(ab) : pl->p<int32_t>(b); };
+        pl->init_steps.push_back([=]() { return run_small_gemm_weights(ctx, g, sg, false, pl->p<int8_t>(w), pl->p<int32_t>(b), xzp, pl->scratch(aw), bias_of()); });
         if (fz.add_node >= 0 && yd == ZANT_I8) {
             fz.add_done = true;
             push("QLinearConv" + tail + "+QLinearAdd", [=]() {
                 const QAddTail add = add_of();
-                return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
-                                      pl->ptr(y_sum), false, rq_of(), &add);
+                return run_small_gemm(ctx, g, sg, pl->ptr(x), xd == ZANT_U8, xzp, pl->scratch(aw), (const float*)pl->aux(am), bias_of(), pl->ptr(y_sum), false, rq_of(), &add);
             });
             return ZANT_OK;
         }
         push("QLinearConv" + tail, [=]() {
-            return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
-                                  pl->ptr(y), yd == ZANT_U8, rq_of());
+            return run_small_gemm(ctx, g, sg, pl->ptr(x), xd == ZANT_U8, xzp, pl->scratch(aw), (const float*)pl->aux(am), bias_of(), pl->ptr(y), yd == ZANT_U8, rq_of());
         });
         return ZANT_OK;
     }
@@ -1175,14 +1172,12 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                 g.N = (int)M; g.C = (int)K; g.H = g.W = 1; g.M = (int)N; g.Cg = (int)K; g.KH = g.KW = 1;
                 g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
                 if (small_gemm_eligible(g, bz_zero)) {
-                    auto prep = std::make_shared<SmallGemmPrep>();
-                    small_gemm_prepare(g, (const int8_t*)T(w).host.data(), 1, N, 0, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, ctx->sm_count, *prep);
-                    const int aw = pl->add_aux(prep->wfrag.data(), prep->wfrag.size() * 4), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4);
-                    const int ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
-                    prep->wfrag.clear(); prep->wfrag.shrink_to_fit();
+                    const SmallGemmPlan sg = small_gemm_plan(g, ctx->sm_count);
+                    const int aw = pl->add_scratch(sg.w_bytes), am = pl->add_aux(mult.data(), mult.size() * 4), ab = xzp != 0 ? pl->add_scratch(N * 4) : -1;
+                    auto bias_of = [=]() { return ab >= 0 ? (int32_t*)pl->scratch(ab) : pl->p<int32_t>(b); };
+                    pl->init_steps.push_back([=]() { return run_small_gemm_weights(ctx, g, sg, true, pl->p<int8_t>(w), pl->p<int32_t>(b), xzp, pl->scratch(aw), bias_of()); });
                     push("QLinearMatMul", [=]() {
-                        return run_small_gemm(ctx, g, *prep, pl->ptr(x), xd == ZANT_U8, xzp, (const uint32_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab),
-                                              pl->ptr(y), yd == ZANT_U8, rq);
+                        return run_small_gemm(ctx, g, sg, pl->ptr(x), xd == ZANT_U8, xzp, pl->scratch(aw), (const float*)pl->aux(am), bias_of(), pl->ptr(y), yd == ZANT_U8, rq);
                     });
                     return ZANT_OK;
                 }

@@ -21,8 +21,7 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <cstring>
-#include <vector>
+#include <type_traits>
 
 #include "context.cuh"
 #include "geometry.hpp"
@@ -33,7 +32,7 @@ namespace zb {
 
 struct SmallGemmArgs {
     const uint8_t* x; const uint4* w; void* y;
-    const float* mult; const int32_t* bias;      // bias has -x_zp * sum(w) folded in
+    const float* mult; const int32_t* bias;      // bias has -x_zp * sum(w) folded in; null: zeros
     ConvGeom g;
     int P, OHW;            // output positions in all, per image
     int c_steps;           // K steps of 32 channels per tap
@@ -202,7 +201,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const S
             for (int j = 0; j < 4; ++j) {
                 const int m = m0 + r0 + j;
                 if (m >= g.M) break;
-                int s = __ldg(a.bias + m);
+                int s = a.bias ? __ldg(a.bias + m) : 0;
                 for (int w = 0; w < warps; ++w) s += red[w * (MT * 16 * LD) + (r0 + j) * LD + col];
                 int q = requant_one<YU8>(s, __ldg(a.mult + m), a.rq);
                 if (!YU8 && a.add.res) q = (int)(int8_t)qadd_word<false>((uint32_t)__ldg(a.add.res + (size_t)p * g.M + m), (uint32_t)(q & 255), a.add);
@@ -212,7 +211,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const S
             // four positions of one filter
             const int row = u >> 3, c4 = (u & 7) * 4, m = m0 + row, p = p0 + c4;
             if (m >= g.M || p >= a.P) continue;
-            const int bs = __ldg(a.bias + m);
+            const int bs = a.bias ? __ldg(a.bias + m) : 0;
             const float mu = __ldg(a.mult + m);
             int s[4] = {bs, bs, bs, bs};
             for (int w = 0; w < warps; ++w) {
@@ -242,12 +241,68 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_q8_kernel(const S
     }
 }
 
+// ---------------------------------------------------------------------------- weights
+// Fragment order, on the device: [16-filter tile][K step][32 lanes][4 words], a thread per lane and step.  The weight of (filter, channel,
+// tap) is w[m * sm + c * sc + tap * st] (a convolution's [M][C][KH][KW], or a matrix [K][N]).  A call brings its weights along every time:
+// shuffled by the host, a 4096 x 4096 matrix took 13 of the call's 13.2 ms.
+struct SmallWeightArgs { const int8_t* w; uint4* out; size_t sm, sc, st; int M, C, contiguous, c_steps, k_steps; long long units; };
+__global__ void __launch_bounds__(256) small_gemm_weights_k(const __grid_constant__ SmallWeightArgs a) {
+    ptx::grid_start();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.units; i += (long long)gridDim.x * blockDim.x) {
+        const int lane = (int)(i & 31), gq = lane >> 2, tq = lane & 3;
+        const long long t = i >> 5;
+        const int s = (int)(t % a.k_steps), tile = (int)(t / a.k_steps);
+        const int tap = a.contiguous ? 0 : s / a.c_steps;
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                          // register j: filter gq + 8 * (j & 1), half j >> 1 of the step
+            const int m = tile * 16 + gq + (j & 1) * 8, h = j >> 1;
+            const int c0 = 4 * (a.contiguous ? (s >> 1) * 16 + tq * 4 + (s & 1) * 2 + h : (s - tap * a.c_steps) * 8 + h * 4 + tq);
+            v[j] = 0u;
+            if (m < a.M) {
+                const int8_t* src = a.w + (size_t)m * a.sm + (size_t)tap * a.st;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (c0 + k < a.C) v[j] |= (uint32_t)(uint8_t)__ldg(src + (size_t)(c0 + k) * a.sc) << (8 * k);
+            }
+        }
+        a.out[i] = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// bias - x_zp * (sum of the filter's weights), element k of filter m at w[m * sm + k * sk]: 32 filters a block, 8 threads a filter that
+// walk K (sm == 1: the filters are the contiguous side), or a warp a filter.
+__global__ void __launch_bounds__(256) small_gemm_bias_k(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int32_t* __restrict__ out, int M, int K, size_t sm, size_t sk, int x_zp) {
+    ptx::grid_start();
+    __shared__ int part[256];
+    const int tid = threadIdx.x;
+    if (sm == 1) {
+        const int m = blockIdx.x * 32 + (tid & 31);
+        int s = 0;
+        if (m < M) for (int k = tid >> 5; k < K; k += 8) s += __ldg(w + (size_t)k * sk + m);
+        part[tid] = s;
+        __syncthreads();
+        if (tid < 32 && m < M) {
+            s = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s += part[j * 32 + tid];
+            out[m] = (bias ? __ldg(bias + m) : 0) - x_zp * s;
+        }
+    } else {
+        for (int m = blockIdx.x * 32 + (tid >> 5); m < min(M, (int)blockIdx.x * 32 + 32); m += 8) {
+            int s = 0;
+            for (int k = tid & 31; k < K; k += 32) s += __ldg(w + (size_t)m * sm + (size_t)k * sk);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if ((tid & 31) == 0) out[m] = (bias ? __ldg(bias + m) : 0) - x_zp * s;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------- host side
-struct SmallGemmPrep {
+struct SmallGemmPlan {
     int path = 2, MT = 1, c_steps = 0, k_steps = 0, warps = 1;
-    std::vector<uint32_t> wfrag;      // [16-filter tile][K step][32 lanes][4 words]
-    std::vector<float> mult;
-    std::vector<int32_t> bias;
+    size_t w_bytes = 0;               // weights in fragment order
 };
 
 inline bool small_gemm_eligible(const ConvGeom& g, bool w_zp_all_zero) {
@@ -255,8 +310,8 @@ inline bool small_gemm_eligible(const ConvGeom& g, bool w_zp_all_zero) {
     return g.G == 1 && w_zp_all_zero && P > 0 && P < 256 && (long long)g.Cg * g.KH * g.KW <= (1 << 20) && g.M <= (1 << 20);
 }
 
-// `w`: weight of (filter, channel, tap) at w[m * sm + c * sc + tap * st] (a convolution's [M][C][KH][KW], or a matrix [K][N]).
-inline void small_gemm_prepare(const ConvGeom& g, const int8_t* w, size_t sm, size_t sc, size_t st, const float* mult, const int32_t* bias, int x_zp, int sm_count, SmallGemmPrep& p) {
+inline SmallGemmPlan small_gemm_plan(const ConvGeom& g, int sm_count) {
+    SmallGemmPlan p;
     const int taps = g.KH * g.KW;
     const bool pointwise = taps == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
     p.path = pointwise && g.H * g.W == 1 ? 0 : (pointwise && (g.H * g.W) % 4 == 0 ? 1 : 2);
@@ -267,30 +322,27 @@ inline void small_gemm_prepare(const ConvGeom& g, const int8_t* w, size_t sm, si
     p.MT = (long long)((g.M + 15) / 16) * cols > 2LL * sm_count ? 2 : 1;
     p.warps = std::max(1, std::min(kSmallWarps, p.path == 0 ? p.k_steps / 2 : p.k_steps));
     const int tiles = (g.M + 16 * p.MT - 1) / (16 * p.MT) * p.MT;
-    p.wfrag.assign((size_t)tiles * p.k_steps * 128, 0u);
-    p.mult.assign(mult, mult + g.M);
-    p.bias.resize(g.M);
-    std::vector<int32_t> sums((size_t)g.M, 0);
-    // four channels of a filter are one register word; the loop runs along the weight tensor's contiguous side
-    auto put = [&](int m, int tap, int c4) {
-        const int8_t* src = w + (size_t)m * sm + (size_t)c4 * 4 * sc + (size_t)tap * st;
-        const int n = std::min(4, g.Cg - c4 * 4);
-        uint32_t word = 0;
-        int sum = 0;
-        for (int i = 0; i < n; ++i) { const int8_t v = src[i * sc]; word |= (uint32_t)(uint8_t)v << (8 * i); sum += v; }
-        sums[m] += sum;
-        // K step, lane column and half of the step of channels 4 * c4 .. 4 * c4 + 3
-        const int s = p.path == 0 ? c4 / 16 * 2 + (c4 >> 1 & 1) : tap * p.c_steps + c4 / 8;
-        const int tq = p.path == 0 ? (c4 & 15) >> 2 : c4 & 3, h = p.path == 0 ? c4 & 1 : (c4 & 7) >> 2;
-        p.wfrag[(((size_t)(m >> 4) * p.k_steps + s) * 32 + (m & 7) * 4 + tq) * 4 + h * 2 + (m >> 3 & 1)] = word;
-    };
-    const int c4s = (g.Cg + 3) / 4;
-    if (sm == 1) for (int c4 = 0; c4 < c4s; ++c4) for (int m = 0; m < g.M; ++m) put(m, 0, c4);
-    else for (int m = 0; m < g.M; ++m) for (int tap = 0; tap < taps; ++tap) for (int c4 = 0; c4 < c4s; ++c4) put(m, tap, c4);
-    for (int m = 0; m < g.M; ++m) p.bias[m] = (bias ? bias[m] : 0) - x_zp * sums[m];
+    p.w_bytes = (size_t)tiles * p.k_steps * 512;
+    return p;
 }
 
-inline int32_t run_small_gemm(zant_ctx* ctx, const ConvGeom& g, const SmallGemmPrep& p, const void* x, bool x_u8, int x_zp, const uint32_t* w_dev, const float* mult_dev,
+// `matrix`: w is [K][N] (g.Cg rows, g.M columns).  With a zero point `bias_out` (g.M values) receives the folded bias; without one it
+// is not written and the tensor's own bias goes to run_small_gemm.
+inline int32_t run_small_gemm_weights(zant_ctx* ctx, const ConvGeom& g, const SmallGemmPlan& p, bool matrix, const int8_t* w, const int32_t* bias, int x_zp, void* out, int32_t* bias_out) {
+    const size_t taps = (size_t)g.KH * g.KW;
+    SmallWeightArgs a{};
+    a.w = w; a.out = (uint4*)out; a.M = g.M; a.C = g.Cg; a.contiguous = p.path == 0 ? 1 : 0; a.c_steps = p.c_steps; a.k_steps = p.k_steps;
+    a.sm = matrix ? 1 : (size_t)g.Cg * taps; a.sc = matrix ? (size_t)g.M : taps; a.st = 1;
+    a.units = (long long)(p.w_bytes / 16);
+    launch(ctx, small_gemm_weights_k, grid_for((size_t)a.units, 256, ctx->sm_count), 256, 0, a);
+    ZB_TRY(check_launch(ctx, "small_gemm_weights_k"));
+    if (x_zp == 0) return ZANT_OK;
+    launch(ctx, small_gemm_bias_k, (unsigned)((g.M + 31) / 32), 256, 0, w, bias, bias_out, g.M, g.Cg * (int)taps, a.sm, matrix ? (size_t)g.M : (size_t)1, x_zp);
+    return check_launch(ctx, "small_gemm_bias_k");
+}
+
+// `w_dev`, `bias_dev`: as run_small_gemm_weights leaves them; `bias_dev` may be null.
+inline int32_t run_small_gemm(zant_ctx* ctx, const ConvGeom& g, const SmallGemmPlan& p, const void* x, bool x_u8, int x_zp, const void* w_dev, const float* mult_dev,
                               const int32_t* bias_dev, void* y, bool y_u8, const Requant& rq, const QAddTail* add = nullptr) {
     SmallGemmArgs a{};
     if (add) a.add = *add;
