@@ -149,7 +149,8 @@ int32_t zant_b200_ctx_set_tf32(zant_ctx* ctx, int32_t enable);
 int32_t zant_b200_ctx_get_tf32(zant_ctx* ctx);
 
 /* Caps the staging arena that host-pointer calls grow on demand (0 = no cap, the default).  A call
- * whose host buffers and workspace need more returns ZANT_E_ARENA_EXHAUSTED and changes nothing;
+ * whose host buffers and workspace need more returns ZANT_E_ARENA_EXHAUSTED and changes nothing
+ * (QLinearConv and QLinearMatMul run on a slower kernel without workspace where only that does not fit);
  * device-pointer calls and plans (which own their arena) are not affected.  No reference
  * counterpart: the reference allocates temporaries from the process heap. */
 int32_t zant_b200_ctx_set_arena_limit(zant_ctx* ctx, size_t max_bytes);

@@ -736,16 +736,32 @@ int32_t zant_b200_qlinearconv_nhwc(zant_ctx* ctx, int32_t x_dtype, const void* x
     if (w_zp) for (size_t i = 0; i < n_w_scale; ++i) wz_zero = wz_zero && w_zp[i] == 0;
     TcConvPlan tcp;
     if (!tc_conv_nhwc_plan(g, wz_zero, x_zp, tcp)) return fail(ZANT_E_UNSUPPORTED, "shape not taken by the channels-last QLinearConv kernel");
-    mult.resize(tcp.a.m_pad, 1.0f);
-    const WBlockArgs wb = weight_blocks_of(tcp, x_zp, true);
+    const Requant rq{y_scale, y_zp, activation};
+    {
+        std::vector<float> mp(mult);
+        mp.resize(tcp.a.m_pad, 1.0f);
+        const WBlockArgs wb = weight_blocks_of(tcp, x_zp, true);
+        Stager s(ctx);
+        const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
+        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+        const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                                    s.ptr<char>(iy), y_dtype == ZANT_U8, rq, weight_blocks_max_product(mult, bias, true, g.M, (long long)g.Cg * g.KH * g.KW)));
+            return s.finish();
+        }
+    }
+    // no room for the weights in both orders: blocked by the host
+    std::vector<int8_t> w_blk; std::vector<float> mp; std::vector<int32_t> bp;
+    tc_conv_nhwc_prepare(tcp, w, mult.data(), bias, x_zp, w_blk, mp, bp);
     Stager s(ctx);
     const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-    const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
-    const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
+    const int iw = s.in(w_blk.data(), w_blk.size()), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bp.data(), bp.size() * 4);
     ZB_TRY(s.commit());
-    ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
-    ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                            s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, weight_blocks_max_product(mult, bias, true, g.M, (long long)g.Cg * g.KH * g.KW)));
+    ZB_TRY(tc_conv_nhwc_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iw), s.ptr<float>(im), s.ptr<int32_t>(ib),
+                            s.ptr<char>(iy), y_dtype == ZANT_U8, rq, tc_conv_max_product(mp, bp, (long long)g.Cg * g.KH * g.KW)));
     return s.finish();
 }
 
@@ -773,6 +789,7 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
     bool wz_zero = true;
     for (int32_t v : wz) wz_zero = wz_zero && v == 0;
     const bool host_consts = !is_device_ptr(w) && !(bias && is_device_ptr(bias));
+    // the kernels in order of preference; one whose workspace finds no room in the arena leaves the call to the next, the last needs none
     PwConvPlan pwp;
     if ((!is_device_ptr(x) || pw_conv_ptr_ok(x, nullptr)) && (!is_device_ptr(y) || pw_conv_ptr_ok(nullptr, y)) &&
         (pw_stem_plan(g, wz_zero, x_zp, ctx->sm_count, pwp) || pw_conv_plan(g, wz_zero, ctx->sm_count, pwp))) {
@@ -788,11 +805,13 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int ic = capped ? s.in(caps.data(), caps.size() * 4) : -1;
         const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
-        ZB_TRY(s.commit());
-        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
-        ZB_TRY(pw_conv_run(ctx, pwp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                           s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, finite, capped ? s.ptr<int32_t>(ic) : nullptr));
-        return s.finish();
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            ZB_TRY(pw_conv_run(ctx, pwp, s.ptr<char>(ix), x_dtype == ZANT_U8, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                               s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}, finite, capped ? s.ptr<int32_t>(ic) : nullptr));
+            return s.finish();
+        }
     }
     if (host_consts && qconv_smallc_eligible(g, wz_zero) && (!is_device_ptr(x) || qconv_smallc_ptr_ok(x))) {
         // 3x3 on at most four input channels (network stems): warp-level MMAs with the filters as rows
@@ -817,12 +836,14 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
         const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
-        ZB_TRY(s.commit());
-        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
-        ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                           s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation},
-                           weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, g.M, (long long)g.Cg * g.KH * g.KW)));
-        return s.finish();
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                               s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation},
+                               weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, g.M, (long long)g.Cg * g.KH * g.KW)));
+            return s.finish();
+        }
     }
     if (host_consts && qdwconv_eligible(g, wz_zero) && (!is_device_ptr(x) || qdwconv_ptr_ok(x)) && (!is_device_ptr(y) || qdwconv_ptr_ok(y))) {
         // depthwise 3x3: one HBM-bound pass
@@ -858,20 +879,22 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
         const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = bias_here ? s.in(bp.data(), bp.size() * 4) : s.in(bias, (size_t)g.M * 4);
         const int ixl = s.scratch((size_t)g.N * hw * pix), iwb = s.scratch(nhp.w_bytes), ibb = s.scratch((size_t)nhp.a.const_n * 4);
-        ZB_TRY(s.commit());
-        const uint64_t launched = ctx->launches;
-        ZB_TRY(run_nh_weights(ctx, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb)));
-        if (!bias_here) {
-            launch(ctx, nh_bias_k, (unsigned)((nhp.a.const_n + 7) / 8), 256, 0, (const int8_t*)s.ptr<int8_t>(iw), (const int32_t*)s.ptr<int32_t>(ib), s.ptr<int32_t>(ibb), g.M, K, nhp.a.const_n, x_zp);
-            ZB_TRY(check_launch(ctx, "nh_bias_k"));
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            const uint64_t launched = ctx->launches;
+            ZB_TRY(run_nh_weights(ctx, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb)));
+            if (!bias_here) {
+                launch(ctx, nh_bias_k, (unsigned)((nhp.a.const_n + 7) / 8), 256, 0, (const int8_t*)s.ptr<int8_t>(iw), (const int32_t*)s.ptr<int32_t>(ib), s.ptr<int32_t>(ibb), g.M, K, nhp.a.const_n, x_zp);
+                ZB_TRY(check_launch(ctx, "nh_bias_k"));
+            }
+            ctx->launches = launched;                       // (not operator launches)
+            ZB_TRY(run_to_nhwc_bytes(ctx, s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix));
+            NhConvArgs a = nhp.a;
+            a.w = s.ptr<uint8_t>(iwb); a.mult = s.ptr<float>(im); a.bias = s.ptr<int32_t>(bias_here ? ib : ibb);
+            a.y = s.ptr<uint8_t>(iy); a.nchw = 1; a.act = activation; a.six = lean_six(y_scale);
+            ZB_TRY(nh_conv_run(ctx, nhp, a, NhView{s.ptr<char>(ixl), pix, g.H, g.W, 0}));
+            return s.finish();
         }
-        ctx->launches = launched;                       // (not operator launches)
-        ZB_TRY(run_to_nhwc_bytes(ctx, s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix));
-        NhConvArgs a = nhp.a;
-        a.w = s.ptr<uint8_t>(iwb); a.mult = s.ptr<float>(im); a.bias = s.ptr<int32_t>(bias_here ? ib : ibb);
-        a.y = s.ptr<uint8_t>(iy); a.nchw = 1; a.act = activation; a.six = lean_six(y_scale);
-        ZB_TRY(nh_conv_run(ctx, nhp, a, NhView{s.ptr<char>(ixl), pix, g.H, g.W, 0}));
-        return s.finish();
     }
     if (qconv_tc_eligible(g, wz_zero)) {
         // tensor-core path: im2col into the GEMM-blocked layout, tcgen05 GEMM, NCHW requantised store
@@ -884,11 +907,13 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int iw = s.in(w, numel(w_shape, 4)), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int ia = s.scratch(qgemm_a_bytes((size_t)g.N * g.OH * g.OW, prep));
         const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
-        ZB_TRY(s.commit());
-        ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
-        ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                            s.ptr<uint8_t>(ia), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-        return s.finish();
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                                s.ptr<uint8_t>(ia), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+            return s.finish();
+        }
     }
     if (host_consts && small_gemm_eligible(g, wz_zero)) {
         // few output positions: warp-level MMAs, K split over the warps of many small CTAs
@@ -897,13 +922,15 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
         const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int iwf = s.scratch(sg.w_bytes), ibf = s.scratch(x_zp != 0 ? (size_t)g.M * 4 : 0);
-        ZB_TRY(s.commit());
-        const uint64_t launched = ctx->launches;
-        ZB_TRY(run_small_gemm_weights(ctx, g, sg, false, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), x_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
-        ctx->launches = launched;                       // (not operator launches)
-        ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(x_zp != 0 ? ibf : ib),
-                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-        return s.finish();
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            const uint64_t launched = ctx->launches;
+            ZB_TRY(run_small_gemm_weights(ctx, g, sg, false, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), x_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
+            ctx->launches = launched;                       // (not operator launches)
+            ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(x_zp != 0 ? ibf : ib),
+                                  s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+            return s.finish();
+        }
     }
     Stager s(ctx);
     const int ix = s.in(x, numel(x_shape, 4)), iw = s.in(w, numel(w_shape, 4)), iy = s.out(y, numel(y_shape, 4));
@@ -957,11 +984,13 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
             const int iw = s.in(b, K * N), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, N * 4);
             const int isc = s.scratch(qgemm_a_bytes(M, prep));
             const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
-            ZB_TRY(s.commit());
-            ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
-            ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
-                                s.ptr<uint8_t>(isc), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-            return s.finish();
+            if (s.room()) {
+                ZB_TRY(s.commit());
+                ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+                ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
+                                    s.ptr<uint8_t>(isc), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+                return s.finish();
+            }
         }
     }
     if (M < 256 && N <= (1u << 20) && K <= (1u << 20) && y_dtype != ZANT_I32 && bz_zero && !is_device_ptr(b) && !(bias && is_device_ptr(bias))) {
@@ -973,13 +1002,15 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
         const int ix = s.in(a, M * K), iy = s.out(y, M * N);
         const int iw = s.in(b, K * N), im = s.in(mult.data(), mult.size() * 4), ib = s.in(bias, N * 4);
         const int iwf = s.scratch(sg.w_bytes), ibf = s.scratch(a_zp != 0 ? N * 4 : 0);
-        ZB_TRY(s.commit());
-        const uint64_t launched = ctx->launches;
-        ZB_TRY(run_small_gemm_weights(ctx, g, sg, true, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), a_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
-        ctx->launches = launched;                       // (not operator launches)
-        ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(a_zp != 0 ? ibf : ib),
-                              s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
-        return s.finish();
+        if (s.room()) {
+            ZB_TRY(s.commit());
+            const uint64_t launched = ctx->launches;
+            ZB_TRY(run_small_gemm_weights(ctx, g, sg, true, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), a_zp, s.ptr<char>(iwf), s.ptr<int32_t>(ibf)));
+            ctx->launches = launched;                       // (not operator launches)
+            ZB_TRY(run_small_gemm(ctx, g, sg, s.ptr<char>(ix), a_dtype == ZANT_U8, a_zp, s.ptr<char>(iwf), s.ptr<float>(im), s.ptr<int32_t>(a_zp != 0 ? ibf : ib),
+                                  s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
+            return s.finish();
+        }
     }
     Stager s(ctx);
     const int ia = s.in(a, M * K), ib = s.in(b, K * N), iy = s.out(y, M * N * dtype_size(y_dtype));

@@ -214,11 +214,18 @@ class Stager {
         return (int)slots_.size() - 1;
     }
 
+    // Arena space for every staged slot.  False when the arena may not or cannot grow that far: a kernel that wants less workspace is
+    // tried then.  (Anything else that is wrong with the buffers is left to commit.)
+    bool room() {
+        if (foreign_ || stream_capturing(ctx_)) return true;
+        const int32_t st = arena_reserve(ctx_, layout());
+        return st != ZANT_E_ARENA_EXHAUSTED && st != ZANT_E_MEM_ERROR;
+    }
+
     // Allocates arena space for every staged slot and issues the H2D copies.
     int32_t commit() {
         if (foreign_) return fail(ZANT_E_INVALID_INPUT, "a device buffer belongs to another GPU than the context's device %d", ctx_->device);
-        size_t total = 0;
-        for (auto& s : slots_) if (s.staged) { s.off = total; total += align_up(s.bytes ? s.bytes : 1, kArenaAlign); }
+        const size_t total = layout();
         if (total) {
             // the arena is the next call's as soon as this one returns: a replay would find that call's data there
             if (stream_capturing(ctx_)) return fail(ZANT_E_CUDA, "a call with host buffers or a workspace cannot be captured into a CUDA graph");
@@ -255,6 +262,11 @@ class Stager {
     }
 
   private:
+    size_t layout() {
+        size_t total = 0;
+        for (auto& s : slots_) if (s.staged) { s.off = total; total += align_up(s.bytes ? s.bytes : 1, kArenaAlign); }
+        return total;
+    }
     int add(const void* pin, void* pout, size_t bytes, bool is_in) {
         const void* p = is_in ? pin : pout;
         Slot s{nullptr, nullptr, bytes, 0, nullptr, false};
