@@ -1320,6 +1320,8 @@ static int32_t try_fuse_fconv_group(zant_plan* pl, size_t i0, size_t& consumed) 
         if (bias < 0 || T(bias).dtype != ZANT_F32 || T(cur).dtype != ZANT_F32 || T(add.out[0]).shape != ys || ys.empty()) return ZANT_OK;
         // a row vector of the product's columns: the last dimension and nothing else
         if (T(bias).shape.empty() || T(bias).shape.back() != ys.back() || numel(T(bias).shape.data(), T(bias).shape.size()) != ys.back() || T(bias).shape.size() > ys.size()) return ZANT_OK;
+        BcastGeom bg;
+        if (bcast_resolve(ys.data(), ys.size(), T(bias).shape.data(), T(bias).shape.size(), ys.data(), ys.size(), bg) != ZANT_OK) return ZANT_OK;
         interior.push_back(cur);
         cur = add.out[0];
         ++j;
@@ -1769,7 +1771,7 @@ static bool nh_parse(const zant_plan* pl, const ChainCtx& c, size_t i, NhGroup& 
         if (check_zero_point(T(x).dtype, n.a.x_zp, "QLinearConv x") != ZANT_OK) return false;
         if ((g.pt || g.pl || g.pb || g.pr) && n.a.x_zp != 0) return false;            // the halo is zero fill
         const int wz = opt_in(n, 3), b = opt_in(n, 4);
-        if (wz >= 0 && (T(wz).dtype != ZANT_I32 || !all_zero_i32(T(wz)))) return false;
+        if (wz >= 0 && (T(wz).dtype != ZANT_I32 || (T(wz).bytes != 4 && T(wz).bytes != (size_t)g.M * 4) || !all_zero_i32(T(wz)))) return false;
         if (b >= 0 && (T(b).dtype != ZANT_I32 || T(b).bytes != (size_t)g.M * 4)) return false;
         const size_t nws = T(n.in[2]).bytes / 4;
         if (nws != 1 && nws != (size_t)g.M) return false;
@@ -1838,11 +1840,12 @@ static bool nh_parse(const zant_plan* pl, const ChainCtx& c, size_t i, NhGroup& 
         if (rs.in.size() == 1 && T(rs.out[0]).dtype == T(cur).dtype && rs.a.n_scales == 4 && so.size() == 4 && so[0] == si[0] && so[1] == si[1] && so[2] == 2 * si[2] && so[3] == 2 * si[3]) {
             std::vector<int32_t> table, off;
             resize_index_table(si.data(), so.data(), 4, rs.a.coord_mode, table, off);
-            bool ok = true;
+            size_t os[4];
+            bool ok = resize_output_shape(si.data(), 4, rs.a.scales, rs.a.n_scales, nullptr, 0, os) == ZANT_OK && std::equal(so.begin(), so.end(), os);
             for (int d = 0; d < 4; ++d) for (size_t o = 0; o < so[d]; ++o) ok = ok && table[off[d] + o] == (int32_t)(d < 2 ? o : o / 2);
             if (ok) { q.up2 = true; take(); }
         }
-    } else if (i8 && next(ZANT_OP_DEQUANTIZE_LINEAR) && T(pl->nodes[j].out[0]).dtype == ZANT_F32 && T(pl->nodes[j].out[0]).shape == T(cur).shape) {
+    } else if (i8 && next(ZANT_OP_DEQUANTIZE_LINEAR) && pl->nodes[j].in.size() == 1 && T(pl->nodes[j].out[0]).dtype == ZANT_F32 && T(pl->nodes[j].out[0]).shape == T(cur).shape) {
         q.dequant = (int)j;
         take();
     }
