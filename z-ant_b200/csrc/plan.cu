@@ -117,6 +117,18 @@ struct zant_plan {
         aux_host.emplace_back((const char*)data, (const char*)data + bytes);
         return (int)aux_host.size() - 1;
     }
+    // Takes back what an earlier finalize that failed has derived: tensors, nodes and initializers stay as they were declared.
+    void reset_build() {
+        if (arena) { cudaStreamSynchronize(ctx->stream); cudaFree(arena); arena = nullptr; arena_bytes = 0; }
+        steps.clear(); init_steps.clear(); step_names.clear(); step_macs.clear(); step_bytes.clear();
+        aux_host.clear(); aux_off.clear(); scratch_bytes.clear(); scratch_off.clear(); nh_groups.clear();
+        im2col_scratch = -1;
+        pending_fact = 0; pending_slope = 0.0f; pending_y = -1; pending_used = false; pending_pool = -1;
+        for (PlanTensor& x : t) {
+            x.alias = -1; x.elided = false; x.arena_ptr = nullptr; x.bound = nullptr;
+            x.nh = false; x.nh_root = -1; x.nh_off = x.nh_pix = 0; x.nh_lo = 0;
+        }
+    }
 };
 
 namespace {
@@ -306,7 +318,7 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     ZB_CUDA(cudaSetDevice(ctx->device));
 
     // 1. validate nodes, derive constants, record launch closures
-    plan->steps.clear(); plan->step_names.clear(); plan->step_macs.clear(); plan->step_bytes.clear();
+    plan->reset_build();
     size_t i = 0;
     if (fuse) nh_layout(plan);
     while (i < plan->nodes.size()) {
@@ -361,7 +373,6 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     plan->init_steps.clear();
     ctx->launches = launched;
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (auto& t : plan->t) { t.host.clear(); t.host.shrink_to_fit(); }
 
     // 3. one dry count of launches
     plan->finalized = true;
@@ -371,6 +382,7 @@ int32_t zant_b200_plan_finalize(zant_plan* plan, int32_t input_id, int32_t outpu
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
     plan->launches_per_run = (int)(ctx->launches - before);
     ctx->launches = before;
+    for (auto& t : plan->t) { t.host.clear(); t.host.shrink_to_fit(); }
     log_line("zant_b200 plan: %zu tensors, %zu nodes, %zu steps, %d launches, arena %zu bytes", plan->t.size(), plan->nodes.size(), plan->steps.size(), plan->launches_per_run, plan->arena_bytes);
     return ZANT_OK;
 }
