@@ -104,9 +104,10 @@ class HostStage {
             e = cudaMemcpyAsync((char*)dst + off, slot(s), n, cudaMemcpyHostToDevice, stream);
             if (e == cudaSuccess) e = cudaEventRecord(ev_[s], stream);
         }
-        // whatever was claimed is finished before src goes back to the caller
-        limit_.store(0, std::memory_order_release);
-        while (busy_.load(std::memory_order_acquire) != 0) pause();
+        // whatever was claimed is finished before src goes back to the caller, and nothing is claimed any more: a thread counts itself
+        // busy before it looks at the limit, the limit falls before the count is read, and all four accesses are in one order
+        limit_.store(0, std::memory_order_seq_cst);
+        while (busy_.load(std::memory_order_seq_cst) != 0) pause();
         cur_ = (first + pieces) % kSlots;
         used_ = 0; dirty_ = false;
         const bool skip = idle_ && pieces < kSlots;
@@ -168,10 +169,10 @@ class HostStage {
     bool done(int i) { return done_[i].load(std::memory_order_acquire) != 0; }
     // claims and fills one open piece; false when there is none
     bool copy_one() {
-        busy_.fetch_add(1, std::memory_order_acq_rel);
+        busy_.fetch_add(1, std::memory_order_seq_cst);
         int i = next_.load(std::memory_order_acquire);
         bool got = false;
-        while (i < limit_.load(std::memory_order_acquire)) {
+        while (i < limit_.load(std::memory_order_seq_cst)) {
             if (next_.compare_exchange_weak(i, i + 1)) { got = true; break; }
         }
         if (got) {
