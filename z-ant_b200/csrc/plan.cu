@@ -93,6 +93,7 @@ struct zant_plan {
     size_t prof_used = 0;                   // events recorded since the last read
 
     std::vector<NhGroup> nh_groups;   // channels-last convolution groups found by the layout pass, by first node
+    std::vector<std::pair<int, char*>> nchw_copies;   // channels-last tensors whose address was asked for, and buffers that hold them in the graph's order after each run
     void* ptr(int id) const {
         int r = id;
         while (t[r].alias >= 0) r = t[r].alias;
@@ -200,6 +201,7 @@ int32_t zant_b200_plan_destroy(zant_plan* plan) {
     cudaStreamSynchronize(plan->ctx->stream);
     if (plan->graph_exec) cudaGraphExecDestroy(plan->graph_exec);
     if (plan->arena) cudaFree(plan->arena);
+    for (auto& c : plan->nchw_copies) cudaFree(c.second);
     for (cudaEvent_t e : plan->prof_events) cudaEventDestroy(e);
     cudaGetLastError();
     delete plan;
@@ -255,6 +257,7 @@ static int32_t try_fuse_qconv_group(zant_plan* pl, size_t node_index, size_t& co
 static int32_t try_fuse_fconv_group(zant_plan* pl, size_t node_index, size_t& consumed);
 static void nh_layout(zant_plan* pl);
 static int32_t build_nh(zant_plan* pl, size_t node_index, size_t& consumed);
+static int32_t refresh_nchw_copy(zant_plan* pl, int id, char* y);
 
 // Multiply-accumulates of one node (contractions only; everything else counts as 0).
 static double node_macs(const zant_plan* pl, const PlanNode& n) {
@@ -420,6 +423,7 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
         ZB_CUDA(copy_in());
         ZB_CUDA(cudaGraphLaunch(plan->graph_exec, ctx->stream));
         ctx->launches += (uint64_t)plan->launches_per_run;
+        for (auto& c : plan->nchw_copies) ZB_TRY(refresh_nchw_copy(plan, c.first, c.second));
         return copy_out();
     }
     ti.bound = in_dev ? const_cast<void*>(input) : nullptr;
@@ -442,6 +446,7 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
     }
     if (plan->profiling) { int32_t st = mark(); if (st != ZANT_OK) return st; }
     ti.bound = nullptr; tor.bound = nullptr;
+    for (auto& c : plan->nchw_copies) ZB_TRY(refresh_nchw_copy(plan, c.first, c.second));
     return out_dev ? ZANT_OK : copy_out();
 }
 
@@ -481,7 +486,15 @@ void* zant_b200_plan_tensor_ptr(zant_plan* plan, int32_t id) {
     if (!plan || !plan->finalized || id < 0 || id >= (int)plan->t.size()) return nullptr;
     int r = id;
     while (plan->t[r].alias >= 0) r = plan->t[r].alias;
-    if (plan->t[r].nh) return nullptr;        // kept in another layout: zant_b200_plan_read_tensor converts
+    if (plan->t[r].nh) {
+        // kept in another layout: the address of a copy in the graph's order, which every run from now on brings up to date
+        for (auto& c : plan->nchw_copies) if (c.first == r) return c.second;
+        char* y = nullptr;
+        if (cudaSetDevice(plan->ctx->device) != cudaSuccess || dev_malloc((void**)&y, plan->t[r].bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (refresh_nchw_copy(plan, r, y) != ZANT_OK) { cudaFree(y); return nullptr; }
+        plan->nchw_copies.emplace_back(r, y);
+        return y;
+    }
     return plan->ptr(id);
 }
 
@@ -1967,6 +1980,14 @@ static void nh_layout(zant_plan* pl) {
 static NhView nh_view(zant_plan* pl, int id) {
     const PlanTensor& t = pl->t[id];
     return NhView{t.arena_ptr, (long long)t.nh_pix, (int)t.shape[2], (int)t.shape[3], t.nh_lo};
+}
+
+static int32_t refresh_nchw_copy(zant_plan* pl, int id, char* y) {
+    const PlanTensor& t = pl->t[id];
+    const uint64_t launched = pl->ctx->launches;
+    const int32_t st = run_from_nhwc(pl->ctx, nh_view(pl, id), y, t.shape[0], t.shape[1], dtype_size(t.dtype));
+    pl->ctx->launches = launched;                    // (not an operator launch)
+    return st;
 }
 
 static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {

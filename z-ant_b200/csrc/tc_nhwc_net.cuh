@@ -898,6 +898,29 @@ inline int32_t run_to_nhwc_bytes(zant_ctx* ctx, const void* x, void* y, int N, i
     return check_launch(ctx, "to_nhwc_bytes_k");
 }
 
+// A channels-last tensor in the graph's order, for a caller that asked for its address; split form: hi + lo.
+struct FromNhwcArgs { const uint8_t* x; uint8_t* y; long long pix, hw, total; int C, lo; };
+template <typename T>
+__global__ void __launch_bounds__(256) from_nhwc_k(const __grid_constant__ FromNhwcArgs a) {
+    ptx::grid_start();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.total; i += (long long)gridDim.x * blockDim.x) {
+        const long long t = i / a.hw, p = i - t * a.hw, n = t / a.C, c = t - n * a.C;
+        const T* s = reinterpret_cast<const T*>(a.x + (n * a.hw + p) * a.pix) + c;
+        T v = *s;
+        if constexpr (sizeof(T) == 4) { if (a.lo) v = __fadd_rn(v, s[a.lo]); }
+        reinterpret_cast<T*>(a.y)[i] = v;
+    }
+}
+inline int32_t run_from_nhwc(zant_ctx* ctx, const NhView& x, void* y, size_t N, size_t C, size_t esz) {
+    FromNhwcArgs a{};
+    a.x = (const uint8_t*)x.ptr; a.y = (uint8_t*)y; a.pix = x.pix; a.hw = (long long)x.H * x.W; a.C = (int)C; a.lo = x.lo;
+    a.total = (long long)(N * C) * a.hw;
+    const int grid = grid_for((size_t)a.total, 256, ctx->sm_count);
+    if (esz == 1) launch(ctx, from_nhwc_k<uint8_t>, grid, 256, 0, a);
+    else launch(ctx, from_nhwc_k<float>, grid, 256, 0, a);
+    return check_launch(ctx, "from_nhwc_k");
+}
+
 // MaxPool: a thread owns 16 bytes of one output pixel's channels.  KIND as above; split form: the larger hi + lo.
 struct NhPoolArgs { const uint8_t* x; uint8_t* y; long long x_pix, y_pix, total; int chunks, H, W, OH, OW, KH, KW, sh, sw, dh, dw, pt, pl; int lo_in, lo_out; };
 template <int KIND>
