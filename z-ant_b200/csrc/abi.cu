@@ -130,6 +130,7 @@ void* zant_b200_ctx_stream(zant_ctx* ctx) { return ctx ? (void*)ctx->stream : nu
 
 int32_t zant_b200_ctx_synchronize(zant_ctx* ctx) {
     ZB_NEED_CTX(ctx);
+    ZB_TRY(refuse_capture(ctx));
     return drain_and_check_status(ctx);
 }
 

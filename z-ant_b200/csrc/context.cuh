@@ -101,27 +101,30 @@ inline bool stream_capturing(zant_ctx* ctx) {
     return s != cudaStreamCaptureStatusNone;
 }
 
-// Host buffer -> device, ordered on the context's stream; `src` may be changed as soon as this returns.  (In a capture the copy
-// becomes a node that reads `src` at every replay; the ring's slots would hold something else by then.)
+inline int32_t refuse_capture(zant_ctx* ctx) {
+    return stream_capturing(ctx) ? fail(ZANT_E_CUDA, "the context's stream is being captured: it cannot be waited for") : ZANT_OK;
+}
+
+// Host buffer -> device, ordered on the context's stream; `src` may be changed as soon as this returns.  Not in a capture: the copy would
+// become a node that reads the ring's slot at every replay, which holds something else by then.
 inline cudaError_t copy_to_device(zant_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return cudaSuccess;
-    if (stream_capturing(ctx)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (HostStage* st = host_stage(ctx)) return st->to_device(dst, src, bytes, ctx->stream);
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);      // no page-locked memory to be had
 }
 
 // Drains the stream and reads the device status word that kernels with bounded waits write when
 // they give up; a non-zero value is reported once and cleared.  With `host_dst` the same wait also brings a result back
-// (`bytes` from device memory): one synchronisation for both.
-inline int32_t drain_and_check_status(zant_ctx* ctx, void* host_dst = nullptr, const void* dev_src = nullptr, size_t bytes = 0) {
-    if (stream_capturing(ctx)) return fail(ZANT_E_CUDA, "the context's stream is being captured: it cannot be waited for");
+// (`bytes` from device memory): one synchronisation for both.  A small one for pageable memory lands in the ring first; page-locked
+// memory (`dst_pinned`) takes it directly.  The stream must not be in a capture (refuse_capture).
+inline int32_t drain_and_check_status(zant_ctx* ctx, void* host_dst = nullptr, const void* dev_src = nullptr, size_t bytes = 0, bool dst_pinned = false) {
     int h = 0;
     char* slot = nullptr;
-    if (ctx->stage || (host_dst && bytes && bytes + 256 <= HostStage::kSlot)) {
-        const size_t want = 256 + ((bytes + 256 <= HostStage::kSlot) ? bytes : 0);
-        if (HostStage* st = host_stage(ctx)) slot = (char*)st->result_slot(want, ctx->stream);
+    const bool ring = host_dst && bytes && !dst_pinned && bytes + 256 <= HostStage::kSlot;
+    if (ctx->stage || ring) {
+        if (HostStage* st = host_stage(ctx)) slot = (char*)st->result_slot(256 + (ring ? bytes : 0), ctx->stream);
     }
-    const bool via_slot = slot && bytes && bytes + 256 <= HostStage::kSlot;
+    const bool via_slot = slot && ring;
     if (host_dst && bytes) ZB_CUDA(cudaMemcpyAsync(via_slot ? (void*)(slot + 256) : host_dst, dev_src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     ZB_CUDA(cudaMemcpyAsync(slot ? (void*)slot : (void*)&h, ctx->status_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ZB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -258,7 +261,7 @@ class Stager {
         if (!last && !wait_) return ZANT_OK;
         // the call waits anyway: also pick up the status word that a bounded device-side wait writes
         // when it gives up, so that the time-out is reported by the call that suffered it
-        return last ? drain_and_check_status(ctx_, last->host_out, last->dev, last->bytes) : drain_and_check_status(ctx_);
+        return last ? drain_and_check_status(ctx_, last->host_out, last->dev, last->bytes, last->pinned) : drain_and_check_status(ctx_);
     }
 
   private:

@@ -408,16 +408,19 @@ int32_t zant_b200_plan_run(zant_plan* plan, const void* input, void* output) {
     const bool async = out_dev || (ko.pinned && (in_dev || ki.pinned));
     auto copy_in = [&]() -> cudaError_t {
         if (in_dev || ki.pinned) return cudaMemcpyAsync(ti.arena_ptr, input, ti.bytes, in_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream);
+        // (captured by the caller: a plain copy, which reads `input` at every replay)
+        if (stream_capturing(ctx)) return cudaMemcpyAsync(ti.arena_ptr, input, ti.bytes, cudaMemcpyHostToDevice, ctx->stream);
         return copy_to_device(ctx, ti.arena_ptr, input, ti.bytes);
     };
     // copies the result out; a call that has to wait reads the status word with the same synchronisation
     auto copy_out = [&]() -> int32_t {
-        if (!async) return drain_and_check_status(ctx, output, tor.arena_ptr, to.bytes);
+        if (!async) return drain_and_check_status(ctx, output, tor.arena_ptr, to.bytes, ko.pinned);
         ZB_CUDA(cudaMemcpyAsync(output, tor.arena_ptr, to.bytes, out_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
         return ZANT_OK;
     };
     if (ki.foreign || ko.foreign)
         return fail(ZANT_E_INVALID_INPUT, "input/output is device memory of another GPU than the plan's device %d", ctx->device);
+    if (!async) ZB_TRY(refuse_capture(ctx));
     if (plan->graph_exec && !plan->profiling) {
         // replay: everything runs on the arena's own buffers
         ZB_CUDA(copy_in());
