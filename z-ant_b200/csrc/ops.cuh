@@ -30,18 +30,31 @@ inline int32_t launch_contract_tile(zant_ctx* ctx, const ContractArgs& p) {
     return check_launch(ctx, "contract_f32_tile");
 }
 
-// Tile by cost: waves of tiles over the SMs times the tile's outputs over the share of the FP32 rate a tile of that shape
-// reaches (8 x 8 sums per thread keep the pipe busy; fewer spend more of their slots on operands).
+// Tile by time: what n tiles of a shape cost an SM for each k, in ns, and 25 k's worth per tile for its results.  Up to three tiles get an SM's
+// shared memory in equal shares and overlap (lone + n * per); more queue (base + n * slope).  The numbers are medians over 220 convolutions, as
+// calls and as plans (whose weights are in slab order), and 200 products of 5 us to 2 ms with every shape forced: the choice is 1.5 % slower
+// than the best shape in the mean.  By waves and the rate of a full SM alone, which knows no latency, it was 4 to 15 %, and up to 20 %
+// slower than 64 x 64 tiles where a few narrow tiles met a long k (convolution 2312 x 155 x 800: 115 us there, 125, now 75).
+struct ContractTime { double lone, per, base, slope; };
+inline double contract_cost(const ContractTime& t, double tiles_per_sm, double k) {
+    const double ns = tiles_per_sm <= 3.0 ? t.lone + t.per * tiles_per_sm : t.base + t.slope * tiles_per_sm;
+    return ns * k + 25.0 * t.slope * tiles_per_sm;
+}
 template <bool CONV, bool POOL>
 inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     p.neg_zero = 0x8000000080000000ull;
-    struct Shape { int bm, bn; double rate; };
-    static const Shape shapes[] = {{128, 128, 1.0}, {128, 64, 0.85}, {128, 32, 0.75}, {128, 16, 0.5}, {32, 32, 0.4}, {CF_BM, CF_BN, 0.12}};
+    static const int shapes[6][2] = {{128, 128}, {128, 64}, {128, 32}, {128, 16}, {32, 32}, {CF_BM, CF_BN}};
+    static const ContractTime times[3][6] = {
+        {{0, 204, 50, 195}, {45, 87, 40, 92}, {95, 36, 130, 46}, {72, 23, 90, 31}, {52, 9, 55, 17.5}, {0, 33, 30, 26}},        // B runs along k (a convolution's weights as the tensor has them, a transposed matrix)
+        {{0, 186, 30, 180}, {32, 81, 30, 83}, {78, 35, 115, 42}, {62, 23, 85, 28.5}, {38, 8, 45, 14.5}, {0, 14.5, 12, 10.2}},  // convolution, weights in slab order
+        {{0, 167, 0, 165}, {12, 83, 10, 83}, {22, 48, 25, 49}, {55, 16.5, 65, 32}, {19, 9, 42, 11}, {1, 9, 12, 8}},            // product with B in rows
+    };
+    const ContractTime* t = times[!p.b_vec && p.sbk == 1 ? 0 : (CONV ? 1 : 2)];
     int best = -1; double cost = 1e300;
     for (int i = 0; i < 6; ++i) {
-        const double row_tiles = std::ceil((double)p.M / shapes[i].bm), col_tiles = std::ceil((double)p.N / shapes[i].bn);
-        if (col_tiles > 65535.0 || row_tiles * shapes[i].bm > 2147483648.0) continue;        // (grid.y; a tile's rows are ints)
-        const double c = std::ceil(row_tiles * col_tiles / ctx->sm_count) * shapes[i].bm * shapes[i].bn / shapes[i].rate;
+        const double row_tiles = std::ceil((double)p.M / shapes[i][0]), col_tiles = std::ceil((double)p.N / shapes[i][1]);
+        if (col_tiles > 65535.0 || row_tiles * shapes[i][0] > 2147483648.0) continue;        // (grid.y; a tile's rows are ints)
+        const double c = contract_cost(t[i], std::ceil(row_tiles * col_tiles / ctx->sm_count), p.K);
         if (c < cost) { cost = c; best = i; }
     }
     if (best < 0) return fail(ZANT_E_TOO_LARGE, "too many output columns");
