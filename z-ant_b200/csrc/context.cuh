@@ -138,7 +138,7 @@ inline int32_t drain_and_check_status(zant_ctx* ctx, void* host_dst = nullptr, c
     return ZANT_OK;
 }
 
-// What a caller's pointer is: one driver query per buffer.
+// What a caller's pointer is: everything the library asks about it, in one driver query.
 struct PtrKind { bool device = false, foreign = false, pinned = false; };
 inline PtrKind ptr_kind(const void* p, int device) {
     PtrKind k;

@@ -1812,7 +1812,7 @@ static bool nh_parse(const zant_plan* pl, const ChainCtx& c, size_t i, NhGroup& 
         const int b = opt_in(n, 2);
         if (b >= 0 && (T(b).dtype != ZANT_F32 || T(b).bytes != (size_t)g.M * 4)) return false;
     }
-    // the input has to come channels-last from somewhere, or be a first layer's (the search for a tiling below takes 75 us a shape)
+    // the input has to come channels-last from somewhere, or be a first layer's (no search for a tiling otherwise)
     if (T(x).shape[1] > 4) {
         bool from = false;
         for (size_t k = 0; k < i; ++k) {

@@ -350,7 +350,6 @@ inline bool tc_conv_nhwc_plan(const ConvGeom& g, bool w_zp_all_zero, int x_zp, T
     p.NT *= 2;                                                   // (the loop has halved it once more)
     p.smem_bytes = (size_t)a.off_out + kTcConvTail;
     p.w_bytes = (size_t)a.n_tiles * a.c_stages * w_stage;
-    p.row_efficiency = (double)a.OH * a.OW / ((double)a.hseg * a.RB * a.wseg * 128.0);
     const long long tiles = (long long)a.N * a.hseg * a.wseg * a.n_tiles;
     return tiles <= 0x7fffffffLL;
 }

@@ -4,7 +4,8 @@
 // A call brings its weights along every time, so re-blocking them is part of the call: on the host the byte shuffle of a
 // 512 x 256 x 3 x 3 tensor took 1.1 of 1.5 ms (the convolution itself takes 0.05), here the raw tensor is uploaded as it is
 // and one launch of a few microseconds shuffles it.  One block per (padded) filter row; a thread moves 16-byte chunks of K
-// and the block adds the row up for the bias (bias - x_zp * sum).  A plan blocks its weights once, on the host.
+// and the block adds the row up for the bias (bias - x_zp * sum).  A plan blocks its weights once, when it is finalized: those of the
+// channels-last and few-position kernels on the device, the others on the host.
 #pragma once
 #include <cuda_runtime.h>
 
