@@ -90,6 +90,7 @@ struct NhConvArgs {
 
 constexpr int kNhThreads = 608;
 constexpr int kNhMaxStages = 8, kNhMaxW = 12;
+constexpr int kNhOrderN = 8;                             // batch whose best tiling fixes the order of float sums
 constexpr int kNhTail = 48 * 8 + 256 + 64;               // barriers, TMEM slot, flag, activation table
 
 struct NhMaps { CUtensorMap m[4]; };
@@ -551,8 +552,9 @@ inline double nh_cost(const NhConvArgs& a, int kind, int mode, long long tiles, 
     return std::ceil((double)tiles / sm_count) * tile + epi;
 }
 
-// `g`: the convolution on NCHW shapes.  False when the kernel does not take it.
-inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, NhConvPlan& p) {
+// `g`: the convolution on NCHW shapes.  False when the kernel does not take it.  `same`: only tilings that add an output's products up in
+// the order of that one (channel stages, and the way the views of a pool are taken).
+inline bool nh_conv_search(const ConvGeom& g, int kind, bool pool, int sm_count, NhConvPlan& p, const NhConvPlan* same) {
     const bool i8 = kind <= NH_U8;
     const int esz = i8 ? 1 : 4, parts = kind == NH_TF32X3 ? 2 : 1;
     const bool s2 = g.sh == 2 && (g.KH > 1 || g.KW > 1), planed = pool || s2;
@@ -570,7 +572,7 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
     base.BH = std::max(1, std::min(base.GH, 128 / base.PW));
     // images whose whole patch is at most half a row block share one (7 x 7 outputs with stride 2: two, of 64 rows each)
     base.imgs = g.N; base.IB = 1;
-    if (!pool && base.wseg == 1 && base.BH == base.GH) base.IB = std::max(1, std::min(g.N, 128 / ((base.GH + halo_h) * base.PW)));
+    if (!pool && base.wseg == 1 && base.BH == base.GH) base.IB = std::max(1, std::min(i8 ? g.N : std::min(g.N, kNhOrderN), 128 / ((base.GH + halo_h) * base.PW)));
     base.N = (g.N + base.IB - 1) / base.IB;
     base.parts = parts;
     const int cin = parts > 1 ? (g.C + 7) / 8 * 8 : g.C;             // (a stage of the hi half must not run into the lo half)
@@ -587,6 +589,7 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
                 if (2 * sets * rb * NT > 512 || (NT > 32 && NT / 2 >= g.M) || (mode == NH_POOL_PAIRS && KC == 16)) continue;
                 if (KC > (s2 ? 32 : 16) && KC / 2 >= cbytes) continue;               // (channels past C arrive as zeros)
                 if (KC == 16 && (cbytes > 16 || parts > 1 || s2)) continue;
+                if (same && (KC != same->a.KC || mode != same->pool)) continue;
                 NhConvArgs a = base;
                 a.n_tiles = (g.M + NT - 1) / NT;
                 a.KC = KC; a.c_stages = (cbytes + KC - 1) / KC;
@@ -635,6 +638,16 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
                 }
             }
     return best < 1e300;
+}
+
+// Float sums depend on their order: the one that suits 8 images is kept for every batch, so that an image's result does not depend on how
+// many others it is run with (a sharded batch equals the whole one).  int8 sums are exact and take the best tiling of each batch.
+inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, NhConvPlan& p) {
+    if (kind <= NH_U8) return nh_conv_search(g, kind, pool, sm_count, p, nullptr);
+    ConvGeom few = g;
+    few.N = kNhOrderN;
+    NhConvPlan order;
+    return nh_conv_search(few, kind, pool, sm_count, order, nullptr) && nh_conv_search(g, kind, pool, sm_count, p, &order);
 }
 
 // Weights [M][C][KH][KW] -> [filter tile][channel stage][iteration][part][NB rows of KC bytes], rows swizzled as the tensor core reads
