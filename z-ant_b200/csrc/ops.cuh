@@ -18,14 +18,18 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // What a fused step applies to a contraction's finished sums.
 struct ContractFusion { int act = CT_ACT_NONE; float slope = 0.0f; const float* bias = nullptr; bool pool = false; };
 
+// Up to three tiles per SM: so much shared memory that no SM takes more than its share.  A grid that starts while its predecessor
+// drains would otherwise pile up on the SMs that are free first (128 tiles, two to an SM: 290 -> 540 us).
+inline size_t contract_share(zant_ctx* ctx, const dim3& grid, size_t smem) {
+    const long long share = ((long long)grid.x * grid.y + ctx->sm_count - 1) / ctx->sm_count;
+    return std::max<size_t>(smem, share == 1 ? 122880 : (share == 2 ? 81920 : (share == 3 ? 61440 : 0)));
+}
+
 template <bool CONV, bool POOL, int BM, int BN, int TM, int TN>
 inline int32_t launch_contract_tile(zant_ctx* ctx, const ContractArgs& p) {
     ZB_SMEM_ATTR(ctx, (contract_f32_tile<CONV, POOL, BM, BN, TM, TN>), 122880);
     const dim3 grid(((unsigned)p.M + BM - 1) / BM, ((unsigned)p.N + BN - 1) / BN);
-    // Up to three tiles per SM: ask for so much shared memory that no SM takes more than its share.  A grid that starts while
-    // its predecessor drains would otherwise pile up on the SMs that are free first (128 tiles, two to an SM: 290 -> 540 us).
-    const long long share = ((long long)grid.x * grid.y + ctx->sm_count - 1) / ctx->sm_count;
-    const size_t smem = std::max<size_t>(contract_smem<BM, BN>(), share == 1 ? 122880 : (share == 2 ? 81920 : (share == 3 ? 61440 : 0)));
+    const size_t smem = contract_share(ctx, grid, contract_smem<BM, BN>());
     launch(ctx, contract_f32_tile<CONV, POOL, BM, BN, TM, TN>, grid, (BM / TM) * (BN / TN), smem, p);
     return check_launch(ctx, "contract_f32_tile");
 }
@@ -66,10 +70,9 @@ inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
         case 4: return launch_contract_tile<CONV, POOL, 32, 32, 4, 2>(ctx, p);
         default: break;
     }
-    constexpr int smem = contract_few_smem();
-    ZB_SMEM_ATTR(ctx, (contract_f32_few<CONV, POOL>), smem);
+    ZB_SMEM_ATTR(ctx, (contract_f32_few<CONV, POOL>), 122880);
     const dim3 grid(((unsigned)p.M + CF_BM - 1) / CF_BM, ((unsigned)p.N + CF_BN - 1) / CF_BN);
-    launch(ctx, contract_f32_few<CONV, POOL>, grid, 256, smem, p);
+    launch(ctx, contract_f32_few<CONV, POOL>, grid, 256, contract_share(ctx, grid, contract_few_smem()), p);
     return check_launch(ctx, "contract_f32_few");
 }
 
