@@ -1,12 +1,10 @@
 // Fused kernels for quantized 3x3 convolution stages followed by ReLU and a 2x2/2 MaxPool.
 //
-// Internal activation layout between the two stages, "parity planes": every pixel of a 16-channel group is one
-// 16-byte chunk, and the chunks of the pixels with the same (row parity, column parity) form one plane in
-// row-major order of (row/2, column/2), images one after the other.  With that layout the A operand of an
-// implicit-GEMM convolution FOLLOWED BY a 2x2/2 pool needs no im2col at all: for member (dy,dx) of a pool
-// window and filter tap (kh,kw) the rows of A (one per pool window) are consecutive chunks of one plane,
-// shifted by a constant, so the tcgen05 shared-memory descriptor (K-major, no swizzle: 8 rows = 8
-// consecutive 16-byte chunks) simply starts a few rows further.
+// Internal activation layout between the two stages, "image blocks": [N / 128][12 x 12 pixels][2 chunks of 16 channels][128 images][16]
+// (a batch below 128: one block of as many images, whose MMA rows beyond them read the bytes behind and are not stored), so that the 128 rows of an MMA are the same pixel of 128 images.  With that layout the A operand of an implicit-GEMM convolution
+// FOLLOWED BY a 2x2/2 pool needs no im2col and computes nothing twice: the view (ry, rx) of a pool window - input pixel (2py + ry, 2px + rx),
+// ry = dy + kh, rx = dx + kw - is one 4 KB block (K-major, no swizzle: 8 rows = 8 consecutive 16-byte chunks), and every one of the
+// 25 windows of an image is a tile row that is kept.
 //
 // MaxPool is applied to the int32 accumulators BEFORE requantisation.  That is exact because the
 // requantisation y = sat(rne(float(acc + bias) * M) + zp) is non-decreasing in acc whenever M > 0
@@ -16,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 
 #include "kernels_q8.cuh"
 #include "ptx_sm100.cuh"
@@ -29,7 +28,7 @@ enum DeviceError : int {
 
 // =============================================================================================
 // Stage 1: QuantizeLinear(uint8) + QLinearConv(1 -> 32, 3x3, stride 1, no pad) + ReLU + MaxPool 2x2/2
-//          float [N,1,28,28]  ->  int8 parity planes (Conv1MmaArgs::plane_bytes)
+//          float [N,1,28,28]  ->  int8 image blocks (c2_block_bytes)
 // Host-side description of the stage (the plan fills it from the graph; the kernel below takes its
 // own argument block derived from it).
 // =============================================================================================
@@ -60,17 +59,15 @@ struct Conv1Args {
 struct Conv1MmaArgs {
     const float* x;
     int8_t* y;
-    int n_images;
+    int n_images, ib;
     float x_scale; int x_zp;
+    float q_rh, q_rl;        // the quotient of the quantisation in two instructions (quant_steps); q_rl == 0: by division
     const uint32_t* wfrag;   // [4 members][4 groups][32 lanes] B-fragment words
-    const int32_t* biasfrag; // [4 groups][32 lanes][2]  (bias - x_zp * sum(w)) of the lane's two columns
+    const float* floorfrag;  // [4 groups][32 lanes][2]  kAccBase - (bias - x_zp * sum(w)) of the lane's two columns (or the bits of the bias)
     const float* multfrag;   // [4 groups][32 lanes][2]
     int* status;             // device status word: DEV_ERR_WAIT_TIMEOUT when a bounded wait gave up
-    // Output layout: parity planes for tc_conv3x3_pool_parity_kernel, [2 chunks][4 parities][N*36 rows (+ padding)][16],
-    // `plane_bytes` apart: pooled pixel (y, x), y and x below 12, lies in plane (y&1)*2 + (x&1) at row
-    // n*36 + (y>>1)*6 + (x>>1); row and column 12 are neither computed nor stored (the next stage's pool never
-    // reads them).
-    long long plane_bytes;
+    // Output layout: image blocks for tc_conv3x3_pool_kernel; pooled row and column 12 are neither computed nor stored (the next
+    // stage's pool never reads them).
 };
 
 __device__ __forceinline__ void mma_m16n8k16_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, const int (&c)[4]) {
@@ -79,10 +76,26 @@ __device__ __forceinline__ void mma_m16n8k16_u8s8(int (&d)[4], uint32_t a0, uint
                  : "r"(a0), "r"(a1), "r"(b0), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
 
+// Accumulators that start at the bit pattern of 1.5 * 2^23 are, read as floats, 1.5 * 2^23 + acc exactly (|acc| < 2^22), and order as
+// integers the way the sums do.  With floor = 1.5 * 2^23 - bias, max(acc', floor) as integers is the ReLU and one subtraction of floats
+// then gives float(max(acc + bias, 0)): no register moves of the bias into the MMAs' C operand (one quad serves all of
+// them) and no integer -> float conversion, which shares the half-rate ALU pipe with the maxima.
+constexpr int kAccBaseBits = 0x4b400000;
+constexpr float kAccBase = 12582912.0f;
+// biases that keep floor and the sums of nine products of 255 x 128 inside [2^23, 2^24)
+inline bool acc_base_ok(int32_t bias) { return bias > -3800000 && bias < 3800000; }
+
+inline float int_bits_as_float(int32_t v) { float f; std::memcpy(&f, &v, 4); return f; }
+
+// Image blocks between the stages: ib = min(128, N) images, a pixel is both their 16-channel chunks, 144 pixels are a block.
+__host__ __device__ constexpr int c2_pixel_bytes(int ib) { return 2 * ib * 16; }
+__host__ __device__ constexpr int c2_block_bytes(int ib) { return 144 * c2_pixel_bytes(ib); }
+
 // Images per CTA iteration: 4 x 144 pooled pixels = 36 units of 16.
 constexpr int C1M_G = 4;
-constexpr int C1M_THREADS = 256;
-constexpr int C1M_UNITS = (C1M_G * 144 + 15) / 16;
+constexpr int C1M_THREADS = 384;
+// words of a quantized image in shared memory: the four images of a unit's rows lie in different banks
+constexpr int C1M_IMG_WORDS = 28 * 8 + 2;
 
 constexpr int C1M_IMG_FLOATS = 28 * 28;
 constexpr int C1M_GROUP_BYTES = C1M_G * C1M_IMG_FLOATS * 4;   // 9408: a multiple of 16, as the bulk copy wants
@@ -90,17 +103,18 @@ constexpr int C1M_GROUP_BYTES = C1M_G * C1M_IMG_FLOATS * 4;   // 9408: a multipl
 // The float images of a group arrive by one bulk async copy into a two-deep shared-memory ring: the copy
 // of group i+1 is issued when the MMA phase of group i starts, so no thread waits on global loads.  The
 // quantized bytes are double-buffered too, which leaves one __syncthreads per group.
-// Three CTAs per SM (80 registers per thread; a fourth would need 64 registers and spills).
-__global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(const Conv1MmaArgs a) {
+// A group is 36 units of 16 rows: four neighbouring pixels of a pooled row times its four images.  Twelve warps take three units each, the same
+// third of every fourth row, and a thread's rows are one image's pixels of one column parity, so that everything about a unit but
+// constant offsets is known before the loop (a table of pixels and eight warps, 4.5 units each, cost 870 of 1880 warp instructions an image).
+// Two CTAs per SM (80 registers per thread).
+// BASE false: biases that do not qualify (acc_base_ok); the accumulators start at 0 and are converted.
+template <bool BASE>
+__global__ void __launch_bounds__(C1M_THREADS, 2) conv1_mma_relu_pool_kernel(const Conv1MmaArgs a) {
     ptx::grid_start();
     __shared__ __align__(128) float stage[2][C1M_G * C1M_IMG_FLOATS];
-    __shared__ uint32_t img2[2][C1M_G][28][8];   // quantized uint8 rows of 32 bytes (28 pixels + 4 pad)
+    __shared__ uint32_t img2[2][C1M_G * C1M_IMG_WORDS];   // quantized uint8 rows of 32 bytes (28 pixels + 4 pad)
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ int abort_flag;
-    // Per pooled pixel of an iteration (the same in every iteration): x = word of img that holds the patch's
-    // first byte | odd column << 16 | image within the group << 17 (3 bits) | exists << 20; y = byte offset of the
-    // pixel's first 16-channel chunk from the group's first image (and, with parity planes, from plane 0).  Keeps divisions out of the main loop.
-    __shared__ uint2 pix_tab[C1M_UNITS * 16];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int stride = gridDim.x * C1M_G;
@@ -116,19 +130,7 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
             ptx::bulk_g2s(ptx::smem_u32(&stage[0][0]), a.x + (size_t)base * C1M_IMG_FLOATS, bytes, bar0);
         }
     }
-    // Parity planes: only the 12 x 12 pooled pixels that the next stage reads are computed, enumerated plane by
-    // plane (a unit's 16 pixels are 16 consecutive rows of one plane: contiguous stores).
-    constexpr int n_pix = C1M_G * 144, n_units = (n_pix + 15) / 16;
-    for (int i = tid; i < C1M_UNITS * 16; i += C1M_THREADS) {
-        const bool exists = i < n_pix;
-        const int pc = exists ? i : 0;
-        const int gi = pc / 144, rem = pc - gi * 144;
-        const int plane = rem / 36, rloc = rem - plane * 36;
-        const int py = 2 * (rloc / 6) + (plane >> 1), px = 2 * (rloc % 6) + (plane & 1);
-        const uint32_t off = (uint32_t)(plane * a.plane_bytes) + (uint32_t)((gi * 36 + rloc) * 16);
-        pix_tab[i] = make_uint2((uint32_t)(gi * 224 + 2 * py * 8 + (px >> 1)) | ((uint32_t)(px & 1) << 16) | ((uint32_t)gi << 17) | ((uint32_t)exists << 20), off);
-    }
-    uint32_t wf[4][4]; int bias[4][2]; float mult[4][2];
+    uint32_t wf[4][4]; float flr[4][2]; float mult[4][2];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -136,13 +138,28 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) { bias[j][b] = __ldg(a.biasfrag + (j * 32 + lane) * 2 + b); mult[j][b] = __ldg(a.multfrag + (j * 32 + lane) * 2 + b); }
+        for (int b = 0; b < 2; ++b) { flr[j][b] = __ldg(a.floorfrag + (j * 32 + lane) * 2 + b); mult[j][b] = __ldg(a.multfrag + (j * 32 + lane) * 2 + b); }
+    int base_q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) asm volatile("mov.b32 %0, %1;" : "=r"(base_q[k]) : "n"(BASE ? kAccBaseBits : 0));   // (opaque: kept in a register quad)
     __syncthreads();                               // barriers and the abort flag are set up
 
     const float q_lo = (float)(-a.x_zp), q_hi = (float)(255 - a.x_zp);
-    // this thread's 8 channels: chunk t >> 1 (four parity planes further), half t & 1
-    int8_t* const y_thread = a.y + (size_t)(t >> 1) * 4 * (size_t)a.plane_bytes + (t & 1) * 8;
-    constexpr size_t img_bytes = 36 * 16;
+    // Only the 12 x 12 pooled pixels that the next stage reads are computed.  Rows g and g + 8 of unit k of this warp: image g % 4, pooled row
+    // warp / 3 + 4k, columns 4 (warp % 3) + g / 4 and the one two further; patch row t.  This thread's 8 channels: chunk t >> 1, half t & 1.
+    const int my_img = g & 3, odd = g >> 2;
+    const uint32_t sel = odd ? 0x5432u : 0x3210u;
+    const int word0 = my_img * C1M_IMG_WORDS + (warp / 3) * 16 + t * 8 + (warp % 3) * 2;
+    const int pixel = c2_pixel_bytes(a.ib);
+    int8_t* const y_thread = a.y + ((warp / 3) * 12 + (warp % 3) * 4 + odd) * pixel + (t >> 1) * (pixel >> 1) + my_img * 16 + (t & 1) * 8;
+    // The float4s that this thread quantizes: pooled rows and columns 0..11 read input rows 0..25 (26 rows of 7 float4)
+    constexpr int n_f4 = C1M_G * 182, F4 = (n_f4 + C1M_THREADS - 1) / C1M_THREADS;
+    int f_src[F4], f_dst[F4], f_img[F4];
+#pragma unroll
+    for (int k = 0; k < F4; ++k) {
+        const int i = tid + k * C1M_THREADS, gi = i / 182, p4 = i - gi * 182, r = p4 / 7;
+        f_src[k] = gi * 196 + p4; f_dst[k] = gi * C1M_IMG_WORDS + r * 8 + (p4 - r * 7); f_img[k] = i < n_f4 ? gi : C1M_G;
+    }
     int it = 0;
     for (int base = blockIdx.x * C1M_G; base < a.n_images; base += stride, ++it) {
         const int s = it & 1;
@@ -150,35 +167,32 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
         //      status word says so)
         ptx::mbar_wait(bar0 + 8 * s, (uint32_t)(it >> 1) & 1u, &abort_flag);
         // ---- quantize C1M_G images: float4 in, four uint8 out
-        uint32_t (*img)[28][8] = img2[s];
+        uint32_t* img = img2[s];
         const int n_here = min(C1M_G, a.n_images - base);
-        // pooled rows and columns 0..11 read input rows 0..25 only (26 rows of 7 float4)
-        constexpr int f4_per_img = 182;
-        for (int i = tid; i < C1M_G * f4_per_img; i += C1M_THREADS) {
-            const int gi = i / f4_per_img, p4 = i - gi * f4_per_img;        // 7 float4 per row
-            uint32_t word = 0;
-            if (gi < n_here && a.x_zp == 0) {
-                // zero point 0: sat_u8(rne(clamp(t, -512, 511))) is the float -> int32 conversion (rne, a NaN gives 0) followed
-                // by the pack instruction's own saturation to [0, 255]; no clamps, no adds (the ALU pipe bounds this kernel)
-                const float4 v = reinterpret_cast<const float4*>(stage[s])[gi * 196 + p4];
-                const int q0 = __float2int_rn(__fdiv_rn(v.x, a.x_scale)), q1 = __float2int_rn(__fdiv_rn(v.y, a.x_scale));
-                const int q2 = __float2int_rn(__fdiv_rn(v.z, a.x_scale)), q3 = __float2int_rn(__fdiv_rn(v.w, a.x_scale));
-                uint32_t hi;
-                asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q3), "r"(q2));
-                asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(word) : "r"(q1), "r"(q0), "r"(hi));
-            } else if (gi < n_here) {
-                const float4 v = reinterpret_cast<const float4*>(stage[s])[gi * 196 + p4];
-                // sat_u8(rne(clamp(t, -512, 511)) + zp) == rne(clamp(t, -zp, 255 - zp)) + zp: the bounds are integers
-                // inside [-512, 511] and rounding is monotonic; a NaN becomes the lower bound either way.
-                // (the proof-by-residual form of quantize_fast costs this kernel more issue slots than the division it saves)
-                const int q0 = __float2int_rn(fminf(fmaxf(__fdiv_rn(v.x, a.x_scale), q_lo), q_hi)) + a.x_zp;
-                const int q1 = __float2int_rn(fminf(fmaxf(__fdiv_rn(v.y, a.x_scale), q_lo), q_hi)) + a.x_zp;
-                const int q2 = __float2int_rn(fminf(fmaxf(__fdiv_rn(v.z, a.x_scale), q_lo), q_hi)) + a.x_zp;
-                const int q3 = __float2int_rn(fminf(fmaxf(__fdiv_rn(v.w, a.x_scale), q_lo), q_hi)) + a.x_zp;
-                word = (uint32_t)q0 | ((uint32_t)q1 << 8) | ((uint32_t)q2 << 16) | ((uint32_t)q3 << 24);
+#pragma unroll
+        for (int k = 0; k < F4; ++k) {
+            if (f_img[k] < n_here) {
+                uint32_t word;
+                float4 v = reinterpret_cast<const float4*>(stage[s])[f_src[k]];
+                if (a.q_rl != 0.0f) {
+                    v.x = quant_quotient(v.x, a.q_rh, a.q_rl); v.y = quant_quotient(v.y, a.q_rh, a.q_rl);
+                    v.z = quant_quotient(v.z, a.q_rh, a.q_rl); v.w = quant_quotient(v.w, a.q_rh, a.q_rl);
+                } else {
+                    v.x = __fdiv_rn(v.x, a.x_scale); v.y = __fdiv_rn(v.y, a.x_scale); v.z = __fdiv_rn(v.z, a.x_scale); v.w = __fdiv_rn(v.w, a.x_scale);
+                }
+                if (a.x_zp == 0) {
+                    // zero point 0: sat_u8(rne(clamp(t, -512, 511))) is the float -> int32 conversion (rne, a NaN gives 0) followed
+                    // by the pack instruction's own saturation to [0, 255]; no clamps, no adds (the ALU pipe bounds this kernel)
+                    word = pack_sat_u8x4(__float2int_rn(v.x), __float2int_rn(v.y), __float2int_rn(v.z), __float2int_rn(v.w));
+                } else {
+                    // sat_u8(rne(clamp(t, -512, 511)) + zp) == rne(clamp(t, -zp, 255 - zp)) + zp: the bounds are integers
+                    // inside [-512, 511] and rounding is monotonic; a NaN becomes the lower bound either way.
+                    const int q0 = __float2int_rn(fminf(fmaxf(v.x, q_lo), q_hi)) + a.x_zp, q1 = __float2int_rn(fminf(fmaxf(v.y, q_lo), q_hi)) + a.x_zp;
+                    const int q2 = __float2int_rn(fminf(fmaxf(v.z, q_lo), q_hi)) + a.x_zp, q3 = __float2int_rn(fminf(fmaxf(v.w, q_lo), q_hi)) + a.x_zp;
+                    word = (uint32_t)q0 | ((uint32_t)q1 << 8) | ((uint32_t)q2 << 16) | ((uint32_t)q3 << 24);
+                }
+                img[f_dst[k]] = word;
             }
-            const int r = p4 / 7, c4 = p4 - r * 7;
-            img[gi][r][c4] = word;
         }
         __syncthreads();
         // ---- every thread is done with the other ring slot (it was read one group ago): refill it
@@ -189,17 +203,14 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
             ptx::mbar_arrive_expect_tx(bar, bytes);
             ptx::bulk_g2s(ptx::smem_u32(&stage[s ^ 1][0]), a.x + (size_t)nb * C1M_IMG_FLOATS, bytes, bar);
         }
-        // ---- 16 pooled pixels per warp iteration
-        for (int u = warp; u < n_units; u += C1M_THREADS / 32) {
-            bool ok[2]; uint32_t afrag[2], out_off[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint2 e = pix_tab[u * 16 + g + 8 * h];
-                ok[h] = (e.x >> 20) != 0 && base + (int)((e.x >> 17) & 7u) < a.n_images;
-                out_off[h] = e.y;
-                const uint32_t* row = &img[0][0][0] + (e.x & 0xffffu) + t * 8;       // patch row t of the pooled pixel
-                afrag[h] = __byte_perm(row[0], row[1], (e.x & 0x10000u) ? 0x5432u : 0x3210u);
-            }
+        // ---- 16 pooled pixels per warp iteration (a group does not straddle blocks of 128 images)
+        int8_t* const y_group = y_thread + (size_t)(base >> 7) * (144 * 4096) + (base & 127) * 16;
+        const bool ok = base + my_img < a.n_images;
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t* row = img + word0 + k * 64;
+            const uint32_t x0 = row[0], x1 = row[1], x2 = row[2];
+            const uint32_t afrag[2] = {__byte_perm(x0, x1, sel), __byte_perm(x1, x2, sel)};
             uint32_t outw[2][2];
 #pragma unroll
             for (int jp = 0; jp < 2; ++jp) {          // two channel groups at a time -> one packed word per pixel
@@ -207,24 +218,27 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {
                     const int j = jp * 2 + jj;
-                    const int c[4] = {bias[j][0], bias[j][1], bias[j][0], bias[j][1]};
                     int d0[4], d1[4], d2[4], d3[4];
-                    mma_m16n8k16_u8s8(d0, afrag[0], afrag[1], wf[0][j], c);
-                    mma_m16n8k16_u8s8(d1, afrag[0], afrag[1], wf[1][j], c);
-                    mma_m16n8k16_u8s8(d2, afrag[0], afrag[1], wf[2][j], c);
-                    mma_m16n8k16_u8s8(d3, afrag[0], afrag[1], wf[3][j], c);
+                    mma_m16n8k16_u8s8(d0, afrag[0], afrag[1], wf[0][j], base_q);
+                    mma_m16n8k16_u8s8(d1, afrag[0], afrag[1], wf[1][j], base_q);
+                    mma_m16n8k16_u8s8(d2, afrag[0], afrag[1], wf[2][j], base_q);
+                    mma_m16n8k16_u8s8(d3, afrag[0], afrag[1], wf[3][j], base_q);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        r[jj][k] = rq_round(__vimax_s32_relu(__vimax3_s32(d0[k], d1[k], d2[k]), d3[k]), mult[j][k & 1]);   // max of the window and ReLU: two instructions
+                    for (int k = 0; k < 4; ++k) {
+                        const int mx = __vimax3_s32(d0[k], d1[k], d2[k]);
+                        const float f = flr[j][k & 1];                 // BASE: kAccBase - bias, else the bits of the bias
+                        const float v = BASE ? __fsub_rn(__int_as_float(__vimax3_s32(mx, d3[k], __float_as_int(f))), f)
+                                             : __int2float_rn(max(max(mx, d3[k]) + __float_as_int(f), 0));
+                        r[jj][k] = __float2int_rn(__fmul_rn(v, mult[j][k & 1]));
+                    }
                 }
                 outw[0][jp] = pack_sat_s8x4(r[0][0], r[0][1], r[1][0], r[1][1]);   // row g   : ch 8t+4jp .. +3
                 outw[1][jp] = pack_sat_s8x4(r[0][2], r[0][3], r[1][2], r[1][3]);   // row g+8
             }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (!ok[h]) continue;
-                int8_t* yo = y_thread + (size_t)base * img_bytes + out_off[h];
-                *reinterpret_cast<uint2*>(yo) = make_uint2(outw[h][0], outw[h][1]);
+            if (ok) {
+                int8_t* yo = y_group + k * (48 * pixel);
+                *reinterpret_cast<uint2*>(yo) = make_uint2(outw[0][0], outw[0][1]);
+                *reinterpret_cast<uint2*>(yo + 2 * pixel) = make_uint2(outw[1][0], outw[1][1]);
             }
         }
     }
@@ -232,68 +246,66 @@ __global__ void __launch_bounds__(C1M_THREADS, 3) conv1_mma_relu_pool_kernel(con
 }
 
 // =============================================================================================
-// Stage 2, pool windows on the MMA rows: QLinearConv(32 -> 64, 3x3, no pad) + ReLU + MaxPool 2x2/2 from the
-// parity-plane layout that stage 1 writes (Conv1MmaArgs::plane_bytes).
+// Stage 2: QLinearConv(32 -> 64, 3x3, no pad) + ReLU + MaxPool 2x2/2 on the image blocks that stage 1 writes.
 //
-// MMA row r of tile t is pool window R = t*128 + r of the whole batch: image R / 36, window (py, px) =
-// ((R % 36) / 6, (R % 36) % 6) (py, px < 5 exist).  The four members (dy, dx) of a window are four
-// accumulators (TMEM columns m*64 ..): member (dy, dx), tap (kh, kw) reads input pixel
-// (2py + dy + kh, 2px + dx + kw), which lies in parity plane ((dy+kh)&1, (dx+kw)&1) at row
-// R + ((dy+kh)>>1)*6 + ((dx+kw)>>1) -- the same 128 consecutive rows of that plane, shifted.  So a tile is
-// eight bulk copies (2 chunks x 4 planes, 136 rows of 16 bytes each) and 24 MMAs (12 of 128x128x32 that serve two
-// members at once, 12 of 128x64x32), and a thread
-// of the epilogue holds all four members of its window: max, bias, ReLU and requantisation happen in
-// registers on a quarter of the values, with no staging; a window's 64 channels leave as four 16-byte stores
-// into the GEMM-blocked layout [N/128][1600/16][128 images][16].
-//   warp 0 producer, warp 1 MMA issuer (TMEM: two sets of 4 x 64 columns, so the epilogue of a tile overlaps the
-//   MMAs of the next), warps 2-17 epilogue.
+// A tile is one pool window (py, px) of 128 images: MMA row r is image 128 * block + r.  The four members (dy, dx) of the window are four
+// accumulators of 64 columns, in the order (0,0), (0,1), (1,1), (1,0), so that nearly every view's members are neighbours: the view
+// (ry, rx), 0..3 each, serves the members with ry - dy and rx - dx in 0..2 - the four inner views all of them (one 128x256x32 MMA), the
+// edges two (128x128x32; for rx = 0 the two are the outer ones: two of 128x64x32), the corners one.  18 MMAs a tile, 1152 cycles of math and 1152
+// of shared-memory operands.  (Windows of a row-major plane on the MMA rows, 36 rows per image of which 25 are windows, took 24 MMAs of N = 64 and
+// 128 for 3.6 images' worth: 133 us at batch 65536, against 99 here.)
+//
+// An item is a row of five windows (block, py), or one window where the rows are fewer than the SMs.  Its input is six (two) column pairs of 4 x 2
+// pixels, 32 KB each, of which a window reads two: a ring of five stages, each read by two windows.
+//   warp 0 producer, warp 1 MMA issuer (the whole warp runs the loop, one lane issues; TMEM: two sets of 4 x 64 columns, so the epilogue of a
+//   tile overlaps the MMAs of the next), warps 2-17 epilogue: a thread holds all four members of its window for 16 filters - max, bias, ReLU
+//   and requantisation in registers, one 16-byte store into the GEMM-blocked layout [N/128][1600/16][ib images][16], 512 contiguous bytes a warp.
 // =============================================================================================
-// Optional per-role cycle counters of the kernel below (debug builds with -DZB_TC_CONV_TIMERS only).
-#ifdef ZB_TC_CONV_TIMERS
-__device__ unsigned long long g_c2_timers[256 * 8];
-#define ZB_C2T_DECL() long long c2t_[8] = {0, 0, 0, 0, 0, 0, 0, 0}; long long c2t0_ = clock64()
-#define ZB_C2T(slot) do { const long long n_ = clock64(); c2t_[slot] += n_ - c2t0_; c2t0_ = n_; } while (0)
-#define ZB_C2T_DUMP(lo, hi) do { for (int i_ = (lo); i_ < (hi); ++i_) g_c2_timers[blockIdx.x * 8 + i_] = (unsigned long long)c2t_[i_]; } while (0)
-#else
-#define ZB_C2T_DECL() do {} while (0)
-#define ZB_C2T(slot) do {} while (0)
-#define ZB_C2T_DUMP(lo, hi) do {} while (0)
-#endif
-
-struct TcConvParityArgs {
-    const int8_t* x; long long plane_bytes;
-    const int8_t* w;                 // [9 taps][2 chunks][64][16] int8, then the paired blocks (TcConvParityCfg::W_ALL_BYTES)
-    float mult[64]; int32_t bias[64];   // per filter; bias includes -x_zp * sum(w); constant-bank operands
+struct TcConvPoolArgs {
+    const int8_t* x;
+    const int8_t* w;                    // tc_conv_pool_weights
+    float mult[64], bias[64];           // per filter, constant-bank operands; bias - x_zp * sum(w) as kAccBase - bias (BASE), else its bits
     int8_t* y;
-    int n_images, n_tiles;           // n_tiles = ceil(n_images * 36 / 128)
+    int n_images, ib, items, wins;      // images per block, items, windows per item (5 or 1)
     int* status;
 };
 
-struct TcConvParityCfg {
-    static constexpr int ROWS = 136;                         // 128 + the largest shift (7), rounded up to 8
-    static constexpr int PLANE_BYTES = ROWS * 16;
-    static constexpr int STAGE_BYTES = 8 * PLANE_BYTES;
-    static constexpr int STAGES = 6;                         // 104 KB of stages: also keeps a second CTA (which would wait for TMEM) off the SM
-    static constexpr int W_TAP_BYTES = 2 * 64 * 16;
-    static constexpr int W_BYTES = 9 * W_TAP_BYTES;
-    // paired blocks after the nine taps: [kh][j][2 chunks][128 rows][16]; j = 0: rows 0-63 tap (kh,1), rows 64-127 tap
-    // (kh,0); j = 1: rows 0-63 tap (kh,2), rows 64-127 tap (kh,1)   (member dx = 0 first, then dx = 1)
-    static constexpr int W_PAIR_BYTES = 2 * 128 * 16;
-    static constexpr int W_ALL_BYTES = W_BYTES + 6 * W_PAIR_BYTES;
-    static constexpr int OFF_W = 0;
-    static constexpr int OFF_A = OFF_W + W_ALL_BYTES;
-    static constexpr int OFF_BAR = OFF_A + STAGES * STAGE_BYTES;
-    static constexpr int SMEM_BYTES = OFF_BAR + 256;
-    static constexpr int TMEM_COLS = 512;                    // 2 sets x 4 members x 64 filters
-    static constexpr int THREADS = 576;                      // producer, MMA issuer, 16 epilogue warps
-    // rows of a plane that a batch needs: every tile copies ROWS rows from its first row
-    static long long plane_rows(long long n_tiles) { return n_tiles * 128 + (ROWS - 128); }
+struct TcConvPoolCfg {
+    static constexpr int STAGES = 5, STAGE_BYTES = 8 * c2_pixel_bytes(128);      // [ry][column of the pair][chunk][128][16]
+    // weights: for each inner view [chunk][4 members][64][16]; then three chains [chunk][3 taps][64][16] for the edges and corners
+    static constexpr int W_VIEW_BYTES = 2 * 256 * 16, W_CHAIN_BYTES = 2 * 192 * 16;
+    static constexpr int W_BYTES = 4 * W_VIEW_BYTES + 3 * W_CHAIN_BYTES;
+    static constexpr int OFF_A = W_BYTES, OFF_BAR = OFF_A + STAGES * STAGE_BYTES, SMEM_BYTES = OFF_BAR + 256;
+    static constexpr int TMEM_COLS = 512, THREADS = 576;
 };
+static_assert(TcConvPoolCfg::OFF_A % 128 == 0 && TcConvPoolCfg::SMEM_BYTES <= 227 * 1024, "");
 
-__global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_parity_kernel(const __grid_constant__ TcConvParityArgs a) {
-    using Cfg = TcConvParityCfg;
+// One MMA of a tile: the view it reads, where its filters start (bytes into the weights) and how far their second K chunk lies, N, accumulator column.
+struct TcConvPoolMma { int ry, rx, w, lbo, n, col; };
+
+// w: [64][32][3][3]
+inline void tc_conv_pool_weights(const int8_t* w, int8_t* out) {
+    auto block = [&](int8_t* dst, int chunk, int tap) {
+        for (int m = 0; m < 64; ++m)
+            for (int c = 0; c < 16; ++c) dst[m * 16 + c] = w[(m * 32 + chunk * 16 + c) * 9 + tap];
+    };
+    const int order[4][2] = {{0, 0}, {0, 1}, {1, 1}, {1, 0}};
+    for (int v = 0; v < 4; ++v)
+        for (int chunk = 0; chunk < 2; ++chunk)
+            for (int j = 0; j < 4; ++j)
+                block(out + v * TcConvPoolCfg::W_VIEW_BYTES + (chunk * 4 + j) * 1024, chunk, (1 + v / 2 - order[j][0]) * 3 + 1 + v % 2 - order[j][1]);
+    const int chains[3][3] = {{2, 1, 0}, {6, 7, 8}, {8, 5, 2}};
+    for (int e = 0; e < 3; ++e)
+        for (int chunk = 0; chunk < 2; ++chunk)
+            for (int j = 0; j < 3; ++j)
+                block(out + 4 * TcConvPoolCfg::W_VIEW_BYTES + e * TcConvPoolCfg::W_CHAIN_BYTES + (chunk * 3 + j) * 1024, chunk, chains[e][j]);
+}
+
+template <bool BASE>
+__global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_kernel(const __grid_constant__ TcConvPoolArgs a) {
+    using Cfg = TcConvPoolCfg;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sW = smem + Cfg::OFF_W;
+    uint8_t* sW = smem;
     uint8_t* sA = smem + Cfg::OFF_A;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 128);
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_parity_kernel(const __
         *abort_flag = 0;
         ptx::mbar_fence_init();
     }
-    for (int i = tid; i < Cfg::W_ALL_BYTES / 16; i += Cfg::THREADS)
+    for (int i = tid; i < Cfg::W_BYTES / 16; i += Cfg::THREADS)
         reinterpret_cast<uint4*>(sW)[i] = __ldg(reinterpret_cast<const uint4*>(a.w) + i);
     ptx::fence_proxy_async_smem();
     if (warp == 1) {
@@ -325,123 +337,121 @@ __global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_parity_kernel(const __
     ptx::grid_trigger();
     ptx::grid_wait();
 
+    const int pixel = c2_pixel_bytes(a.ib);
     if (warp == 0) {
-        // ------------------------------------------------------------------ producer
+        // ------------------------------------------------------------------ producer: the column pairs of the items
         if (ptx::elect_one()) {
-            int it = 0;
-            ZB_C2T_DECL();
-            for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (uint32_t)(it / Cfg::STAGES) & 1u;
-                if (!ptx::mbar_wait(empty(s), ph ^ 1u, abort_flag)) break;
-                ZB_C2T(3);
-                ptx::mbar_arrive_expect_tx(full(s), Cfg::STAGE_BYTES);
-                const int8_t* src = a.x + (size_t)t * (128 * 16);
-                const uint32_t dst = ptx::smem_u32(sA + s * Cfg::STAGE_BYTES);
+            int s = 0; uint32_t ph = 0;
+            bool alive = true;
+            for (int item = blockIdx.x; item < a.items && alive; item += gridDim.x) {
+                const int win = item * a.wins, nb = win / 25, py = (win - nb * 25) / 5, px0 = win % 5;
+                const int8_t* src = a.x + (size_t)nb * (144 * pixel) + (size_t)((2 * py) * 12 + 2 * px0) * pixel;
+                for (int cp = 0; cp <= a.wins; ++cp, src += 2 * pixel) {
+                    if (!ptx::mbar_wait(empty(s), ph ^ 1u, abort_flag)) { alive = false; break; }
+                    const uint32_t dst = ptx::smem_u32(sA + s * Cfg::STAGE_BYTES);
+                    // (a last block's images that do not exist: whatever is there)
+                    ptx::mbar_arrive_expect_tx(full(s), (uint32_t)(8 * pixel));
 #pragma unroll
-                for (int pl = 0; pl < 8; ++pl)
-                    ptx::bulk_g2s(dst + (uint32_t)(pl * Cfg::PLANE_BYTES), src + (size_t)pl * (size_t)a.plane_bytes, Cfg::PLANE_BYTES, full(s));
-                ZB_C2T(7);
+                    for (int ry = 0; ry < 4; ++ry)
+                        ptx::bulk_g2s(dst + (uint32_t)(ry * 2 * pixel), src + (size_t)(ry * 12) * pixel, (uint32_t)(2 * pixel), full(s));
+                    if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+                }
             }
-            ZB_C2T_DUMP(3, 4);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (ptx::elect_one()) {
-            constexpr uint32_t idesc64 = ptx::idesc_i8(128, 64, true, true), idesc128 = ptx::idesc_i8(128, 128, true, true);
-            const uint32_t w_addr = ptx::smem_u32(sW);
-            int it = 0;
-            ZB_C2T_DECL();
-            for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (uint32_t)(it / Cfg::STAGES) & 1u;
+        // In this order an MMA rarely follows one that writes part of its columns in another shape: it would wait for that one to drain.
+        constexpr TcConvPoolMma M[18] = {
+            // inner views: member (dy, dx) takes tap (ry - dy, rx - dx)
+            {1, 1, 0, 4096, 256, 0}, {1, 2, 8192, 4096, 256, 0}, {2, 1, 16384, 4096, 256, 0}, {2, 2, 24576, 4096, 256, 0},
+            // chain 2, taps (2,2) (1,2) (0,2): members (0,1) and (1,1)
+            {1, 3, 45056 + 1024, 3072, 128, 64}, {2, 3, 45056, 3072, 128, 64},
+            // rx = 0, members (0,0) and (1,0): tap (1,0) is the second block of the first inner view
+            {1, 0, 1024, 4096, 64, 0}, {2, 0, 38912, 3072, 64, 0}, {0, 0, 32768 + 2048, 3072, 64, 0},
+            {1, 0, 32768 + 2048, 3072, 64, 192}, {2, 0, 1024, 4096, 64, 192}, {3, 0, 38912, 3072, 64, 192},
+            {0, 3, 32768, 3072, 64, 64}, {3, 3, 38912 + 2048, 3072, 64, 128},
+            // chain 0, taps (0,2) (0,1) (0,0), and chain 1, taps (2,0) (2,1) (2,2)
+            {0, 1, 32768 + 1024, 3072, 128, 0}, {0, 2, 32768, 3072, 128, 0}, {3, 1, 38912, 3072, 128, 128}, {3, 2, 38912 + 1024, 3072, 128, 128},
+        };
+        const uint32_t leader = ptx::elect_one() ? 1u : 0u;
+        auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag)) != 0; };
+        const uint64_t da = ptx::smem_desc_kmajor(0, (uint32_t)pixel >> 1, 128);
+        const uint32_t pixel_u = (uint32_t)pixel >> 4;
+        const uint32_t hi = (uint32_t)(da >> 32), a_lo0 = (uint32_t)da + (ptx::smem_u32(sA) >> 4), w_lo0 = ptx::smem_u32(sW) >> 4;
+        int s = 0, it = 0; uint32_t ph = 0;                       // stage of the window's left column pair
+        bool alive = true;
+        for (int item = blockIdx.x; item < a.items && alive; item += gridDim.x) {
+            for (int px = 0; px < a.wins; ++px, ++it) {
                 const int b = it & 1;
-                const uint32_t bph = (uint32_t)(it >> 1) & 1u;
-                if (!ptx::mbar_wait(tempty(b), bph ^ 1u, abort_flag)) break;
-                ZB_C2T(0);
-                if (!ptx::mbar_wait(full(s), ph, abort_flag)) break;
-                ZB_C2T(1);
+                const int s1 = s + 1 == Cfg::STAGES ? 0 : s + 1;
+                const uint32_t ph1 = s1 == 0 ? ph ^ 1u : ph;
+                alive = wait(tempty(b), ((uint32_t)(it >> 1) & 1u) ^ 1u) && (px > 0 || wait(full(s), ph)) && wait(full(s1), ph1);
+                if (!alive) break;
                 ptx::tc_fence_after();
-                const uint32_t a_addr = ptx::smem_u32(sA + s * Cfg::STAGE_BYTES);
-                // Input pixel (2py + ry, 2px + rx), ry = dy + kh, rx = dx + kw, 0..3 each: one shifted view of one plane.
-                // The view (ry, rx = 1 or 2) serves both members dx = 0 (kw = rx) and dx = 1 (kw = rx - 1) of a row dy:
-                // one MMA of 128 filters-times-members over the paired weight block instead of two of 64 (an N = 64
-                // MMA is bound by its 6 KB of shared-memory operands, not by its 32 cycles of math).
+                const uint32_t left = a_lo0 + (uint32_t)(s * (Cfg::STAGE_BYTES / 16)), right = a_lo0 + (uint32_t)(s1 * (Cfg::STAGE_BYTES / 16));
+                const uint32_t d = tmem_base + (uint32_t)(b * 256);
 #pragma unroll
-                for (int kh = 0; kh < 3; ++kh) {
-#pragma unroll
-                    for (int dy = 0; dy < 2; ++dy) {
-                        const int ry = dy + kh;
-                        auto view = [&](int rx) {
-                            const int plane = (ry & 1) * 2 + (rx & 1), shift = (ry >> 1) * 6 + (rx >> 1);
-                            return ptx::smem_desc_kmajor(a_addr + (uint32_t)(plane * Cfg::PLANE_BYTES + shift * 16), 4 * Cfg::PLANE_BYTES, 128);
-                        };
-                        auto w64 = [&](int kw) { return ptx::smem_desc_kmajor(w_addr + (uint32_t)((kh * 3 + kw) * Cfg::W_TAP_BYTES), 64 * 16, 128); };
-                        auto w128 = [&](int j) { return ptx::smem_desc_kmajor(w_addr + (uint32_t)(Cfg::W_BYTES + (kh * 2 + j) * Cfg::W_PAIR_BYTES), 128 * 16, 128); };
-                        const uint32_t d = tmem_base + (uint32_t)(b * 256 + dy * 128);     // members (dy, 0) and (dy, 1): 2 x 64 columns
-                        ptx::mma_i8(d, view(1), w128(0), idesc128, kh > 0);               // the first MMA of a set initialises both members
-                        ptx::mma_i8(d, view(2), w128(1), idesc128, true);
-                        ptx::mma_i8(d, view(0), w64(0), idesc64, true);
-                        ptx::mma_i8(d + 64u, view(3), w64(2), idesc64, true);
-                    }
+                for (int i = 0; i < 18; ++i) {
+                    const uint32_t al = (M[i].rx < 2 ? left : right) + (uint32_t)(M[i].ry * 2 + (M[i].rx & 1)) * pixel_u;
+                    const uint32_t bl = w_lo0 + (uint32_t)((M[i].w >> 4) | ((M[i].lbo >> 4) << 16));
+                    ptx::mma_i8_if(leader, d + (uint32_t)M[i].col, al, hi, bl, hi, ptx::idesc_i8(128, M[i].n, true, true), i > 0 ? 1u : 0u);   // the first initialises all members
                 }
-                ptx::mma_commit(empty(s));
-                ptx::mma_commit(tfull(b));
-                ZB_C2T(2);
+                ptx::mma_commit_if(leader, empty(s));
+                if (px == a.wins - 1) ptx::mma_commit_if(leader, empty(s1));
+                ptx::mma_commit_if(leader, tfull(b));
+                s = s1; ph = ph1;
             }
-            ZB_C2T_DUMP(0, 3);
+            if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }          // the next item starts behind the last pair
         }
     } else {
         // ------------------------------------------------------------------ epilogue: 16 warps, four per TMEM lane
-        // quarter; each takes 16 of the 64 filters of its quarter's 32 windows, in every tile (a single warp per
+        // quarter; each takes 16 of the 64 filters of its quarter's 32 images, in every tile (a single warp per
         // quarter and tile would be latency-bound and slower than the MMAs of the next tile).
         const int quarter = warp & 3;               // TMEM lane quarter this warp may access
         const int cg = (warp - 2) >> 2;             // 16-filter group of this warp
-        const int row = quarter * 32 + lane;        // MMA row = pool window within the tile
-        float mult[16]; int bias[16];
+        const int row = quarter * 32 + lane;        // MMA row = image within the block
+        float mult[16], flr[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) { mult[j] = a.mult[cg * 16 + j]; bias[j] = a.bias[cg * 16 + j]; }
+        for (int j = 0; j < 16; ++j) { mult[j] = a.mult[cg * 16 + j]; flr[j] = a.bias[cg * 16 + j]; }
         int it = 0;
-        ZB_C2T_DECL();
-        for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-            const int b = it & 1;
-            const uint32_t bph = (uint32_t)(it >> 1) & 1u;
-            int ok = 1;
-            if (lane == 0) ok = ptx::mbar_wait(tfull(b), bph, abort_flag) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
-            ZB_C2T(4);
-            ptx::tc_fence_after();
-            const int R = t * 128 + row;
-            const int n = R / 36, q = R - 36 * n;
-            const int py = q / 6, px = q - py * 6;
-            const bool live = n < a.n_images && py < 5 && px < 5;
-            int8_t* yw = a.y + (size_t)(n >> 7) * (1600 / 16) * 2048 + (size_t)(n & 127) * 16 + (size_t)((py * 5 + px) * 4 + cg) * 2048;
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 256 + cg * 16);
-            uint32_t v[4][16];
+        bool alive = true;
+        for (int item = blockIdx.x; item < a.items && alive; item += gridDim.x) {
+            const int win = item * a.wins, nb = win / 25;
+            const bool live = nb * 128 + row < a.n_images;
+            int8_t* yw = a.y + ((size_t)nb * 100 + (win - nb * 25) * 4 + cg) * (size_t)(a.ib * 16) + (size_t)row * 16;
+            for (int px = 0; px < a.wins; ++px, ++it, yw += 4 * a.ib * 16) {
+                const int b = it & 1;
+                int ok = 1;
+                if (lane == 0) ok = ptx::mbar_wait(tfull(b), (uint32_t)(it >> 1) & 1u, abort_flag) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) { alive = false; break; }
+                ptx::tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 256 + cg * 16);
+                uint32_t v[4][16];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * 64), v[m]);
-            ptx::tmem_wait_ld();
-            ZB_C2T(5);
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(tempty(b));   // this warp has its values: the set may be overwritten once all 16 arrived
-            uint32_t pk[4];
+                for (int m = 0; m < 4; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * 64), v[m]);
+                ptx::tmem_wait_ld();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(tempty(b));   // this warp has its values: the set may be overwritten once all 16 arrived
+                uint32_t pk[4];
 #pragma unroll
-            for (int j4 = 0; j4 < 4; ++j4) {
-                int r[4];
+                for (int j4 = 0; j4 < 4; ++j4) {
+                    int r[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c = j4 * 4 + j;
-                    const int mx = max(__vimax3_s32((int)v[0][c], (int)v[1][c], (int)v[2][c]), (int)v[3][c]);
-                    r[j] = rq_round(mx + bias[c], mult[c]);
+                    for (int j = 0; j < 4; ++j) {
+                        const int c = j4 * 4 + j;
+                        const int mx = max(__vimax3_s32((int)v[0][c], (int)v[1][c], (int)v[2][c]), (int)v[3][c]);
+                        // bias and ReLU (kAccBase: one instruction, and a subtraction gives the float)
+                        const float f = BASE ? __fsub_rn(__int_as_float(__viaddmax_s32(mx, kAccBaseBits, __float_as_int(flr[c]))), flr[c])
+                                             : __int2float_rn(max(mx + __float_as_int(flr[c]), 0));
+                        r[j] = __float2int_rn(__fmul_rn(f, mult[c]));
+                    }
+                    pk[j4] = pack_sat_s8x4(r[0], r[1], r[2], r[3]);
                 }
-                pk[j4] = relu_s8x4(pack_sat_s8x4(r[0], r[1], r[2], r[3]));
+                if (live) *reinterpret_cast<uint4*>(yw) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             }
-            if (live) *reinterpret_cast<uint4*>(yw) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            ZB_C2T(6);
         }
-        if (warp == 2 && lane == 0) ZB_C2T_DUMP(4, 7);
     }
 
     // ---------------------------------------------------------------------- teardown

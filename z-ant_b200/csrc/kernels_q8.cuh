@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "geometry.hpp"
@@ -49,6 +50,38 @@ __device__ __forceinline__ int quantize_fast(float x, const QuantFast& q) {
     if (proved) return (int)k;
     return __float2int_rn(fminf(fmaxf(__fdiv_rn(x, q.scale), q.lo), q.hi));
 }
+
+// fl(x / scale) before the rounding to an integer, in two instructions: fma(x, rh, x * rl) with rh the largest float below
+// 1 / scale and rl = fl(1 / scale - rh) > 0.  Both products and the sum are non-decreasing in x, as is the reference's
+// rne(clamp(fl(x / scale), lo, hi)), so the two agree for every x if and only if they agree on both sides of each of the hi - lo steps of
+// the reference: quant_steps finds the steps by bisection over the floats and compares there.  Infinities keep their sign (rl > 0), a NaN
+// stays one.  The division itself costs eight instructions and a branch.
+struct QuantSteps { float rh, rl; };
+
+inline bool quant_steps(float scale, int lo, int hi, QuantSteps& q) {
+    if (!(scale > 1.0e-30f) || !(scale < 1.0e30f) || lo >= hi || lo < -512 || hi > 511) return false;
+    const double inv = 1.0 / (double)scale;
+    float rh = (float)inv;
+    if ((double)rh >= inv) rh = std::nextafterf(rh, 0.0f);
+    q.rh = rh; q.rl = (float)(inv - (double)rh);
+    if (!(q.rl > 0.0f)) return false;
+    auto code = [&](float t) { return (int)std::nearbyintf(std::fmin(std::fmax(t, (float)lo), (float)hi)); };
+    auto ref = [&](float x) { volatile float t = x / scale; return code(t); };
+    auto fast = [&](float x) { volatile float p = x * q.rl; return code(std::fma(x, q.rh, p)); };
+    // floats in ascending order as integers
+    auto to_float = [](int32_t i) { const int32_t b = i >= 0 ? i : (int32_t)(0x80000000u - (uint32_t)i); float f; std::memcpy(&f, &b, 4); return f; };
+    auto to_int = [](float f) { int32_t b; std::memcpy(&b, &f, 4); return b >= 0 ? b : (int32_t)(0x80000000u - (uint32_t)b); };
+    for (int k = lo; k < hi; ++k) {
+        // the smallest x whose code is above k: close to (k + 0.5) * scale
+        int32_t a = to_int((float)(((double)k + 0.5) * scale)) - 8, b = a + 16;
+        if (ref(to_float(a)) > k || ref(to_float(b)) <= k) return false;
+        while (b - a > 1) { const int32_t mid = a + (b - a) / 2; if (ref(to_float(mid)) > k) b = mid; else a = mid; }
+        if (ref(to_float(b)) != k + 1 || fast(to_float(b)) != k + 1 || fast(to_float(a)) != k) return false;
+    }
+    return true;
+}
+
+__device__ __forceinline__ float quant_quotient(float x, float rh, float rl) { return __fmaf_rn(x, rh, __fmul_rn(x, rl)); }
 
 template <bool U8> __device__ __forceinline__ int sat_q(int t) {
     return U8 ? min(max(t, 0), 255) : min(max(t, -128), 127);

@@ -1593,33 +1593,26 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     // ---- stage 2 parameters
     std::vector<float> m2; std::vector<int32_t> b2;
     if (!scales_of(c2, 64, m2) || !bias_of(c2, 64, b2)) return ZANT_OK;
-    std::vector<int8_t> w2arr(TcConvParityCfg::W_ALL_BYTES);      // nine taps, then the paired blocks
+    std::vector<int8_t> w2arr(TcConvPoolCfg::W_BYTES);
+    bool acc_base2 = true;                                          // accumulators and biases small enough for kAccBase
     {
         const int8_t* w = (const int8_t*)T(c2.in[1]).host.data();   // [64][32][3][3]
         for (int m = 0; m < 64; ++m) {
             int sum = 0;
-            for (int ch = 0; ch < 32; ++ch)
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int8_t v = w[(m * 32 + ch) * 9 + tap];
-                    w2arr[((tap * 2 + ch / 16) * 64 + m) * 16 + ch % 16] = v;
-                    sum += v;
-                }
+            long long abs_sum = 0;
+            for (int i = 0; i < 288; ++i) { sum += w[m * 288 + i]; abs_sum += std::abs((int)w[m * 288 + i]); }
             b2[m] -= c2.a.x_zp * sum;
+            acc_base2 = acc_base2 && acc_base_ok(b2[m]) && std::abs((long long)b2[m]) + 128 * abs_sum < (1 << 22);
         }
-        // paired blocks [kh][j][chunk][128 rows][16]: rows 0-63 tap (kh, j + 1), rows 64-127 tap (kh, j)
-        for (int kh = 0; kh < 3; ++kh)
-            for (int j = 0; j < 2; ++j)
-                for (int chunk = 0; chunk < 2; ++chunk)
-                    for (int r = 0; r < 128; ++r) {
-                        const int tap = kh * 3 + (r < 64 ? j + 1 : j), m = r & 63;
-                        std::memcpy(&w2arr[TcConvParityCfg::W_BYTES + (size_t)(((kh * 2 + j) * 2 + chunk) * 128 + r) * 16],
-                                    &w2arr[(size_t)((tap * 2 + chunk) * 64 + m) * 16], 16);
-                    }
+        tc_conv_pool_weights(w, w2arr.data());
     }
     // ---- fc1: rows re-ordered from the graph's (c,h,w) flatten order to the (h,w,c) order stage 2 writes
     std::vector<float> m3; std::vector<int32_t> b3;
     if (!scales_of(f1, 512, m3) || !bias_of(f1, 512, b3)) return ZANT_OK;
-    constexpr int FC_NT = 256, FC_KC = 4, FC_STAGES = 8;
+    // the narrowest column tile whose grid fits the SMs: a CTA streams all of K for its columns (batch 1: 12.6 us with two CTAs of 256)
+    constexpr int FC_KC = 4, FC_STAGES = 8;
+    int FC_NT = 256;
+    while (FC_NT > 32 && (int)((B + 127) / 128) * (512 / (FC_NT / 2)) <= pl->ctx->sm_count) FC_NT /= 2;
     std::vector<int8_t> w3blk(1600 * 512);      // [512/NT][100 chunks][NT][16], K in (h,w,c) order
     {
         const int8_t* w = (const int8_t*)T(f1.in[1]).host.data();   // [1600][512], row = c*25 + h*5 + w
@@ -1628,9 +1621,10 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
             for (int hw = 0; hw < 25; ++hw) {
                 const int k = hw * 64 + ch;                         // position in the order stage 2 writes
                 const int8_t* src = &w[(size_t)(ch * 25 + hw) * 512];
-                for (int n = 0; n < 512; ++n) {
-                    w3blk[(((size_t)(n / FC_NT) * 100 + k / 16) * FC_NT + n % FC_NT) * 16 + k % 16] = src[n];
-                    colsum[n] += src[n];
+                for (int n = 0; n < 512; ++n) colsum[n] += src[n];
+                for (int n0 = 0; n0 < 512; n0 += FC_NT) {
+                    int8_t* dst = &w3blk[((size_t)n0 * 100 + (size_t)(k / 16) * FC_NT) * 16 + k % 16];
+                    for (int n = 0; n < FC_NT; ++n) dst[n * 16] = src[n0 + n];
                 }
             }
         for (int n = 0; n < 512; ++n) b3[n] -= f1.a.x_zp * colsum[n];
@@ -1646,12 +1640,10 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         }
     }
 
-    // stage 1 -> stage 2 hand-over: parity planes (TcConvParityCfg), every tile of stage 2 copies 136 rows of each plane
-    const long long c2_tiles = ((long long)B * 36 + 127) / 128;
-    const long long plane_bytes = (TcConvParityCfg::plane_rows(c2_tiles) * 16 + 255) / 256 * 256;
-    const int s_pool1 = pl->add_scratch((size_t)(8 * plane_bytes));
-    const size_t Bpad = (B + 127) / 128 * 128;
-    const int s_pool2 = pl->add_scratch(Bpad * 1600);
+    // stage 1 -> stage 2 hand-over: image blocks
+    const int ib = (int)std::min<size_t>(B, 128), blocks128 = (int)((B + 127) / 128);
+    const int s_pool1 = pl->add_scratch(blocks128 * (size_t)c2_block_bytes(ib));
+    const int s_pool2 = pl->add_scratch((size_t)blocks128 * ib * 1600);
     const int s_fc1 = pl->add_scratch(B * 512);
     const int a_w2 = pl->add_aux(w2arr.data(), w2arr.size());
     const int a_w3 = pl->add_aux(w3blk.data(), w3blk.size());
@@ -1661,8 +1653,9 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
 
     // B-fragment words, bias and multipliers in the per-lane order of the warp-level MMA
     std::vector<uint32_t> wfrag(4 * 4 * 32);
-    std::vector<int32_t> biasfrag(4 * 32 * 2);
-    std::vector<float> multfrag(4 * 32 * 2);
+    bool acc_base = true;
+    for (int m = 0; m < 32; ++m) acc_base = acc_base && acc_base_ok(a1.bias[m]);
+    std::vector<float> floorfrag(4 * 32 * 2), multfrag(4 * 32 * 2);
     {
         const int8_t* w = (const int8_t*)T(c1.in[1]).host.data();   // [32][1][3][3]
         for (int lane = 0; lane < 32; ++lane) {
@@ -1680,48 +1673,62 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
                 }
                 for (int b = 0; b < 2; ++b) {
                     const int cc = 8 * t + 2 * j + b;                // the lane's accumulator columns 2t, 2t+1
-                    biasfrag[(j * 32 + lane) * 2 + b] = a1.bias[cc];
+                    floorfrag[(j * 32 + lane) * 2 + b] = acc_base ? kAccBase - (float)a1.bias[cc] : int_bits_as_float(a1.bias[cc]);
                     multfrag[(j * 32 + lane) * 2 + b] = a1.mult[cc];
                 }
             }
         }
     }
+    QuantSteps steps{};
+    if (a1.x_zp < 0 || a1.x_zp > 255 || !quant_steps(a1.x_scale, -a1.x_zp, 255 - a1.x_zp, steps)) steps = QuantSteps{0.0f, 0.0f};
     const int a_wf = pl->add_aux(wfrag.data(), wfrag.size() * 4);
-    const int a_bf = pl->add_aux(biasfrag.data(), biasfrag.size() * 4);
+    const int a_bf = pl->add_aux(floorfrag.data(), floorfrag.size() * 4);
     const int a_mf = pl->add_aux(multfrag.data(), multfrag.size() * 4);
     push("Fused[QuantizeLinear+QLinearConv+Relu+MaxPool] mma", [=]() {
         Conv1MmaArgs k{};
-        k.x = pl->p<float>(x); k.y = (int8_t*)pl->scratch(s_pool1); k.n_images = (int)B;
-        k.x_scale = a1.x_scale; k.x_zp = a1.x_zp;
-        k.wfrag = (const uint32_t*)pl->aux(a_wf); k.biasfrag = (const int32_t*)pl->aux(a_bf); k.multfrag = (const float*)pl->aux(a_mf); k.status = ctx->status_word; k.plane_bytes = plane_bytes;
-        const int blocks = std::min<int>((int)((B + C1M_G - 1) / C1M_G), ctx->sm_count * 8);
-        launch(ctx, conv1_mma_relu_pool_kernel, blocks, C1M_THREADS, 0, k);
+        k.x = pl->p<float>(x); k.y = (int8_t*)pl->scratch(s_pool1); k.n_images = (int)B; k.ib = ib;
+        k.x_scale = a1.x_scale; k.x_zp = a1.x_zp; k.q_rh = steps.rh; k.q_rl = steps.rl;
+        k.wfrag = (const uint32_t*)pl->aux(a_wf); k.floorfrag = (const float*)pl->aux(a_bf); k.multfrag = (const float*)pl->aux(a_mf); k.status = ctx->status_word;
+        const int blocks = std::min<int>((int)((B + C1M_G - 1) / C1M_G), ctx->sm_count * 2);
+        launch(ctx, acc_base ? conv1_mma_relu_pool_kernel<true> : conv1_mma_relu_pool_kernel<false>, blocks, C1M_THREADS, 0, k);
         return check_launch(ctx, "conv1_mma_relu_pool_kernel");
     });
     push("Fused[QLinearConv+Relu+MaxPool] tcgen05", [=]() {
-        using Cfg = TcConvParityCfg;
-        ZB_SMEM_ATTR(ctx, (tc_conv3x3_pool_parity_kernel), Cfg::SMEM_BYTES);
-        TcConvParityArgs k{};
-        k.x = (const int8_t*)pl->scratch(s_pool1); k.plane_bytes = plane_bytes; k.w = (const int8_t*)pl->aux(a_w2);
-        for (int m = 0; m < 64; ++m) { k.mult[m] = m2[m]; k.bias[m] = b2[m]; }
-        k.y = (int8_t*)pl->scratch(s_pool2); k.n_images = (int)B; k.n_tiles = (int)c2_tiles; k.status = ctx->status_word;
-        const int blocks = std::min<int>((int)c2_tiles, ctx->sm_count);
-        launch_const(ctx, tc_conv3x3_pool_parity_kernel, blocks, Cfg::THREADS, Cfg::SMEM_BYTES, k);
-        return check_launch(ctx, "tc_conv3x3_pool_parity_kernel");
+        using Cfg = TcConvPoolCfg;
+        TcConvPoolArgs k{};
+        k.x = (const int8_t*)pl->scratch(s_pool1); k.w = (const int8_t*)pl->aux(a_w2);
+        for (int m = 0; m < 64; ++m) { k.mult[m] = m2[m]; k.bias[m] = acc_base2 ? kAccBase - (float)b2[m] : int_bits_as_float(b2[m]); }
+        k.y = (int8_t*)pl->scratch(s_pool2); k.n_images = (int)B; k.ib = ib; k.status = ctx->status_word;
+        k.wins = blocks128 * 25 <= ctx->sm_count ? 1 : 5;
+        k.items = blocks128 * 25 / k.wins;
+        const int blocks = std::min<int>(k.items, ctx->sm_count);
+        auto with = [&](auto base) -> int32_t {
+            ZB_SMEM_ATTR(ctx, (tc_conv3x3_pool_kernel<decltype(base)::value>), Cfg::SMEM_BYTES);
+            launch_const(ctx, tc_conv3x3_pool_kernel<decltype(base)::value>, blocks, Cfg::THREADS, Cfg::SMEM_BYTES, k);
+            return check_launch(ctx, "tc_conv3x3_pool_kernel");
+        };
+        return acc_base2 ? with(std::true_type{}) : with(std::false_type{});
     });
     const zant_node_attrs f1a = f1.a, f2a = f2.a, dqa = N[11].a;
     push("Fused[Reshape+QLinearMatMul+Relu] tcgen05", [=]() {
-        using Cfg = TcGemmCfg<FC_NT, FC_KC, FC_STAGES>;
-        ZB_SMEM_ATTR(ctx, (tc_gemm_i8_kernel<FC_NT, FC_KC, FC_STAGES>), Cfg::SMEM_BYTES);
         TcGemmArgs k{};
-        k.a = (const int8_t*)pl->scratch(s_pool2); k.w = (const int8_t*)pl->aux(a_w3);
+        k.a = (const int8_t*)pl->scratch(s_pool2); k.w = (const int8_t*)pl->aux(a_w3); k.a_rows = ib;
         k.mult = (const float*)pl->aux(a_m3); k.bias = (const int32_t*)pl->aux(a_b3);
         k.y = (int8_t*)pl->scratch(s_fc1); k.M = (int)B; k.N = 512; k.K16 = 100;
         k.y_scale = f1a.y_scale; k.y_zp = f1a.y_zp; k.act = ZANT_QACT_RELU; k.status = ctx->status_word;
-        const int tiles = (int)((B + 127) / 128) * (512 / FC_NT);
-        const int blocks = std::min(tiles, ctx->sm_count);
-        launch_const(ctx, tc_gemm_i8_kernel<FC_NT, FC_KC, FC_STAGES>, blocks, Cfg::THREADS, Cfg::SMEM_BYTES, k);
-        return check_launch(ctx, "tc_gemm_i8_kernel");
+        auto with = [&](auto nt) -> int32_t {
+            constexpr int NT = decltype(nt)::value;
+            using Cfg = TcGemmCfg<NT, FC_KC, FC_STAGES>;
+            ZB_SMEM_ATTR(ctx, (tc_gemm_i8_kernel<NT, FC_KC, FC_STAGES>), Cfg::SMEM_BYTES);
+            launch_const(ctx, tc_gemm_i8_kernel<NT, FC_KC, FC_STAGES>, std::min(blocks128 * (512 / NT), ctx->sm_count), Cfg::THREADS, Cfg::SMEM_BYTES, k);
+            return check_launch(ctx, "tc_gemm_i8_kernel");
+        };
+        switch (FC_NT) {
+            case 32: return with(std::integral_constant<int, 32>{});
+            case 64: return with(std::integral_constant<int, 64>{});
+            case 128: return with(std::integral_constant<int, 128>{});
+            default: return with(std::integral_constant<int, 256>{});
+        }
     });
     push("Fused[QLinearMatMul+DequantizeLinear]", [=]() {
         FcOutArgs k{};

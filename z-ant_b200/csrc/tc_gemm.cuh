@@ -27,11 +27,12 @@
 namespace zb {
 
 struct TcGemmArgs {
-    const int8_t* a;       // [ceil(M/128)][K16][128][16]
+    const int8_t* a;       // [ceil(M/128)][K16][128][16], or for fewer than 128 rows [K16][a_rows][16]
     const int8_t* w;       // [N/NT][K16][NT][16]
     const float* mult;     // [N]
     const int32_t* bias;   // [N]
     int8_t* y;             // [M][N] row-major
+    int a_rows;            // rows of a tile of A in memory: 128, or M where that is less (0: 128); the MMA rows beyond them read what lies behind
     int M, N, K16;         // N = padded column count (multiple of NT), K16 = K/16, a multiple of KC
     float y_scale; int y_zp; int act;
     const uint8_t* lut;       // MODE 2 only: optional table applied to the output codes (see Requant)
@@ -57,13 +58,14 @@ struct TcGemmCfg {
     static constexpr int TMEM_COLS = 2 * NT;
     // warps per TMEM lane quarter (they split the tile's columns): two for the row-major epilogue, which is bound by the
     // operand feed anyway; four for the NCHW-storing one (with two per scheduler it was latency-bound: 35 % issue-active)
-    static constexpr int PARTS = ((MODE & 2) && NT >= 128) ? 4 : 2;
+    // (32 columns: one)
+    static constexpr int PARTS = ((MODE & 2) && NT >= 128) ? 4 : (NT == 32 ? 1 : 2);
     static constexpr int COLS_PER_WARP = NT / PARTS;
     static constexpr int EPI_WARPS = 4 * PARTS;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;      // producer, MMA issuer, epilogue warps
     static_assert(KC % 2 == 0, "a stage must hold whole 32-byte MMA K steps");
-    static_assert(NT % 64 == 0 && NT <= 256, "tile width");
-    static_assert(TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
+    static_assert((NT % 64 == 0 || NT == 32) && NT <= 256, "tile width");
+    static_assert(TMEM_COLS == 64 || TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
     static_assert(2 * STAGES + 4 <= 48, "barrier slots");
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(TcGemmCfg<NT, KC, STAGES, MODE>::THREADS, 1) t
     const int m_tiles = (a.M + 127) / 128;
     const int tiles = m_tiles * n_tiles;
     const int k_stages = a.K16 / KC;
+    const uint32_t a_chunk = a.a_rows ? (uint32_t)a.a_rows * 16u : 2048u;      // bytes of a K chunk of A
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { ptx::mbar_init(full(s), 1); ptx::mbar_init(empty(s), 1); }
@@ -119,15 +122,15 @@ __global__ void __launch_bounds__(TcGemmCfg<NT, KC, STAGES, MODE>::THREADS, 1) t
             int it = 0;
             for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
                 const int m = t / n_tiles, n = t - m * n_tiles;
-                const int8_t* ga = a.a + (size_t)m * a.K16 * 2048;
+                const int8_t* ga = a.a + (size_t)m * a.K16 * a_chunk;
                 const int8_t* gw = a.w + (size_t)n * a.K16 * (NT * 16);
                 for (int ks = 0; ks < k_stages; ++ks, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
                     if (!ptx::mbar_wait(empty(s), ph ^ 1u, abort_flag)) goto producer_done;
-                    ptx::mbar_arrive_expect_tx(full(s), Cfg::STAGE);
+                    ptx::mbar_arrive_expect_tx(full(s), KC * a_chunk + Cfg::W_STAGE);
                     const uint32_t dst = ptx::smem_u32(sStages + s * Cfg::STAGE);
-                    ptx::bulk_g2s(dst, ga + (size_t)ks * Cfg::A_STAGE, Cfg::A_STAGE, full(s));
+                    ptx::bulk_g2s(dst, ga + (size_t)ks * (KC * a_chunk), KC * a_chunk, full(s));
                     ptx::bulk_g2s(dst + Cfg::A_STAGE, gw + (size_t)ks * Cfg::W_STAGE, Cfg::W_STAGE, full(s));
                 }
             }
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(TcGemmCfg<NT, KC, STAGES, MODE>::THREADS, 1) t
                     const uint32_t sw = sa + Cfg::A_STAGE;
 #pragma unroll
                     for (int kk = 0; kk < KC / 2; ++kk) {
-                        const uint64_t da = ptx::smem_desc_kmajor(sa + (uint32_t)(kk * 2 * 2048), 2048, 128);
+                        const uint64_t da = ptx::smem_desc_kmajor(sa + (uint32_t)(kk * 2) * a_chunk, a_chunk, 128);
                         const uint64_t db = ptx::smem_desc_kmajor(sw + (uint32_t)(kk * 2 * NT * 16), NT * 16, 128);
                         ptx::mma_i8(d_tmem, da, db, idesc, (ks | kk) != 0);
                     }
