@@ -1,0 +1,534 @@
+// Inverted residual block on small planes as one kernel: QLinearConv 1x1 (expand, ReLU / ReLU6) -> QLinearConv depthwise 3x3 (pads 1,
+// stride 1, ReLU / ReLU6) -> QLinearConv 1x1 (project) [-> QLinearAdd with the block's input], int8 with zero point 0 between them.
+//
+// The expanded tensor, six times the input, never exists in memory.  A tile is one image (planes up to 16 wide; two where the planes are
+// at most 8 wide).  Per chunk of 128 expanded channels:
+//   expand    D1 (TMEM: lane = channel, column = pixel)  =  W1 chunk [128][C]  x  X [C][pixels]            tcgen05, kind::i8
+//   epilogue  a thread owns a channel: it requantises the accumulators of (eight columns of) a plane row into packed bytes, keeps three
+//             rows of sums in registers, runs the depthwise filter (dp4a on windows cut by byte permutes; no shuffles, no shared memory),
+//             requantises and stores the row to shared memory as rows of the next product's operand
+//   project   D2 (lane = filter)  +=  W2 [filters][128 channels]  x  Y [128 channels][pixels]
+// and after the last chunk the project epilogue requantises D2, adds the block's input from the operand X that is still in shared memory, stages
+// the tile and sends it with one bulk copy.  Plane rows lie PITCH = 16 (or 8) columns apart, so that a row is one or half a 16-byte chunk of an
+// MN-major operand row and one TMEM load; the columns past the width hold whatever, are masked behind the expansion and never stored.
+//
+// What bounds it: instruction issue in the epilogue warps, about 12 instructions per expanded value for both requantisations and the
+// depthwise filter together (as separate kernels the depthwise one alone took 31).
+//
+// Warp roles (640 threads, 96 registers each, one persistent CTA per SM):
+//   warp 0 weights (a chunk's W1, W2 and per-channel constants are one bulk copy into a ring)     warp 1 TMEM owner + MMA issuer
+//   warps 2-17 epilogue: four per TMEM lane quarter, one for each half of the rows and of the columns (or each of the two images); two per
+//   quarter with whole rows had a scheduler issue 43 % of the time (14 x 14, 384 channels: 14.9 us a tile)
+//   warps 18-19 builders: the input's rows from NCHW into the MN-major operand X
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+#include "context.cuh"
+#include "fused_cnn.cuh"
+#include "geometry.hpp"
+#include "kernels_q8.cuh"
+#include "ptx_sm100.cuh"
+#include "tc_pw_nchw.cuh"
+
+namespace zb {
+
+// Per expanded channel: kAccBase - bias and multiplier of the expansion, multiplier and (as bits) kAccBase plus bias of the depthwise filter,
+// its three rows packed for dp4a.
+struct IrbConst { float e_floor, e_mult, d_mult; int32_t d_base; uint32_t k[3], pad; };
+
+struct IrbArgs {
+    const uint8_t* x; uint8_t* y; const uint8_t* w;        // w: per chunk [W1 | W2 | constants]
+    const float* mult2; const int32_t* bias2;              // project
+    int N, C, M, H, W;
+    int IB, tiles;                 // images per tile
+    int n_cols;                    // columns of an accumulator: IB * H * PITCH, a multiple of 16, at most 256
+    int chunks, last_live;         // chunks of 128 expanded channels; channels of the last one
+    int kp;                        // C rounded up to K steps of 32
+    int mt2;                       // 128-filter tiles of the project product
+    int d1_bufs, x_bufs, y_bufs, w_stages;
+    int w_bytes, x_bytes, y_bytes; // one stage / buffer
+    int off_x, off_y, off_out, off_tail;
+    int* status;
+};
+
+constexpr int kIrbMinTiles = 8;
+constexpr int kIrbThreads = 640, kIrbEpiWarps = 16, kIrbMaxStages = 3;
+
+// N accumulators of consecutive columns, N at most 9.
+template <int N>
+__device__ __forceinline__ void irb_tmem_cols(uint32_t taddr, uint32_t (&v)[9]) {
+    static_assert(N >= 1 && N <= 9, "");
+    ptx::tmem_ld8(taddr, v);
+    if constexpr (N == 9) ptx::tmem_ld1(taddr + 8u, v + 8);
+}
+
+// Expand epilogue and depthwise filter of one channel's output rows [r0, r1) at OUT consecutive columns.  `src`: TMEM column of the first input column at row
+// 0 (LEFT: the one left of the outputs, else the first output's own, with nothing to its left; RIGHT: one more on the right), rows PITCH apart;
+// valid[j]: byte mask of the columns that exist.  put(row, packed codes); drained() once the accumulators have been read.
+template <int OUT, bool LEFT, bool RIGHT, int PITCH, typename Put, typename Drained>
+__device__ __forceinline__ void irb_rows(uint32_t src, int H, int r0, int r1, const uint32_t (&valid)[3], float ef, float em, float dm, int dbase,
+                                         uint32_t k0, uint32_t k1, uint32_t k2, Put put, Drained drained) {
+    constexpr int IN = OUT + (LEFT ? 1 : 0) + (RIGHT ? 1 : 0), NW = (IN + 3) / 4, NO = (OUT + 3) / 4;
+    const int lo = max(r0 - 1, 0), hi = min(r1, H - 1);                      // input rows
+    int acc[3][OUT];
+#pragma unroll
+    for (int x = 0; x < OUT; ++x) acc[0][x] = acc[1][x] = acc[2][x] = dbase;
+    uint32_t v[9];
+    src += (uint32_t)(lo * PITCH);
+    irb_tmem_cols<IN>(src, v);
+    for (int base = lo; base <= r1; base += 3) {
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const int ir = base + u;
+            if (ir > r1) break;
+            int* up = acc[(u + 2) % 3];                                      // output row ir - 1: this is its filter row 2
+            int* at = acc[u];
+            int* dn = acc[(u + 1) % 3];
+            if (ir <= hi) {
+                uint32_t A[NW + 1];
+                ptx::tmem_wait_ld();
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    int k4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int x = 4 * w + e;
+                        k4[e] = x < IN ? __float2int_rn(__fmul_rn(__fsub_rn(__int_as_float(__viaddmax_s32((int)v[x < 9 ? x : 0], kAccBaseBits, __float_as_int(ef))), ef), em)) : 0;
+                    }
+                    A[w] = pack_sat_s8x4(k4[0], k4[1], k4[2], k4[3]) & valid[w];
+                }
+                A[NW] = 0u;
+                src += (uint32_t)PITCH;
+                if (ir < hi) irb_tmem_cols<IN>(src, v);
+                else drained();
+#pragma unroll
+                for (int x = 0; x < OUT; ++x) {
+                    constexpr int shift = LEFT ? 0 : 3;                      // the window starts at byte x, or at byte x - 1 = 4 * (x / 4 - 1) + x % 4 + 3
+                    const int p = x + shift, w = p / 4 - (LEFT ? 0 : 1), o = p % 4;
+                    const uint32_t a0 = w < 0 ? 0u : A[w < 0 ? 0 : w], a1 = A[w + 1];
+                    const uint32_t win = o == 0 ? a0 : __byte_perm(a0, a1, o == 1 ? 0x4321 : (o == 2 ? 0x5432 : 0x6543));
+                    up[x] = dw_dp4a<false>(win, k2, up[x]);
+                    at[x] = dw_dp4a<false>(win, k1, at[x]);
+                    dn[x] = dw_dp4a<false>(win, k0, dbase);
+                }
+            }
+            if (ir - 1 >= r0) {
+                uint32_t pk[2] = {0u, 0u};
+#pragma unroll
+                for (int w = 0; w < NO; ++w) {
+                    int k4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int x = 4 * w + e;
+                        k4[e] = x < OUT ? __float2int_rn(__fmul_rn(__fsub_rn(__int_as_float(max(up[x < OUT ? x : 0], kAccBaseBits)), kAccBase), dm)) : 0;
+                    }
+                    pk[w] = pack_sat_s8x4(k4[0], k4[1], k4[2], k4[3]);
+                }
+                put(ir - 1, pk[0], pk[1]);
+            }
+        }
+    }
+}
+
+// WC: columns computed per row (the width rounded up to an instantiated value).
+template <int WC, bool ADD>
+__global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_constant__ IrbArgs a, const __grid_constant__ QAddTail add) {
+    constexpr int PITCH = WC > 8 ? 16 : 8;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* tail = smem + a.off_tail;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 256);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 260);
+    const uint32_t smem0 = ptx::smem_u32(smem), bar0 = ptx::smem_u32(bars);
+    auto wfull = [&](int s) { return bar0 + 8u * s; };
+    auto wempty = [&](int s) { return bar0 + 8u * (3 + s); };
+    auto xfull = [&](int b) { return bar0 + 8u * (6 + b); };
+    auto xempty = [&](int b) { return bar0 + 8u * (8 + b); };
+    auto d1full = [&](int b) { return bar0 + 8u * (10 + b); };
+    auto d1empty = [&](int b) { return bar0 + 8u * (12 + b); };
+    auto yfull = [&](int b) { return bar0 + 8u * (14 + b); };
+    auto yempty = [&](int b) { return bar0 + 8u * (16 + b); };
+    const uint32_t d2full = bar0 + 8u * 18, d2empty = bar0 + 8u * 19, out_free = bar0 + 8u * 20, out_full = bar0 + 8u * 21;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cols = (a.d1_bufs + a.mt2) * a.n_cols;
+    const uint32_t tmem_cols = cols <= 64 ? 64u : (cols <= 128 ? 128u : (cols <= 256 ? 256u : 512u));
+
+    if (tid == 0) {
+        for (int s = 0; s < kIrbMaxStages; ++s) { ptx::mbar_init(wfull(s), 1); ptx::mbar_init(wempty(s), 1 + kIrbEpiWarps); }
+        for (int b = 0; b < 2; ++b) {
+            ptx::mbar_init(xfull(b), 2); ptx::mbar_init(xempty(b), ADD ? 1 + kIrbEpiWarps : 1);
+            ptx::mbar_init(d1full(b), 1); ptx::mbar_init(d1empty(b), kIrbEpiWarps);
+            ptx::mbar_init(yfull(b), kIrbEpiWarps); ptx::mbar_init(yempty(b), 1);
+        }
+        ptx::mbar_init(d2full, 1); ptx::mbar_init(d2empty, kIrbEpiWarps);
+        ptx::mbar_init(out_free, 1); ptx::mbar_init(out_full, kIrbEpiWarps);
+        *abort_flag = 0;
+        ptx::mbar_fence_init();
+    }
+    if (warp == 1) {
+        ptx::tmem_alloc(ptx::smem_u32(tmem_slot), tmem_cols);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_trigger();
+    if (warp != 0) ptx::grid_wait();                     // (weights are constants)
+    const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int total = my_tiles * a.chunks;               // chunks of this CTA, in order
+
+    if (warp == 0) {
+        // ------------------------------------------------------------------ weights
+        if (lane == 0) {
+            int s = 0, c = 0; uint32_t ph = 0;
+            for (int j = 0; j < total; ++j) {
+                if (!ptx::mbar_wait(wempty(s), ph ^ 1u, abort_flag)) break;
+                ptx::mbar_arrive_expect_tx(wfull(s), (uint32_t)a.w_bytes);
+                ptx::bulk_g2s(smem0 + (uint32_t)(s * a.w_bytes), a.w + (size_t)c * a.w_bytes, (uint32_t)a.w_bytes, wfull(s));
+                if (++c == a.chunks) c = 0;
+                if (++s == a.w_stages) { s = 0; ph ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer (the whole warp runs the loop, one lane issues): expand of
+        // chunk j, then project of chunk j - 1, so that the epilogue's next accumulators are on their way while it works
+        const uint32_t leader = ptx::elect_one() ? 1u : 0u;
+        auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag)) != 0; };
+        const uint32_t n0 = (uint32_t)min(a.n_cols, 128), n1 = (uint32_t)(a.n_cols - 128);
+        const uint32_t id0 = ptx::idesc_i8(128, (int)n0, true, true) | kIdescBMnMajor, id1 = a.n_cols > 128 ? (ptx::idesc_i8(128, (int)n1, true, true) | kIdescBMnMajor) : 0u;
+        const uint64_t da = ptx::smem_desc_kmajor(0, 128 * 16, 128);
+        const uint32_t a_hi = (uint32_t)(da >> 32), a_lo = (uint32_t)da, w1_bytes = (uint32_t)a.kp * 128u;
+        const uint32_t xblk = (uint32_t)a.kp * 128u, yblk = 16384u;
+        const uint64_t dbx = ptx::smem_desc_mnmajor_sw128(0, xblk, 1024), dby = ptx::smem_desc_mnmajor_sw128(0, yblk, 1024);
+        const uint32_t b_hi = (uint32_t)(dbx >> 32);                     // the high halves of both are the same
+        const uint32_t d2 = tmem_base + (uint32_t)(a.d1_bufs * a.n_cols);
+        int s = 0, b = 0, c = 0, xb = 0; uint32_t wph = 0, bph = 0, xph = 0;          // of the expand
+        int ps = 0, yb = 0, pc = 0; uint32_t yph = 0, d2ph = 0;                       // of the project, a chunk behind
+        for (int j = 0; j <= total; ++j) {
+            if (j < total) {
+                if (!wait(wfull(s), wph) || (c == 0 && !wait(xfull(xb), xph)) || !wait(d1empty(b), bph ^ 1u)) break;
+                ptx::tc_fence_after();
+                const uint32_t d = tmem_base + (uint32_t)(b * a.n_cols);
+                uint32_t al = a_lo + ((smem0 + (uint32_t)(s * a.w_bytes)) >> 4), bl = (uint32_t)dbx + ((smem0 + (uint32_t)(a.off_x + xb * a.x_bytes)) >> 4);
+                for (int k = 0; k < a.kp; k += 32, al += 256u, bl += 256u) {
+                    ptx::mma_i8_if(leader, d, al, a_hi, bl, b_hi, id0, k > 0 ? 1u : 0u);
+                    if (id1) ptx::mma_i8_if(leader, d + 128u, al, a_hi, bl + (xblk >> 4), b_hi, id1, k > 0 ? 1u : 0u);
+                }
+                ptx::mma_commit_if(leader, d1full(b));
+                if (++s == a.w_stages) { s = 0; wph ^= 1u; }
+                if (++b == a.d1_bufs) { b = 0; bph ^= 1u; }
+                if (++c == a.chunks) {
+                    c = 0;
+                    ptx::mma_commit_if(leader, xempty(xb));
+                    if (++xb == a.x_bufs) { xb = 0; xph ^= 1u; }
+                }
+            }
+            if (j > 0) {
+                if (!wait(yfull(yb), yph) || (pc == 0 && !wait(d2empty, d2ph ^ 1u))) break;
+                ptx::tc_fence_after();
+                const int ks = pc == a.chunks - 1 ? (a.last_live + 31) >> 5 : 4;
+                const uint32_t w2 = (smem0 + (uint32_t)(ps * a.w_bytes) + w1_bytes) >> 4, y0 = (smem0 + (uint32_t)(a.off_y + yb * a.y_bytes)) >> 4;
+                for (int m = 0; m < a.mt2; ++m) {
+                    const uint32_t d = d2 + (uint32_t)(m * a.n_cols);
+                    uint32_t al = a_lo + w2 + (uint32_t)m * 1024u, bl = (uint32_t)dby + y0;
+                    for (int k = 0; k < ks; ++k, al += 256u, bl += 256u) {
+                        const uint32_t acc = (pc | k) != 0 ? 1u : 0u;
+                        ptx::mma_i8_if(leader, d, al, a_hi, bl, b_hi, id0, acc);
+                        if (id1) ptx::mma_i8_if(leader, d + 128u, al, a_hi, bl + (yblk >> 4), b_hi, id1, acc);
+                    }
+                }
+                ptx::mma_commit_if(leader, yempty(yb));
+                ptx::mma_commit_if(leader, wempty(ps));
+                if (++ps == a.w_stages) ps = 0;
+                if (++yb == a.y_bufs) { yb = 0; yph ^= 1u; }
+                if (++pc == a.chunks) { pc = 0; ptx::mma_commit_if(leader, d2full); d2ph ^= 1u; }
+            }
+        }
+    } else if (warp >= 18) {
+        // ------------------------------------------------------------------ builders: 16-byte chunk q of channel c, at chunk position q ^ (c % 8) of the
+        // channel's 128-byte row in block q / 8 (the form a box with the 128-byte swizzle has).  Whole aligned words are read: the input's
+        // size is a multiple of four, and words past its end are not.
+        const int bt = tid - 576, nq = a.n_cols >> 4, HW = a.H * a.W;
+        const long long words = (long long)a.N * a.C * HW / 4;
+        const uint32_t* xw = reinterpret_cast<const uint32_t*>(a.x);
+        int xb = 0; uint32_t xph = 0;
+        for (int i = 0; i < my_tiles; ++i) {
+            const int t = (int)blockIdx.x + i * (int)gridDim.x;
+            int ok = 1;
+            if (lane == 0) ok = ptx::mbar_wait(xempty(xb), xph ^ 1u, abort_flag) ? 1 : 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            const uint32_t dst = smem0 + (uint32_t)(a.off_x + xb * a.x_bytes);
+            const int n_chunks = a.C * nq;
+            constexpr int RW = PITCH / 4;                   // words of a row; a chunk is 16 / PITCH rows
+            constexpr int R = 16 / PITCH;
+#pragma unroll 4
+            for (int k = bt; k < n_chunks; k += 64) {
+                const int c = k / nq, q = k - c * nq;
+                uint32_t o[4];
+#pragma unroll
+                for (int h = 0; h < R; ++h) {
+                    const int rr = q * R + h, img = R == 1 ? 0 : rr / a.H, r = rr - img * a.H, n = t * a.IB + img;
+                    const long long off = ((long long)(n * (long long)a.C + c) * a.H + r) * a.W;
+                    const long long w0 = off >> 2;
+                    const uint32_t sh = 8u * (uint32_t)(off & 3);
+                    uint32_t v[RW + 1];
+#pragma unroll
+                    for (int e = 0; e <= RW; ++e) v[e] = (n < a.N && img < a.IB && w0 + e < words) ? __ldg(xw + w0 + e) : 0u;
+#pragma unroll
+                    for (int e = 0; e < RW; ++e) o[h * RW + e] = __funnelshift_r(v[e], v[e + 1], sh);
+                }
+                sts_u128(dst + (uint32_t)(q >> 3) * (uint32_t)a.kp * 128u + (uint32_t)c * 128u + ((((uint32_t)q & 7u) ^ ((uint32_t)c & 7u)) << 4), o[0], o[1], o[2], o[3]);
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(xfull(xb));
+            if (++xb == a.x_bufs) { xb = 0; xph ^= 1u; }
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue
+        const int quarter = warp & 3, part = (warp - 2) >> 2, ch = quarter * 32 + lane;
+        const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16), d2 = lane_base + (uint32_t)(a.d1_bufs * a.n_cols);
+        const bool leader = warp == 2 && lane == 0;
+        const int HW = a.H * a.W;
+        // this warp's rows (a half of them) and columns (left eight or the rest; all of them of one of the two images)
+        const int sub = part >> 1, r0 = (part & 1) ? (a.H + 1) / 2 : 0, r1 = (part & 1) ? a.H : (a.H + 1) / 2;
+        const int img = PITCH == 16 ? 0 : sub, c0 = PITCH == 16 ? sub * 8 : 0, cols_here = PITCH == 16 ? (sub ? a.W - 8 : 8) : a.W;
+        uint32_t valid[3];
+        {
+            const int n = PITCH == 16 && sub ? a.W - 7 : a.W;        // (the right part's first input column is 7)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) valid[j] = n >= 4 * j + 4 ? 0xffffffffu : (n <= 4 * j ? 0u : 0xffffffffu >> (8 * (4 * j + 4 - n)));
+        }
+        auto wait = [&](uint32_t bar, uint32_t parity) {
+            int ok = 1;
+            if (lane == 0) ok = ptx::mbar_wait(bar, parity, abort_flag) ? 1 : 0;
+            return __shfl_sync(0xffffffffu, ok, 0) != 0;
+        };
+
+        // The project epilogue of this CTA's tile number i: behind the next tile's first chunk, so that its last MMAs have had time.
+        auto project = [&](int i) -> bool {
+            const int t = (int)blockIdx.x + i * (int)gridDim.x;
+            const int n_here = min(a.IB, a.N - t * a.IB);
+            if (leader) { ptx::bulk_wait_read<0>(); ptx::mbar_arrive(out_free); }
+            if (!wait(out_free, (uint32_t)i & 1u) || !wait(d2full, (uint32_t)i & 1u)) return false;
+            if (ADD && __all_sync(0xffffffffu, ptx::mbar_wait(xfull(i % a.x_bufs), (uint32_t)(i / a.x_bufs) & 1u, abort_flag)) == 0) return false;
+            ptx::tc_fence_after();
+            uint8_t* out = smem + a.off_out;
+            const uint32_t xs = smem0 + (uint32_t)(a.off_x + (i % a.x_bufs) * a.x_bytes);
+            for (int mt = 0; mt < a.mt2; ++mt) {
+                if (mt * 128 + quarter * 32 >= a.M || img >= n_here) break;
+                const int m = mt * 128 + ch;
+                const bool live = m < a.M;
+                const float mlt = live ? __ldg(a.mult2 + m) : 1.0f;
+                const int bs = live ? __ldg(a.bias2 + m) : 0;
+                uint32_t src = d2 + (uint32_t)(mt * a.n_cols + (img * a.H + r0) * PITCH + c0);
+                uint8_t* o = out + ((size_t)img * a.M + m) * HW + r0 * a.W + c0;
+                uint32_t v[9];
+                irb_tmem_cols<8>(src, v);
+                for (int r = r0; r < r1; ++r, o += a.W) {
+                    ptx::tmem_wait_ld();
+                    uint32_t pk[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        pk[j] = pack_sat_s8x4(rq_round((int)v[4 * j] + bs, mlt), rq_round((int)v[4 * j + 1] + bs, mlt), rq_round((int)v[4 * j + 2] + bs, mlt), rq_round((int)v[4 * j + 3] + bs, mlt));
+                    src += (uint32_t)PITCH;
+                    if (r + 1 < r1) irb_tmem_cols<8>(src, v);
+                    if constexpr (ADD) {
+                        // the block's input at this channel (m < C == M) and row, from the operand
+                        const uint32_t rr = (uint32_t)(img * a.H + r), q = PITCH == 16 ? rr : rr >> 1;
+                        const uint32_t ad = xs + (q >> 3) * (uint32_t)a.kp * 128u + (uint32_t)min(m, a.kp - 1) * 128u + (((q & 7u) ^ ((uint32_t)m & 7u)) << 4) + (PITCH == 16 ? (uint32_t)c0 : (rr & 1u) * 8u);
+                        pk[0] = qadd_word<false>(lds_u32<0>(ad), pk[0], add);
+                        pk[1] = qadd_word<false>(lds_u32<4>(ad), pk[1], add);
+                        __syncwarp();
+                    }
+                    if (live) {
+                        if ((a.W & 3) == 0) {
+                            *reinterpret_cast<uint32_t*>(o) = pk[0];
+                            if (cols_here > 4) *reinterpret_cast<uint32_t*>(o + 4) = pk[1];
+                        } else if ((a.W & 1) == 0) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) if (2 * k < cols_here) *reinterpret_cast<uint16_t*>(o + 2 * k) = (uint16_t)(pk[k / 2] >> (16 * (k % 2)));
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) if (k < cols_here) o[k] = (uint8_t)(pk[k / 4] >> (8 * (k % 4)));
+                        }
+                    }
+                }
+            }
+            ptx::tc_fence_before();
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                ptx::mbar_arrive(d2empty);
+                if (ADD) ptx::mbar_arrive(xempty(i % a.x_bufs));
+                ptx::mbar_arrive(out_full);
+            }
+            if (warp == 2) {
+                if (!wait(out_full, (uint32_t)i & 1u)) return false;
+                if (leader) ptx::bulk_s2g(a.y + (size_t)t * a.IB * a.M * HW, ptx::smem_u32(out), (uint32_t)(n_here * a.M * HW));
+            }
+            return true;
+        };
+
+        int s = 0, b = 0, yb = 0, c = 0, tile_i = 0; uint32_t wph = 0, bph = 0, yph = 0;
+        bool alive = true;
+        for (int j = 0; j < total; ++j) {
+            // (every lane waits for the weights: each reads its channel's constants)
+            alive = __all_sync(0xffffffffu, ptx::mbar_wait(wfull(s), wph, abort_flag)) != 0 && wait(yempty(yb), yph ^ 1u) && wait(d1full(b), bph);
+            if (!alive) break;
+            ptx::tc_fence_after();
+            auto drained = [&]() {
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(d1empty(b));         // this warp has read its accumulators
+            };
+            if (c < a.chunks - 1 || quarter * 32 < a.last_live) {
+                const uint32_t cs = smem0 + (uint32_t)(s * a.w_bytes + a.kp * 128 + a.mt2 * 16384 + ch * 32);
+                const uint4 k0 = lds_u128(cs), k1 = lds_u128(cs + 16u);
+                const float ef = __uint_as_float(k0.x), em = __uint_as_float(k0.y), dm = __uint_as_float(k0.z);
+                const uint32_t d1 = lane_base + (uint32_t)(b * a.n_cols + img * a.H * PITCH), yrow = smem0 + (uint32_t)(a.off_y + yb * a.y_bytes + ch * 128);
+                auto put = [&](int r, uint32_t p0, uint32_t p1) {
+                    const uint32_t rr = (uint32_t)(img * a.H + r), q = PITCH == 16 ? rr : rr >> 1;
+                    const uint32_t ad = yrow + (q >> 3) * 16384u + (((q & 7u) ^ ((uint32_t)ch & 7u)) << 4) + (PITCH == 16 ? (uint32_t)c0 : (rr & 1u) * 8u);
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ad), "r"(p0), "r"(p1) : "memory");
+                };
+                if constexpr (PITCH == 16) {
+                    if (sub == 0) irb_rows<8, false, true, 16>(d1, a.H, r0, r1, valid, ef, em, dm, (int)k0.w, k1.x, k1.y, k1.z, put, drained);
+                    else irb_rows<WC - 8, true, false, 16>(d1 + 7u, a.H, r0, r1, valid, ef, em, dm, (int)k0.w, k1.x, k1.y, k1.z, put, drained);
+                } else {
+                    irb_rows<WC, false, false, 8>(d1, a.H, r0, r1, valid, ef, em, dm, (int)k0.w, k1.x, k1.y, k1.z, put, drained);
+                }
+            } else {
+                drained();
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) { ptx::mbar_arrive(yfull(yb)); ptx::mbar_arrive(wempty(s)); }
+            if (++s == a.w_stages) { s = 0; wph ^= 1u; }
+            if (++b == a.d1_bufs) { b = 0; bph ^= 1u; }
+            if (++yb == a.y_bufs) { yb = 0; yph ^= 1u; }
+            if (c == 0 && tile_i > 0) {
+                alive = project(tile_i - 1);
+                if (!alive) break;
+            }
+            if (++c == a.chunks) { c = 0; ++tile_i; }
+        }
+        if (alive && my_tiles > 0) project(my_tiles - 1);
+        if (leader) ptx::bulk_wait_all();
+    }
+
+    if (*abort_flag) {
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) ptx::tmem_dealloc(tmem_base, tmem_cols);
+    if (tid == 0 && *abort_flag) atomicExch(a.status, (int)DEV_ERR_WAIT_TIMEOUT);
+}
+
+// =============================================================================================
+// Host side
+// =============================================================================================
+struct IrbPlan {
+    IrbArgs a{};
+    int wc = 0, E = 0;
+    size_t smem_bytes = 0;
+};
+
+// Geometry of the three convolutions; false when the kernel does not take them.  With the addition the operand X of a tile is read by the
+// project epilogue, behind the next tile's first chunk: it needs a second buffer.
+inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bool add, IrbPlan& q) {
+    auto pointwise = [](const ConvGeom& g) { return g.G == 1 && g.KH == 1 && g.KW == 1 && g.sh == 1 && g.sw == 1 && !g.pt && !g.pl && !g.pb && !g.pr; };
+    if (!pointwise(e) || !pointwise(p)) return false;
+    if (d.G != d.C || d.M != d.C || d.KH != 3 || d.KW != 3 || d.sh != 1 || d.sw != 1 || d.dh != 1 || d.dw != 1 || d.pt != 1 || d.pl != 1 || d.pb != 1 || d.pr != 1) return false;
+    if (e.N <= 0 || e.H > 16 || e.W > 16 || e.H < 2 || e.W < 3 || e.C > 512 || p.M > 512 || e.M < 128 || e.M > 4096) return false;
+    if ((long long)e.N * e.C * e.H * e.W % 4 != 0 || (long long)p.M * e.H * e.W % 16 != 0 || (long long)e.N * std::max(e.C, p.M) * e.H * e.W > 0x7fffffffLL) return false;
+    IrbArgs& a = q.a;
+    a = IrbArgs{};
+    a.N = e.N; a.C = e.C; a.M = p.M; a.H = e.H; a.W = e.W;
+    q.E = e.M;
+    q.wc = e.W <= 4 ? 4 : (e.W <= 6 ? 6 : (e.W == 7 ? 7 : (e.W <= 8 ? 8 : (e.W <= 10 ? 10 : (e.W <= 12 ? 12 : (e.W <= 14 ? 14 : 16))))));
+    a.IB = e.W > 8 ? 1 : 2;
+    a.tiles = (e.N + a.IB - 1) / a.IB;
+    a.n_cols = e.H * 16;
+    a.chunks = (q.E + 127) / 128; a.last_live = q.E - (a.chunks - 1) * 128;
+    a.kp = (e.C + 31) / 32 * 32;
+    a.mt2 = (p.M + 127) / 128;
+    if ((1 + a.mt2) * a.n_cols > 512) return false;
+    a.d1_bufs = (2 + a.mt2) * a.n_cols <= 512 ? 2 : 1;
+    a.w_bytes = a.kp * 128 + a.mt2 * 16384 + 128 * (int)sizeof(IrbConst);
+    const int blocks = (a.n_cols + 127) / 128;
+    a.x_bytes = blocks * a.kp * 128; a.y_bytes = blocks * 16384;
+    const int out_bytes = (a.IB * a.M * e.H * e.W + 127) / 128 * 128;
+    // as many buffers as fit: weights first (their loads have the longest way), then the input's, then the operand between the products
+    for (int n = 0; n < (add ? 2 : 4); ++n) {
+        a.w_stages = 2; a.x_bufs = n < 2 ? 2 : 1; a.y_bufs = n % 2 == 0 ? 2 : 1;
+        a.off_x = (a.w_stages * a.w_bytes + 1023) / 1024 * 1024;
+        a.off_y = a.off_x + a.x_bufs * a.x_bytes;
+        a.off_out = a.off_y + a.y_bufs * a.y_bytes;
+        a.off_tail = a.off_out + out_bytes;
+        q.smem_bytes = (size_t)a.off_tail + 512;
+        if (q.smem_bytes <= 227 * 1024) return true;
+    }
+    return false;
+}
+
+// Weights and constants per chunk; false when an accumulator could leave the range of kAccBase.  eb, db: biases with -x_zp * sum(w) folded in.
+inline bool irb_prepare(const IrbPlan& q, const int8_t* we, const float* em, const int32_t* eb, const int8_t* wd, const float* dm, const int32_t* db,
+                        const int8_t* wp, std::vector<uint8_t>& out) {
+    const IrbArgs& a = q.a;
+    out.assign((size_t)a.chunks * a.w_bytes, 0);
+    for (int e = 0; e < q.E; ++e) {
+        uint8_t* stage = out.data() + (size_t)(e / 128) * a.w_bytes;
+        const int r = e % 128;
+        const int8_t* w = we + (size_t)e * a.C;
+        int s1 = 0, s2 = 0;
+        for (int c = 0; c < a.C; ++c) s1 += std::abs((int)w[c]);
+        for (int c = 0; c < a.C; c += 16) std::memcpy(stage + ((size_t)(c / 16) * 128 + r) * 16, w + c, std::min(16, a.C - c));
+        IrbConst k{};
+        for (int i = 0; i < 9; ++i) { k.k[i / 3] |= (uint32_t)(uint8_t)wd[e * 9 + i] << (8 * (i % 3)); s2 += std::abs((int)wd[e * 9 + i]); }
+        if (!acc_base_ok(eb[e]) || !acc_base_ok(db[e]) || s1 * 128 + std::abs(eb[e]) >= (1 << 22) || s2 * 128 + std::abs(db[e]) >= (1 << 22)) return false;
+        k.e_floor = kAccBase - (float)eb[e]; k.e_mult = em[e]; k.d_mult = dm[e]; k.d_base = kAccBaseBits + db[e];
+        std::memcpy(stage + (size_t)a.kp * 128 + (size_t)a.mt2 * 16384 + (size_t)r * sizeof(IrbConst), &k, sizeof k);
+    }
+    for (int m = 0; m < a.M; ++m)
+        for (int e = 0; e < q.E; e += 16)
+            std::memcpy(out.data() + (size_t)(e / 128) * a.w_bytes + (size_t)a.kp * 128 + (size_t)(m / 128) * 16384 + ((size_t)(e % 128 / 16) * 128 + m % 128) * 16,
+                        wp + (size_t)m * q.E + e, std::min(16, q.E - e));
+    return true;
+}
+
+// x: 4-byte aligned, y: 16-byte aligned.
+inline int32_t irb_run(zant_ctx* ctx, const IrbPlan& q, const void* x, const uint8_t* w, const float* mult2, const int32_t* bias2, void* y, const QAddTail* add) {
+    IrbArgs a = q.a;
+    a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.w = w; a.mult2 = mult2; a.bias2 = bias2; a.status = ctx->status_word;
+    const int grid = std::min(a.tiles, ctx->sm_count);
+    auto go = [&](auto wc, auto with) -> int32_t {
+        constexpr int WC = decltype(wc)::value;
+        constexpr bool ADD = decltype(with)::value;
+        ZB_SMEM_ATTR(ctx, (irb_kernel<WC, ADD>), 227 * 1024);
+        launch_const(ctx, irb_kernel<WC, ADD>, grid, kIrbThreads, q.smem_bytes, a, add ? *add : QAddTail{});
+        return check_launch(ctx, "irb_kernel");
+    };
+    auto pick = [&](auto wc) -> int32_t { return add ? go(wc, std::true_type{}) : go(wc, std::false_type{}); };
+    switch (q.wc) {
+        case 4: return pick(std::integral_constant<int, 4>{});
+        case 6: return pick(std::integral_constant<int, 6>{});
+        case 7: return pick(std::integral_constant<int, 7>{});
+        case 8: return pick(std::integral_constant<int, 8>{});
+        case 10: return pick(std::integral_constant<int, 10>{});
+        case 12: return pick(std::integral_constant<int, 12>{});
+        case 14: return pick(std::integral_constant<int, 14>{});
+        default: return pick(std::integral_constant<int, 16>{});
+    }
+}
+
+}  // namespace zb

@@ -28,6 +28,7 @@
 #include "tc_gemm_tf32.cuh"
 #include "small_gemm_q8.cuh"
 #include "tc_nhwc_net.cuh"
+#include "irb_q8.cuh"
 #include "status.hpp"
 
 using namespace zb;
@@ -92,6 +93,19 @@ struct zant_plan {
     std::vector<cudaEvent_t> prof_events;   // pool, reused between reads
     size_t prof_used = 0;                   // events recorded since the last read
 
+    // additions inside a convolution's step, with the proof of their short form (once for equal parameters)
+    std::vector<QAddTail> proved_adds;
+    QAddTail prove(QAddTail t) {
+        for (const QAddTail& p : proved_adds) {
+            QAddTail q = p;
+            q.proved = 0;
+            if (std::memcmp(&q, &t, sizeof q) == 0) return p;
+        }
+        QAddTail p = t;
+        qadd_prove(p);
+        proved_adds.push_back(p);
+        return p;
+    }
     std::vector<NhGroup> nh_groups;   // channels-last convolution groups found by the layout pass, by first node
     std::vector<std::pair<int, char*>> nchw_copies;   // channels-last tensors whose address was asked for, and buffers that hold them in the graph's order after each run
     void* ptr(int id) const {
@@ -255,6 +269,7 @@ static int32_t try_fuse(zant_plan* pl, size_t node_index, size_t& consumed);
 static int32_t try_fuse_small_cnn(zant_plan* pl, size_t node_index, size_t& consumed, bool probe = false);
 static int32_t try_fuse_qconv_group(zant_plan* pl, size_t node_index, size_t& consumed);
 static int32_t try_fuse_fconv_group(zant_plan* pl, size_t node_index, size_t& consumed);
+static int32_t try_fuse_irb(zant_plan* pl, size_t node_index, size_t& consumed);
 static void nh_layout(zant_plan* pl);
 static int32_t build_nh(zant_plan* pl, size_t node_index, size_t& consumed);
 static int32_t refresh_nchw_copy(zant_plan* pl, int id, char* y);
@@ -650,7 +665,7 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
     if (fz.add_node >= 0) {
         const PlanNode& an = pl->nodes[fz.add_node];
         const bool first = an.in[0] == add_res;
-        add0 = qadd_tail<false>(first ? an.a.x_scale : an.a.b_scale, first ? an.a.x_zp : an.a.b_zp, first ? an.a.b_scale : an.a.x_scale, first ? an.a.b_zp : an.a.x_zp, an.a.y_scale, an.a.y_zp, an.a.activation);
+        add0 = pl->prove(qadd_tail<false>(first ? an.a.x_scale : an.a.b_scale, first ? an.a.x_zp : an.a.b_zp, first ? an.a.b_scale : an.a.x_scale, first ? an.a.b_zp : an.a.x_zp, an.a.y_scale, an.a.y_zp, an.a.activation));
     }
     auto add_of = [pl, add0, add_res]() { QAddTail t = add0; t.res = (const uint8_t*)pl->ptr(add_res); return t; };
 
@@ -1321,9 +1336,96 @@ static int32_t try_fuse(zant_plan* pl, size_t i0, size_t& consumed) {
     consumed = 0;
     ZB_TRY(try_fuse_small_cnn(pl, i0, consumed));
     if (consumed) return ZANT_OK;
+    ZB_TRY(try_fuse_irb(pl, i0, consumed));
+    if (consumed) return ZANT_OK;
     ZB_TRY(try_fuse_qconv_group(pl, i0, consumed));
     if (consumed) return ZANT_OK;
     return try_fuse_fconv_group(pl, i0, consumed);
+}
+
+// QLinearConv 1x1 -> QLinearConv depthwise 3x3 -> QLinearConv 1x1 [-> QLinearAdd with the group's input] on small planes as one step
+// (irb_q8.cuh).  Both activations are ReLU or a ReLU6 whose bound is the type's own, all tensors int8, zero points 0 between the convolutions,
+// interior tensors read by the next node only.  Whatever does not qualify is left to the steps of its own.
+static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
+    consumed = 0;
+    if (i0 + 3 > pl->nodes.size()) return ZANT_OK;
+    const PlanNode *e = &pl->nodes[i0], *d = e + 1, *p = e + 2;
+    for (const PlanNode* n : {e, d, p})
+        if (n->op != ZANT_OP_QLINEAR_CONV || n->in.size() < 3 || n->in.size() > 5 || n->out.size() != 1 || n->a.channels_last) return ZANT_OK;
+    ChainCtx c{pl, std::vector<int>(pl->t.size(), 0)};
+    for (const PlanNode& n : pl->nodes) for (int id : n.in) if (id >= 0) c.consumers[id]++;
+    auto T = [&](int id) -> const PlanTensor& { return pl->t[id]; };
+    const int x = e->in[0], t1 = e->out[0], t2 = d->out[0], y0 = p->out[0];
+    if (x < 0 || d->in[0] != t1 || p->in[0] != t2 || !only_feeds_next(c, t1) || !only_feeds_next(c, t2)) return ZANT_OK;
+    auto plain = [&](int id) { return T(id).dtype == ZANT_I8 && T(id).shape.size() == 4 && !T(id).nh && T(id).alias < 0 && !T(id).elided && !T(id).is_const; };
+    if (!plain(x) || !plain(t1) || !plain(t2) || !plain(y0) || x == pl->input || y0 == pl->output) return ZANT_OK;
+    // parameters of the three convolutions
+    ConvGeom g[3];
+    std::vector<float> mult[3]; std::vector<int32_t> bias[3];
+    const PlanNode* conv[3] = {e, d, p};
+    for (int i = 0; i < 3; ++i) {
+        const PlanNode& n = *conv[i];
+        const int w = n.in[1], ws = n.in[2], wz = opt_in(n, 3), b = opt_in(n, 4);
+        if (w < 0 || ws < 0 || !T(w).is_const || T(w).dtype != ZANT_I8 || !T(ws).is_const || T(ws).dtype != ZANT_F32 || T(w).shape.size() != 4) return ZANT_OK;
+        if (b >= 0 && (!T(b).is_const || T(b).dtype != ZANT_I32)) return ZANT_OK;
+        if (wz >= 0 && (!T(wz).is_const || T(wz).dtype != ZANT_I32 || !all_zero_i32(T(wz)))) return ZANT_OK;
+        if (check_zero_point(ZANT_I8, n.a.x_zp, "x") != ZANT_OK || n.a.y_zp != 0 || (i > 0 && n.a.x_zp != 0)) return ZANT_OK;
+        if (conv_resolve_onnx(T(n.in[0]).shape.data(), 4, T(w).shape.data(), 4, T(n.out[0]).shape.data(), 4, n.a.strides, n.a.n_strides, n.a.pads, n.a.n_pads,
+                              n.a.dilations, n.a.n_dilations, n.a.group, n.a.auto_pad < 0 ? 0 : n.a.auto_pad, g[i]) != ZANT_OK) return ZANT_OK;
+        const size_t M = (size_t)g[i].M, nws = T(ws).bytes / 4;
+        if ((nws != 1 && nws != M) || (b >= 0 && T(b).bytes != M * 4)) return ZANT_OK;
+        if (wz >= 0 && T(wz).bytes != 4 && T(wz).bytes != M * 4) return ZANT_OK;
+        requant_multipliers(n.a.x_scale, (const float*)T(ws).host.data(), nws, n.a.y_scale, M, mult[i]);
+        if (!positive_finite(mult[i])) return ZANT_OK;
+        bias[i].assign(M, 0);
+        if (b >= 0) std::memcpy(bias[i].data(), T(b).host.data(), M * 4);
+        if (i < 2) {
+            std::vector<int32_t> caps;
+            if (!requant_relu_caps(mult[i].data(), M, n.a.activation, lean_six(n.a.y_scale), caps)) return ZANT_OK;
+            for (int32_t v : caps) if (v != 0x7fffffff) return ZANT_OK;
+        } else if (n.a.activation != ZANT_QACT_NONE) return ZANT_OK;
+    }
+    if (e->a.x_zp != 0) {
+        const int8_t* w = (const int8_t*)T(e->in[1]).host.data();
+        for (int m = 0; m < g[0].M; ++m) {
+            int sum = 0;
+            for (int k = 0; k < g[0].C; ++k) sum += w[(size_t)m * g[0].C + k];
+            bias[0][m] -= e->a.x_zp * sum;
+        }
+    }
+    // the residual addition: its other operand is the group's input
+    int y = y0;
+    consumed = 3;
+    QAddTail add{};
+    bool with_add = false;
+    if (i0 + 3 < pl->nodes.size() && only_feeds_next(c, y0)) {
+        const PlanNode& n = pl->nodes[i0 + 3];
+        if (n.op == ZANT_OP_QLINEAR_ADD && n.in.size() == 2 && n.out.size() == 1 && ((n.in[0] == x && n.in[1] == y0) || (n.in[0] == y0 && n.in[1] == x)) &&
+            plain(n.out[0]) && n.out[0] != pl->output && T(n.out[0]).bytes == T(x).bytes && T(x).bytes == T(y0).bytes && g[0].C == g[2].M &&
+            check_zero_point(ZANT_I8, n.a.y_zp, "QLinearAdd y") == ZANT_OK) {
+            const bool first = n.in[0] == x;
+            add = pl->prove(qadd_tail<false>(first ? n.a.x_scale : n.a.b_scale, first ? n.a.x_zp : n.a.b_zp, first ? n.a.b_scale : n.a.x_scale, first ? n.a.b_zp : n.a.x_zp, n.a.y_scale, n.a.y_zp, n.a.activation));
+            with_add = true;
+            y = n.out[0];
+            consumed = 4;
+        }
+    }
+    IrbPlan q;
+    if (!irb_plan(g[0], g[1], g[2], with_add, q) || q.a.tiles < kIrbMinTiles) { consumed = 0; return ZANT_OK; }
+    std::vector<uint8_t> stages;
+    if (!irb_prepare(q, (const int8_t*)T(e->in[1]).host.data(), mult[0].data(), bias[0].data(), (const int8_t*)T(d->in[1]).host.data(), mult[1].data(), bias[1].data(),
+                     (const int8_t*)T(p->in[1]).host.data(), stages)) { consumed = 0; return ZANT_OK; }
+    const int aw = pl->add_aux(stages.data(), stages.size()), am = pl->add_aux(mult[2].data(), mult[2].size() * 4), ab = pl->add_aux(bias[2].data(), bias[2].size() * 4);
+    const size_t first_step = pl->steps.size();
+    zant_ctx* ctx = pl->ctx;
+    pl->step_names.push_back(with_add ? "QLinearConv(expand+depthwise+project)+QLinearAdd" : "QLinearConv(expand+depthwise+project)");
+    pl->steps.push_back([=]() {
+        return irb_run(ctx, q, pl->ptr(x), (const uint8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y), with_add ? &add : nullptr);
+    });
+    pl->t[t1].elided = pl->t[t2].elided = true;
+    if (with_add) pl->t[y0].elided = true;
+    record_step_cost(pl, first_step, i0, consumed);
+    return ZANT_OK;
 }
 
 // Float Conv -> [Relu | LeakyRelu] -> [MaxPool 2x2 / 2] and MatMul -> Add(row vector) -> [Relu | LeakyRelu] as one step: what
