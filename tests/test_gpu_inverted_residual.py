@@ -8,48 +8,54 @@ pytestmark = pytest.mark.gpu
 
 CONV = dict(dilations=(1, 1), auto_pad="NOTSET")
 
-# N C E M H W, input zero point, project bias, residual addition: 0 none, 1 input first, 2 input second
+# N C E M H W, input zero point, biases, residual addition: 0 none, 1 input first, 2 input second; stride
 CASES = [
-    (9, 64, 384, 64, 14, 14, 0, True, 1),        # whole chunks, one image a tile
-    (160, 96, 576, 96, 14, 14, 0, False, 2),     # half a chunk at the end, CTAs with two tiles
-    (310, 32, 128, 32, 7, 7, 0, True, 1),        # two images a tile, CTAs with two tiles, one chunk
-    (17, 160, 960, 160, 7, 7, 0, True, 1),       # two filter tiles, an odd image
-    (16, 160, 960, 320, 7, 7, -3, True, 0),      # three filter tiles, input zero point
-    (8, 40, 200, 48, 16, 16, 2, True, 0),        # 256 columns
-    (21, 24, 144, 24, 12, 9, 5, True, 1),        # ragged width, K step partly empty
-    (33, 40, 240, 112, 5, 16, -1, False, 0),
-    (18, 32, 192, 32, 11, 13, 0, True, 2),       # odd plane
-    (40, 48, 288, 48, 3, 3, 0, True, 1),
-    (19, 64, 136, 16, 2, 5, 9, True, 0),         # eight channels in the last chunk
-    (24, 32, 256, 32, 10, 10, 0, True, 1),
-    (30, 64, 384, 64, 6, 8, 0, True, 1),
-    (17, 64, 384, 64, 16, 4, 0, True, 1),        # 256 columns of two narrow images
-    (16, 32, 160, 32, 4, 6, 0, True, 1),
-    (12, 32, 160, 32, 8, 11, 0, True, 2),
+    (9, 64, 384, 64, 14, 14, 0, True, 1, 1),        # whole chunks, one image a tile, both halves in one accumulator
+    (160, 96, 576, 96, 14, 14, 0, False, 2, 1),     # half a chunk at the end, CTAs with two tiles
+    (310, 32, 128, 32, 7, 7, 0, True, 1, 1),        # two images a tile, CTAs with two tiles, one chunk
+    (17, 160, 960, 160, 7, 7, 0, True, 1, 1),       # two filter tiles, an odd image
+    (16, 160, 960, 320, 7, 7, -3, True, 0, 1),      # three filter tiles, input zero point
+    (8, 40, 200, 48, 14, 16, 2, True, 0, 1),
+    (21, 24, 144, 24, 12, 9, 5, True, 1, 1),        # ragged width, K step partly empty
+    (33, 40, 240, 112, 5, 16, -1, False, 0, 1),     # odd rows, halves apart
+    (18, 32, 192, 32, 11, 13, 0, True, 2, 1),       # odd plane
+    (40, 48, 288, 48, 3, 3, 0, True, 1, 1),
+    (19, 64, 136, 16, 2, 5, 9, True, 0, 1),         # eight channels in the last chunk
+    (150, 32, 256, 32, 10, 10, 0, True, 1, 1),
+    (30, 64, 384, 64, 6, 8, 0, True, 1, 1),
+    (17, 64, 384, 64, 8, 4, 0, True, 1, 1),
+    (16, 32, 160, 32, 4, 6, 0, True, 1, 1),
+    (12, 32, 160, 32, 8, 11, 0, True, 2, 1),
+    (9, 16, 128, 16, 2, 12, 0, True, 1, 1),         # one output row a half
+    (9, 96, 576, 160, 14, 14, 2, True, 0, 2),       # stride 2, two filter tiles
+    (150, 32, 192, 64, 10, 10, 1, True, 0, 2),      # both halves in one accumulator, three and two output rows, CTAs with two tiles
+    (20, 24, 144, 80, 12, 12, 3, False, 0, 2),      # the second half reads more rows than the first
+    (11, 40, 130, 16, 4, 14, -4, True, 0, 2),
 ]
 
 
-@pytest.mark.parametrize("case", CASES, ids=["x".join(map(str, c[:6])) for c in CASES])
+@pytest.mark.parametrize("case", CASES, ids=["x".join(map(str, c[:6] + c[9:])) for c in CASES])
 def test_block(zb, ctx, oracle, case):
-    N, C, E, M, H, W, xzp, bias, res = case
+    N, C, E, M, H, W, xzp, bias, res, stride = case
+    OH, OW = (H + stride - 1) // stride, (W + stride - 1) // stride
     rng = np.random.default_rng(C + E + H * 16 + W)
     g = zb.Graph("irb")
     x0 = g.tensor("x", zb.I8, (N, 4, H, W))
 
-    def conv(src, cin, cout, k, group, name, sx, zx, sy, zy, act):
+    def conv(src, cin, cout, k, group, name, sx, zx, sy, zy, act, oh=H, ow=W, s=1):
         w = g.tensor("w" + name, zb.I8, (cout, cin // group, k, k), rng.integers(-127, 128, (cout, cin // group, k, k), dtype=np.int8))
         target = 60.0 * sy / (sx * 40.0 * 73.0 * np.sqrt(cin // group * k * k))        # outputs spread over the codes
         ws = g.tensor("s" + name, zb.F32, (cout,), (rng.uniform(0.7, 1.4, cout) * target).astype(np.float32))
         b = g.tensor("b" + name, zb.I32, (cout,), rng.integers(-3000, 3000, cout).astype(np.int32)) if bias else -1
-        y = g.tensor("y" + name, zb.I8, (N, cout, H, W))
-        g.node("QLinearConv", [src, w, ws, -1, b], [y], x_scale=sx, x_zp=zx, y_scale=sy, y_zp=zy, pads=(k // 2,) * 4, strides=(1, 1), group=group, activation=act, **CONV)
+        y = g.tensor("y" + name, zb.I8, (N, cout, oh, ow))
+        g.node("QLinearConv", [src, w, ws, -1, b], [y], x_scale=sx, x_zp=zx, y_scale=sy, y_zp=zy, pads=(k // 2,) * 4, strides=(s, s), group=group, activation=act, **CONV)
         return y
 
     x = conv(x0, 4, C, 1, 1, "0", 0.05, 0, 0.1, xzp, None)
     six = float(np.float32(6.0) / np.float32(127.0))
     t1 = conv(x, C, E, 1, 1, "e", 0.1, xzp, six, 0, "relu6")
-    t2 = conv(t1, E, E, 3, E, "d", six, 0, six, 0, "relu")
-    cur = conv(t2, E, M, 1, 1, "p", six, 0, 0.12, 0, None)
+    t2 = conv(t1, E, E, 3, E, "d", six, 0, six, 0, "relu", OH, OW, stride)
+    cur = conv(t2, E, M, 1, 1, "p", six, 0, 0.12, 0, None, OH, OW)
     if res:
         y = g.tensor("sum", zb.I8, (N, M, H, W))
         if res == 1:
@@ -57,7 +63,7 @@ def test_block(zb, ctx, oracle, case):
         else:
             g.node("QLinearAdd", [cur, x], [y], x_scale=0.12, x_zp=0, b_scale=0.1, b_zp=xzp, y_scale=0.2, y_zp=0)
         cur = y
-    out = g.tensor("out", zb.F32, (N, M, H, W))
+    out = g.tensor("out", zb.F32, (N, M, OH, OW))
     g.node("DequantizeLinear", [cur], [out], x_scale=0.2, x_zp=0)
     g.input, g.output = x0, out
     xv = rng.integers(-128, 128, (N, 4, H, W)).astype(np.int8)
