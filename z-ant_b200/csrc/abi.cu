@@ -977,7 +977,7 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
         g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
         if (y_dtype != ZANT_I32 && qconv_tc_eligible(g, bz_zero)) {
             QGemmPrep prep;
-            qgemm_sizes((int)N, (int)K, mult.data(), prep);
+            qgemm_sizes((int)N, (int)K, mult.data(), prep, (long long)M);
             WBlockArgs wb = weight_blocks_of(prep, (int)N, (int)K, 1, a_zp);
             wb.sm = 1; wb.sc = N;                                       // [K][N]
             Stager s(ctx);

@@ -1198,7 +1198,7 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                     const int8_t* bw = (const int8_t*)T(w).host.data();
                     for (size_t k = 0; k < K; ++k) for (size_t j = 0; j < N; ++j) bt[j * K + k] = bw[k * N + j];
                     auto prep = std::make_shared<QGemmPrep>();
-                    qgemm_prepare(bt.data(), (int)N, (int)K, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep);
+                    qgemm_prepare(bt.data(), (int)N, (int)K, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep, (long long)M);
                     const int aw = pl->add_aux(prep->w_blk.data(), prep->w_blk.size()), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4);
                     const int ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
                     const int sa = pl->shared_im2col_scratch(qgemm_a_bytes(M, *prep));

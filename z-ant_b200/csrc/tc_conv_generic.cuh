@@ -109,6 +109,15 @@ __global__ void __launch_bounds__(256) pointwise_blocked_kernel(const PwBlockArg
     }
 }
 
+// Matrix products (one position per image): a row of K bytes is a run of 16-byte chunks already.
+__global__ void __launch_bounds__(256) rows_blocked_kernel(const uint4* x, uint4* a, int M, int c16, int K16, int chunks) {
+    ptx::grid_start();
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < chunks; i += gridDim.x * 256) {
+        const int r = i & 127, q = i >> 7, mt = q / K16, k = q - mt * K16, m = mt * 128 + r;
+        a[i] = m < M && k < c16 ? __ldg(x + (size_t)m * c16 + k) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
 // Convolutions whose channel count is a multiple of 16 use the K order (tap, channel) instead of the
 // weight tensor's (channel, tap): a 16-byte K chunk is then 16 channels of ONE tap, and the im2col
 // matrix is built like the 1x1 case, tap by tap.  A CTA takes one tap, 64 channels and 128 output
@@ -193,6 +202,8 @@ inline void qgemm_sizes(int n_out, int K, const float* mult, QGemmPrep& p, long 
         const long long c256 = (t256 + 147) / 148 * 256, c128 = (t128 + 147) / 148 * 128;
         if (c128 < c256) p.NT = 128;
     }
+    // few rows: narrower tiles while the grid still fits the SMs (1024 x 1280 times 1000 columns: 32 CTAs of 256, 128 of 64)
+    while (p.NT > 64 && rows > 0 && (rows + 127) / 128 * ((n_out + p.NT / 2 - 1) / (p.NT / 2)) <= 148) p.NT /= 2;
     p.N_pad = (n_out + p.NT - 1) / p.NT * p.NT;
     p.K = K;
     p.K16 = K <= 32 ? 2 : (K + 63) / 64 * 4;      // a stage holds 4 chunks of K (2 when K fits 32: first layers with 3 channels)
@@ -262,7 +273,11 @@ inline int32_t run_qconv_tc(zant_ctx* ctx, const ConvGeom& g, const void* x, boo
     ia.x = (const uint8_t*)x; ia.a = a_blk; ia.g = g; ia.K = p.K; ia.K16 = p.K16; ia.M = (int)M; ia.pad_value = x_zp;
     const bool pointwise = g.KH == 1 && g.KW == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
     const int m_tiles = (int)((M + 127) / 128);
-    if (pointwise && (g.H * g.W) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 3u) == 0 && m_tiles <= 0x7fffffff / 128 && (p.K16 + 3) / 4 <= 65535) {
+    if (pointwise && g.H * g.W == 1 && g.C % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (long long)m_tiles * p.K16 * 128 < 0x7fffffffLL) {
+        const int chunks = m_tiles * p.K16 * 128;
+        launch(ctx, rows_blocked_kernel, std::min((chunks + 255) / 256, ctx->sm_count * 8), 256, 0, (const uint4*)x, (uint4*)a_blk, (int)M, g.C / 16, p.K16, chunks);
+        ZB_TRY(check_launch(ctx, "rows_blocked_kernel"));
+    } else if (pointwise && (g.H * g.W) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 3u) == 0 && m_tiles <= 0x7fffffff / 128 && (p.K16 + 3) / 4 <= 65535) {
         PwBlockArgs pa{};
         pa.x = (const uint8_t*)x; pa.a = a_blk; pa.C = g.C; pa.HW = g.H * g.W; pa.M = (int)M; pa.K16 = p.K16;
         launch(ctx, pointwise_blocked_kernel, dim3((unsigned)m_tiles, (unsigned)((p.K16 + 3) / 4)), 256, 0, pa);
@@ -289,6 +304,7 @@ inline int32_t run_qconv_tc(zant_ctx* ctx, const ConvGeom& g, const void* x, boo
         v6 = std::fmin(std::fmax(v6, -512.0f), 511.0f);
         k.six = std::min(std::max((int)std::nearbyintf(v6), -128), 127);
     }
+    k.word_store = k.ohw == 1 && g.M % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 3u) == 0 ? 1 : 0;
     const int tiles = (int)((M + 127) / 128) * (p.N_pad / p.NT);
     if (p.NT == 64) return x_u8 ? launch_tc_gemm<64, 3>(ctx, k, tiles) : launch_tc_gemm<64, 2>(ctx, k, tiles);
     if (p.NT == 128) return x_u8 ? launch_tc_gemm<128, 3>(ctx, k, tiles) : launch_tc_gemm<128, 2>(ctx, k, tiles);

@@ -43,6 +43,7 @@ struct TcGemmArgs {
     // MODE & 2: int8 output with zero point 0 and finite multipliers (host-checked): requantisation by rni and a saturating
     // pack, the activation as a clamp of the packed codes to [0 | -128, six | 127]
     int lean; int six;
+    int word_store;           // MODE & 2, lean: one position per image, n_valid and y multiples of four: a row's four columns are one word
 };
 
 template <int NT, int KC, int STAGES, int MODE = 0>
@@ -239,7 +240,9 @@ __global__ void __launch_bounds__(TcGemmCfg<NT, KC, STAGES, MODE>::THREADS, 1) t
                             const int q2 = rq_round((int)v[j4 * 4 + 2] + b4.z, m4.z), q3 = rq_round((int)v[j4 * 4 + 3] + b4.w, m4.w);
                             uint32_t w4 = relu_act ? __vminu4(pack_sat_u8x4(q0, q1, q2, q3), hi4) : pack_sat_s8x4(q0, q1, q2, q3);
                             if (a.lut) w4 = lut4(a.lut, w4);
-                            if (row_ok && all_cols) {
+                            if (a.word_store) {
+                                if (row_ok && col0 + j4 * 4 < a.n_valid) *reinterpret_cast<uint32_t*>(yc) = w4;
+                            } else if (row_ok && all_cols) {
                                 yc[0] = (uint8_t)w4; yc[st1] = (uint8_t)(w4 >> 8); yc[st2] = (uint8_t)(w4 >> 16); yc[st3] = (uint8_t)(w4 >> 24);
                             } else if (row_ok) {
 #pragma unroll
