@@ -696,9 +696,9 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         std::vector<int32_t> caps;
         const bool capped = finite && yd == ZANT_I8 && rq0.y_zp == 0 && requant_relu_caps(mult.data(), mult.size(), rq0.act, lean_six(rq0.y_scale), caps);
         const int ac = capped ? pl->add_aux(caps.data(), caps.size() * 4) : -1;
-        // from 8 MB of output on (below, a CTA has a tile or two, whose epilogue the addition makes longer by more than the launch it
-        // saves: 37 images of 160 x 160 took 512 us with it, 484 without; 1024 of 224 x 224 go from 114 + 80 to 165 us in the largest)
-        if (!stem && fz.add_node >= 0 && (long long)g.N * g.M * g.OH * g.OW >= (8LL << 20) && xd == ZANT_I8 && yd == ZANT_I8 && rq0.y_zp == 0 && finite) {
+        // In the short form (proved) from 64 KB of output on, else from 8 MB (below, a CTA has a tile or two, whose epilogue the long form
+        // makes longer by more than the launch it saves: 37 images of 160 x 160 took 512 us with it, 484 without).
+        if (!stem && fz.add_node >= 0 && (long long)g.N * g.M * g.OH * g.OW >= (add0.proved ? 64LL << 10 : 8LL << 20) && xd == ZANT_I8 && yd == ZANT_I8 && rq0.y_zp == 0 && finite) {
             fz.add_done = true;
             push("QLinearConv(tc-pointwise)" + tail + "+QLinearAdd", [=]() {
                 if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y_sum))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");

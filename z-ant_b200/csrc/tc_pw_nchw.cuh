@@ -636,8 +636,22 @@ inline bool pw_conv_plan(const ConvGeom& g, bool w_zp_all_zero, int sm_count, Pw
         // the groups the pixels-on-lanes form of the implicit-GEMM kernel is the better one
         if (a.G == 1 && g.M <= 32) return false;
         const long long tile_max = 256LL * a.G;
+        // Pixels per tile: 256; with less than four rounds of the CTAs as many tiles as make the last round short, a tile costing about as
+        // much as 48 pixels beside its pixels.  (96 filters to 24 on 3136 pixels, one image: 4 tiles of four groups took 7.3 us, 25 take 6.1; from
+        // four rounds on it costs: 24 to 144 on 3136 pixels, 1024 images 175 -> 186.)
         a.px_tiles = (int)((hw + tile_max - 1) / tile_max);
-        a.n_px = (int)(((hw + (long long)a.px_tiles * a.G - 1) / ((long long)a.px_tiles * a.G) + 15) / 16 * 16);
+        auto px_of = [&](int pt) { return (int)(((hw + (long long)pt * a.G - 1) / ((long long)pt * a.G) + 15) / 16 * 16); };
+        a.n_px = px_of(a.px_tiles);
+        const long long ctas = std::max(1, sm_count / p.m_tiles);
+        if ((long long)g.N * a.px_tiles < 4 * ctas) {
+            const int px_min = a.px_tiles;
+            long long best = -1;
+            for (int pt = px_min; pt <= px_min * 8 && (pt == px_min || pt <= (hw + 32LL * a.G - 1) / (32LL * a.G)); ++pt) {
+                const int n_px = px_of(pt);
+                const long long tiles = (hw + (long long)n_px * a.G - 1) / ((long long)n_px * a.G), cost = (g.N * tiles + ctas - 1) / ctas * (n_px + 48);
+                if (best < 0 || cost < best) { best = cost; a.px_tiles = (int)tiles; a.n_px = n_px; }
+            }
+        }
         a.wide_store = (hw % 32 == 0 && a.n_px % 32 == 0) ? 1 : 0;
     } else {
         if (hw > 256 || hw % 4 != 0) return false;      // rows that are not whole words stay with the im2col path (the byte copies cost more than they save)
