@@ -31,6 +31,8 @@ CASES = [
     (150, 32, 192, 64, 10, 10, 1, True, 0, 2),      # both halves in one accumulator, three and two output rows, CTAs with two tiles
     (20, 24, 144, 80, 12, 12, 3, False, 0, 2),      # the second half reads more rows than the first
     (11, 40, 130, 16, 4, 14, -4, True, 0, 2),
+    (31, 48, 700, 48, 5, 5, 0, True, 1, 1),         # six chunks on six CTAs a tile, 60 channels in the last, an odd image
+    (90, 64, 1100, 64, 4, 6, 0, True, 2, 1),        # nine chunks on three CTAs
 ]
 
 

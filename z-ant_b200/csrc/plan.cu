@@ -1411,16 +1411,22 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
         }
     }
     IrbPlan q;
-    if (!irb_plan(g[0], g[1], g[2], with_add, q) || q.a.tiles < kIrbMinTiles) { consumed = 0; return ZANT_OK; }
+    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || q.a.tiles < kIrbMinTiles) { consumed = 0; return ZANT_OK; }
     std::vector<uint8_t> stages;
     if (!irb_prepare(q, (const int8_t*)T(e->in[1]).host.data(), mult[0].data(), bias[0].data(), (const int8_t*)T(d->in[1]).host.data(), mult[1].data(), bias[1].data(),
                      (const int8_t*)T(p->in[1]).host.data(), stages)) { consumed = 0; return ZANT_OK; }
     const int aw = pl->add_aux(stages.data(), stages.size()), am = pl->add_aux(mult[2].data(), mult[2].size() * 4), ab = pl->add_aux(bias[2].data(), bias[2].size() * 4);
     const size_t first_step = pl->steps.size();
     zant_ctx* ctx = pl->ctx;
+    int as = -1;
+    if (q.sums_bytes) {
+        const size_t bytes = q.sums_bytes + (size_t)q.a.tiles * sizeof(int);
+        as = pl->add_scratch(bytes);
+        pl->init_steps.push_back([=]() -> int32_t { ZB_CUDA(cudaMemsetAsync(pl->scratch(as), 0, bytes, ctx->stream)); return ZANT_OK; });
+    }
     pl->step_names.push_back(with_add ? "QLinearConv(expand+depthwise+project)+QLinearAdd" : "QLinearConv(expand+depthwise+project)");
     pl->steps.push_back([=]() {
-        return irb_run(ctx, q, pl->ptr(x), (const uint8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y), with_add ? &add : nullptr);
+        return irb_run(ctx, q, pl->ptr(x), (const uint8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y), as >= 0 ? pl->scratch(as) : nullptr, with_add ? &add : nullptr);
     });
     pl->t[t1].elided = pl->t[t2].elided = true;
     if (with_add) pl->t[y0].elided = true;
