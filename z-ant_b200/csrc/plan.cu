@@ -2133,7 +2133,9 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
         const int N = (int)T(y).shape[0], C = (int)T(y).shape[1];
         const long long hw = (long long)(T(y).shape[2] * T(y).shape[3]);
         const float sc = n.a.y_scale; const int zp = n.a.y_zp; const bool u8 = T(y).dtype == ZANT_U8;
-        push("QuantizeLinear", [=]() { return run_to_nhwc(ctx, 0, pl->ptr(x), pl->t[y].arena_ptr, N, C, hw, sc, zp, u8); });
+        QuantSteps steps{};
+        if (!quant_steps(sc, (u8 ? 0 : -128) - zp, (u8 ? 255 : 127) - zp, steps)) steps = QuantSteps{0.0f, 0.0f};
+        push("QuantizeLinear", [=]() { return run_to_nhwc(ctx, 0, pl->ptr(x), pl->t[y].arena_ptr, N, C, hw, sc, zp, u8, steps); });
         record_step_cost(pl, first_step, i, 1);
         consumed = 1;
         return ZANT_OK;
