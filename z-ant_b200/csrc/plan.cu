@@ -1725,14 +1725,15 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     {
         const int8_t* w = (const int8_t*)T(f1.in[1]).host.data();   // [1600][512], row = c*25 + h*5 + w
         std::vector<int> colsum(512, 0);
-        for (int ch = 0; ch < 64; ++ch)
-            for (int hw = 0; hw < 25; ++hw) {
-                const int k = hw * 64 + ch;                         // position in the order stage 2 writes
-                const int8_t* src = &w[(size_t)(ch * 25 + hw) * 512];
-                for (int n = 0; n < 512; ++n) colsum[n] += src[n];
-                for (int n0 = 0; n0 < 512; n0 += FC_NT) {
-                    int8_t* dst = &w3blk[((size_t)n0 * 100 + (size_t)(k / 16) * FC_NT) * 16 + k % 16];
-                    for (int n = 0; n < FC_NT; ++n) dst[n * 16] = src[n0 + n];
+        for (int k = 0; k < 1600; ++k)
+            for (int n = 0; n < 512; ++n) colsum[n] += w[(size_t)k * 512 + n];
+        // 16 channels of a position are a K chunk: 16 rows of the matrix, transposed
+        for (int hw = 0; hw < 25; ++hw)
+            for (int c16 = 0; c16 < 4; ++c16) {
+                const int8_t* src = &w[(size_t)(c16 * 16 * 25 + hw) * 512];
+                for (int n = 0; n < 512; ++n) {
+                    int8_t* dst = &w3blk[((size_t)(n / FC_NT) * 100 * FC_NT + (size_t)(hw * 4 + c16) * FC_NT + n % FC_NT) * 16];
+                    for (int c = 0; c < 16; ++c) dst[c] = src[(size_t)c * 25 * 512 + n];
                 }
             }
         for (int n = 0; n < 512; ++n) b3[n] -= f1.a.x_zp * colsum[n];
