@@ -67,3 +67,9 @@ def test_biases_beyond_the_float_form(zb, ctx, oracle, models, scales, layer):
 def test_blocks_of_images(zb, ctx, oracle, models, scales, batch):
     g = models.small_cnn_int8(batch, act_scales=scales, bias_amplitude=(100, 1000, 5000, 300))
     _run(zb, ctx, oracle, g, models.small_cnn_input(batch, batch))
+
+
+@pytest.mark.parametrize("batch", [700, 1025])
+def test_several_single_windows_a_cta(zb, ctx, oracle, models, scales, batch):
+    g = models.small_cnn_int8(batch, act_scales=scales, bias_amplitude=(100, 1000, 5000, 300))
+    _run(zb, ctx, oracle, g, models.small_cnn_input(batch, batch))
