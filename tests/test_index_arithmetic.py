@@ -1,4 +1,4 @@
-"""Index arithmetic of two shared-memory kernels, restated on the CPU and checked over many shapes.
+"""Index arithmetic of shared-memory kernels, restated on the CPU and checked over many shapes.
 
 The stem mode of the pointwise kernel (`z-ant_b200/csrc/tc_pw_nchw.cuh`: `pw_stem_plan`, the loader's bulk
 copies, `pw_stem_builder`) and the rows-form depthwise kernel (`z-ant_b200/csrc/dwconv_q8.cuh`: the batch
@@ -8,10 +8,13 @@ invariants the kernels rely on: every bulk copy starts on 16 bytes, is a multipl
 stays inside its buffer; every input row a builder reads was loaded; every load and store stays inside
 its buffer (with the 16 bytes in front and behind that the kernels reserve); the one-multiplication
 division by the output width is exact; only the first pixel of tap 0 and the last pixel of a tap can lie
-outside the image.  No GPU is involved; the formulas must be kept in step with the kernels.
+outside the image.  The pooled convolution of the small CNN (`z-ant_b200/csrc/fused_cnn.cuh`: `tc_conv_pool_weights`, the operand addresses
+of `tc_conv3x3_pool_kernel`) is run on bytes: the MMAs' operands are gathered as the descriptors say and their sums compared with the
+convolution's.  No GPU is involved; the formulas must be kept in step with the kernels.
 """
 import itertools
 
+import numpy as np
 import pytest
 
 
@@ -129,3 +132,47 @@ def test_rows_form_depthwise_batches_and_offsets():
                         assert j < NA and (o == 0 or j + 1 <= NA) and S * x + 2 <= W + 1, where
                     assert pl * PO + r * OW + OW <= out, where
     assert configs > 100
+
+
+def kmajor(mem, start, rows, lbo):
+    """[rows][32] bytes of a K-major operand without swizzle: two chunks of 16 bytes `lbo` apart, rows 16 bytes apart."""
+    return np.concatenate([mem[start + c * lbo: start + c * lbo + rows * 16].reshape(rows, 16) for c in range(2)], axis=1).astype(np.int32)
+
+
+@pytest.mark.parametrize("ib", [128, 5])
+def test_pooled_convolution_operands(ib):
+    rng = np.random.default_rng(ib)
+    w = rng.integers(-128, 128, (64, 32, 3, 3), dtype=np.int8)
+    x = rng.integers(-128, 128, (ib, 32, 4, 4), dtype=np.int8)         # one window's input pixels
+    # weights: [kh][rx][chunk][dx][64][16]
+    block = 2 * 128 * 16
+    wm = np.zeros(12 * block, np.int8)
+    for kh, rx, dx in itertools.product(range(3), range(4), range(2)):
+        if 0 <= rx - dx <= 2:
+            for ch in range(32):
+                at = (kh * 4 + rx) * block + (ch // 16 * 128 + dx * 64 + np.arange(64)) * 16 + ch % 16
+                wm[at] = w[:, ch, kh, rx - dx]
+    # two stages of 4 x 2 pixels, as the bulk copies of a block of `ib` images leave them; what lies behind is whatever was there
+    pixel, stage = 2 * ib * 16, 8 * 2 * 128 * 16
+    am = rng.integers(-128, 128, 2 * stage, dtype=np.int8)
+    for ry, rx in itertools.product(range(4), range(4)):
+        for chunk in range(2):
+            at = (rx // 2) * stage + (ry * 2 + rx % 2) * pixel + chunk * (pixel // 2)
+            am[at:at + ib * 16] = x[:, chunk * 16:chunk * 16 + 16, ry, rx].reshape(-1)
+    d = np.zeros((128, 256), np.int64)
+    written = {}
+    for i, dy in itertools.product(range(12), range(2)):
+        kh, rx = i >> 2, i & 3
+        a = (0 if rx < 2 else stage) + (kh * 2 + (rx & 1)) * pixel + dy * 2 * pixel
+        assert a + pixel // 2 + 128 * 16 <= 2 * stage and a % 16 == 0
+        col, n = dy * 128, 128
+        # TMEM is written in the order of issue only by MMAs of one shape on one accumulator: no two others may overlap
+        for c0, n0 in written:
+            assert (c0, n0) == (col, n) or col + n <= c0 or c0 + n0 <= col
+        acc = kmajor(am, a, 128, pixel // 2) @ kmajor(wm, i * block, n, 2048).T
+        d[:, col:col + n] = acc + (d[:, col:col + n] if i > 0 else 0)
+        assert (i > 0) == ((col, n) in written)
+        written[(col, n)] = True
+    for dy, dx in itertools.product(range(2), range(2)):
+        want = np.einsum("nckl,mckl->nm", x[:, :, dy:dy + 3, dx:dx + 3].astype(np.int64), w.astype(np.int64))
+        assert np.array_equal(d[:ib, dy * 128 + dx * 64: dy * 128 + dx * 64 + 64], want)

@@ -248,15 +248,15 @@ __global__ void __launch_bounds__(C1M_THREADS, 2) conv1_mma_relu_pool_kernel(con
 // =============================================================================================
 // Stage 2: QLinearConv(32 -> 64, 3x3, no pad) + ReLU + MaxPool 2x2/2 on the image blocks that stage 1 writes.
 //
-// A tile is one pool window (py, px) of 128 images: MMA row r is image 128 * block + r.  The four members (dy, dx) of the window are four
-// accumulators of 64 columns, in the order (0,0), (0,1), (1,1), (1,0), so that nearly every view's members are neighbours: the view
-// (ry, rx), 0..3 each, serves the members with ry - dy and rx - dx in 0..2 - the four inner views all of them (one 128x256x32 MMA), the
-// edges two (128x128x32; for rx = 0 the two are the outer ones: two of 128x64x32), the corners one.  18 MMAs a tile, 1152 cycles of math and 1152
-// of shared-memory operands.  (Windows of a row-major plane on the MMA rows, 36 rows per image of which 25 are windows, took 24 MMAs of N = 64 and
-// 128 for 3.6 images' worth: 133 us at batch 65536, against 99 here.)
+// A tile is one pool window (py, px) of 128 images: MMA row r is image 128 * block + r.  The members (dy, dx) of the window are four accumulators
+// of 64 columns; the two of a row dy are one MMA accumulator of 128: filter row kh of member row dy reads the views (dy + kh, rx), rx 0..3, and
+// the block (kh, rx) of the weights holds tap (kh, rx) for dx = 0 and tap (kh, rx - 1) for dx = 1, zeros where that tap does not exist: 24 MMAs of
+// 128x128x32 a tile.  MMAs write TMEM in the order of issue only when they have the same accumulator and the same shape; hence two accumulators
+// that do not overlap and one shape.  (18 MMAs of 64, 128 and 256 columns, all of them useful, accumulated into columns that overlap: 102 us at
+// batch 65536, 117 with this form; one 128x256x32 MMA for each of the 16 views 130.)
 //
-// An item is a row of five windows (block, py), or one window where the rows are fewer than the SMs.  Its input is six (two) column pairs of 4 x 2
-// pixels, 32 KB each, of which a window reads two: a ring of five stages, each read by two windows.
+// An item is a row of five windows (block, py), or one window where that takes the rounds of the SMs less time (the plan's rule).  Its input is
+// six (two) column pairs of 4 x 2 pixels, 32 KB each, of which a window reads two: a ring of five stages, each read by two windows.
 //   warp 0 producer, warp 1 MMA issuer (the whole warp runs the loop, one lane issues; TMEM: two sets of 4 x 64 columns, so the epilogue of a
 //   tile overlaps the MMAs of the next), warps 2-17 epilogue: a thread holds all four members of its window for 16 filters - max, bias, ReLU
 //   and requantisation in registers, one 16-byte store into the GEMM-blocked layout [N/128][1600/16][ib images][16], 512 contiguous bytes a warp.
@@ -272,33 +272,24 @@ struct TcConvPoolArgs {
 
 struct TcConvPoolCfg {
     static constexpr int STAGES = 5, STAGE_BYTES = 8 * c2_pixel_bytes(128);      // [ry][column of the pair][chunk][128][16]
-    // weights: for each inner view [chunk][4 members][64][16]; then three chains [chunk][3 taps][64][16] for the edges and corners
-    static constexpr int W_VIEW_BYTES = 2 * 256 * 16, W_CHAIN_BYTES = 2 * 192 * 16;
-    static constexpr int W_BYTES = 4 * W_VIEW_BYTES + 3 * W_CHAIN_BYTES;
+    static constexpr int W_BLOCK_BYTES = 2 * 128 * 16, W_BYTES = 12 * W_BLOCK_BYTES;     // [kh][rx][chunk][dx][64][16]
     static constexpr int OFF_A = W_BYTES, OFF_BAR = OFF_A + STAGES * STAGE_BYTES, SMEM_BYTES = OFF_BAR + 256;
     static constexpr int TMEM_COLS = 512, THREADS = 576;
 };
 static_assert(TcConvPoolCfg::OFF_A % 128 == 0 && TcConvPoolCfg::SMEM_BYTES <= 227 * 1024, "");
 
-// One MMA of a tile: the view it reads, where its filters start (bytes into the weights) and how far their second K chunk lies, N, accumulator column.
-struct TcConvPoolMma { int ry, rx, w, lbo, n, col; };
-
 // w: [64][32][3][3]
 inline void tc_conv_pool_weights(const int8_t* w, int8_t* out) {
-    auto block = [&](int8_t* dst, int chunk, int tap) {
-        for (int m = 0; m < 64; ++m)
-            for (int c = 0; c < 16; ++c) dst[m * 16 + c] = w[(m * 32 + chunk * 16 + c) * 9 + tap];
-    };
-    const int order[4][2] = {{0, 0}, {0, 1}, {1, 1}, {1, 0}};
-    for (int v = 0; v < 4; ++v)
-        for (int chunk = 0; chunk < 2; ++chunk)
-            for (int j = 0; j < 4; ++j)
-                block(out + v * TcConvPoolCfg::W_VIEW_BYTES + (chunk * 4 + j) * 1024, chunk, (1 + v / 2 - order[j][0]) * 3 + 1 + v % 2 - order[j][1]);
-    const int chains[3][3] = {{2, 1, 0}, {6, 7, 8}, {8, 5, 2}};
-    for (int e = 0; e < 3; ++e)
-        for (int chunk = 0; chunk < 2; ++chunk)
-            for (int j = 0; j < 3; ++j)
-                block(out + 4 * TcConvPoolCfg::W_VIEW_BYTES + e * TcConvPoolCfg::W_CHAIN_BYTES + (chunk * 3 + j) * 1024, chunk, chains[e][j]);
+    std::memset(out, 0, TcConvPoolCfg::W_BYTES);
+    for (int kh = 0; kh < 3; ++kh)
+        for (int rx = 0; rx < 4; ++rx)
+            for (int dx = 0; dx < 2; ++dx) {
+                const int kw = rx - dx;
+                if (kw < 0 || kw > 2) continue;
+                for (int ch = 0; ch < 32; ++ch)
+                    for (int m = 0; m < 64; ++m)
+                        out[(kh * 4 + rx) * TcConvPoolCfg::W_BLOCK_BYTES + (ch / 16 * 128 + dx * 64 + m) * 16 + ch % 16] = w[(m * 32 + ch) * 9 + kh * 3 + kw];
+            }
 }
 
 template <bool BASE>
@@ -360,24 +351,11 @@ __global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_kernel(const __grid_co
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        // In this order an MMA rarely follows one that writes part of its columns in another shape: it would wait for that one to drain.
-        constexpr TcConvPoolMma M[18] = {
-            // inner views: member (dy, dx) takes tap (ry - dy, rx - dx)
-            {1, 1, 0, 4096, 256, 0}, {1, 2, 8192, 4096, 256, 0}, {2, 1, 16384, 4096, 256, 0}, {2, 2, 24576, 4096, 256, 0},
-            // chain 2, taps (2,2) (1,2) (0,2): members (0,1) and (1,1)
-            {1, 3, 45056 + 1024, 3072, 128, 64}, {2, 3, 45056, 3072, 128, 64},
-            // rx = 0, members (0,0) and (1,0): tap (1,0) is the second block of the first inner view
-            {1, 0, 1024, 4096, 64, 0}, {2, 0, 38912, 3072, 64, 0}, {0, 0, 32768 + 2048, 3072, 64, 0},
-            {1, 0, 32768 + 2048, 3072, 64, 192}, {2, 0, 1024, 4096, 64, 192}, {3, 0, 38912, 3072, 64, 192},
-            {0, 3, 32768, 3072, 64, 64}, {3, 3, 38912 + 2048, 3072, 64, 128},
-            // chain 0, taps (0,2) (0,1) (0,0), and chain 1, taps (2,0) (2,1) (2,2)
-            {0, 1, 32768 + 1024, 3072, 128, 0}, {0, 2, 32768, 3072, 128, 0}, {3, 1, 38912, 3072, 128, 128}, {3, 2, 38912 + 1024, 3072, 128, 128},
-        };
         const uint32_t leader = ptx::elect_one() ? 1u : 0u;
         auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag)) != 0; };
         const uint64_t da = ptx::smem_desc_kmajor(0, (uint32_t)pixel >> 1, 128);
         const uint32_t pixel_u = (uint32_t)pixel >> 4;
-        const uint32_t hi = (uint32_t)(da >> 32), a_lo0 = (uint32_t)da + (ptx::smem_u32(sA) >> 4), w_lo0 = ptx::smem_u32(sW) >> 4;
+        const uint32_t hi = (uint32_t)(da >> 32), a_lo0 = (uint32_t)da + (ptx::smem_u32(sA) >> 4), w_lo0 = (uint32_t)ptx::smem_desc_kmajor(ptx::smem_u32(sW), 2048, 128);
         int s = 0, it = 0; uint32_t ph = 0;                       // stage of the window's left column pair
         bool alive = true;
         for (int item = blockIdx.x; item < a.items && alive; item += gridDim.x) {
@@ -391,10 +369,12 @@ __global__ void __launch_bounds__(576, 1) tc_conv3x3_pool_kernel(const __grid_co
                 const uint32_t left = a_lo0 + (uint32_t)(s * (Cfg::STAGE_BYTES / 16)), right = a_lo0 + (uint32_t)(s1 * (Cfg::STAGE_BYTES / 16));
                 const uint32_t d = tmem_base + (uint32_t)(b * 256);
 #pragma unroll
-                for (int i = 0; i < 18; ++i) {
-                    const uint32_t al = (M[i].rx < 2 ? left : right) + (uint32_t)(M[i].ry * 2 + (M[i].rx & 1)) * pixel_u;
-                    const uint32_t bl = w_lo0 + (uint32_t)((M[i].w >> 4) | ((M[i].lbo >> 4) << 16));
-                    ptx::mma_i8_if(leader, d + (uint32_t)M[i].col, al, hi, bl, hi, ptx::idesc_i8(128, M[i].n, true, true), i > 0 ? 1u : 0u);   // the first initialises all members
+                for (int i = 0; i < 12; ++i) {                    // block (kh, rx) of the weights
+                    const int kh = i >> 2, rx = i & 3;
+                    const uint32_t al = (rx < 2 ? left : right) + (uint32_t)(kh * 2 + (rx & 1)) * pixel_u, bl = w_lo0 + (uint32_t)(i * (Cfg::W_BLOCK_BYTES >> 4));
+#pragma unroll
+                    for (int dy = 0; dy < 2; ++dy)
+                        ptx::mma_i8_if(leader, d + (uint32_t)(dy * 128), al + (uint32_t)(dy * 2) * pixel_u, hi, bl, hi, ptx::idesc_i8(128, 128, true, true), i > 0 ? 1u : 0u);
                 }
                 ptx::mma_commit_if(leader, empty(s));
                 if (px == a.wins - 1) ptx::mma_commit_if(leader, empty(s1));
