@@ -36,8 +36,8 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("case", CASES, ids=["x".join(map(str, c[:6] + c[9:])) for c in CASES])
-def test_block(zb, ctx, oracle, case):
+def block(zb, case):
+    """Graph up to the block's result `cur`, and the tensors t1, t2 between the convolutions."""
     N, C, E, M, H, W, xzp, bias, res, stride = case
     OH, OW = (H + stride - 1) // stride, (W + stride - 1) // stride
     rng = np.random.default_rng(C + E + H * 16 + W)
@@ -65,14 +65,47 @@ def test_block(zb, ctx, oracle, case):
         else:
             g.node("QLinearAdd", [cur, x], [y], x_scale=0.12, x_zp=0, b_scale=0.1, b_zp=xzp, y_scale=0.2, y_zp=0)
         cur = y
-    out = g.tensor("out", zb.F32, (N, M, OH, OW))
+    g.input = x0
+    return g, t1, t2, cur, rng.integers(-128, 128, (N, 4, H, W)).astype(np.int8)
+
+
+@pytest.mark.parametrize("case", CASES, ids=["x".join(map(str, c[:6] + c[9:])) for c in CASES])
+def test_block(zb, ctx, oracle, case):
+    g, t1, t2, cur, xv = block(zb, case)
+    out = g.tensor("out", zb.F32, g.tensors[cur]["shape"])
     g.node("DequantizeLinear", [cur], [out], x_scale=0.2, x_zp=0)
-    g.input, g.output = x0, out
-    xv = rng.integers(-128, 128, (N, 4, H, W)).astype(np.int8)
+    g.output = out
     want = graph_oracle.run(oracle, g, xv)
     plan = zb.Plan(ctx, g, fuse=True)
     assert any("expand+depthwise+project" in n for n in plan.step_names())
     for _ in range(2):
         assert np.array_equal(plan.run(xv), want[g.output])
     assert len(np.unique(want[t1])) > 30 and len(np.unique(want[t2])) > 20 and len(np.unique(want[cur])) > 30
+    plan.close()
+
+
+@pytest.mark.parametrize("res", [0, 1])
+def test_result_behind_a_reshape_is_the_output(zb, ctx, oracle, res):
+    """The block's result is then the caller's buffer, which need not have the alignment that the kernel's stores want."""
+    import torch
+    case = (160, 64, 384, 64, 14, 14, 0, True, res, 1)
+    g, t1, t2, cur, xv = block(zb, case)
+    flat = g.tensor("flat", zb.I8, (160, 64 * 14 * 14))
+    g.node("Reshape", [cur], [flat])
+    g.output = flat
+    want = graph_oracle.run(oracle, g, xv)[flat]
+    plan = zb.Plan(ctx, g, fuse=True)
+    steps = [n for n in plan.step_names() if "expand+depthwise+project" in n]
+    assert not steps or (res and not steps[0].endswith("+QLinearAdd"))         # (the addition, a step of its own, takes any alignment)
+    x = torch.from_numpy(xv).cuda()
+    buf = torch.zeros(want.size + 64, dtype=torch.int8, device="cuda")
+    for offset in (0, 32, 4, 1):
+        y = buf[offset:offset + want.size].view(want.shape)
+        try:
+            plan.run(x, y)
+        except zb.ZantError as e:
+            assert e.name == "InvalidInput" and offset % 32 != 0
+            continue
+        ctx.synchronize()
+        assert np.array_equal(y.cpu().numpy(), want)
     plan.close()

@@ -1296,6 +1296,14 @@ bool only_feeds_next(const ChainCtx& c, int tensor) {
     return c.consumers[tensor] == 1 && tensor != c.pl->output && !c.pl->t[tensor].is_const;
 }
 
+// The graph's output, or a tensor whose memory a Reshape hands on as the output's: in a run the caller's buffer, of whatever alignment.
+bool holds_output(const zant_plan* pl, int id) {
+    std::vector<int> same{id};
+    auto has = [&](int k) { return std::find(same.begin(), same.end(), k) != same.end(); };
+    for (const PlanNode& n : pl->nodes) if (n.op == ZANT_OP_RESHAPE && n.in.size() == 1 && n.out.size() == 1 && has(n.in[0])) same.push_back(n.out[0]);
+    return has(pl->output);
+}
+
 bool shape_is(const PlanTensor& t, std::initializer_list<size_t> s) { return t.shape == std::vector<size_t>(s); }
 
 bool plain_conv3x3(const zant_node_attrs& a) {
@@ -1358,7 +1366,7 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
     const int x = e->in[0], t1 = e->out[0], t2 = d->out[0], y0 = p->out[0];
     if (x < 0 || d->in[0] != t1 || p->in[0] != t2 || !only_feeds_next(c, t1) || !only_feeds_next(c, t2)) return ZANT_OK;
     auto plain = [&](int id) { return T(id).dtype == ZANT_I8 && T(id).shape.size() == 4 && !T(id).nh && T(id).alias < 0 && !T(id).elided && !T(id).is_const; };
-    if (!plain(x) || !plain(t1) || !plain(t2) || !plain(y0) || x == pl->input || y0 == pl->output) return ZANT_OK;
+    if (!plain(x) || !plain(t1) || !plain(t2) || !plain(y0) || x == pl->input || holds_output(pl, x) || holds_output(pl, y0)) return ZANT_OK;
     // parameters of the three convolutions
     ConvGeom g[3];
     std::vector<float> mult[3]; std::vector<int32_t> bias[3];
@@ -1401,7 +1409,7 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
     if (i0 + 3 < pl->nodes.size() && only_feeds_next(c, y0)) {
         const PlanNode& n = pl->nodes[i0 + 3];
         if (n.op == ZANT_OP_QLINEAR_ADD && n.in.size() == 2 && n.out.size() == 1 && ((n.in[0] == x && n.in[1] == y0) || (n.in[0] == y0 && n.in[1] == x)) &&
-            plain(n.out[0]) && n.out[0] != pl->output && T(n.out[0]).bytes == T(x).bytes && T(x).bytes == T(y0).bytes && g[0].C == g[2].M &&
+            plain(n.out[0]) && !holds_output(pl, n.out[0]) && T(n.out[0]).bytes == T(x).bytes && T(x).bytes == T(y0).bytes && g[0].C == g[2].M &&
             check_zero_point(ZANT_I8, n.a.y_zp, "QLinearAdd y") == ZANT_OK) {
             const bool first = n.in[0] == x;
             add = pl->prove(qadd_tail<false>(first ? n.a.x_scale : n.a.b_scale, first ? n.a.x_zp : n.a.b_zp, first ? n.a.b_scale : n.a.x_scale, first ? n.a.b_zp : n.a.x_zp, n.a.y_scale, n.a.y_zp, n.a.activation));
