@@ -71,3 +71,32 @@ def test_fused(zb, ctx, oracle, case):
     fused = any("+QLinearAdd" in n for n in plan.step_names())
     assert fused == (case != CASES[-1]), plan.step_names()
     plan.close()
+
+
+def test_operand_that_is_the_output(zb, ctx, oracle):
+    """A Reshape of the residual operand is the graph's output: the operand lies in the caller's buffer then, so the addition, whose
+    loads in the convolution's epilogue are words, stays a step of its own."""
+    rng = np.random.default_rng(3)
+    g = zb.Graph("res")
+    x = g.tensor("x", zb.I8, (64, 8, 64, 64))
+
+    def conv(src, cin, name):
+        w = g.tensor(f"w{name}", zb.I8, (32, cin, 1, 1), rng.integers(-127, 128, (32, cin, 1, 1), dtype=np.int8))
+        ws = g.tensor(f"s{name}", zb.F32, (32,), (rng.random(32, dtype=np.float32) * 0.01 + 0.002).astype(np.float32))
+        y = g.tensor(f"c{name}", zb.I8, (64, 32, 64, 64))
+        g.node("QLinearConv", [src, w, ws, -1, -1], [y], x_scale=0.05, x_zp=0, y_scale=0.3, y_zp=0, pads=(0,) * 4, strides=(1, 1), group=1, **CONV)
+        return y
+
+    r = conv(x, 8, "r")
+    cur = conv(r, 32, "c")
+    y = g.tensor("sum", zb.I8, (64, 32, 64, 64))
+    g.node("QLinearAdd", [r, cur], [y], x_scale=0.3, x_zp=0, b_scale=0.3, b_zp=0, y_scale=0.5, y_zp=0)
+    flat = g.tensor("flat", zb.I8, (64, 32 * 64 * 64))
+    g.node("Reshape", [r], [flat])
+    g.input, g.output = x, flat
+    xv = rng.integers(-128, 128, (64, 8, 64, 64)).astype(np.int8)
+    want = graph_oracle.run(oracle, g, xv)
+    plan = zb.Plan(ctx, g, fuse=True)
+    assert not any("+QLinearAdd" in n for n in plan.step_names())
+    assert np.array_equal(plan.run(xv), want[flat]) and np.array_equal(plan.read_tensor(y), want[y])
+    plan.close()

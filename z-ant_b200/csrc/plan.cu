@@ -1587,7 +1587,7 @@ static int32_t try_fuse_qconv_group(zant_plan* pl, size_t i0, size_t& consumed) 
             const int r = add.in[0] == cur ? add.in[1] : add.in[0], y = add.out[0];
             bool there = false;
             for (size_t k = 0; k < i0; ++k) for (int id : pl->nodes[k].out) there = there || id == r;
-            if (r >= 0 && there && !T(r).elided && !T(r).nh && T(r).alias < 0 && r != pl->input && r != pl->output && y != pl->output && T(cur).dtype == ZANT_I8 &&
+            if (r >= 0 && there && !T(r).elided && !T(r).nh && T(r).alias < 0 && r != pl->input && !holds_output(pl, r) && y != pl->output && T(cur).dtype == ZANT_I8 &&
                 T(r).dtype == ZANT_I8 && T(y).dtype == ZANT_I8 && T(r).bytes == T(cur).bytes && T(y).bytes == T(cur).bytes && check_zero_point(ZANT_I8, add.a.y_zp, "QLinearAdd y") == ZANT_OK) {
                 fz.add_node = (int)j;
                 fz.add_res = r;
