@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
                 if (warp == 2) {
                     if (!wait(sum_full, 0)) return false;
                     if (lane == 0) {
+                        __threadfence();                                  // (the other warps' additions, which sum_full ordered before this thread, before the counter)
                         const bool last = atomicAdd(a.arrived + t, 1) == splits - 1;
                         if (last) a.arrived[t] = 0;
                         *finish = last ? 1 : 0;
