@@ -109,3 +109,30 @@ def test_result_behind_a_reshape_is_the_output(zb, ctx, oracle, res):
         ctx.synchronize()
         assert np.array_equal(y.cpu().numpy(), want)
     plan.close()
+
+
+@pytest.mark.parametrize("case,ctas", [((31, 48, 700, 48, 5, 5, 0, True, 1, 1), 96), ((16, 160, 960, 320, 7, 7, -3, True, 0, 1), 64)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_sums_are_clean_after_a_time_out(zb, oracle, case, ctas, graph):
+    """A CTA that gives up half way through its additions reports a time-out in its run; the runs behind it are right."""
+    ctx = zb.Context(0)
+    g, t1, t2, cur, xv = block(zb, case)
+    out = g.tensor("out", zb.F32, g.tensors[cur]["shape"])
+    g.node("DequantizeLinear", [cur], [out], x_scale=0.2, x_zp=0)
+    g.output = out
+    want = graph_oracle.run(oracle, g, xv)[out]
+    plan = zb.Plan(ctx, g, fuse=True)
+    assert any("expand+depthwise+project" in n for n in plan.step_names())
+    for cta in (0, 1, ctas // 2, ctas - 1):
+        ctx.selftest_give_up(cta)
+        if graph:
+            plan.use_graph(True)                 # (the kernel that gives up is part of this graph)
+        with pytest.raises(zb.ZantError) as e:
+            plan.run(xv)
+        assert e.value.name == "DeviceTimeout"
+        if graph:
+            plan.use_graph(True)
+        for _ in range(2):
+            assert np.array_equal(plan.run(xv), want)
+    plan.close()
+    ctx.close()

@@ -324,6 +324,10 @@ class Context:
         """Launches the bounded-wait self test; the next synchronize() raises DeviceTimeout once."""
         check(lib().zant_b200_selftest_bounded_wait(self._h, C.c_uint32(int(budget_us))))
 
+    def selftest_give_up(self, cta):
+        """CTA `cta` of the next kernel that adds up partial sums gives up; that run raises DeviceTimeout."""
+        check(lib().zant_b200_selftest_give_up(self._h, C.c_int32(int(cta))))
+
     def measure_int8_peak(self, iters=20000):
         """Attainable int8 tensor rate (TOP/s) from the resident-tile tcgen05 probe."""
         v = C.c_double(0.0)

@@ -203,6 +203,12 @@ int32_t zant_b200_selftest_bounded_wait(zant_ctx* ctx, uint32_t budget_us) {
     return check_launch(ctx, "bounded_wait_selftest_kernel");
 }
 
+int32_t zant_b200_selftest_give_up(zant_ctx* ctx, int32_t cta) {
+    ZB_NEED_CTX(ctx);
+    ctx->give_up_cta = cta < 0 ? -1 : cta;
+    return ZANT_OK;
+}
+
 int32_t zant_b200_debug_fail_alloc(int32_t nth) {
     alloc_failures_armed().store(nth > 0 ? nth : 0);
     return ZANT_OK;

@@ -18,7 +18,9 @@
 // operand of unit u holds the filters in lanes 64 u .. and zeros elsewhere, and all four lane quarters take part in the project epilogue.
 //
 // SPLITS.  Where the tiles leave SMs idle the chunks of a tile are dealt to `splits` CTAs, each adds its D2 to 32-bit sums in global memory
-// (exact in any order) and the last of them to come runs the project epilogue from there and leaves the sums zero for the next run.
+// (exact in any order) and the last of them to come runs the project epilogue from there and leaves the sums zero for the next run.  A CTA whose
+// wait ran out counts itself all the same, when its warps are done, and the last one zeroes the tile's sums if it gave up itself: a run that
+// reported a time-out leaves the next one (a graph's replay too) what a run in order leaves.
 //
 // What bounds it: instruction issue in the epilogue warps, 31 thousand of the warp instructions of a 14 x 14 x 384 image are the two
 // requantisations, the filter and the project epilogue (as separate kernels the depthwise one alone took 31 instructions an output).
@@ -65,6 +67,7 @@ struct IrbArgs {
     int d1_bufs;                   // one unit: buffers of D1
     int splits;                    // CTAs per tile; above 1 a CTA has one tile
     int32_t* sums; int* arrived;   // splits: [tile][D2 column][128 lanes], all zero between runs, and a counter per tile
+    int give_up;                   // splits: self test, a CTA half of whose epilogue warps give up (-1: none)
     int x_bufs, y_bufs, w_stages;
     int w_bytes, x_bytes, y_bytes; // one stage / buffer
     int off_x, off_y, off_out, off_tail;
@@ -73,7 +76,7 @@ struct IrbArgs {
 
 // fewer tiles: the separate kernels use more of the chip (one image of 224 x 224: 250 us with them, 288 with this)
 constexpr int kIrbMinTiles = 8;
-constexpr int kIrbThreads = 640, kIrbEpiWarps = 16, kIrbMaxStages = 2;
+constexpr int kIrbThreads = 640, kIrbEpiWarps = 16;
 
 // N accumulators of consecutive columns, N at most 9.
 template <int N>
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 256);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 260);
     volatile int* finish = reinterpret_cast<volatile int*>(tail + 264);      // this CTA has the tile's sums
+    volatile int* counted = reinterpret_cast<volatile int*>(tail + 268);     // splits: this CTA is in the tile's counter (2: as the last)
     const uint32_t smem0 = ptx::smem_u32(smem), bar0 = ptx::smem_u32(bars);
     auto wfull = [&](int s) { return bar0 + 8u * s; };
     auto wempty = [&](int s) { return bar0 + 8u * (2 + s); };
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
         ptx::mbar_init(d2full, 1); ptx::mbar_init(d2empty, kIrbEpiWarps);
         ptx::mbar_init(out_free, 1); ptx::mbar_init(out_full, kIrbEpiWarps);
         ptx::mbar_init(sum_full, kIrbEpiWarps); ptx::mbar_init(sum_done, 1);
-        *abort_flag = 0; *finish = 1;
+        *abort_flag = 0; *finish = 1; *counted = 0;
         ptx::mbar_fence_init();
     }
     if (warp == 1) {
@@ -433,6 +437,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
             ptx::tc_fence_after();
             int32_t* sums = nullptr;
             if constexpr (SPLIT) {
+                if ((int)blockIdx.x == a.give_up && (warp & 1)) { *abort_flag = 1; return false; }
                 sums = a.sums + (size_t)t * d2_cols * 128 + ch;
                 // this warp's part of D2 into the tile's sums
                 for (int mt = 0; mt < a.mt2; ++mt) {
@@ -457,6 +462,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
                         const bool last = atomicAdd(a.arrived + t, 1) == splits - 1;
                         if (last) a.arrived[t] = 0;
                         *finish = last ? 1 : 0;
+                        *counted = last ? 2 : 1;
                         __threadfence();
                         ptx::mbar_arrive(sum_done);
                     }
@@ -582,6 +588,19 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 1) ptx::tmem_dealloc(tmem_base, tmem_cols);
+    if (SPLIT && my_tiles > 0 && *abort_flag) {
+        // nothing of this CTA adds or waits any more
+        if (tid == 0 && *counted == 0) {
+            __threadfence();
+            const bool last = atomicAdd(a.arrived + tile0, 1) == splits - 1;
+            if (last) a.arrived[tile0] = 0;
+            *counted = last ? 2 : 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (*counted == 2)
+            for (int i = tid; i < d2_cols * 128; i += kIrbThreads) a.sums[(size_t)tile0 * d2_cols * 128 + i] = 0;
+    }
     if (tid == 0 && *abort_flag) atomicExch(a.status, (int)DEV_ERR_WAIT_TIMEOUT);
 }
 
@@ -679,7 +698,8 @@ inline bool irb_prepare(const IrbPlan& q, const int8_t* we, const float* em, con
 inline int32_t irb_run(zant_ctx* ctx, const IrbPlan& q, const void* x, const uint8_t* w, const float* mult2, const int32_t* bias2, void* y, void* sums, const QAddTail* add) {
     IrbArgs a = q.a;
     a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.w = w; a.mult2 = mult2; a.bias2 = bias2; a.status = ctx->status_word;
-    if (a.splits > 1) { a.sums = (int32_t*)sums; a.arrived = (int*)((char*)sums + q.sums_bytes); }
+    a.give_up = -1;
+    if (a.splits > 1) { a.sums = (int32_t*)sums; a.arrived = (int*)((char*)sums + q.sums_bytes); std::swap(a.give_up, ctx->give_up_cta); }
     const int grid = std::min(a.tiles * a.splits, ctx->sm_count);
     auto go = [&](auto wc, auto stride, auto with, auto split) -> int32_t {
         constexpr int WC = decltype(wc)::value, S = decltype(stride)::value;
