@@ -176,3 +176,15 @@ def test_pooled_convolution_operands(ib):
     for dy, dx in itertools.product(range(2), range(2)):
         want = np.einsum("nckl,mckl->nm", x[:, :, dy:dy + 3, dx:dx + 3].astype(np.int64), w.astype(np.int64))
         assert np.array_equal(d[:ib, dy * 128 + dx * 64: dy * 128 + dx * 64 + 64], want)
+
+
+def test_row_copy_counter_stays_in_its_type():
+    """rows_blocked_kernel (tc_conv_generic.cuh) steps an unsigned by the whole grid, at most 148 * 8 CTAs of 256 threads, up to the largest
+    number of chunks that the host admits: the last value compared, one step behind the last chunk, must not wrap.  (It does in an int.)"""
+    step, most = 148 * 8 * 256, 0x7fffffff - 1
+    for chunks in (most, most - step, most - step + 1, 1 << 30):
+        for first in (0, 1, step - 1):
+            last = first + (chunks - 1 - first) // step * step + step
+            assert last < 1 << 32 and last >= chunks
+            for i in (chunks - 1, chunks - 129, 127):
+                assert 0 <= (i >> 7) < 1 << 24 and (i >> 7) * 128 + (i & 127) == i

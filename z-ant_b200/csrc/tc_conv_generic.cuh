@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(256) pointwise_blocked_kernel(const PwBlockArg
 // Matrix products (one position per image): a row of K bytes is a run of 16-byte chunks already.
 __global__ void __launch_bounds__(256) rows_blocked_kernel(const uint4* x, uint4* a, int M, int c16, int K16, int chunks) {
     ptx::grid_start();
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < chunks; i += gridDim.x * 256) {
+    // (unsigned: the step behind the last chunk may leave the range of int, the host admits up to 2^31 - 1 chunks)
+    for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < (unsigned)chunks; i += gridDim.x * 256) {
         const int r = i & 127, q = i >> 7, mt = q / K16, k = q - mt * K16, m = mt * 128 + r;
         a[i] = m < M && k < c16 ? __ldg(x + (size_t)m * c16 + k) : make_uint4(0u, 0u, 0u, 0u);
     }
