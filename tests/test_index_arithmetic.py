@@ -97,6 +97,20 @@ def test_stem_mode_offsets_stay_inside_their_buffers():
     assert checked > 200
 
 
+def rows_unit(P, PO):
+    unit = 16
+    while unit > 1 and (P * (unit // 2)) % 16 == 0 and (PO * (unit // 2)) % 16 == 0:
+        unit //= 2
+    return unit
+
+
+def rows_buffers(PB, P, PO, limit):
+    """Bytes of a batch in and out, and the distance of the buffers; None beyond the dispatch's limit."""
+    buf, out = PB * P, PB * PO
+    in_stride, out_stride = (buf + 32 + 127) // 128 * 128, (out + 127) // 128 * 128
+    return None if 3 * in_stride + 2 * out_stride + 32 > limit else (buf, out, in_stride, out_stride)
+
+
 def test_rows_form_depthwise_batches_and_offsets():
     configs = 0
     for S, widths in ((1, (7, 14, 28)), (2, (14, 28))):
@@ -105,16 +119,11 @@ def test_rows_form_depthwise_batches_and_offsets():
             if OH > 64:
                 continue
             P, PO = H * W, OH * OW
-            unit = 16
-            while unit > 1 and (P * (unit // 2)) % 16 == 0 and (PO * (unit // 2)) % 16 == 0:
-                unit //= 2
+            unit = rows_unit(P, PO)
             PB = 256 // OH // unit * unit
-            if PB < unit:
+            if PB < unit or rows_buffers(PB, P, PO, 48 * 1024) is None:
                 continue
-            buf, out = PB * P, PB * PO
-            in_stride, out_stride = (buf + 32 + 127) // 128 * 128, (out + 127) // 128 * 128
-            if 3 * in_stride + 2 * out_stride + 32 > 48 * 1024:
-                continue
+            buf, out, in_stride, out_stride = rows_buffers(PB, P, PO, 48 * 1024)
             configs += 1
             where = (S, W, H, PB)
             assert buf % 16 == 0 and out % 16 == 0 and PB * OH <= 256, where
@@ -132,6 +141,48 @@ def test_rows_form_depthwise_batches_and_offsets():
                         assert j < NA and (o == 0 or j + 1 <= NA) and S * x + 2 <= W + 1, where
                     assert pl * PO + r * OW + OW <= out, where
     assert configs > 100
+
+
+def test_two_rows_form_depthwise_batches_and_offsets():
+    """A thread's two output rows of a plane 28 wide: whole words in and out, every row of every plane by exactly one thread, and the
+    columns that a window takes from the words to its left and right."""
+    configs = 0
+    W, NW = 28, 7
+    for H in range(1, 65):
+        P, tpp = H * W, (H + 1) // 2
+        unit = rows_unit(P, P)
+        PB = 256 // tpp // unit * unit
+        if PB < unit or rows_buffers(PB, P, P, 96 * 1024) is None:
+            continue
+        buf, out, in_stride, out_stride = rows_buffers(PB, P, P, 96 * 1024)
+        configs += 1
+        assert buf % 16 == 0 and out % 16 == 0 and PB * tpp <= 256 and 3 * in_stride + 2 * out_stride + 32 <= 96 * 1024, H
+        rows = set()
+        for t in range(256):
+            pl, r = t // tpp, t % tpp * 2
+            if pl >= PB:
+                continue
+            for i in range(4):
+                iy = r - 1 + i
+                if 0 <= iy < H:
+                    at = 16 + pl * P + iy * W
+                    assert at % 4 == 0 and 16 <= at and at + 4 * NW <= in_stride, (H, t)
+            for row in (r, r + 1):
+                if row < H:
+                    at = pl * P + row * W
+                    assert at % 4 == 0 and at + W <= out and (pl, row) not in rows, (H, t)
+                    rows.add((pl, row))
+        assert len(rows) == PB * H, H
+    assert configs > 50
+    # windows of the four columns of word w: bytes 4w - 1 .. 4w + 4 of left, middle and right words
+    line = [None] + list(range(W)) + [None] * 4
+    word = lambda w: [line[4 * w + 1 + k] if 0 <= w < NW else None for k in range(4)]
+    for w in range(NW):
+        both, right = word(w - 1) + word(w), word(w) + word(w + 1)
+        windows = [[both[s] for s in (3, 4, 5, 6)], word(w), [right[s] for s in (1, 2, 3, 4)], [right[s] for s in (2, 3, 4, 5)]]
+        for x, win in enumerate(windows):
+            col = 4 * w + x
+            assert win[:3] == [c if 0 <= c < W else None for c in (col - 1, col, col + 1)], (w, x)
 
 
 def kmajor(mem, start, rows, lbo):

@@ -411,10 +411,11 @@ __global__ void __launch_bounds__(256) qdwconv3x3_s1w8_kernel(const QDwParam<BAN
 // stored to the output batch bytewise (two bytes at a time when the rows are 2-byte aligned).  Three input and two output
 // buffers: the next two batches are in flight and the previous one is being written back while a batch is computed.
 // PB * H * W and PB * OH * OW are multiples of 16 (bulk copies), and a trailing batch of fewer planes is copied by the threads.
-// Rows of whole words at stride 1 (28 wide): a thread owns TWO output rows.  Their four input rows are words as they lie, kept in registers; four
-// columns at a time the windows of an input row serve both outputs and the results leave as words: 12 instructions an output instead of
-// 31.  192 channels of 28 x 28, 1024 images, inside a plan: 102 us (46 % of the measured HBM rate; 71 KB of buffers, three CTAs an SM), 118 us with a
-// row per thread.
+// PAIR, rows of whole words at stride 1 (28 wide): a thread owns TWO output rows.  Their four input rows are words as they lie, kept in registers;
+// four columns at a time the windows of an input row serve both outputs and the results leave as words: 12 instructions an output instead of
+// 31, on half the threads a plane, so twice the planes a batch (71 KB of buffers, three CTAs an SM).  From two batches an SM on: 196608 planes of
+// 28 x 28 98 us (46 % of the measured HBM rate), 113 with a row per thread; 6144 planes 5.9, 7.3; with fewer the longer chain of a thread shows:
+// 4608 planes 6.1, 5.1, 192 planes 5.3, 3.5.
 struct QDwRowsArgs {
     QDwArgs p;
     int PB;                    // planes per batch
@@ -424,12 +425,12 @@ struct QDwRowsArgs {
     int* status;               // device status word: DEV_ERR_WAIT_TIMEOUT when a bounded wait gave up
 };
 
-template <bool XU8, bool LEAN, int W, int S>
+template <bool XU8, bool LEAN, int W, int S, bool PAIR>
 __global__ void __launch_bounds__(256) qdwconv3x3_rows_kernel(const QDwRowsArgs a) {
     ptx::grid_start();
     constexpr int NA = (W + 2 + 3) / 4;                             // words that hold the bytes col -1 .. col W
     constexpr int OW = S == 1 ? W : W / 2;
-    constexpr bool PAIR = S == 1 && W % 4 == 0;
+    static_assert(!PAIR || (S == 1 && W % 4 == 0), "");
     extern __shared__ __align__(128) uint8_t dw_rows_smem[];
     const QDwArgs& p = a.p;
     const int P = p.H * W, PO = p.OH * OW;
@@ -832,34 +833,37 @@ inline int32_t run_qdwconv(zant_ctx* ctx, const ConvGeom& g, const void* x, bool
         while (unit > 1 && (P * (unit / 2)) % 16 == 0 && (PO * (unit / 2)) % 16 == 0) unit /= 2;
         QDwRowsArgs ra{};
         ra.p = a;
-        // a thread owns two output rows: half the threads a plane, so twice the planes a batch, and 96 KB for the five buffers instead of 48
-        const bool pair = rows_s1 && g.W % 4 == 0;
-        ra.PB = 256 / (pair ? (g.OH + 1) / 2 : g.OH) / unit * unit;
-        if (ra.PB >= unit && a.planes >= 4 * ra.PB) {
+        ra.status = ctx->status_word;
+        size_t smem = 0;
+        // batches for `tpp` threads a plane and `limit` bytes of buffers; at least `min_batches`
+        auto batches = [&](int tpp, long long min_batches, size_t limit) {
+            ra.PB = 256 / tpp / unit * unit;
+            if (ra.PB < unit || a.planes < min_batches * ra.PB) return false;
             ra.batches = (a.planes + ra.PB - 1) / ra.PB;
             ra.buf_bytes = ra.PB * P;
             ra.out_bytes = ra.PB * PO;
-            ra.status = ctx->status_word;
-            const int in_stride = (ra.buf_bytes + 32 + 127) / 128 * 128, out_stride = (ra.out_bytes + 127) / 128 * 128;
-            const size_t smem = (size_t)3 * in_stride + 2 * out_stride + 32;
-            const int rgrid = (int)std::min<long long>(ra.batches, (long long)ctx->sm_count * 8);
-            auto pick = [&](auto w_tag, auto s_tag) -> int32_t {
-                constexpr int KW = decltype(w_tag)::value, KS = decltype(s_tag)::value;
-                auto go = [&](auto u8_tag, auto lean_tag) -> int32_t {
-                    constexpr bool XU8 = decltype(u8_tag)::value, LEAN = decltype(lean_tag)::value;
-                    if (KS == 1 && KW % 4 == 0) ZB_SMEM_ATTR(ctx, (qdwconv3x3_rows_kernel<XU8, LEAN, KW, KS>), 96 * 1024);
-                    launch(ctx, qdwconv3x3_rows_kernel<XU8, LEAN, KW, KS>, rgrid, 256, smem, ra);
-                    return check_launch(ctx, "qdwconv3x3_rows_kernel");
-                };
-                if (x_u8) return lean ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
-                return lean ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+            smem = (size_t)3 * ((ra.buf_bytes + 32 + 127) / 128 * 128) + 2 * ((ra.out_bytes + 127) / 128 * 128) + 32;
+            return smem <= limit;
+        };
+        auto pick = [&](auto w_tag, auto s_tag, auto pair_tag) -> int32_t {
+            constexpr int KW = decltype(w_tag)::value, KS = decltype(s_tag)::value;
+            constexpr bool PAIR = decltype(pair_tag)::value;
+            auto go = [&](auto u8_tag, auto lean_tag) -> int32_t {
+                constexpr bool XU8 = decltype(u8_tag)::value, LEAN = decltype(lean_tag)::value;
+                if (PAIR) ZB_SMEM_ATTR(ctx, (qdwconv3x3_rows_kernel<XU8, LEAN, KW, KS, PAIR>), 96 * 1024);
+                launch(ctx, qdwconv3x3_rows_kernel<XU8, LEAN, KW, KS, PAIR>, (int)std::min<long long>(ra.batches, (long long)ctx->sm_count * 8), 256, smem, ra);
+                return check_launch(ctx, "qdwconv3x3_rows_kernel");
             };
-            if (smem <= (pair ? 96 : 48) * 1024) {
-                using std::integral_constant;
-                if (rows_s1 && g.W == 28) return pick(integral_constant<int, 28>{}, integral_constant<int, 1>{});
-                if (rows_s1) return g.W == 14 ? pick(integral_constant<int, 14>{}, integral_constant<int, 1>{}) : pick(integral_constant<int, 7>{}, integral_constant<int, 1>{});
-                return g.W == 28 ? pick(integral_constant<int, 28>{}, integral_constant<int, 2>{}) : pick(integral_constant<int, 14>{}, integral_constant<int, 2>{});
-            }
+            if (x_u8) return lean ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+            return lean ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+        };
+        using std::integral_constant;
+        // two rows a thread from two batches an SM on (qdwconv3x3_rows_kernel), at least four batches of the other form
+        if (rows_s1 && g.W == 28 && batches((g.OH + 1) / 2, 2LL * ctx->sm_count, 96 * 1024)) return pick(integral_constant<int, 28>{}, integral_constant<int, 1>{}, std::true_type{});
+        if (batches(g.OH, 4, 48 * 1024)) {
+            if (rows_s1 && g.W == 28) return pick(integral_constant<int, 28>{}, integral_constant<int, 1>{}, std::false_type{});
+            if (rows_s1) return g.W == 14 ? pick(integral_constant<int, 14>{}, integral_constant<int, 1>{}, std::false_type{}) : pick(integral_constant<int, 7>{}, integral_constant<int, 1>{}, std::false_type{});
+            return g.W == 28 ? pick(integral_constant<int, 28>{}, integral_constant<int, 2>{}, std::false_type{}) : pick(integral_constant<int, 14>{}, integral_constant<int, 2>{}, std::false_type{});
         }
     }
     if (!aligned && g.sh == 1) {
