@@ -807,26 +807,42 @@ inline int32_t nh_conv_run(zant_ctx* ctx, const NhConvPlan& p, NhConvArgs a, con
 // ---------------------------------------------------------------------------------------------
 // First layers: an NCHW tensor of at most four channels -> pixels of 16 bytes.  MODE 0: float, quantised (QuantizeLinear);
 // 1: 8-bit codes as they are; 2: float, rounded to TF32 (pixels of 4 floats); 3: hi and lo halves of 8 floats each.
-// A CTA takes 1024 pixels of one image, a lane every 32nd of its warp's 128: loads and 16-byte pixel stores are contiguous over the warp
+// A CTA takes 1024 pixels, a lane every 32nd of its warp's 128: loads and 16-byte pixel stores are contiguous over the warp
 // whatever the plane's alignment.  (Four neighbouring pixels a thread stored 16 bytes of every 64: 32 images of 3 x 416 x 416 took 43 us,
-// 155 MB.)
-struct ToNhwcArgs { const void* x; uint8_t* y; int C, HW, blocks_per_image; QuantFast qf; QuantSteps qs; int zp; };
-template <int MODE>
+// 155 MB.)  PACKED, planes of at most 512 pixels: as many whole images as 1024 pixels hold, a pixel's image is a division (one image a
+// CTA: 4096 of 3 x 8 x 8 14.7 us, packed 7.2); larger planes: 1024 pixels of one image.
+struct ToNhwcArgs { const void* x; uint8_t* y; int C, N, imgs; long long HW, blocks_per_image; QuantFast qf; QuantSteps qs; int zp; };
+template <int MODE, bool PACKED>
 __global__ void __launch_bounds__(256) to_nhwc_small_k(const __grid_constant__ ToNhwcArgs a) {
     ptx::grid_start();
-    const int n = (int)blockIdx.x / a.blocks_per_image, p0 = ((int)blockIdx.x - n * a.blocks_per_image) * 1024 + (int)(threadIdx.x >> 5) * 128 + (int)(threadIdx.x & 31);
-    const long long px0 = (long long)n * a.HW + p0;
+    const int t = (int)(threadIdx.x >> 5) * 128 + (int)(threadIdx.x & 31);
+    long long px0, off[4];                   // the first pixel, in the whole run; element of channel 0
+    bool on[4];
+    if (PACKED) {
+        const int hw = (int)a.HW, n0 = (int)blockIdx.x * a.imgs, here = min(a.imgs, a.N - n0) * hw;
+        px0 = (long long)n0 * hw + t;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = t + 32 * j, dn = (int)((unsigned)r / (unsigned)hw);
+            off[j] = (long long)n0 * a.C * hw + dn * a.C * hw + (r - dn * hw); on[j] = r < here;
+        }
+    } else {
+        const long long n = (long long)blockIdx.x / a.blocks_per_image, p0 = ((long long)blockIdx.x - n * a.blocks_per_image) * 1024 + t;
+        px0 = n * a.HW + p0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { off[j] = n * a.C * a.HW + p0 + 32 * j; on[j] = p0 + 32 * j < a.HW; }
+    }
     float f[4][4] = {};
     uint32_t q[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         if (c >= a.C) break;
-        const long long at = ((long long)n * a.C + c) * a.HW + p0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (p0 + 32 * j >= a.HW) continue;
-            if (MODE == 1) q[j] |= (uint32_t)__ldg((const uint8_t*)a.x + at + 32 * j) << (8 * c);
-            else f[j][c] = __ldg((const float*)a.x + at + 32 * j);
+            if (!on[j]) continue;
+            const long long at = off[j] + c * a.HW;
+            if (MODE == 1) q[j] |= (uint32_t)__ldg((const uint8_t*)a.x + at) << (8 * c);
+            else f[j][c] = __ldg((const float*)a.x + at);
         }
     }
     if (MODE == 0) {
@@ -845,7 +861,7 @@ __global__ void __launch_bounds__(256) to_nhwc_small_k(const __grid_constant__ T
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (p0 + 32 * j >= a.HW) break;
+        if (!on[j]) break;
         const long long px = px0 + 32 * j;
         if (MODE <= 1) {
             *reinterpret_cast<uint4*>(a.y + px * 16) = make_uint4(q[j], 0u, 0u, 0u);
@@ -862,17 +878,21 @@ __global__ void __launch_bounds__(256) to_nhwc_small_k(const __grid_constant__ T
 // `steps`: the quantisation's quotient without a division, where the caller has it (quant_steps).
 inline int32_t run_to_nhwc(zant_ctx* ctx, int mode, const void* x, void* y, int N, int C, long long HW, float scale, int zp, bool u8, const QuantSteps& steps = QuantSteps{0.0f, 0.0f}) {
     ToNhwcArgs a{};
-    const long long per = (HW + 1023) / 1024;
-    if (HW > 0x3fffffffLL || per * N > 0x7fffffffLL) return fail(ZANT_E_TOO_LARGE, "too many pixels for the channels-last conversion");
-    if (per * N == 0) return ZANT_OK;
-    a.x = x; a.y = (uint8_t*)y; a.C = C; a.HW = (int)HW; a.blocks_per_image = (int)per; a.zp = zp; a.qs = steps;
+    const bool packed = HW <= 512;
+    const long long imgs = packed && HW > 0 ? 1024 / HW : 1, per = (HW + 1023) / 1024, grid = (N + imgs - 1) / imgs * per;
+    if (grid > 0x7fffffffLL) return fail(ZANT_E_TOO_LARGE, "too many pixels for the channels-last conversion");
+    if (grid == 0) return ZANT_OK;
+    a.x = x; a.y = (uint8_t*)y; a.C = C; a.N = N; a.imgs = (int)imgs; a.HW = HW; a.blocks_per_image = per; a.zp = zp; a.qs = steps;
     if (mode == 0) a.qf = quant_fast(scale, (float)((u8 ? 0 : -128) - zp), (float)((u8 ? 255 : 127) - zp));
-    const int grid = (int)(per * N);
+    auto go = [&](auto m) {
+        if (packed) launch(ctx, to_nhwc_small_k<decltype(m)::value, true>, (unsigned)grid, 256, 0, a);
+        else launch(ctx, to_nhwc_small_k<decltype(m)::value, false>, (unsigned)grid, 256, 0, a);
+    };
     switch (mode) {
-        case 0: launch(ctx, to_nhwc_small_k<0>, grid, 256, 0, a); break;
-        case 1: launch(ctx, to_nhwc_small_k<1>, grid, 256, 0, a); break;
-        case 2: launch(ctx, to_nhwc_small_k<2>, grid, 256, 0, a); break;
-        default: launch(ctx, to_nhwc_small_k<3>, grid, 256, 0, a); break;
+        case 0: go(std::integral_constant<int, 0>{}); break;
+        case 1: go(std::integral_constant<int, 1>{}); break;
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        default: go(std::integral_constant<int, 3>{}); break;
     }
     return check_launch(ctx, "to_nhwc_small_k");
 }
