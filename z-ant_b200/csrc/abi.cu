@@ -906,7 +906,7 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
     if (qconv_tc_eligible(g, wz_zero)) {
         // tensor-core path: im2col into the GEMM-blocked layout, tcgen05 GEMM, NCHW requantised store
         QGemmPrep prep;
-        qgemm_sizes(g.M, g.Cg * g.KH * g.KW, mult.data(), prep, (long long)g.N * g.OH * g.OW);
+        qgemm_sizes(g.M, g.Cg * g.KH * g.KW, mult.data(), prep, (long long)g.N * g.OH * g.OW, ctx->sm_count);
         prep.tap_major = qconv_tap_major(g);
         const WBlockArgs wb = weight_blocks_of(prep, g.M, g.Cg, g.KH * g.KW, x_zp);
         Stager s(ctx);
@@ -983,7 +983,7 @@ int32_t zant_b200_qlinearmatmul(zant_ctx* ctx, int32_t a_dtype, const void* a, c
         g.sh = g.sw = g.dh = g.dw = 1; g.OH = g.OW = 1; g.G = 1;
         if (y_dtype != ZANT_I32 && qconv_tc_eligible(g, bz_zero)) {
             QGemmPrep prep;
-            qgemm_sizes((int)N, (int)K, mult.data(), prep, (long long)M);
+            qgemm_sizes((int)N, (int)K, mult.data(), prep, (long long)M, ctx->sm_count);
             WBlockArgs wb = weight_blocks_of(prep, (int)N, (int)K, 1, a_zp);
             wb.sm = 1; wb.sc = N;                                       // [K][N]
             Stager s(ctx);

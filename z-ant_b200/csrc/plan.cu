@@ -790,7 +790,7 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
     if (qconv_tc_eligible(g, wz_zero) && const_bias) {
         // tensor-core path: weights re-blocked once here, im2col + tcgen05 GEMM per run
         auto prep = std::make_shared<QGemmPrep>();
-        qconv_gemm_prepare(g, (const int8_t*)T(w).host.data(), mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep);
+        qconv_gemm_prepare(g, (const int8_t*)T(w).host.data(), mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep, ctx->sm_count);
         const int aw = pl->add_aux(prep->w_blk.data(), prep->w_blk.size()), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4);
         const int ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
         const int sa = pl->shared_im2col_scratch(qgemm_a_bytes((size_t)g.N * g.OH * g.OW, *prep));
@@ -1198,7 +1198,7 @@ static int32_t build_node_impl(zant_plan* pl, size_t node_index, int32_t /*fuse*
                     const int8_t* bw = (const int8_t*)T(w).host.data();
                     for (size_t k = 0; k < K; ++k) for (size_t j = 0; j < N; ++j) bt[j * K + k] = bw[k * N + j];
                     auto prep = std::make_shared<QGemmPrep>();
-                    qgemm_prepare(bt.data(), (int)N, (int)K, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep, (long long)M);
+                    qgemm_prepare(bt.data(), (int)N, (int)K, mult.data(), b >= 0 ? (const int32_t*)T(b).host.data() : nullptr, xzp, *prep, (long long)M, ctx->sm_count);
                     const int aw = pl->add_aux(prep->w_blk.data(), prep->w_blk.size()), am = pl->add_aux(prep->mult.data(), prep->mult.size() * 4);
                     const int ab = pl->add_aux(prep->bias.data(), prep->bias.size() * 4);
                     const int sa = pl->shared_im2col_scratch(qgemm_a_bytes(M, *prep));

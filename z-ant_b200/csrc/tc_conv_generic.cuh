@@ -193,18 +193,18 @@ struct QGemmPrep {
 };
 
 // w: [n_out][K] int8 row-major (a convolution's [M][C][KH][KW] weight is exactly that).
-// `rows` (when known) lets wide outputs pick the tile width that wastes the least of the last wave of
-// 148 persistent CTAs: 256-wide tiles halve the number of tiles but a partly filled wave costs a full one.
-inline void qgemm_sizes(int n_out, int K, const float* mult, QGemmPrep& p, long long rows = 0) {
+// The tile width of wide outputs is the one that wastes the least of the last wave of persistent CTAs, one an SM: 256-wide tiles halve the
+// number of tiles but a partly filled wave costs a full one.
+inline void qgemm_sizes(int n_out, int K, const float* mult, QGemmPrep& p, long long rows, int sm_count) {
     p.NT = n_out <= 64 ? 64 : (n_out <= 128 ? 128 : 256);
     if (p.NT == 256 && rows > 0) {
         const long long mt = (rows + 127) / 128;
         const long long t256 = mt * ((n_out + 255) / 256), t128 = mt * ((n_out + 127) / 128);
-        const long long c256 = (t256 + 147) / 148 * 256, c128 = (t128 + 147) / 148 * 128;
+        const long long c256 = (t256 + sm_count - 1) / sm_count * 256, c128 = (t128 + sm_count - 1) / sm_count * 128;
         if (c128 < c256) p.NT = 128;
     }
     // few rows: narrower tiles while the grid still fits the SMs (1024 x 1280 times 1000 columns: 32 CTAs of 256, 128 of 64)
-    while (p.NT > 64 && rows > 0 && (rows + 127) / 128 * ((n_out + p.NT / 2 - 1) / (p.NT / 2)) <= 148) p.NT /= 2;
+    while (p.NT > 64 && rows > 0 && (rows + 127) / 128 * ((n_out + p.NT / 2 - 1) / (p.NT / 2)) <= sm_count) p.NT /= 2;
     p.N_pad = (n_out + p.NT - 1) / p.NT * p.NT;
     p.K = K;
     p.K16 = K <= 32 ? 2 : (K + 63) / 64 * 4;      // a stage holds 4 chunks of K (2 when K fits 32: first layers with 3 channels)
@@ -215,8 +215,8 @@ inline void qgemm_sizes(int n_out, int K, const float* mult, QGemmPrep& p, long 
     }
 }
 
-inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p, long long rows = 0) {
-    qgemm_sizes(n_out, K, mult, p, rows);
+inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p, long long rows, int sm_count) {
+    qgemm_sizes(n_out, K, mult, p, rows, sm_count);
     p.w_blk.assign((size_t)p.N_pad * p.K16 * 16, 0);
     p.bias.assign(p.N_pad, 0);
     for (int n = 0; n < n_out; ++n) {
@@ -236,15 +236,15 @@ inline void qgemm_prepare(const int8_t* w, int n_out, int K, const float* mult, 
 // tensor's own order.
 inline bool qconv_tap_major(const ConvGeom& g) { return g.KH * g.KW > 1 && g.Cg % 16 == 0; }
 
-inline void qconv_gemm_prepare(const ConvGeom& g, const int8_t* w, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p) {
+inline void qconv_gemm_prepare(const ConvGeom& g, const int8_t* w, const float* mult, const int32_t* bias, int x_zp, QGemmPrep& p, int sm_count) {
     const int taps = g.KH * g.KW, C = g.Cg, K = C * taps;
     const long long rows = (long long)g.N * g.OH * g.OW;
-    if (!qconv_tap_major(g)) { qgemm_prepare(w, g.M, K, mult, bias, x_zp, p, rows); return; }
+    if (!qconv_tap_major(g)) { qgemm_prepare(w, g.M, K, mult, bias, x_zp, p, rows, sm_count); return; }
     std::vector<int8_t> wt((size_t)g.M * K);
     for (int m = 0; m < g.M; ++m)
         for (int c = 0; c < C; ++c)
             for (int t = 0; t < taps; ++t) wt[(size_t)m * K + (size_t)t * C + c] = w[((size_t)m * C + c) * taps + t];
-    qgemm_prepare(wt.data(), g.M, K, mult, bias, x_zp, p, rows);
+    qgemm_prepare(wt.data(), g.M, K, mult, bias, x_zp, p, rows, sm_count);
     p.tap_major = true;
 }
 
