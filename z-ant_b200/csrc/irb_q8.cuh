@@ -74,8 +74,6 @@ struct IrbArgs {
     int* status;
 };
 
-// fewer tiles: the separate kernels use more of the chip (one image of 224 x 224: 250 us with them, 288 with this)
-constexpr int kIrbMinTiles = 8;
 constexpr int kIrbThreads = 640, kIrbEpiWarps = 16;
 
 // N accumulators of consecutive columns, N at most 9.
@@ -645,10 +643,12 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
     const int d2_cols = (a.paired ? 1 : a.mt2 * (two ? 2 : 1)) * a.n2;
     if ((two ? 2 : 1) * a.n1 + d2_cols > 512 || a.n1 > 128) return false;
     a.d1_bufs = !two && 2 * a.n1 + d2_cols <= 512 ? 2 : 1;
-    // as many CTAs a tile as the SMs hold, none with less than a chunk, where that saves a CTA four chunks: adding up costs as much as three or
-    // four (37 images: 960 channels at 5 x 5 24 -> 18 us in eight chunks, 384 and 576 at 10 x 10 16 -> 18 and 22 -> 23 in three and five)
+    // As many CTAs a tile as the SMs hold, none with less than a chunk, where that saves a CTA four chunks and while adding up and reading back,
+    // which grow with the filter tiles and with the CTAs that add at once, take less than the chunks saved (160 channels at 7 x 7, eight chunks,
+    // in one CTA a tile against several: 8 tiles 56 -> 42 us, 20 52, 40 54, 74 62; 320 filters: 8 tiles 56 -> 46, 16 56, 24 66, 74 99; at 5 x 5 and
+    // 160 filters 48 -> 35, 43, 45, 53.  384 and 576 channels at 10 x 10 in three and five: 16 -> 18 and 22 -> 23.)
     a.splits = two ? 1 : std::max(1, std::min(a.chunks, sm_count / a.tiles));
-    if (a.chunks - (a.chunks + a.splits - 1) / a.splits < 4) a.splits = 1;
+    if (a.chunks - (a.chunks + a.splits - 1) / a.splits < 4 || a.tiles * a.mt2 * a.mt2 > 160) a.splits = 1;
     q.sums_bytes = a.splits > 1 ? (size_t)a.tiles * d2_cols * 512 : 0;
     a.w2_bytes = a.paired ? 8 * 192 * 16 : a.mt2 * 16384;
     a.w_bytes = a.kp * 128 + a.w2_bytes + 128 * (int)sizeof(IrbConst);
@@ -665,6 +665,28 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
         if (q.smem_bytes <= 227 * 1024) return true;
     }
     return false;
+}
+
+// Whether the block is faster as one kernel than as three, or four with the addition.  One kernel takes rounds of the SMs whose time is a
+// tile's; the separate ones, a launch each more and the expanded tensor through memory, take a time that grows with the images.  Measured inside
+// plans, 28 shapes of 3 to 14 rows, 16 to 160 channels, 1 to 1500 images, us as one kernel / separate, with 14 us of other steps:
+//   two units, stride 1: a tile costs about 2 + 5 us a chunk, at least 13.5, at 14 rows; the separate kernels 16 + 2.25 us per million expanded
+//     values.  96 -> 576 at 14 x 14: 8 images 43 / 34, 48 44 / 42, 64 44 / 48, 148 47 / 66, 1024 245 / 330; 64 -> 384: 8 images 32 / 31, 12 31 / 32,
+//     148 34 / 53; 16 -> 128: 148 images 27 / 37, 768 119 / 86; 32 -> 192 at 12 x 12: 148 images 29 / 41, 768 106 / 89.
+//   two units, stride 2: always (8 images 30 / 33, 1024 132 / 197)
+//   one unit, chunks on one CTA: from about three tiles a chunk on (160 -> 960 -> 320 at 7 x 7: 16 tiles 56 / 48, 24 56 / 58, 74 56 / 79; 64 -> 384
+//     at 4 x 4: 8 tiles 21 / 26), and planes of less than 16 pixels, a quarter of whose columns exist, while there are few rounds of few chunks
+//     (160 -> 960 at 3 x 3: 592 images 63 / 77, 1024 109 / 96; 64 -> 384: 1024 60 / 66, 1500 81 / 75)
+// Below eight tiles the separate kernels use more of the chip (160 -> 960 at 4 x 4: 6 tiles 24 / 22).
+inline bool irb_pays(const IrbPlan& q, int sm_count) {
+    const IrbArgs& a = q.a;
+    if (a.tiles < 8) return false;
+    const long long rounds = ((long long)a.tiles * a.splits + sm_count - 1) / sm_count;
+    if (a.IB == 1) {
+        if (q.stride == 2) return true;
+        return rounds * std::max(13.5, 2.0 + 5.0 * a.chunks) * a.H / 14 <= 16.0 + 2.25e-6 * a.N * q.E * a.H * a.W;
+    }
+    return (a.splits > 1 || a.tiles + 1 >= 3 * a.chunks) && (a.H * a.W >= 16 || rounds * a.chunks <= 16);
 }
 
 // Weights and constants per chunk; false when an accumulator could leave the range of kAccBase.  eb, db: biases with -x_zp * sum(w) folded in.

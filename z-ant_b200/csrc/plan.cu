@@ -1419,7 +1419,7 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
         }
     }
     IrbPlan q;
-    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || q.a.tiles < kIrbMinTiles) { consumed = 0; return ZANT_OK; }
+    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || !irb_pays(q, pl->ctx->sm_count)) { consumed = 0; return ZANT_OK; }
     std::vector<uint8_t> stages;
     if (!irb_prepare(q, (const int8_t*)T(e->in[1]).host.data(), mult[0].data(), bias[0].data(), (const int8_t*)T(d->in[1]).host.data(), mult[1].data(), bias[1].data(),
                      (const int8_t*)T(p->in[1]).host.data(), stages)) { consumed = 0; return ZANT_OK; }
