@@ -73,3 +73,10 @@ def test_blocks_of_images(zb, ctx, oracle, models, scales, batch):
 def test_several_single_windows_a_cta(zb, ctx, oracle, models, scales, batch):
     g = models.small_cnn_int8(batch, act_scales=scales, bias_amplitude=(100, 1000, 5000, 300))
     _run(zb, ctx, oracle, g, models.small_cnn_input(batch, batch))
+
+
+@pytest.mark.parametrize("batch", [384, 390, 512, 513])
+def test_column_tiles_of_fc1(zb, ctx, oracle, models, scales, batch):
+    """Around four blocks of 128 images, where fc1's column tiles are wider than the grid alone asks for."""
+    g = models.small_cnn_int8(batch, act_scales=scales, bias_amplitude=(100, 1000, 5000, 300))
+    _run(zb, ctx, oracle, g, models.small_cnn_input(batch, batch))

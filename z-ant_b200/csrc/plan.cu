@@ -1725,10 +1725,20 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     // ---- fc1: rows re-ordered from the graph's (c,h,w) flatten order to the (h,w,c) order stage 2 writes
     std::vector<float> m3; std::vector<int32_t> b3;
     if (!scales_of(f1, 512, m3) || !bias_of(f1, 512, b3)) return ZANT_OK;
-    // the narrowest column tile whose grid fits the SMs: a CTA streams all of K for its columns (batch 1: 12.6 us with two CTAs of 256)
+    // images per block of stages 1 and 2, blocks; windows per item of stage 2.  Five windows of a row share their column pairs; single windows
+    // fill the SMs better while there are few of them.  A single window is counted as 1.2 of a shared one.  (Whole network, fives -> singles: 512
+    // images 24.7 -> 20.3 us, 1024 28.4 -> 22.4, 2048 32.7 -> 27.4.)
+    const int ib = (int)std::min<size_t>(B, 128), blocks128 = (int)((B + 127) / 128);
+    const long long sms = pl->ctx->sm_count, singles = (blocks128 * 25 + sms - 1) / sms * 6, fives = (blocks128 * 5 + sms - 1) / sms * 25;
+    const int c2_wins = singles <= fives ? 1 : 5, c2_items = blocks128 * 25 / c2_wins;
+    // The narrowest column tile whose grid fits the SMs: a CTA streams all of K for its columns (batch 1: 12.6 us with two CTAs of 256).  Its CTAs
+    // start on the SMs that stage 2 leaves free, two to an SM; where that takes all of them in, but not one to an SM, those that share one
+    // finish last and a wider tile is faster (385 to 512 images, 64 CTAs for 48 SMs: 23.3 us, 20.3 with 32 CTAs).
     constexpr int FC_KC = 4, FC_STAGES = 8;
-    int FC_NT = 256;
-    while (FC_NT > 32 && (int)((B + 127) / 128) * (512 / (FC_NT / 2)) <= pl->ctx->sm_count) FC_NT /= 2;
+    int FC_NT = 32;
+    const int free_sms = std::max(0, (int)sms - c2_items);
+    auto fc_ctas = [&](int nt) { return blocks128 * (512 / nt); };
+    while (FC_NT < 256 && (fc_ctas(FC_NT) > sms || (fc_ctas(FC_NT) > free_sms && fc_ctas(FC_NT) <= 2 * free_sms))) FC_NT *= 2;
     std::vector<int8_t> w3blk(1600 * 512);      // [512/NT][100 chunks][NT][16], K in (h,w,c) order
     {
         const int8_t* w = (const int8_t*)T(f1.in[1]).host.data();   // [1600][512], row = c*25 + h*5 + w
@@ -1758,7 +1768,6 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     }
 
     // stage 1 -> stage 2 hand-over: image blocks
-    const int ib = (int)std::min<size_t>(B, 128), blocks128 = (int)((B + 127) / 128);
     const int s_pool1 = pl->add_scratch(blocks128 * (size_t)c2_block_bytes(ib));
     const int s_pool2 = pl->add_scratch((size_t)blocks128 * ib * 1600);
     const int s_fc1 = pl->add_scratch(B * 512);
@@ -1816,12 +1825,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         k.x = (const int8_t*)pl->scratch(s_pool1); k.w = (const int8_t*)pl->aux(a_w2);
         for (int m = 0; m < 64; ++m) { k.mult[m] = m2[m]; k.bias[m] = acc_base2 ? kAccBase - (float)b2[m] : int_bits_as_float(b2[m]); }
         k.y = (int8_t*)pl->scratch(s_pool2); k.n_images = (int)B; k.ib = ib; k.status = ctx->status_word;
-        // Five windows of a row share their column pairs; single windows fill the SMs better while there are few of them.  A single window is
-        // counted as 1.2 of a shared one.  (Stage alone, fives -> singles: 1024 images 14.2 -> 12.4 us, 2048
-        // 14.6 -> 14.1, 4096 18.9 -> 16.7; whole network 27.5 -> 21.9, 31.8 -> 26.7, 41.0 -> 36.1.)
-        const long long sms = ctx->sm_count, singles = (blocks128 * 25 + sms - 1) / sms * 6, fives = (blocks128 * 5 + sms - 1) / sms * 25;
-        k.wins = singles <= fives ? 1 : 5;
-        k.items = blocks128 * 25 / k.wins;
+        k.wins = c2_wins; k.items = c2_items;
         const int blocks = std::min<int>(k.items, ctx->sm_count);
         auto with = [&](auto base) -> int32_t {
             ZB_SMEM_ATTR(ctx, (tc_conv3x3_pool_kernel<decltype(base)::value>), Cfg::SMEM_BYTES);
