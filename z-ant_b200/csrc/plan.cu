@@ -1743,8 +1743,13 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     {
         const int8_t* w = (const int8_t*)T(f1.in[1]).host.data();   // [1600][512], row = c*25 + h*5 + w
         std::vector<int> colsum(512, 0);
-        for (int k = 0; k < 1600; ++k)
-            for (int n = 0; n < 512; ++n) colsum[n] += w[(size_t)k * 512 + n];
+        // (16-bit sums of 200 rows, at most 25600: the host adds twice as many at a time)
+        for (int k0 = 0; k0 < 1600; k0 += 200) {
+            int16_t part[512] = {};
+            for (int k = k0; k < k0 + 200; ++k)
+                for (int n = 0; n < 512; ++n) part[n] = (int16_t)(part[n] + w[(size_t)k * 512 + n]);
+            for (int n = 0; n < 512; ++n) colsum[n] += part[n];
+        }
         // 16 channels of a position are a K chunk: 16 rows of the matrix, transposed
         for (int hw = 0; hw < 25; ++hw)
             for (int c16 = 0; c16 < 4; ++c16) {
