@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 CONV = dict(dilations=(1, 1), auto_pad="NOTSET")
 
-# N C E M H W, input zero point, biases, residual addition: 0 none, 1 input first, 2 input second; stride
+# N C E M H W, input zero point, biases, residual addition: 0 none, 1 input first, 2 input second; stride; activation of the addition
 CASES = [
     (9, 64, 384, 64, 14, 14, 0, True, 1, 1),        # whole chunks, one image a tile, both halves in one accumulator
     (160, 96, 576, 96, 14, 14, 0, False, 2, 1),     # half a chunk at the end, CTAs with two tiles
@@ -33,12 +33,15 @@ CASES = [
     (11, 40, 130, 16, 4, 14, -4, True, 0, 2),
     (31, 48, 700, 48, 5, 5, 0, True, 1, 1),         # six chunks on six CTAs a tile, 60 channels in the last, an odd image
     (90, 64, 1100, 64, 4, 6, 0, True, 2, 1),        # nine chunks on three CTAs
+    (160, 64, 384, 64, 14, 14, 0, True, 1, 1, "relu"),
+    (31, 48, 700, 48, 5, 5, 0, True, 2, 1, "relu6"),
 ]
 
 
 def block(zb, case):
     """Graph up to the block's result `cur`, and the tensors t1, t2 between the convolutions."""
-    N, C, E, M, H, W, xzp, bias, res, stride = case
+    N, C, E, M, H, W, xzp, bias, res, stride = case[:10]
+    act = case[10] if len(case) > 10 else None
     OH, OW = (H + stride - 1) // stride, (W + stride - 1) // stride
     rng = np.random.default_rng(C + E + H * 16 + W)
     g = zb.Graph("irb")
@@ -61,9 +64,9 @@ def block(zb, case):
     if res:
         y = g.tensor("sum", zb.I8, (N, M, H, W))
         if res == 1:
-            g.node("QLinearAdd", [x, cur], [y], x_scale=0.1, x_zp=xzp, b_scale=0.12, b_zp=0, y_scale=0.2, y_zp=2)
+            g.node("QLinearAdd", [x, cur], [y], x_scale=0.1, x_zp=xzp, b_scale=0.12, b_zp=0, y_scale=0.2, y_zp=2, activation=act)
         else:
-            g.node("QLinearAdd", [cur, x], [y], x_scale=0.12, x_zp=0, b_scale=0.1, b_zp=xzp, y_scale=0.2, y_zp=0)
+            g.node("QLinearAdd", [cur, x], [y], x_scale=0.12, x_zp=0, b_scale=0.1, b_zp=xzp, y_scale=0.2, y_zp=0, activation=act)
         cur = y
     g.input = x0
     return g, t1, t2, cur, rng.integers(-128, 128, (N, 4, H, W)).astype(np.int8)

@@ -239,3 +239,114 @@ def test_row_copy_counter_stays_in_its_type():
             assert last < 1 << 32 and last >= chunks
             for i in (chunks - 1, chunks - 129, 127):
                 assert 0 <= (i >> 7) < 1 << 24 and (i >> 7) * 128 + (i & 127) == i
+
+
+def irb_plan(N, C, E, M, H, W, stride, add):
+    """irb_plan of irb_q8.cuh: a block's tiles, accumulator columns and shared memory; None where the kernel does not take it."""
+    two = W > 8
+    if H > (14 if two else 8) or W > 16 or H < 2 or W < 3 or C > 512 or M > 512 or not 128 <= E <= 4096:
+        return None
+    if stride == 2 and (not two or add or H % 2 or W % 2 or H < 4 or W > 14):
+        return None
+    OH, OW = (H + stride - 1) // stride, (W + stride - 1) // stride
+    if N * C * H * W % 4 or M * OH * OW % 16:
+        return None
+    p = dict(N=N, C=C, E=E, M=M, H=H, W=W, OH=OH, OW=OW, S=stride, U=2 if two else 1, IB=1 if two else 2, pitch=16 if two else 8)
+    p["opitch"] = p["pitch"] if stride == 1 else 8
+    p["rh"] = rh = (OH + 1) // 2
+    if two:
+        p["n1"] = 16 * (rh + 1 if stride == 1 else max(2 * rh, H - 2 * rh + 1))
+        p["n2"] = 16 * rh if stride == 1 else (8 * rh + 15) // 16 * 16
+    else:
+        p["n1"] = p["n2"] = 16 * H
+    p["kp"], p["mt2"] = (C + 31) // 32 * 32, (M + 127) // 128
+    p["paired"] = two and M <= 64
+    d2_cols = (1 if p["paired"] else p["mt2"] * p["U"]) * p["n2"]
+    if p["U"] * p["n1"] + d2_cols > 512 or p["n1"] > 128:
+        return None
+    p["slots"] = 2 if two or 2 * p["n1"] + d2_cols <= 512 else 1
+    p["tmem"] = p["slots"] * p["n1"] + d2_cols
+    w_bytes = p["kp"] * 128 + (8 * 192 * 16 if p["paired"] else p["mt2"] * 16384) + 128 * 32
+    x_bytes, y_bytes, out_bytes = p["U"] * p["kp"] * 128, p["U"] * 16384, (p["IB"] * M * OH * OW + 127) // 128 * 128
+    for n in range(2 if add else 4):
+        off_x = (2 * w_bytes + 1023) // 1024 * 1024
+        off_y = off_x + (2 if n < 2 else 1) * x_bytes
+        off_out = off_y + (2 if n % 2 == 0 else 1) * y_bytes
+        if off_out + out_bytes + 512 <= 227 * 1024:
+            p.update(off_x=off_x, off_y=off_y, off_out=off_out, out_bytes=out_bytes)
+            return p
+    return None
+
+
+IRB_GRID = [(N, C, E, M, H, W, s, add) for N in (8, 33) for C, E, M in ((32, 192, 32), (40, 200, 48), (64, 384, 96), (160, 960, 160), (24, 144, 320))
+            for H, W in itertools.product((2, 3, 5, 7, 8, 10, 11, 14), (3, 4, 5, 7, 8, 9, 10, 12, 13, 14, 16)) for s in (1, 2) for add in (False, True)
+            if not add or C == M]
+
+
+def test_inverted_residual_offsets():
+    checked = 0
+    for case in IRB_GRID:
+        p = irb_plan(*case)
+        if p is None:
+            continue
+        checked += 1
+        N, C, M, H, W, OH, OW, S, U, IB = (p[k] for k in ("N", "C", "M", "H", "W", "OH", "OW", "S", "U", "IB"))
+        n1, n2, rh, pitch, opitch = p["n1"], p["n2"], p["rh"], p["pitch"], p["opitch"]
+        assert p["tmem"] <= 512 and n1 % 16 == 0 and n2 % 16 == 0 and n2 <= 128 and p["off_x"] % 1024 == 0 and p["off_y"] % 1024 == 0 and p["off_out"] % 128 == 0, case
+        words, row_words = N * C * H * W // 4, pitch // 4
+        in1 = rh - 1 if S == 1 else 2 * rh - 1                          # first input row of the second unit
+        # the builder: chunk positions of a unit, and the aligned words that a row is cut out of
+        where = {}
+        for t in (0, (N + IB - 1) // IB - 1):
+            for u in range(U):
+                for q in range(n1 // 16):
+                    for h in range(16 // pitch):
+                        rr = q * (16 // pitch) + h
+                        img, r = (0, rr + (in1 if u else 0)) if U == 2 else (rr // H if rr >= H else 0, rr - H if rr >= H else rr)
+                        n = t * IB + img
+                        if n >= N or r >= H or img >= IB:
+                            continue
+                        where[(t, u, img, r)] = q * 16 + h * 8 if U == 1 else q * 16
+                        for c in (0, C - 1):
+                            first = (n * C * H + r) * W + c * H * W
+                            for x in range(W):
+                                w = (first + x) // 4 - first // 4
+                                assert w <= row_words and (first + x) // 4 < words, case
+        # the rows that the filter reads, and the accumulator columns of their loads
+        for u in range(U):
+            for img in range(IB):
+                for sub in range(2):
+                    u0, u1 = (rh if u else 0), (rh if U == 2 and u == 0 else OH)
+                    hr = (OH + 1) // 2
+                    r0, r1 = (u0, u1) if U == 2 else ((hr, OH) if sub else (0, hr))
+                    if r0 >= r1:
+                        continue
+                    lo, hi = max(S * r0 - 1, 0), (min(r1, H - 1) if S == 1 else 2 * r1 - 1)
+                    assert hi < H, case
+                    col = 0 if U == 2 else (img * H + lo) * pitch
+                    for i, r in enumerate(range(lo, hi + 1)):
+                        c = col + i * pitch
+                        assert where.get((0, u, img if U == 1 else 0, r)) == c, (case, u, img, sub, r)
+                        assert c + (7 if U == 2 and sub else 0) + (9 if S == 1 and U == 2 else 8) <= n1, (case, u, r)
+                    for r in range(r0, r1):                            # the filtered row's place in the second operand
+                        rr = r - u0 if U == 2 else img * OH + r
+                        assert rr * opitch + opitch <= n2 + (8 if opitch == 8 else 0) and rr * opitch < 128, case
+        # the project epilogue: every byte of a tile's output exactly once
+        out = np.zeros(IB * M * OH * OW, np.int32)
+        for quarter, part in itertools.product(range(4), range(4)):
+            pu = quarter >> 1 if p["paired"] else part & 1
+            pu0, pu1 = (rh if U == 2 and pu else 0), (rh if U == 2 and pu == 0 else OH)
+            pc0 = (part >> 1) * 8 if opitch == 16 else 0
+            pcols = min(8, OW - pc0)
+            step = (2 if p["paired"] else 1) if opitch == 16 else (4 if p["paired"] else 2)
+            p0 = pu0 + ((part & 1 if p["paired"] else 0) if opitch == 16 else (part if p["paired"] else part >> 1))
+            for mt in range(p["mt2"]):
+                first = mt * 128 + ((quarter & 1) * 32 if p["paired"] else quarter * 32)
+                for r in range(p0, pu1, step):
+                    d2 = (r - pu0 if U == 2 else pu * OH + r) * opitch + pc0
+                    assert d2 + 8 <= n2, (case, r)
+                    for m in range(first, min(first + 32, M)):
+                        o = ((0 if U == 2 else pu) * M + m) * OH * OW + r * OW + pc0
+                        out[o:o + pcols] += 1
+        assert (out == 1).all(), case
+    assert checked > 300

@@ -668,25 +668,34 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
 }
 
 // Whether the block is faster as one kernel than as three, or four with the addition.  One kernel takes rounds of the SMs whose time is a
-// tile's; the separate ones, a launch each more and the expanded tensor through memory, take a time that grows with the images.  Measured inside
-// plans, 28 shapes of 3 to 14 rows, 16 to 160 channels, 1 to 1500 images, us as one kernel / separate, with 14 us of other steps:
-//   two units, stride 1: a tile costs about 2 + 5 us a chunk, at least 13.5, at 14 rows; the separate kernels 16 + 2.25 us per million expanded
-//     values.  96 -> 576 at 14 x 14: 8 images 43 / 34, 48 44 / 42, 64 44 / 48, 148 47 / 66, 1024 245 / 330; 64 -> 384: 8 images 32 / 31, 12 31 / 32,
-//     148 34 / 53; 16 -> 128: 148 images 27 / 37, 768 119 / 86; 32 -> 192 at 12 x 12: 148 images 29 / 41, 768 106 / 89.
-//   two units, stride 2: always (8 images 30 / 33, 1024 132 / 197)
-//   one unit, chunks on one CTA: from about three tiles a chunk on (160 -> 960 -> 320 at 7 x 7: 16 tiles 56 / 48, 24 56 / 58, 74 56 / 79; 64 -> 384
-//     at 4 x 4: 8 tiles 21 / 26), and planes of less than 16 pixels, a quarter of whose columns exist, while there are few rounds of few chunks
-//     (160 -> 960 at 3 x 3: 592 images 63 / 77, 1024 109 / 96; 64 -> 384: 1024 60 / 66, 1500 81 / 75)
-// Below eight tiles the separate kernels use more of the chip (160 -> 960 at 4 x 4: 6 tiles 24 / 22).
-inline bool irb_pays(const IrbPlan& q, int sm_count) {
+// tile's; the separate ones, a launch each more and the expanded tensor through memory, take a time that grows with the images.  `long_add`: an
+// addition whose short form is not proved (15 instructions a value instead of 6.5), which costs the one kernel more.  Measured inside plans, 43 shapes
+// of 3 to 14 rows, 16 to 160 channels, 1 to 1500 images; below, us as one kernel / separate, with 14 us of other steps:
+//   two units, stride 1, planes of whole words: a tile takes about 6.6 us a chunk less 1.3, at 14 rows, the separate kernels 17.5, or 21.5 where rows
+//     are not whole words too, and 3.2 per million expanded values (96 -> 576 at 14 x 14: 8 images 36 / 33, 32 36 / 38, 148 39 / 61, 1024 192 / 282; at
+//     12 x 12: 24 images 35 / 30, 64 35 / 36, 148 37 / 50; at 10 x 10: 16 images 30 / 32; 32 -> 192 at 12 x 12: 148 images 26 / 36, 768 86 / 84, 1500
+//     150 / 144); with the long addition 2 + 5 us a chunk, at least 13.5, against 16 and 2.25 (96 -> 576 at 14 x 14: 8 images 43 / 34, 48 44 / 42, 148
+//     47 / 66; 16 -> 128: 148 images 27 / 37, 768 119 / 86)
+//   two units, stride 2 or planes that are not whole words, which the separate kernels put through an im2col pass: always (stride 2, 8 images 30 /
+//     33, 1024 132 / 197; 96 -> 576 at 11 x 11: 8 images 45 / 51, 160 84 / 104, 1500 368 / 557; 32 -> 192 at 13 x 13: 34 / 45, 48 / 80, 247 / 357)
+//   one unit, chunks on one CTA: from about three tiles a chunk on (160 -> 960 -> 320 at 7 x 7: 16 tiles 56 / 48, 24 51 / 54, 74 55 / 79; 64 -> 384 at
+//     4 x 4: 8 tiles 21 / 26); dealt to several, three filter tiles, seven rows or more: up to 12 tiles (the same block: 8 tiles 46 / 46, 16 54 / 47;
+//     at 5 x 5 16 tiles 42 / 45)
+//   planes of less than 16 pixels, a quarter of whose columns exist: while there are few rounds of few chunks (160 -> 960 at 3 x 3: 768 images 77 / 85,
+//     1024 95 / 93, 1500 127 / 115; with the long addition 768 90 / 91, 1024 109 / 96)
+// Below eight tiles the separate kernels use more of the chip (160 -> 960 at 4 x 4: 4 tiles 19 / 19, 64 -> 384 at 6 x 6: 2 tiles 20 / 19).
+inline bool irb_pays(const IrbPlan& q, bool long_add, int sm_count) {
     const IrbArgs& a = q.a;
     if (a.tiles < 8) return false;
     const long long rounds = ((long long)a.tiles * a.splits + sm_count - 1) / sm_count;
     if (a.IB == 1) {
-        if (q.stride == 2) return true;
-        return rounds * std::max(13.5, 2.0 + 5.0 * a.chunks) * a.H / 14 <= 16.0 + 2.25e-6 * a.N * q.E * a.H * a.W;
+        if (q.stride == 2 || a.H * a.W % 4 != 0) return true;
+        const double values = 1e-6 * a.N * q.E * a.H * a.W;
+        const double tile = long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : std::max(8.0, 6.6 * a.chunks - 1.3);
+        return rounds * tile * a.H / 14 <= (long_add ? 16.0 + 2.25 * values : (a.W % 4 != 0 ? 21.5 : 17.5) + 3.2 * values);
     }
-    return (a.splits > 1 || a.tiles + 1 >= 3 * a.chunks) && (a.H * a.W >= 16 || rounds * a.chunks <= 16);
+    if (a.splits > 1 ? a.mt2 >= 3 && a.H >= 7 && a.tiles > 12 : a.tiles + 1 < 3 * a.chunks) return false;
+    return a.H * a.W >= 16 || rounds * a.chunks <= (long_add ? 16 : 30);
 }
 
 // Weights and constants per chunk; false when an accumulator could leave the range of kAccBase.  eb, db: biases with -x_zp * sum(w) folded in.

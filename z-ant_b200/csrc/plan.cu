@@ -1419,7 +1419,7 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
         }
     }
     IrbPlan q;
-    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || !irb_pays(q, pl->ctx->sm_count)) { consumed = 0; return ZANT_OK; }
+    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || !irb_pays(q, with_add && !add.proved, pl->ctx->sm_count)) { consumed = 0; return ZANT_OK; }
     std::vector<uint8_t> stages;
     if (!irb_prepare(q, (const int8_t*)T(e->in[1]).host.data(), mult[0].data(), bias[0].data(), (const int8_t*)T(d->in[1]).host.data(), mult[1].data(), bias[1].data(),
                      (const int8_t*)T(p->in[1]).host.data(), stages)) { consumed = 0; return ZANT_OK; }
@@ -1666,7 +1666,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         for (size_t k = 1; k < q->in.size(); ++k)
             if (q->in[k] >= 0 && !T(q->in[k]).is_const) return ZANT_OK;
 
-    if (NCLS > 16 || B > (1u << 20)) return ZANT_OK;         // two column blocks of classes; 32-bit plane offsets in stage 1
+    if (NCLS > 16 || B > (1u << 20)) return ZANT_OK;         // two column blocks of classes; counts of images, tiles and windows far inside 32 bits
     if (probe) { consumed = 12; return ZANT_OK; }
     zant_ctx* ctx = pl->ctx;
     auto push = [&](const char* name, std::function<int32_t()> fn) { pl->steps.push_back(std::move(fn)); pl->step_names.push_back(name); };

@@ -15,6 +15,9 @@
 //   NH_POOL_VIEWS (up to 32 filters)  one MMA of 4 NT columns per view, 16 in all, zero weights where a member has no such tap
 //   NH_POOL_PAIRS (64-filter tiles)   per filter row and member row: the two middle views with both members' filters (2 NT columns),
 //                                     the outer ones with one member's - 24 MMAs, no zeros
+//                                     (MMAs of 2 NT and of NT columns write TMEM columns that overlap, in the order of issue; that order is
+//                                     documented for equal shapes only and otherwise what every run has shown, with the sums compared bit
+//                                     for bit in the channels-last tests.  One shape would need zeros, and zero times an infinite input is a NaN)
 //
 // Stride 2 reads the four parity planes as well, with one accumulator: tap (kh, kw) is plane ((kh - pt) & 1, (kw - pl) & 1) shifted by
 // ((kh - pt) >> 1, (kw - pl) >> 1).  (A 1x1 filter with stride 2 reads one plane, as an image of its own.)
