@@ -109,8 +109,8 @@ def measured_peaks():
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the four fused steps of the int8 CNN at batch 65536,
-# from the ncu captures summarised under profiles/ (index = fused step).
-NCU_DRAM_TRAFFIC_B65536 = [205.9e6 + 253.1e6, 302.1e6 + 80.6e6, 105.7e6 + 9.6e6, 33.6e6 + 0.0]
+# from the one-pass ncu capture in profiles/int8_cnn_b65536_launch_list.md (index = fused step).
+NCU_DRAM_TRAFFIC_B65536 = [205.6e6 + 254.5e6, 302.1e6 + 78.6e6, 105.7e6 + 5.8e6, 33.6e6 + 0.0]
 
 
 # ------------------------------------------------------------------------------------------------

@@ -676,7 +676,9 @@ int32_t zant_b200_plan_step_cost(zant_plan* plan, int32_t step, double* macs, do
 int32_t zant_b200_plan_profile(zant_plan* plan, int32_t enable);
 int32_t zant_b200_plan_profile_read(zant_plan* plan, float* sum_ms, int32_t* runs);
 /* Device pointer of a tensor's buffer (for tests that inspect intermediates).  A fused plan (`fuse` != 0) does not store every tensor:
- * for one interior to a fused step the result is NULL (here) or ZANT_E_UNSUPPORTED (zant_b200_plan_read_tensor).  Tensors that it keeps
+ * for one interior to a fused step the result is NULL (here) or ZANT_E_UNSUPPORTED (zant_b200_plan_read_tensor): between a convolution and
+ * the activation or pool behind it, inside the small CNN's stages, and the expanded tensors (with an addition also the projection's
+ * result) of an inverted residual block that runs as one step.  Tensors that it keeps
  * channels-last between convolutions get a buffer in the graph's order at the first call that asks for theirs; every later run brings
  * that buffer up to date.  In TF32 mode such a tensor holds what the convolutions behind it read: values rounded to TF32 (mode 1), or the
  * sum of two TF32 parts (mode 2).  `fuse` = 0 stores every tensor in full. */
