@@ -100,3 +100,35 @@ def test_operand_that_is_the_output(zb, ctx, oracle):
     assert not any("+QLinearAdd" in n for n in plan.step_names())
     assert np.array_equal(plan.run(xv), want[flat]) and np.array_equal(plan.read_tensor(y), want[y])
     plan.close()
+
+
+@pytest.mark.parametrize("N,M,H,W,fused", [(16, 24, 32, 32, True), (15, 24, 32, 32, False), (28, 64, 20, 12, True), (11, 96, 32, 32, True), (10, 96, 32, 32, False), (33, 132, 16, 16, True)])
+def test_short_form_in_the_epilogue(zb, ctx, oracle, N, M, H, W, fused):
+    """Scales for which the rounding needs no division (proved when the plan is built): on either side of the sizes from which the addition is
+    part of the convolution's step."""
+    rng = np.random.default_rng(N + M)
+    g = zb.Graph("res")
+    x = g.tensor("x", zb.I8, (N, 8, H, W))
+    sx, sr, sc, sy = 0.05, 0.0931, 0.1173, 0.2117
+
+    def conv(src, cin, s_in, name, s_out):
+        w = g.tensor(f"w{name}", zb.I8, (M, cin, 1, 1), rng.integers(-127, 128, (M, cin, 1, 1), dtype=np.int8))
+        ws = g.tensor(f"s{name}", zb.F32, (M,), (rng.uniform(0.7, 1.3, M) * 60.0 * s_out / (s_in * 40.0 * 73.0 * np.sqrt(cin))).astype(np.float32))
+        y = g.tensor(f"c{name}", zb.I8, (N, M, H, W))
+        g.node("QLinearConv", [src, w, ws, -1, -1], [y], x_scale=s_in, x_zp=0, y_scale=s_out, y_zp=0, pads=(0,) * 4, strides=(1, 1), group=1, **CONV)
+        return y
+
+    r = conv(x, 8, sx, "r", sr)
+    cur = conv(r, M, sr, "c", sc)
+    y = g.tensor("sum", zb.I8, (N, M, H, W))
+    g.node("QLinearAdd", [r, cur], [y], x_scale=sr, x_zp=0, b_scale=sc, b_zp=0, y_scale=sy, y_zp=0)
+    out = g.tensor("out", zb.F32, (N, M, H, W))
+    g.node("DequantizeLinear", [y], [out], x_scale=sy, x_zp=0)
+    g.input, g.output = x, out
+    xv = rng.integers(-128, 128, (N, 8, H, W)).astype(np.int8)
+    want = graph_oracle.run(oracle, g, xv)
+    plan = zb.Plan(ctx, g, fuse=True)
+    assert any("+QLinearAdd" in n for n in plan.step_names()) == fused, plan.step_names()
+    assert np.array_equal(plan.run(xv), want[g.output])
+    assert len(np.unique(want[y])) > 100
+    plan.close()

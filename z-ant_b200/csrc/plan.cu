@@ -696,9 +696,13 @@ static int32_t build_qconv(zant_plan* pl, const PlanNode& n, QConvFusion& fz) {
         std::vector<int32_t> caps;
         const bool capped = finite && yd == ZANT_I8 && rq0.y_zp == 0 && requant_relu_caps(mult.data(), mult.size(), rq0.act, lean_six(rq0.y_scale), caps);
         const int ac = capped ? pl->add_aux(caps.data(), caps.size() * 4) : -1;
-        // In the short form (proved) from 64 KB of output on, else from 8 MB (below, a CTA has a tile or two, whose epilogue the long form
-        // makes longer by more than the launch it saves: 37 images of 160 x 160 took 512 us with it, 484 without).
-        if (!stem && fz.add_node >= 0 && (long long)g.N * g.M * g.OH * g.OW >= (add0.proved ? 64LL << 10 : 8LL << 20) && xd == ZANT_I8 && yd == ZANT_I8 && rq0.y_zp == 0 && finite) {
+        // In the short form (proved) from 384 KB of output on with at most 64 filters, from 1 MB with more, where a CTA has enough pixels for the
+        // longer epilogue to cost less than a launch (us, in it / as a step of its own: 24 filters at 56 x 56 294 KB 22.1 / 21.9, 882 KB 23.5 / 24.3, 9.4 MB
+        // 59 / 59, 107 MB 491 / 497; 96 at 20 x 20 225 KB 23.2 / 20.4, 900 KB 25.8 / 25.3, 37 MB 240 / 249; 256 at 28 x 28 392 KB 23.1 / 20.5, 1.6 MB 23.5 /
+        // 23.0, 98 MB 251 / 264).  The long form from 8 MB (its 15 instructions a value cost more than the launch at every size: 24 filters at
+        // 56 x 56 9.4 MB 88 / 71, 107 MB 793 / 648; below 8 MB it is a step of its own).
+        const long long add_from = add0.proved ? (g.M <= 64 ? 384LL << 10 : 1LL << 20) : 8LL << 20;
+        if (!stem && fz.add_node >= 0 && (long long)g.N * g.M * g.OH * g.OW >= add_from && xd == ZANT_I8 && yd == ZANT_I8 && rq0.y_zp == 0 && finite) {
             fz.add_done = true;
             push("QLinearConv(tc-pointwise)" + tail + "+QLinearAdd", [=]() {
                 if (!pw_conv_ptr_ok(pl->ptr(x), pl->ptr(y_sum))) return fail(ZANT_E_INVALID_INPUT, "pointwise QLinearConv buffers must be 16-byte (input) and 32-byte (output) aligned");
