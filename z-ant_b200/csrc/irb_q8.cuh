@@ -644,11 +644,12 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
     if ((two ? 2 : 1) * a.n1 + d2_cols > 512 || a.n1 > 128) return false;
     a.d1_bufs = !two && 2 * a.n1 + d2_cols <= 512 ? 2 : 1;
     // As many CTAs a tile as the SMs hold, none with less than a chunk, where that saves a CTA four chunks and while adding up and reading back,
-    // which grow with the filter tiles and with the CTAs that add at once, take less than the chunks saved (160 channels at 7 x 7, eight chunks,
-    // in one CTA a tile against several: 8 tiles 56 -> 42 us, 20 52, 40 54, 74 62; 320 filters: 8 tiles 56 -> 46, 16 56, 24 66, 74 99; at 5 x 5 and
-    // 160 filters 48 -> 35, 43, 45, 53.  384 and 576 channels at 10 x 10 in three and five: 16 -> 18 and 22 -> 23.)
+    // which grow with the rows, the filter tiles and the CTAs that add at once, take less than the chunks saved (us in one CTA a tile / dealt to
+    // several, 960 channels in eight chunks: 160 filters at 7 x 7 8 tiles 42 / 35, 20 46 / 45, 28 46 / 47, 74 56 / 62; at 5 x 5 8 tiles 38 / 30, 40 42 / 40, 48
+    // 42 / 46; 320 filters at 7 x 7 8 tiles 48 / 46, 12 50 / 49, 16 50 / 56, 74 56 / 99; at 5 x 5 8 tiles 43 / 36, 16 44 / 44, 24 45 / 52; at 3 x 3 8 tiles 29 / 25, 19
+    // 34 / 35.  384 and 576 channels at 10 x 10 in three and five: 16 -> 18 and 22 -> 23.)
     a.splits = two ? 1 : std::max(1, std::min(a.chunks, sm_count / a.tiles));
-    if (a.chunks - (a.chunks + a.splits - 1) / a.splits < 4 || a.tiles * a.mt2 * a.mt2 > 160) a.splits = 1;
+    if (a.chunks - (a.chunks + a.splits - 1) / a.splits < 4 || a.tiles * a.mt2 * a.mt2 > (a.H >= 7 ? 100 : 160)) a.splits = 1;
     q.sums_bytes = a.splits > 1 ? (size_t)a.tiles * d2_cols * 512 : 0;
     a.w2_bytes = a.paired ? 8 * 192 * 16 : a.mt2 * 16384;
     a.w_bytes = a.kp * 128 + a.w2_bytes + 128 * (int)sizeof(IrbConst);
@@ -678,9 +679,8 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
 //     47 / 66; 16 -> 128: 148 images 27 / 37, 768 119 / 86)
 //   two units, stride 2 or planes that are not whole words, which the separate kernels put through an im2col pass: always (stride 2, 8 images 30 /
 //     33, 1024 132 / 197; 96 -> 576 at 11 x 11: 8 images 45 / 51, 160 84 / 104, 1500 368 / 557; 32 -> 192 at 13 x 13: 34 / 45, 48 / 80, 247 / 357)
-//   one unit, chunks on one CTA: from about three tiles a chunk on (160 -> 960 -> 320 at 7 x 7: 16 tiles 56 / 48, 24 51 / 54, 74 55 / 79; 64 -> 384 at
-//     4 x 4: 8 tiles 21 / 26); dealt to several, three filter tiles, seven rows or more: up to 12 tiles (the same block: 8 tiles 46 / 46, 16 54 / 47;
-//     at 5 x 5 16 tiles 42 / 45)
+//   one unit, seven rows or more, chunks on one CTA: from about three tiles a chunk on (160 -> 960 -> 320 at 7 x 7: 16 tiles 50 / 47, 24 53 / 54, 52
+//     54 / 67; 64 -> 384 at 8 x 8: 8 tiles 23 / 27); fewer rows: always (160 -> 960 -> 320 at 6 x 6: 19 tiles 39 / 40, 52 40 / 70; at 4 x 4: 19 29 / 38)
 //   planes of less than 16 pixels, a quarter of whose columns exist: while there are few rounds of few chunks (160 -> 960 at 3 x 3: 768 images 77 / 85,
 //     1024 95 / 93, 1500 127 / 115; with the long addition 768 90 / 91, 1024 109 / 96)
 // Below eight tiles the separate kernels use more of the chip (160 -> 960 at 4 x 4: 4 tiles 19 / 19, 64 -> 384 at 6 x 6: 2 tiles 20 / 19).
@@ -694,7 +694,7 @@ inline bool irb_pays(const IrbPlan& q, bool long_add, int sm_count) {
         const double tile = long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : std::max(8.0, 6.6 * a.chunks - 1.3);
         return rounds * tile * a.H / 14 <= (long_add ? 16.0 + 2.25 * values : (a.W % 4 != 0 ? 21.5 : 17.5) + 3.2 * values);
     }
-    if (a.splits > 1 ? a.mt2 >= 3 && a.H >= 7 && a.tiles > 12 : a.tiles + 1 < 3 * a.chunks) return false;
+    if (a.splits == 1 && a.H >= 7 && a.tiles + 1 < 3 * a.chunks) return false;
     return a.H * a.W >= 16 || rounds * a.chunks <= (long_add ? 16 : 30);
 }
 
