@@ -126,6 +126,15 @@ __device__ __forceinline__ int requant_one(int acc, float M, const Requant& r) {
 // sat(rne(clamp(v,-512,511)) + 0) for every v, so the results are bit-identical.
 __device__ __forceinline__ int rq_round(int acc, float M) { return __float2int_rn(__fmul_rn(__int2float_rn(acc), M)); }
 
+// rne((a - f) * m) of two floats given as bits, each difference and product rounded on its own: two packed operations instead of four.
+__device__ __forceinline__ void sub_mul_rn2(int a0, int a1, float f, float m, int& r0, int& r1) {
+    float x, y;
+    asm("{\n\t.reg .b64 v, f, m;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 f, {%4, %4};\n\tmov.b64 m, {%5, %5};\n\t"
+        "sub.rn.f32x2 v, v, f;\n\tmul.rn.f32x2 v, v, m;\n\tmov.b64 {%0, %1}, v;\n\t}\n"
+        : "=f"(x), "=f"(y) : "f"(__int_as_float(a0)), "f"(__int_as_float(a1)), "f"(f), "f"(m));
+    r0 = __float2int_rn(x); r1 = __float2int_rn(y);
+}
+
 // ReLU / ReLU6 of the lean epilogues moved in front of the requantisation.  With a positive multiplier
 // r(a) = rne(fl(float(a) * M)) is non-decreasing in the accumulator a and r(0) = 0, so for int8 codes with zero point 0
 //     clamp(sat8(r(a)), 0, six)  ==  sat8(r(clamp(a, 0, cap)))      where cap = the smallest a >= 0 with r(a) >= six,
