@@ -17,10 +17,7 @@
 // both: 11200 cycles a chunk of 14 x 14, of which a warp computed 5800; with the batched builder, the sender and the paired D2 8700).  Up to 64 filters (`paired`) the halves share the columns of D2: the A
 // operand of unit u holds the filters in lanes 64 u .. and zeros elsewhere, and all four lane quarters take part in the project epilogue.
 //
-// SPLITS.  Where the tiles leave SMs idle the chunks of a tile are dealt to `splits` CTAs, each adds its D2 to 32-bit sums in global memory
-// (exact in any order) and the last of them to come runs the project epilogue from there and leaves the sums zero for the next run.  A CTA whose
-// wait ran out counts itself all the same, when its warps are done, and the last one zeroes the tile's sums if it gave up itself: a run that
-// reported a time-out leaves the next one (a graph's replay too) what a run in order leaves.
+// For few images irb_band.cuh deals a block to more CTAs.
 //
 // What bounds it: instruction issue in the epilogue warps, 31 thousand of the warp instructions of a 14 x 14 x 384 image are the two
 // requantisations, the filter and the project epilogue (as separate kernels the depthwise one alone took 31 instructions an output).
@@ -65,9 +62,6 @@ struct IrbArgs {
     int paired;                    // two units, at most 64 filters: one D2, lanes 64 u + filter
     int w2_bytes;                  // W2 of a chunk: [filter tile][8 k16][128][16], or paired [8 k16][64 zero, 64 filter, 64 zero rows][16]
     int d1_bufs;                   // one unit: buffers of D1
-    int splits;                    // CTAs per tile; above 1 a CTA has one tile
-    int32_t* sums; int* arrived;   // splits: [tile][D2 column][128 lanes], all zero between runs, and a counter per tile
-    int give_up;                   // splits: self test, a CTA half of whose epilogue warps give up (-1: none)
     int x_bufs, y_bufs, w_stages;
     int w_bytes, x_bytes, y_bytes; // one stage / buffer
     int off_x, off_y, off_out, off_tail;
@@ -202,19 +196,15 @@ __device__ __forceinline__ void irb_rows_s2(uint32_t src, int r0, int r1, const 
 }
 
 // WC: columns computed per row (the width rounded up to an instantiated value).  S: stride.
-// SPLIT: the chunks of a tile dealt to several CTAs (planes at most 8 wide only: the blocks with many chunks).
-template <int WC, int S, bool ADD, bool SPLIT>
+template <int WC, int S, bool ADD>
 __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_constant__ IrbArgs a, const __grid_constant__ QAddTail add) {
     constexpr int PITCH = WC > 8 ? 16 : 8, OPITCH = S == 1 ? PITCH : 8, U = PITCH == 16 ? 2 : 1;
     static_assert(S == 1 || (PITCH == 16 && !ADD), "");
-    const int splits = SPLIT ? a.splits : 1;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* tail = smem + a.off_tail;
     uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 256);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 260);
-    volatile int* finish = reinterpret_cast<volatile int*>(tail + 264);      // this CTA has the tile's sums
-    volatile int* counted = reinterpret_cast<volatile int*>(tail + 268);     // splits: this CTA is in the tile's counter (2: as the last)
     const uint32_t smem0 = ptx::smem_u32(smem), bar0 = ptx::smem_u32(bars);
     auto wfull = [&](int s) { return bar0 + 8u * s; };
     auto wempty = [&](int s) { return bar0 + 8u * (2 + s); };
@@ -224,7 +214,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
     auto d1empty = [&](int b) { return bar0 + 8u * (10 + b); };
     auto yfull = [&](int u, int b) { return bar0 + 8u * (12 + 2 * u + b); };
     auto yempty = [&](int u, int b) { return bar0 + 8u * (16 + 2 * u + b); };
-    const uint32_t d2full = bar0 + 8u * 20, d2empty = bar0 + 8u * 21, out_free = bar0 + 8u * 22, out_full = bar0 + 8u * 23, sum_full = bar0 + 8u * 24, sum_done = bar0 + 8u * 25;
+    const uint32_t d2full = bar0 + 8u * 20, d2empty = bar0 + 8u * 21, out_free = bar0 + 8u * 22, out_full = bar0 + 8u * 23;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slots = U == 2 ? 2 : a.d1_bufs;
     const int d2_cols = (a.paired ? 1 : a.mt2 * U) * a.n2, cols = slots * a.n1 + d2_cols;
@@ -239,8 +229,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
         }
         ptx::mbar_init(d2full, 1); ptx::mbar_init(d2empty, kIrbEpiWarps);
         ptx::mbar_init(out_free, 1); ptx::mbar_init(out_full, kIrbEpiWarps);
-        ptx::mbar_init(sum_full, kIrbEpiWarps); ptx::mbar_init(sum_done, 1);
-        *abort_flag = 0; *finish = 1; *counted = 0;
+        *abort_flag = 0;
         ptx::mbar_fence_init();
     }
     if (warp == 1) {
@@ -253,10 +242,8 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
     ptx::grid_trigger();
     if (warp != 0) ptx::grid_wait();                     // (weights are constants)
-    // this CTA's tiles: tile0, tile0 + step, ..; its chunks of each: split, split + splits, ..
-    const int split = SPLIT ? (int)blockIdx.x % splits : 0, tile0 = SPLIT ? (int)blockIdx.x / splits : (int)blockIdx.x, tile_step = (int)gridDim.x;
-    const int my_tiles = SPLIT ? 1 : ((int)blockIdx.x < a.tiles ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0);
-    const int chunks = (a.chunks - split + splits - 1) / splits;
+    const int tile0 = (int)blockIdx.x, tile_step = (int)gridDim.x;               // this CTA's tiles: tile0, tile0 + step, ..
+    const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0, chunks = a.chunks;
     const int total = my_tiles * chunks;                 // chunks of this CTA, in order
     const uint32_t xblk = (uint32_t)a.kp * 128u;         // a unit's part of X
     constexpr uint32_t yblk = 16384u;
@@ -318,7 +305,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
             for (int j = 0; j < total; ++j) {
                 if (!ptx::mbar_wait_sleeping(wempty(s), ph ^ 1u, abort_flag)) break;
                 ptx::mbar_arrive_expect_tx(wfull(s), (uint32_t)a.w_bytes);
-                ptx::bulk_g2s(smem0 + (uint32_t)(s * a.w_bytes), a.w + (size_t)(split + c * splits) * a.w_bytes, (uint32_t)a.w_bytes, wfull(s));
+                ptx::bulk_g2s(smem0 + (uint32_t)(s * a.w_bytes), a.w + (size_t)c * a.w_bytes, (uint32_t)a.w_bytes, wfull(s));
                 if (++c == chunks) c = 0;
                 if (++s == a.w_stages) { s = 0; ph ^= 1u; }
             }
@@ -360,7 +347,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
                 }
             }
             if (j > 0) {
-                const int ks = split + pc * splits == a.chunks - 1 ? (a.last_live + 31) >> 5 : 4;
+                const int ks = pc == a.chunks - 1 ? (a.last_live + 31) >> 5 : 4;
                 const uint32_t w2 = (smem0 + (uint32_t)(ps * a.w_bytes) + w1_bytes) >> 4, y0 = (smem0 + (uint32_t)(a.off_y + yb * a.y_bytes)) >> 4;
                 for (int u = 0; u < U && alive; ++u) {
                     if (!wait(yfull(u, yb), yph) || (pc == 0 && u == 0 && !wait(d2empty, d2ph ^ 1u))) { alive = false; break; }
@@ -399,7 +386,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
         if (lane == 0) {
             for (int i = 0; i < my_tiles; ++i) {
                 const int t = tile0 + i * tile_step;
-                if (!ptx::mbar_wait_sleeping(out_full, (uint32_t)i & 1u, abort_flag) || (SPLIT && !*finish)) break;
+                if (!ptx::mbar_wait_sleeping(out_full, (uint32_t)i & 1u, abort_flag)) break;
                 const int plane = a.M * a.OH * a.OW;
                 ptx::bulk_s2g(a.y + (size_t)t * a.IB * plane, smem0 + (uint32_t)a.off_out, (uint32_t)(min(a.IB, a.N - t * a.IB) * plane));
                 ptx::bulk_wait_read<0>();
@@ -442,44 +429,10 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
             if ((i > 0 && !wait(out_free, (uint32_t)(i - 1) & 1u)) || !wait(d2full, (uint32_t)i & 1u)) return false;
             if (ADD && __all_sync(0xffffffffu, ptx::mbar_wait(xfull(i % a.x_bufs), (uint32_t)(i / a.x_bufs) & 1u, abort_flag)) == 0) return false;
             ptx::tc_fence_after();
-            int32_t* sums = nullptr;
-            if constexpr (SPLIT) {
-                if ((int)blockIdx.x == a.give_up && (warp & 1)) { *abort_flag = 1; return false; }
-                sums = a.sums + (size_t)t * d2_cols * 128 + ch;
-                // this warp's part of D2 into the tile's sums
-                for (int mt = 0; mt < a.mt2; ++mt) {
-                    if (mt * 128 + (a.paired ? (quarter & 1) * 32 : quarter * 32) >= a.M || (U == 1 && pu >= n_here)) break;
-                    for (int r = p0; r < pu1; r += ps) {
-                        const int col = (a.paired ? 0 : (U == 2 ? mt * 2 + pu : mt) * a.n2) + (U == 2 ? r - pu0 : pu * a.OH + r) * OPITCH + pc0;
-                        uint32_t v[9];
-                        irb_tmem_cols<8>(d2 + (uint32_t)col, v);
-                        ptx::tmem_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < pcols) atomicAdd(sums + (size_t)(col + e) * 128, (int)v[e]);
-                    }
-                }
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(sum_full);
-                if (warp == 2) {
-                    if (!wait(sum_full, 0)) return false;
-                    if (lane == 0) {
-                        __threadfence();                                  // (the other warps' additions, which sum_full ordered before this thread, before the counter)
-                        const bool last = atomicAdd(a.arrived + t, 1) == splits - 1;
-                        if (last) a.arrived[t] = 0;
-                        *finish = last ? 1 : 0;
-                        *counted = last ? 2 : 1;
-                        __threadfence();
-                        ptx::mbar_arrive(sum_done);
-                    }
-                }
-                if (!wait(sum_done, 0)) return false;
-            }
             uint8_t* out = smem + a.off_out;
             const uint32_t xs = smem0 + (uint32_t)(a.off_x + (i % a.x_bufs) * a.x_bytes);
             for (int mt = 0; mt < a.mt2; ++mt) {
-                if (mt * 128 + (a.paired ? (quarter & 1) * 32 : quarter * 32) >= a.M || (U == 1 && pu >= n_here) || p0 >= pu1 || (SPLIT && !*finish)) break;
+                if (mt * 128 + (a.paired ? (quarter & 1) * 32 : quarter * 32) >= a.M || (U == 1 && pu >= n_here) || p0 >= pu1) break;
                 const int m = mt * 128 + pm;
                 const bool live = m < a.M;
                 const float mlt = live ? __ldg(a.mult2 + m) : 1.0f;
@@ -487,23 +440,15 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
                 uint32_t src = d2 + (uint32_t)((a.paired ? 0 : (U == 2 ? mt * 2 + pu : mt) * a.n2) + (U == 2 ? p0 - pu0 : pu * a.OH + p0) * OPITCH + pc0);
                 uint8_t* o = out + ((size_t)(U == 2 ? 0 : pu) * a.M + m) * OHW + p0 * a.OW + pc0;
                 uint32_t v[9];
-                if (!SPLIT) irb_tmem_cols<8>(src, v);
+                irb_tmem_cols<8>(src, v);
                 for (int r = p0; r < pu1; r += ps, o += ps * a.OW) {
-                    if (!SPLIT) {
-                        ptx::tmem_wait_ld();
-                    } else {
-                        int32_t* sr = sums + (size_t)(src - d2) * 128;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = e < pcols ? (uint32_t)__ldcg(sr + e * 128) : 0u;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) if (e < pcols) sr[e * 128] = 0;
-                    }
+                    ptx::tmem_wait_ld();
                     uint32_t pk[2];
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
                         pk[j] = pack_sat_s8x4(rq_round((int)v[4 * j] + bs, mlt), rq_round((int)v[4 * j + 1] + bs, mlt), rq_round((int)v[4 * j + 2] + bs, mlt), rq_round((int)v[4 * j + 3] + bs, mlt));
                     src += (uint32_t)(ps * OPITCH);
-                    if (!SPLIT && r + ps < pu1) irb_tmem_cols<8>(src, v);
+                    if (r + ps < pu1) irb_tmem_cols<8>(src, v);
                     if constexpr (ADD) {
                         // the block's input at this channel (m < C == M) and row, from the operand
                         const uint32_t rr = (uint32_t)(U == 2 ? r - (pu ? a.rh - 1 : 0) : pu * a.H + r), q = PITCH == 16 ? rr : rr >> 1;
@@ -550,7 +495,7 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(d1empty(slot));      // this warp has read its accumulators
             };
-            if (split + c * splits < a.chunks - 1 || quarter * 32 < a.last_live) {
+            if (c < a.chunks - 1 || quarter * 32 < a.last_live) {
                 const uint32_t cs = smem0 + (uint32_t)(s * a.w_bytes + a.kp * 128 + a.w2_bytes + ch * 32);
                 const uint4 k0 = lds_u128(cs), k1 = lds_u128(cs + 16u);
                 const float ef = __uint_as_float(k0.x), em = __uint_as_float(k0.y), dm = __uint_as_float(k0.z);
@@ -595,19 +540,6 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 1) ptx::tmem_dealloc(tmem_base, tmem_cols);
-    if (SPLIT && my_tiles > 0 && *abort_flag) {
-        // nothing of this CTA adds or waits any more
-        if (tid == 0 && *counted == 0) {
-            __threadfence();
-            const bool last = atomicAdd(a.arrived + tile0, 1) == splits - 1;
-            if (last) a.arrived[tile0] = 0;
-            *counted = last ? 2 : 1;
-            __threadfence();
-        }
-        __syncthreads();
-        if (*counted == 2)
-            for (int i = tid; i < d2_cols * 128; i += kIrbThreads) a.sums[(size_t)tile0 * d2_cols * 128 + i] = 0;
-    }
     if (tid == 0 && *abort_flag) atomicExch(a.status, (int)DEV_ERR_WAIT_TIMEOUT);
 }
 
@@ -617,12 +549,12 @@ __global__ void __launch_bounds__(kIrbThreads, 1) irb_kernel(const __grid_consta
 struct IrbPlan {
     IrbArgs a{};
     int wc = 0, E = 0, stride = 1;
-    size_t smem_bytes = 0, sums_bytes = 0;
+    size_t smem_bytes = 0;
 };
 
 // Geometry of the three convolutions; false when the kernel does not take them.  With the addition the operand X of a tile is read by the
 // project epilogue, behind the next tile's first chunk: it needs a second buffer.
-inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bool add, int sm_count, IrbPlan& q) {
+inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bool add, IrbPlan& q) {
     auto pointwise = [](const ConvGeom& g) { return g.G == 1 && g.KH == 1 && g.KW == 1 && g.sh == 1 && g.sw == 1 && !g.pt && !g.pl && !g.pb && !g.pr; };
     if (!pointwise(e) || !pointwise(p)) return false;
     if (d.G != d.C || d.M != d.C || d.KH != 3 || d.KW != 3 || d.sh != d.sw || d.sh < 1 || d.sh > 2 || d.dh != 1 || d.dw != 1 || d.pt != 1 || d.pl != 1 || d.pb != 1 || d.pr != 1) return false;
@@ -652,14 +584,6 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
     const int d2_cols = (a.paired ? 1 : a.mt2 * (two ? 2 : 1)) * a.n2;
     if ((two ? 2 : 1) * a.n1 + d2_cols > 512 || a.n1 > 128) return false;
     a.d1_bufs = !two && 2 * a.n1 + d2_cols <= 512 ? 2 : 1;
-    // As many CTAs a tile as the SMs hold, none with less than a chunk, where that saves a CTA four chunks and while adding up and reading back,
-    // which grow with the rows, the filter tiles and the CTAs that add at once, take less than the chunks saved (us in one CTA a tile / dealt to
-    // several, 960 channels in eight chunks: 160 filters at 7 x 7 8 tiles 42 / 35, 20 46 / 45, 28 46 / 47, 74 56 / 62; at 5 x 5 8 tiles 38 / 30, 40 42 / 40, 48
-    // 42 / 46; 320 filters at 7 x 7 8 tiles 48 / 46, 12 50 / 49, 16 50 / 56, 74 56 / 99; at 5 x 5 8 tiles 43 / 36, 16 44 / 44, 24 45 / 52; at 3 x 3 8 tiles 29 / 25, 19
-    // 34 / 35.  384 and 576 channels at 10 x 10 in three and five: 16 -> 18 and 22 -> 23.)
-    a.splits = two ? 1 : std::max(1, std::min(a.chunks, sm_count / a.tiles));
-    if (a.chunks - (a.chunks + a.splits - 1) / a.splits < 4 || a.tiles * a.mt2 * a.mt2 > (a.H >= 7 ? 100 : 160)) a.splits = 1;
-    q.sums_bytes = a.splits > 1 ? (size_t)a.tiles * d2_cols * 512 : 0;
     a.w2_bytes = a.paired ? 8 * 192 * 16 : a.mt2 * 16384;
     a.w_bytes = a.kp * 128 + a.w2_bytes + 128 * (int)sizeof(IrbConst);
     a.x_bytes = (two ? 2 : 1) * a.kp * 128; a.y_bytes = (two ? 2 : 1) * 16384;
@@ -696,14 +620,14 @@ inline bool irb_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& p, bo
 inline bool irb_pays(const IrbPlan& q, bool long_add, int sm_count) {
     const IrbArgs& a = q.a;
     if (a.tiles < 8) return false;
-    const long long rounds = ((long long)a.tiles * a.splits + sm_count - 1) / sm_count;
+    const long long rounds = (a.tiles + sm_count - 1) / sm_count;
     if (a.IB == 1) {
         if (q.stride == 2 || a.H * a.W % 4 != 0) return true;
         const double values = 1e-6 * a.N * q.E * a.H * a.W;
         const double tile = long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : std::max(8.0, 6.6 * a.chunks - 1.3);
         return rounds * tile * a.H / 14 <= (long_add ? 16.0 + 2.25 * values : (a.W % 4 != 0 ? 21.5 : 17.5) + 3.2 * values);
     }
-    if (a.splits == 1 && a.H >= 7 && a.tiles + 1 < 3 * a.chunks) return false;
+    if (a.H >= 7 && a.tiles + 1 < 3 * a.chunks) return false;
     return a.H * a.W >= 16 || rounds * a.chunks <= (long_add ? 16 : 30);
 }
 
@@ -734,27 +658,21 @@ inline bool irb_prepare(const IrbPlan& q, const int8_t* we, const float* em, con
     return true;
 }
 
-// x: 4-byte aligned, y: 16-byte aligned; sums: q.sums_bytes and a word per tile, zero before the first run.
-inline int32_t irb_run(zant_ctx* ctx, const IrbPlan& q, const void* x, const uint8_t* w, const float* mult2, const int32_t* bias2, void* y, void* sums, const QAddTail* add) {
+// x: 4-byte aligned, y: 16-byte aligned.
+inline int32_t irb_run(zant_ctx* ctx, const IrbPlan& q, const void* x, const uint8_t* w, const float* mult2, const int32_t* bias2, void* y, const QAddTail* add) {
     IrbArgs a = q.a;
     a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.w = w; a.mult2 = mult2; a.bias2 = bias2; a.status = ctx->status_word;
-    a.give_up = -1;
-    if (a.splits > 1) { a.sums = (int32_t*)sums; a.arrived = (int*)((char*)sums + q.sums_bytes); std::swap(a.give_up, ctx->give_up_cta); }
-    const int grid = std::min(a.tiles * a.splits, ctx->sm_count);
-    auto go = [&](auto wc, auto stride, auto with, auto split) -> int32_t {
+    const int grid = std::min(a.tiles, ctx->sm_count);
+    auto go = [&](auto wc, auto stride, auto with) -> int32_t {
         constexpr int WC = decltype(wc)::value, S = decltype(stride)::value;
-        constexpr bool ADD = decltype(with)::value, SPLIT = decltype(split)::value;
-        ZB_SMEM_ATTR(ctx, (irb_kernel<WC, S, ADD, SPLIT>), 227 * 1024);
-        launch_const(ctx, irb_kernel<WC, S, ADD, SPLIT>, grid, kIrbThreads, q.smem_bytes, a, add ? *add : QAddTail{});
+        constexpr bool ADD = decltype(with)::value;
+        ZB_SMEM_ATTR(ctx, (irb_kernel<WC, S, ADD>), 227 * 1024);
+        launch_const(ctx, irb_kernel<WC, S, ADD>, grid, kIrbThreads, q.smem_bytes, a, add ? *add : QAddTail{});
         return check_launch(ctx, "irb_kernel");
     };
     using one = std::integral_constant<int, 1>;
-    if (q.stride == 2) return go(std::integral_constant<int, 16>{}, std::integral_constant<int, 2>{}, std::false_type{}, std::false_type{});
-    auto pick = [&](auto wc) -> int32_t {
-        if constexpr (decltype(wc)::value <= 8)
-            if (a.splits > 1) return add ? go(wc, one{}, std::true_type{}, std::true_type{}) : go(wc, one{}, std::false_type{}, std::true_type{});
-        return add ? go(wc, one{}, std::true_type{}, std::false_type{}) : go(wc, one{}, std::false_type{}, std::false_type{});
-    };
+    if (q.stride == 2) return go(std::integral_constant<int, 16>{}, std::integral_constant<int, 2>{}, std::false_type{});
+    auto pick = [&](auto wc) -> int32_t { return add ? go(wc, one{}, std::true_type{}) : go(wc, one{}, std::false_type{}); };
     switch (q.wc) {
         case 4: return pick(std::integral_constant<int, 4>{});
         case 6: return pick(std::integral_constant<int, 6>{});

@@ -175,6 +175,13 @@ __device__ __forceinline__ uint32_t pack_sat_s8x4(int a0, int a1, int a2, int a3
     return d;
 }
 
+// the two low bytes = sat8(a0), sat8(a1), the others 0
+__device__ __forceinline__ uint32_t pack_sat_s8x2(int a0, int a1) {
+    uint32_t d;
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(d) : "r"(a1), "r"(a0));
+    return d;
+}
+
 // bytes (little endian) = satu8(a0) .. satu8(a3), i.e. each clamped to [0, 255]
 __device__ __forceinline__ uint32_t pack_sat_u8x4(int a0, int a1, int a2, int a3) {
     uint32_t hi, d;

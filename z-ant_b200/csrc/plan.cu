@@ -28,6 +28,7 @@
 #include "tc_gemm_tf32.cuh"
 #include "small_gemm_q8.cuh"
 #include "tc_nhwc_net.cuh"
+#include "irb_band.cuh"
 #include "irb_q8.cuh"
 #include "status.hpp"
 
@@ -1355,8 +1356,8 @@ static int32_t try_fuse(zant_plan* pl, size_t i0, size_t& consumed) {
     return try_fuse_fconv_group(pl, i0, consumed);
 }
 
-// QLinearConv 1x1 -> QLinearConv depthwise 3x3 -> QLinearConv 1x1 [-> QLinearAdd with the group's input] on small planes as one step
-// (irb_q8.cuh).  Both activations are ReLU or a ReLU6 whose bound is the type's own, all tensors int8, zero points 0 between the convolutions,
+// QLinearConv 1x1 -> QLinearConv depthwise 3x3 -> QLinearConv 1x1 [-> QLinearAdd with the group's input] as one step (irb_q8.cuh for
+// many images on small planes, irb_band.cuh for few).  Both activations are ReLU or a ReLU6 whose bound is the type's own, all tensors int8, zero points 0 between the convolutions,
 // interior tensors read by the next node only.  Whatever does not qualify is left to the steps of its own.
 static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
     consumed = 0;
@@ -1422,24 +1423,28 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
             consumed = 4;
         }
     }
-    IrbPlan q;
-    if (!irb_plan(g[0], g[1], g[2], with_add, pl->ctx->sm_count, q) || !irb_pays(q, with_add && !add.proved, pl->ctx->sm_count)) { consumed = 0; return ZANT_OK; }
-    std::vector<uint8_t> stages;
-    if (!irb_prepare(q, (const int8_t*)T(e->in[1]).host.data(), mult[0].data(), bias[0].data(), (const int8_t*)T(d->in[1]).host.data(), mult[1].data(), bias[1].data(),
-                     (const int8_t*)T(p->in[1]).host.data(), stages)) { consumed = 0; return ZANT_OK; }
-    const int aw = pl->add_aux(stages.data(), stages.size()), am = pl->add_aux(mult[2].data(), mult[2].size() * 4), ab = pl->add_aux(bias[2].data(), bias[2].size() * 4);
-    const size_t first_step = pl->steps.size();
     zant_ctx* ctx = pl->ctx;
-    int as = -1;
-    if (q.sums_bytes) {
-        const size_t bytes = q.sums_bytes + (size_t)q.a.tiles * sizeof(int);
-        as = pl->add_scratch(bytes);
-        pl->init_steps.push_back([=]() -> int32_t { ZB_CUDA(cudaMemsetAsync(pl->scratch(as), 0, bytes, ctx->stream)); return ZANT_OK; });
+    auto host = [&](int id) { return (const int8_t*)T(id).host.data(); };
+    IrbPlan q;
+    IrbBandPlan qb;
+    const bool can_one = irb_plan(g[0], g[1], g[2], with_add, q), can_band = irb_band_plan(g[0], g[1], g[2], with_add, ctx->sm_count, qb);
+    const IrbForm form = irb_form(can_one ? &q : nullptr, can_band ? &qb : nullptr, g[1], with_add && !add.proved, ctx->sm_count);
+    std::vector<uint8_t> stages;
+    if (form == IrbForm::kSeparate ||
+        !(form == IrbForm::kBand ? irb_band_prepare(qb, host(e->in[1]), mult[0].data(), bias[0].data(), host(d->in[1]), mult[1].data(), bias[1].data(), host(p->in[1]), mult[2].data(), bias[2].data(), stages)
+                                 : irb_prepare(q, host(e->in[1]), mult[0].data(), bias[0].data(), host(d->in[1]), mult[1].data(), bias[1].data(), host(p->in[1]), stages))) {
+        consumed = 0;
+        return ZANT_OK;
     }
+    const int aw = pl->add_aux(stages.data(), stages.size());
+    const size_t first_step = pl->steps.size();
     pl->step_names.push_back(with_add ? "QLinearConv(expand+depthwise+project)+QLinearAdd" : "QLinearConv(expand+depthwise+project)");
-    pl->steps.push_back([=]() {
-        return irb_run(ctx, q, pl->ptr(x), (const uint8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y), as >= 0 ? pl->scratch(as) : nullptr, with_add ? &add : nullptr);
-    });
+    if (form == IrbForm::kBand) {
+        pl->steps.push_back([=]() { return irb_band_run(ctx, qb, pl->ptr(x), (const uint8_t*)pl->aux(aw), pl->ptr(y), with_add ? &add : nullptr); });
+    } else {
+        const int am = pl->add_aux(mult[2].data(), mult[2].size() * 4), ab = pl->add_aux(bias[2].data(), bias[2].size() * 4);
+        pl->steps.push_back([=]() { return irb_run(ctx, q, pl->ptr(x), (const uint8_t*)pl->aux(aw), (const float*)pl->aux(am), (const int32_t*)pl->aux(ab), pl->ptr(y), with_add ? &add : nullptr); });
+    }
     pl->t[t1].elided = pl->t[t2].elided = true;
     if (with_add) pl->t[y0].elided = true;
     record_step_cost(pl, first_step, i0, consumed);
