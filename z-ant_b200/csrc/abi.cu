@@ -888,14 +888,10 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const int ixl = s.scratch((size_t)g.N * hw * pix), iwb = s.scratch(nhp.w_bytes), ibb = s.scratch((size_t)nhp.a.const_n * 4);
         if (s.room()) {
             ZB_TRY(s.commit());
-            const uint64_t launched = ctx->launches;
-            ZB_TRY(run_nh_weights(ctx, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb)));
-            if (!bias_here) {
-                launch(ctx, nh_bias_k, (unsigned)((nhp.a.const_n + 7) / 8), 256, 0, (const int8_t*)s.ptr<int8_t>(iw), (const int32_t*)s.ptr<int32_t>(ib), s.ptr<int32_t>(ibb), g.M, K, nhp.a.const_n, x_zp);
-                ZB_TRY(check_launch(ctx, "nh_bias_k"));
-            }
-            ctx->launches = launched;                       // (not operator launches)
-            ZB_TRY(run_to_nhwc_bytes(ctx, s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix));
+            NhPrepArgs prep = nh_prep_input(s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix);
+            nh_prep_weights(ctx, prep, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb));
+            if (!bias_here) { prep.bw = s.ptr<int8_t>(iw); prep.bias = s.ptr<int32_t>(ib); prep.bias_out = s.ptr<int32_t>(ibb); prep.M = g.M; prep.K = K; prep.bias_n = nhp.a.const_n; prep.x_zp = x_zp; }
+            ZB_TRY(run_nh_prep(ctx, prep));
             NhConvArgs a = nhp.a;
             a.w = s.ptr<uint8_t>(iwb); a.mult = s.ptr<float>(im); a.bias = s.ptr<int32_t>(bias_here ? ib : ibb);
             a.y = s.ptr<uint8_t>(iy); a.nchw = 1; a.act = activation; a.six = lean_six(y_scale);

@@ -661,11 +661,10 @@ inline bool nh_conv_plan(const ConvGeom& g, int kind, bool pool, int sm_count, N
 // host 30 ms).  T: int8_t, or float (rounded to TF32, part 1 the remainder).
 struct NhWeightArgs { const void* w; uint8_t* out; int M, C, taps, NT, NB, KC, T, c_stages, parts, pool; long long chunks; };
 template <typename T>
-__global__ void __launch_bounds__(256) nh_weights_k(const __grid_constant__ NhWeightArgs a) {
-    ptx::grid_start();
+__device__ __forceinline__ void nh_weight_chunks(const NhWeightArgs& a, long long first, long long step) {
     constexpr int PER = 16 / (int)sizeof(T);
     const int per_row = a.KC / 16;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.chunks; i += (long long)gridDim.x * blockDim.x) {
+    for (long long i = first; i < a.chunks; i += step) {
         long long t = i;
         int slot = (int)(t % per_row); t /= per_row;
         const int row = (int)(t % a.NB); t /= a.NB;
@@ -699,27 +698,24 @@ __global__ void __launch_bounds__(256) nh_weights_k(const __grid_constant__ NhWe
         reinterpret_cast<uint4*>(a.out)[i] = u.q;
     }
 }
-inline int32_t run_nh_weights(zant_ctx* ctx, const NhConvPlan& p, const void* w, void* out) {
+template <typename T>
+__global__ void __launch_bounds__(256) nh_weights_k(const __grid_constant__ NhWeightArgs a) {
+    ptx::grid_start();
+    nh_weight_chunks<T>(a, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+inline NhWeightArgs nh_weight_args(const NhConvPlan& p, const void* w, void* out) {
     NhWeightArgs a{};
     a.w = w; a.out = (uint8_t*)out; a.M = p.a.M; a.C = p.w_cin; a.taps = p.a.KH * p.a.KW; a.NT = p.a.NT; a.KC = p.a.KC; a.T = p.a.T; a.c_stages = p.a.c_stages;
     a.NB = p.a.NT * (p.pool == NH_POOL_VIEWS ? 4 : (p.pool == NH_POOL_PAIRS ? 2 : 1));
     a.parts = p.a.parts; a.pool = p.pool; a.chunks = (long long)p.w_bytes / 16;
+    return a;
+}
+inline int32_t run_nh_weights(zant_ctx* ctx, const NhConvPlan& p, const void* w, void* out) {
+    const NhWeightArgs a = nh_weight_args(p, w, out);
     const int grid = grid_for((size_t)a.chunks, 256, ctx->sm_count);
     if (p.kind <= NH_U8) launch(ctx, nh_weights_k<int8_t>, grid, 256, 0, a);
     else launch(ctx, nh_weights_k<float>, grid, 256, 0, a);
     return check_launch(ctx, "nh_weights_k");
-}
-
-// bias - x_zp * (sum of the filter's weights), zeros behind the last filter: a warp per entry.
-__global__ void __launch_bounds__(256) nh_bias_k(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int32_t* __restrict__ out, int M, int K, int n, int x_zp) {
-    ptx::grid_start();
-    const int m = (int)((blockIdx.x * 256 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (m >= n) return;
-    int s = 0;
-    if (m < M && x_zp != 0) for (int k = lane; k < K; k += 32) s += __ldg(w + (size_t)m * K + k);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[m] = m < M ? (bias ? __ldg(bias + m) : 0) - x_zp * s : 0;
 }
 
 // A single call's plan: the search visits some hundred tilings (1 to 2 us of the 30 a small call takes), so a thread keeps the plans of
@@ -900,43 +896,100 @@ inline int32_t run_to_nhwc(zant_ctx* ctx, int mode, const void* x, void* y, int 
     return check_launch(ctx, "to_nhwc_small_k");
 }
 
-// Any 8-bit NCHW tensor -> pixels of `pix` bytes (channels rounded up to 16, zeros behind the last): 64 channels x 128 pixels of one
-// image through shared memory.  The rows of a channel plane start at any byte: a thread cuts its word out of two aligned ones.
-constexpr int kToNhwcPx = 128, kToNhwcCh = 64, kToNhwcPitch = kToNhwcPx + 4;
-__global__ void __launch_bounds__(256) to_nhwc_bytes_k(const uint8_t* __restrict__ x, uint8_t* __restrict__ y, int C, int HW, int pix, long long bytes) {
+// What a single call prepares on the device, one launch, blocks by kind: the input channels-last, the weights in their blocks, the bias.
+//   input  8-bit NCHW -> pixels of `pix` bytes (channels rounded up to 16, zeros behind the last): a block takes 64 channels x 128 pixels of one image
+//          through shared memory; rows of a channel plane start at any byte, so a word is cut out of two aligned ones.  A thread then has four pixels of
+//          16 channels as sixteen words, transposes them by byte permutes (instead of 64 byte loads from shared memory) and four lanes write 64
+//          contiguous bytes of a pixel.  Words of a row are stored at w ^ 8 (channel / 16), so that the four lanes' channels lie in different banks.
+//   bias   bias - x_zp * (sum of the filter's weights), zeros behind the last filter: a warp per entry
+// The kinds do not depend on each other: as launches one after the other, latency chains both, 7.4 + 14.4 us for 256 x 256 x 14 x 14 and 512 filters of
+// 3 x 3 and 6.4 + 6.1 for 33 x 45 x 27 x 27 and 85, together 15.1 and 6.9; the calls 95.8 -> 93.6 (the weights' upload is most of it) and 38.2 -> 32.6.
+struct NhPrepArgs {
+    const uint8_t* x; uint8_t* y; int C, HW, pix; long long bytes;
+    int px_tiles, ch_tiles;
+    unsigned x_blocks, w_blocks;
+    NhWeightArgs w;
+    const int8_t* bw; const int32_t* bias; int32_t* bias_out; int M, K, bias_n, x_zp;      // bias_n 0: the bias is ready
+};
+constexpr int kNhPrepThreads = 128;
+__global__ void __launch_bounds__(kNhPrepThreads) nh_prep_k(const __grid_constant__ NhPrepArgs a) {
     ptx::grid_start();
-    __shared__ __align__(16) uint8_t tile[kToNhwcCh * kToNhwcPitch];
-    const int p0 = (int)blockIdx.x * kToNhwcPx, c0 = (int)blockIdx.y * kToNhwcCh;
-    const long long n = blockIdx.z;
-    for (int i = threadIdx.x; i < kToNhwcCh * (kToNhwcPx / 4); i += 256) {
-        const int c = i / (kToNhwcPx / 4), w = i - c * (kToNhwcPx / 4);
-        uint32_t v = 0;
-        if (c0 + c < C && p0 + 4 * w < HW) {
-            const long long at = (n * C + c0 + c) * (long long)HW + p0 + 4 * w, al = at & ~3LL;
-            const uint32_t* s = reinterpret_cast<const uint32_t*>(x + al);
-            if (al + 8 <= bytes) {
-                const uint32_t lo = __ldg(s), sh = (uint32_t)(at & 3) * 8u;
-                v = sh ? __funnelshift_r(lo, __ldg(s + 1), sh) : lo;
-            } else {
-                for (int k = 0; k < 4; ++k) if (at + k < bytes) v |= (uint32_t)__ldg(x + at + k) << (8 * k);
+    __shared__ uint32_t tile[64 * 32];
+    unsigned b = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (b < a.x_blocks) {
+        const int per = a.px_tiles * a.ch_tiles;
+        const long long n = b / per;
+        const int r = (int)(b - n * per), c0 = r / a.px_tiles * 64, p0 = (r - r / a.px_tiles * a.px_tiles) * 128;
+        for (int i0 = 0; i0 < 16; i0 += 8) {
+            uint32_t lo[8], hi[8], sh[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int c = c0 + warp + 4 * (i0 + i), p = p0 + 4 * lane;
+                lo[i] = hi[i] = sh[i] = 0u;
+                if (c < a.C && p < a.HW) {
+                    const long long at = (n * a.C + c) * (long long)a.HW + p, al = at & ~3LL;
+                    if (al + 8 <= a.bytes) {
+                        const uint32_t* s = reinterpret_cast<const uint32_t*>(a.x + al);
+                        sh[i] = (uint32_t)(at & 3) * 8u;
+                        lo[i] = __ldg(s);
+                        if (sh[i]) hi[i] = __ldg(s + 1);
+                    } else {
+                        for (int k = 0; k < 4; ++k) if (at + k < a.bytes) lo[i] |= (uint32_t)__ldg(a.x + at + k) << (8 * k);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int c = warp + 4 * (i0 + i);
+                tile[c * 32 + (lane ^ (8 * (c >> 4)))] = __funnelshift_r(lo[i], hi[i], sh[i]);
             }
         }
-        *reinterpret_cast<uint32_t*>(tile + c * kToNhwcPitch + 4 * w) = v;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kToNhwcPx * (kToNhwcCh / 16); i += 256) {
-        const int p = i >> 2, c = (i & 3) * 16;
-        if (p0 + p >= HW || c0 + c >= pix) continue;
-        uint32_t q[4] = {0u, 0u, 0u, 0u};
+        __syncthreads();
+        const int j = lane & 3, word = warp * 8 + (lane >> 2), p = p0 + 4 * word, c = c0 + 16 * j;
+        if (p >= a.HW || c >= a.pix) return;
+        uint32_t o[4][4];                                                        // [pixel][four channels]
 #pragma unroll
-        for (int k = 0; k < 16; ++k) q[k >> 2] |= (uint32_t)tile[(c + k) * kToNhwcPitch + p] << (8 * (k & 3));
-        *reinterpret_cast<uint4*>(y + (n * HW + p0 + p) * (long long)pix + c0 + c) = make_uint4(q[0], q[1], q[2], q[3]);
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t* t = tile + (16 * j + 4 * q) * 32 + (word ^ (8 * j));
+            const uint32_t v0 = t[0], v1 = t[32], v2 = t[64], v3 = t[96];
+            const uint32_t a0 = __byte_perm(v0, v1, 0x5140), a1 = __byte_perm(v2, v3, 0x5140), a2 = __byte_perm(v0, v1, 0x7362), a3 = __byte_perm(v2, v3, 0x7362);
+            o[0][q] = __byte_perm(a0, a1, 0x5410); o[1][q] = __byte_perm(a0, a1, 0x7632);
+            o[2][q] = __byte_perm(a2, a3, 0x5410); o[3][q] = __byte_perm(a2, a3, 0x7632);
+        }
+        uint8_t* y = a.y + (n * a.HW + p) * (long long)a.pix + c;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (p + k < a.HW) *reinterpret_cast<uint4*>(y + (long long)k * a.pix) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+        return;
     }
+    b -= a.x_blocks;
+    if (b < a.w_blocks) { nh_weight_chunks<int8_t>(a.w, (long long)b * kNhPrepThreads + tid, (long long)a.w_blocks * kNhPrepThreads); return; }
+    b -= a.w_blocks;
+    const int m = (int)b * (kNhPrepThreads / 32) + warp;
+    if (m >= a.bias_n) return;
+    int s = 0;
+    if (m < a.M && a.x_zp != 0) for (int k = lane; k < a.K; k += 32) s += __ldg(a.bw + (size_t)m * a.K + k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) a.bias_out[m] = m < a.M ? (a.bias ? __ldg(a.bias + m) : 0) - a.x_zp * s : 0;
 }
-inline int32_t run_to_nhwc_bytes(zant_ctx* ctx, const void* x, void* y, int N, int C, int HW, int pix) {
-    const dim3 grid((unsigned)((HW + kToNhwcPx - 1) / kToNhwcPx), (unsigned)((pix + kToNhwcCh - 1) / kToNhwcCh), (unsigned)N);
-    launch(ctx, to_nhwc_bytes_k, grid, 256, 0, (const uint8_t*)x, (uint8_t*)y, C, HW, pix, (long long)N * C * HW);
-    return check_launch(ctx, "to_nhwc_bytes_k");
+inline NhPrepArgs nh_prep_input(const void* x, void* y, int N, int C, int HW, int pix) {
+    NhPrepArgs a{};
+    a.x = (const uint8_t*)x; a.y = (uint8_t*)y; a.C = C; a.HW = HW; a.pix = pix; a.bytes = (long long)N * C * HW;
+    a.px_tiles = (HW + 127) / 128; a.ch_tiles = (pix + 63) / 64;
+    a.x_blocks = (unsigned)((long long)N * a.px_tiles * a.ch_tiles);
+    return a;
+}
+inline void nh_prep_weights(zant_ctx* ctx, NhPrepArgs& a, const NhConvPlan& p, const void* w, void* out) {
+    a.w = nh_weight_args(p, w, out);
+    a.w_blocks = (unsigned)grid_for((size_t)a.w.chunks, kNhPrepThreads, ctx->sm_count, 16);
+}
+inline int32_t run_nh_prep(zant_ctx* ctx, const NhPrepArgs& a) {
+    const unsigned blocks = a.x_blocks + a.w_blocks + (unsigned)((a.bias_n + kNhPrepThreads / 32 - 1) / (kNhPrepThreads / 32));
+    if (blocks == 0) return ZANT_OK;
+    launch(ctx, nh_prep_k, blocks, kNhPrepThreads, 0, a);
+    return check_launch(ctx, "nh_prep_k");
 }
 
 // A channels-last tensor in the graph's order, for a caller that asked for its address; split form: hi + lo.
