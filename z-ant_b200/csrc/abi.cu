@@ -94,6 +94,7 @@ int32_t zant_b200_ctx_destroy(zant_ctx* ctx) {
     if (!ctx) return ZANT_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    delete ctx->lane;
     delete ctx->stage;
     if (ctx->arena) cudaFree(ctx->arena);
     if (ctx->status_word) cudaFree(ctx->status_word);
@@ -841,11 +842,13 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const bool bias_dev = bias && is_device_ptr(bias);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+        const int iw = s.in_early(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
         if (s.room()) {
             ZB_TRY(s.commit());
+            ZB_TRY(s.start_early());
             ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            s.end_early();
             ZB_TRY(tc_conv_run(ctx, tcp, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                                s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation},
                                weight_blocks_max_product(mult, bias_dev ? nullptr : bias, !bias_dev, g.M, (long long)g.Cg * g.KH * g.KW)));
@@ -884,14 +887,21 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         if (bias_here && bias) std::memcpy(bp.data(), bias, (size_t)g.M * 4);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = bias_here ? s.in(bp.data(), bp.size() * 4) : s.in(bias, (size_t)g.M * 4);
+        const int iw = s.in_early(w, numel(w_shape, 4)), im = s.in(mp.data(), mp.size() * 4), ib = bias_here ? s.in(bp.data(), bp.size() * 4) : s.in(bias, (size_t)g.M * 4);
         const int ixl = s.scratch((size_t)g.N * hw * pix), iwb = s.scratch(nhp.w_bytes), ibb = s.scratch((size_t)nhp.a.const_n * 4);
         if (s.room()) {
             ZB_TRY(s.commit());
             NhPrepArgs prep = nh_prep_input(s.ptr<char>(ix), s.ptr<char>(ixl), g.N, g.C, hw, pix);
+            if (s.early()) {                                // the input beside the upload of the weights
+                ZB_TRY(run_nh_prep(ctx, prep));
+                prep.x_blocks = 0;
+                --ctx->launches;                            // (one operator launch with the next)
+                ZB_TRY(s.start_early());
+            }
             nh_prep_weights(ctx, prep, nhp, s.ptr<int8_t>(iw), s.ptr<char>(iwb));
             if (!bias_here) { prep.bw = s.ptr<int8_t>(iw); prep.bias = s.ptr<int32_t>(ib); prep.bias_out = s.ptr<int32_t>(ibb); prep.M = g.M; prep.K = K; prep.bias_n = nhp.a.const_n; prep.x_zp = x_zp; }
             ZB_TRY(run_nh_prep(ctx, prep));
+            s.end_early();
             NhConvArgs a = nhp.a;
             a.w = s.ptr<uint8_t>(iwb); a.mult = s.ptr<float>(im); a.bias = s.ptr<int32_t>(bias_here ? ib : ibb);
             a.y = s.ptr<uint8_t>(iy); a.nchw = 1; a.act = activation; a.six = lean_six(y_scale);
@@ -907,12 +917,14 @@ int32_t zant_b200_qlinearconv(zant_ctx* ctx, int32_t x_dtype, const void* x, con
         const WBlockArgs wb = weight_blocks_of(prep, g.M, g.Cg, g.KH * g.KW, x_zp);
         Stager s(ctx);
         const int ix = s.in(x, numel(x_shape, 4)), iy = s.out(y, numel(y_shape, 4));
-        const int iw = s.in(w, numel(w_shape, 4)), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
+        const int iw = s.in_early(w, numel(w_shape, 4)), im = s.in(prep.mult.data(), prep.mult.size() * 4), ib = s.in(bias, (size_t)g.M * 4);
         const int ia = s.scratch(qgemm_a_bytes((size_t)g.N * g.OH * g.OW, prep));
         const int iwb = s.scratch(weight_blocks_bytes(wb)), ibb = s.scratch(weight_blocks_bias(wb) * 4);
         if (s.room()) {
             ZB_TRY(s.commit());
+            ZB_TRY(s.start_early());
             ZB_TRY(run_weight_blocks(ctx, wb, s.ptr<int8_t>(iw), s.ptr<int32_t>(ib), s.ptr<int8_t>(iwb), s.ptr<int32_t>(ibb)));
+            s.end_early();
             ZB_TRY(run_qconv_tc(ctx, g, s.ptr<char>(ix), x_dtype == ZANT_U8, x_zp, prep, s.ptr<int8_t>(iwb), s.ptr<float>(im), s.ptr<int32_t>(ibb),
                                 s.ptr<uint8_t>(ia), s.ptr<char>(iy), y_dtype == ZANT_U8, Requant{y_scale, y_zp, activation}));
             return s.finish();

@@ -62,14 +62,10 @@ class HostStage {
     // dst (device) <- src (pageable host), ordered on the stream; src is free again when this returns.
     cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
         if (bytes <= kSlot / 4) {
-            if (used_ + bytes > kSlot) { cudaError_t e = next_slot(stream); if (e != cudaSuccess) return e; }
-            char* p = slot(cur_) + used_;
-            stream_copy(p, (const char*)src, bytes);
-            used_ += (bytes + 255) / 256 * 256;
-            dirty_ = true; idle_ = false;
-            return cudaMemcpyAsync(dst, p, bytes, cudaMemcpyHostToDevice, stream);
+            const Part one{src, bytes, 0};
+            return to_device(dst, &one, 1, bytes, stream);
         }
-        cudaError_t e = next_slot(stream);                         // pieces own whole slots, from cur_ on
+        cudaError_t e = next_slot();                               // pieces own whole slots, from cur_ on
         if (e != cudaSuccess) return e;
         int pieces = bytes > kSlot ? (int)((bytes + kSlot - 1) / kSlot) + 3 : 1;
         while (piece_begin(pieces) < bytes) ++pieces;
@@ -116,13 +112,25 @@ class HostStage {
         return e;
     }
 
+    // Several small buffers whose places on the device lie within `span` bytes (at most a quarter of a slot): one copy, which also carries the gaps.
+    struct Part { const void* src; size_t bytes, off; };
+    cudaError_t to_device(void* dst, const Part* parts, size_t n, size_t span, cudaStream_t stream) {
+        if (used_ + span > kSlot || (used_ > 0 && stream != stream_)) { cudaError_t e = next_slot(); if (e != cudaSuccess) return e; }
+        char* p = slot(cur_) + used_;
+        stream_ = stream;
+        for (size_t i = 0; i < n; ++i) stream_copy(p + parts[i].off, (const char*)parts[i].src, parts[i].bytes);
+        used_ += (span + 255) / 256 * 256;
+        dirty_ = true; idle_ = false;
+        return cudaMemcpyAsync(dst, p, span, cudaMemcpyHostToDevice, stream);
+    }
+
     // The stream has been drained: every slot is free.
     void drained() { idle_ = true; used_ = 0; dirty_ = false; }
 
     // Page-locked room for a result of at most a slot; valid until the next transfer of this context.
     void* result_slot(size_t bytes, cudaStream_t stream) {
         if (bytes > kSlot) return nullptr;
-        if (used_ + bytes > kSlot && next_slot(stream) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if ((used_ + bytes > kSlot || (used_ > 0 && stream != stream_)) && next_slot() != cudaSuccess) { cudaGetLastError(); return nullptr; }
         return slot(cur_) + used_;
     }
 
@@ -157,10 +165,10 @@ class HostStage {
         std::this_thread::yield();
 #endif
     }
-    // closes the current slot (its event marks its last DMA) and waits until the next one is free
-    cudaError_t next_slot(cudaStream_t stream) {
+    // closes the current slot (its event marks its last DMA, on the stream that its small copies share) and waits until the next one is free
+    cudaError_t next_slot() {
         if (!dirty_ && used_ == 0) return cudaSuccess;
-        cudaError_t e = cudaEventRecord(ev_[cur_], stream);
+        cudaError_t e = cudaEventRecord(ev_[cur_], stream_);
         if (e != cudaSuccess) return e;
         cur_ = (cur_ + 1) % kSlots;
         used_ = 0; dirty_ = false;
@@ -214,6 +222,7 @@ class HostStage {
     cudaEvent_t ev_[kSlots] = {};
     int cur_ = 0;
     size_t used_ = 0;
+    cudaStream_t stream_ = nullptr;     // of the current slot's small copies
     bool dirty_ = false;
     bool idle_ = true;         // no DMA of this ring is in flight
     bool started_ = false;
