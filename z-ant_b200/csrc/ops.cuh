@@ -44,9 +44,30 @@ inline double contract_cost(const ContractTime& t, double tiles_per_sm, double k
     const double ns = tiles_per_sm <= 3.0 ? t.lone + t.per * tiles_per_sm : t.base + t.slope * tiles_per_sm;
     return ns * k + 25.0 * t.slope * tiles_per_sm;
 }
+// A first layer with its pool in contract_f32.cuh's kernel for it: at any size (1 image of 28 x 28 6.3 -> 4.2 us).  All filters in a thread, or as few as
+// it takes for three CTAs an SM (256 images: 32 filters a thread 10.4 us, 16 8.3; 16 images: 32 6.3, 8 4.4).
+inline bool conv_lowc_takes(const ContractArgs& p) {
+    const ConvGeom& g = p.g;
+    return g.KH == 3 && g.KW == 3 && g.sh == 1 && g.sw == 1 && g.dh == 1 && g.dw == 1 && g.C <= 3 && p.N <= kLowCMaxFilters && (long long)g.C * g.H * g.W < 0x7fffffffLL;
+}
+inline int32_t launch_conv_lowc(zant_ctx* ctx, const ContractArgs& p) {
+    const unsigned gx = ((unsigned)(p.M / 4) + kLowCThreads - 1) / kLowCThreads;
+    int per = (p.N + 7) / 8 * 8;
+    while (per > 8 && (long long)gx * ((p.N + per - 1) / per) < 3LL * ctx->sm_count) per = (per / 2 + 7) / 8 * 8;
+    const dim3 grid(gx, (unsigned)((p.N + per - 1) / per));
+    const size_t smem = (size_t)(p.g.C * 9 + 1) * per * 4;
+    switch (p.g.C) {
+        case 1: launch(ctx, conv3x3_pool_f32_lowc<1>, grid, kLowCThreads, smem, p, per); break;
+        case 2: launch(ctx, conv3x3_pool_f32_lowc<2>, grid, kLowCThreads, smem, p, per); break;
+        default: launch(ctx, conv3x3_pool_f32_lowc<3>, grid, kLowCThreads, smem, p, per); break;
+    }
+    return check_launch(ctx, "conv3x3_pool_f32_lowc");
+}
+
 template <bool CONV, bool POOL>
 inline int32_t launch_contract(zant_ctx* ctx, ContractArgs& p) {
     p.neg_zero = 0x8000000080000000ull;
+    if constexpr (CONV && POOL) if (conv_lowc_takes(p)) return launch_conv_lowc(ctx, p);
     static const int shapes[6][2] = {{128, 128}, {128, 64}, {128, 32}, {128, 16}, {32, 32}, {CF_BM, CF_BN}};
     static const ContractTime times[3][6] = {
         {{0, 204, 50, 195}, {45, 87, 40, 92}, {95, 36, 130, 46}, {72, 23, 90, 31}, {52, 9, 55, 17.5}, {0, 33, 30, 26}},        // B runs along k (a convolution's weights as the tensor has them, a transposed matrix)
