@@ -86,6 +86,18 @@ inline void launch_const(zant_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 bl
     else kernel<<<grid, block, smem, ctx->stream>>>(std::forward<A>(args)...);
 }
 
+// The same in clusters of `n` CTAs (1: none).
+template <typename... P, typename... A>
+inline void launch_cluster(zant_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned n, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension; attr[1].val.clusterDim.x = n; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = n > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 inline int32_t check_launch(zant_ctx* ctx, const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ZANT_E_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));

@@ -543,13 +543,7 @@ template <int S, bool ADD, bool CLUSTER>
 inline int32_t irb_band_launch(zant_ctx* ctx, const IrbBandPlan& q, const IrbBandArgs& a, const QAddTail& add) {
     auto kernel = irb_band_kernel<S, ADD, CLUSTER>;
     ZB_SMEM_ATTR(ctx, kernel, 227 * 1024);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = (unsigned)(a.N * a.bands * a.cs); cfg.blockDim = (unsigned)q.threads; cfg.dynamicSmemBytes = q.smem_bytes; cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[2]{};
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension; attr[1].val.clusterDim.x = (unsigned)a.cs; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = CLUSTER ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, kernel, a, add);
+    launch_cluster(ctx, kernel, (unsigned)(a.N * a.bands * a.cs), (unsigned)q.threads, q.smem_bytes, CLUSTER ? (unsigned)a.cs : 1u, a, add);
     return check_launch(ctx, "irb_band_kernel");
 }
 

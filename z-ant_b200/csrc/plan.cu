@@ -28,6 +28,7 @@
 #include "tc_gemm_tf32.cuh"
 #include "small_gemm_q8.cuh"
 #include "tc_nhwc_net.cuh"
+#include "fused_cnn_few.cuh"
 #include "irb_band.cuh"
 #include "irb_q8.cuh"
 #include "status.hpp"
@@ -1731,6 +1732,14 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         }
         tc_conv_pool_weights(w, w2arr.data());
     }
+    bool acc_base = true;
+    for (int m = 0; m < 32; ++m) acc_base = acc_base && acc_base_ok(a1.bias[m]);
+    // Few images: one kernel, a cluster for as few of them as fill the clusters that run at once, up to two rounds of sixteen a cluster (480 images 20.3
+    // us in four kernels, 19.8 in one; 512, three rounds, 20.3 and 27.3).
+    const int few_clusters = irb_band_resident(1, CnnFewCfg::CTAS, pl->ctx->sm_count);
+    int few_imgs = 1;
+    while (few_imgs < CnnFewCfg::IMGS && (size_t)few_imgs * few_clusters < B) few_imgs *= 2;
+    const bool few = acc_base && acc_base2 && B <= (size_t)2 * CnnFewCfg::IMGS * few_clusters;
     // ---- fc1: rows re-ordered from the graph's (c,h,w) flatten order to the (h,w,c) order stage 2 writes
     std::vector<float> m3; std::vector<int32_t> b3;
     if (!scales_of(f1, 512, m3) || !bias_of(f1, 512, b3)) return ZANT_OK;
@@ -1760,7 +1769,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
             for (int n = 0; n < 512; ++n) colsum[n] += part[n];
         }
         // 16 channels of a position are a K chunk: 16 rows of the matrix, transposed
-        for (int hw = 0; hw < 25; ++hw)
+        for (int hw = 0; hw < 25 && !few; ++hw)
             for (int c16 = 0; c16 < 4; ++c16) {
                 const int8_t* src = &w[(size_t)(c16 * 16 * 25 + hw) * 512];
                 for (int n = 0; n < 512; ++n) {
@@ -1781,20 +1790,12 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         }
     }
 
-    // stage 1 -> stage 2 hand-over: image blocks
-    const int s_pool1 = pl->add_scratch(blocks128 * (size_t)c2_block_bytes(ib));
-    const int s_pool2 = pl->add_scratch((size_t)blocks128 * ib * 1600);
-    const int s_fc1 = pl->add_scratch(B * 512);
-    const int a_w2 = pl->add_aux(w2arr.data(), w2arr.size());
-    const int a_w3 = pl->add_aux(w3blk.data(), w3blk.size());
     const int a_m3 = pl->add_aux(m3.data(), m3.size() * 4), a_b3 = pl->add_aux(b3.data(), b3.size() * 4);
     const int a_m4 = pl->add_aux(m4.data(), m4.size() * 4), a_b4 = pl->add_aux(b4.data(), b4.size() * 4);
     const int w4 = f2.in[1];
 
     // B-fragment words, bias and multipliers in the per-lane order of the warp-level MMA
     std::vector<uint32_t> wfrag(4 * 4 * 32);
-    bool acc_base = true;
-    for (int m = 0; m < 32; ++m) acc_base = acc_base && acc_base_ok(a1.bias[m]);
     std::vector<float> floorfrag(4 * 32 * 2), multfrag(4 * 32 * 2);
     {
         const int8_t* w = (const int8_t*)T(c1.in[1]).host.data();   // [32][1][3][3]
@@ -1824,6 +1825,50 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     const int a_wf = pl->add_aux(wfrag.data(), wfrag.size() * 4);
     const int a_bf = pl->add_aux(floorfrag.data(), floorfrag.size() * 4);
     const int a_mf = pl->add_aux(multfrag.data(), multfrag.size() * 4);
+    for (int k = 0; k < 11; ++k) pl->t[N[k].out[0]].elided = true;   // interior tensors live only inside the fused kernels
+    consumed = 12;
+    // algorithmic work of the fused steps: tensors that cross a kernel boundary once at their storage type,
+    // weights included; of the 13 x 13 pooled pixels of stage 1 only the 12 x 12 that stage 2's pool reads exist
+    const double Bd = (double)B, nc = (double)NCLS;
+    auto costs = [&](std::initializer_list<double> macs, std::initializer_list<double> bytes) {
+        pl->step_macs.resize(pl->steps.size() - macs.size(), 0.0); pl->step_bytes.resize(pl->steps.size() - bytes.size(), 0.0);
+        pl->step_macs.insert(pl->step_macs.end(), macs); pl->step_bytes.insert(pl->step_bytes.end(), bytes);
+    };
+    if (few) {
+        std::vector<uint8_t> blob;
+        cnn_few_weights((const int8_t*)T(c2.in[1]).host.data(), (const int8_t*)T(f1.in[1]).host.data(), (const int8_t*)T(f2.in[1]).host.data(), (int)NCLS, blob);
+        std::vector<float> floor2(64);
+        for (int m = 0; m < 64; ++m) floor2[m] = kAccBase - (float)b2[m];
+        const int a_blob = pl->add_aux(blob.data(), blob.size()), a_f2 = pl->add_aux(floor2.data(), 256), a_m2 = pl->add_aux(m2.data(), 256);
+        CnnFewArgs k{};
+        k.n_images = (int)B; k.imgs = few_imgs;
+        k.x_scale = a1.x_scale; k.x_zp = a1.x_zp; k.q_rh = steps.rh; k.q_rl = steps.rl;
+        k.ncls = (int)NCLS; k.y_scale = f2.a.y_scale; k.y_zp = f2.a.y_zp; k.dq_scale = N[11].a.x_scale; k.dq_zp = N[11].a.x_zp;
+        push("Fused[QuantizeLinear+(QLinearConv+Relu+MaxPool)x2+QLinearMatMul+Relu+QLinearMatMul+DequantizeLinear] mma", [=]() {
+            using Cfg = CnnFewCfg;
+            CnnFewArgs a = k;
+            a.x = pl->p<float>(x); a.y = pl->p<float>(y); a.status = ctx->status_word;
+            a.wfrag = (const uint32_t*)pl->aux(a_wf); a.floor1 = (const float*)pl->aux(a_bf); a.mult1 = (const float*)pl->aux(a_mf);
+            a.w = (const uint8_t*)pl->aux(a_blob); a.floor2 = (const float*)pl->aux(a_f2); a.mult2 = (const float*)pl->aux(a_m2);
+            a.mult3 = (const float*)pl->aux(a_m3); a.bias3 = (const int32_t*)pl->aux(a_b3); a.mult4 = (const float*)pl->aux(a_m4); a.bias4 = (const int32_t*)pl->aux(a_b4);
+            const unsigned grid = (unsigned)((k.n_images + k.imgs - 1) / k.imgs * Cfg::CTAS);
+            auto go = [&](auto two) -> int32_t {
+                ZB_SMEM_ATTR(ctx, (cnn_few_kernel<decltype(two)::value>), Cfg::SMEM_BYTES);
+                launch_cluster(ctx, cnn_few_kernel<decltype(two)::value>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, Cfg::CTAS, a);
+                return ZANT_OK;
+            };
+            ZB_TRY(k.imgs > Cfg::CTAS ? go(std::true_type{}) : go(std::false_type{}));
+            return check_launch(ctx, "cnn_few_kernel");
+        });
+        costs({Bd * (194688.0 + 2230272.0 + 819200.0 + 512.0 * nc)}, {Bd * (784.0 * 4 + 4.0 * nc) + 288.0 + 64.0 * 288 + 1600.0 * 512 + 512.0 * nc});
+        return ZANT_OK;
+    }
+    // stage 1 -> stage 2 hand-over: image blocks
+    const int s_pool1 = pl->add_scratch(blocks128 * (size_t)c2_block_bytes(ib));
+    const int s_pool2 = pl->add_scratch((size_t)blocks128 * ib * 1600);
+    const int s_fc1 = pl->add_scratch(B * 512);
+    const int a_w2 = pl->add_aux(w2arr.data(), w2arr.size());
+    const int a_w3 = pl->add_aux(w3blk.data(), w3blk.size());
     push("Fused[QuantizeLinear+QLinearConv+Relu+MaxPool] mma", [=]() {
         Conv1MmaArgs k{};
         k.x = pl->p<float>(x); k.y = (int8_t*)pl->scratch(s_pool1); k.n_images = (int)B; k.ib = ib;
@@ -1886,18 +1931,8 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
         };
         return NCLS <= 8 ? with(std::integral_constant<int, 8>{}) : with(std::integral_constant<int, 16>{});
     });
-    for (int k = 0; k < 11; ++k) pl->t[N[k].out[0]].elided = true;   // interior tensors live only inside the fused kernels
-    consumed = 12;
-    {
-        // algorithmic work of the four fused steps: tensors that cross a kernel boundary once at their storage type,
-        // weights included; of the 13 x 13 pooled pixels of stage 1 only the 12 x 12 that stage 2's pool reads exist
-        const double Bd = (double)B, nc = (double)NCLS;
-        const double macs[4] = {Bd * 194688.0, Bd * 2230272.0, Bd * 819200.0, Bd * 512.0 * nc};
-        const double bytes[4] = {Bd * (784.0 * 4 + 144.0 * 32) + 288.0, Bd * (144.0 * 32 + 1600.0) + 64.0 * 288, Bd * (1600.0 + 512.0) + 1600.0 * 512,
-                                 Bd * (512.0 + 4.0 * nc) + 512.0 * nc};
-        pl->step_macs.resize(pl->steps.size(), 0.0); pl->step_bytes.resize(pl->steps.size(), 0.0);
-        for (int k = 0; k < 4; ++k) { pl->step_macs[pl->steps.size() - 4 + k] = macs[k]; pl->step_bytes[pl->steps.size() - 4 + k] = bytes[k]; }
-    }
+    costs({Bd * 194688.0, Bd * 2230272.0, Bd * 819200.0, Bd * 512.0 * nc},
+          {Bd * (784.0 * 4 + 144.0 * 32) + 288.0, Bd * (144.0 * 32 + 1600.0) + 64.0 * 288, Bd * (1600.0 + 512.0) + 1600.0 * 512, Bd * (512.0 + 4.0 * nc) + 512.0 * nc});
     return ZANT_OK;
 }
 
