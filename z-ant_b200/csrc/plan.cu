@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstring>
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <functional>
 #include <memory>
@@ -28,6 +29,7 @@
 #include "tc_gemm_tf32.cuh"
 #include "small_gemm_q8.cuh"
 #include "tc_nhwc_net.cuh"
+#include "first_layer_q8.cuh"
 #include "fused_cnn_few.cuh"
 #include "irb_band.cuh"
 #include "irb_q8.cuh"
@@ -70,6 +72,7 @@ struct NhGroup {
     int fact = 0; float slope = 0.0f;    // TF32
     bool pool = false, up2 = false;
     int dequant = -1;                    // DequantizeLinear node
+    int quant = -1;                      // QuantizeLinear node in front of it that the same kernel takes (first_layer_q8.cuh)
     bool on = false;                     // the layout pass took it
 };
 
@@ -2158,7 +2161,18 @@ static void nh_layout(zant_plan* pl) {
             o += t.shape[1] * dtype_size(t.dtype);
         }
     }
-    for (NhGroup& q : pl->nh_groups) if (q.on) for (int id : q.interior) T(id).elided = true;
+    for (NhGroup& q : pl->nh_groups) {
+        if (!q.on) continue;
+        for (int id : q.interior) T(id).elided = true;
+        // a first layer that a QuantizeLinear feeds alone quantises its own input
+        const PlanNode& n = pl->nodes[q.first];
+        ConvGeom g;
+        if (q.first == 0 || !q.pool || q.up2 || !T(q.y).nh || !T(q.x).nh || !only_feeds_next(c, q.x) || !nh_conv_geom(pl, n, g) || !first_q8_takes(g, pl->ctx->sm_count)) continue;
+        const PlanNode& ql = pl->nodes[q.first - 1];
+        if (ql.op != ZANT_OP_QUANTIZE_LINEAR || ql.in.size() != 1 || ql.out.size() != 1 || ql.out[0] != q.x) continue;
+        q.quant = (int)q.first - 1;
+        T(q.x).nh = false; T(q.x).elided = true;
+    }
 }
 
 static NhView nh_view(zant_plan* pl, int id) {
@@ -2172,6 +2186,70 @@ static int32_t refresh_nchw_copy(zant_plan* pl, int id, char* y) {
     const int32_t st = run_from_nhwc(pl->ctx, nh_view(pl, id), y, t.shape[0], t.shape[1], dtype_size(t.dtype));
     pl->ctx->launches = launched;                    // (not an operator launch)
     return st;
+}
+
+// Multipliers and biases (-x_zp * sum of the filter folded in) of `pad` filters: their numbers in the plan.
+static void nh_int8_constants(zant_plan* pl, const NhGroup& q, const ConvGeom& g, size_t pad, int& am, int& ab) {
+    const PlanNode& n = pl->nodes[q.first];
+    auto T = [&](int id) -> const PlanTensor& { return pl->t[id]; };
+    std::vector<float> mp; std::vector<int32_t> bp(pad, 0);
+    const PlanTensor& ws = T(n.in[2]);
+    const int b = opt_in(n, 4);
+    requant_multipliers(n.a.x_scale, (const float*)ws.host.data(), ws.bytes / 4, n.a.y_scale, (size_t)g.M, mp);
+    mp.resize(pad, 1.0f);
+    const int K = g.Cg * g.KH * g.KW;
+    for (int m = 0; m < g.M; ++m) {
+        int sum = 0;
+        if (n.a.x_zp != 0) for (int k = 0; k < K; ++k) sum += ((const int8_t*)T(n.in[1]).host.data())[(size_t)m * K + k];
+        bp[m] = (b >= 0 ? ((const int32_t*)T(b).host.data())[m] : 0) - n.a.x_zp * sum;
+    }
+    am = pl->add_aux(mp.data(), mp.size() * 4); ab = pl->add_aux(bp.data(), bp.size() * 4);
+}
+
+// A group with its QuantizeLinear, whose nodes the caller has checked.
+static int32_t build_first_layer(zant_plan* pl, const NhGroup& q, size_t& consumed) {
+    const PlanNode &ql = pl->nodes[q.quant], &n = pl->nodes[q.first];
+    zant_ctx* ctx = pl->ctx;
+    const size_t first_step = pl->steps.size();
+    ConvGeom g;
+    if (!nh_conv_geom(pl, n, g)) return fail(ZANT_E_INVALID_DIMENSIONS, "convolution geometry");
+    FirstQ8Args base{};
+    const int x = ql.in[0], y = q.y;
+    const bool u8 = pl->t[q.x].dtype == ZANT_U8;
+    base.zp = ql.a.y_zp;
+    base.qf = quant_fast(ql.a.y_scale, (float)((u8 ? 0 : -128) - base.zp), (float)((u8 ? 255 : 127) - base.zp));
+    if (!quant_steps(ql.a.y_scale, (u8 ? 0 : -128) - base.zp, (u8 ? 255 : 127) - base.zp, base.qs)) base.qs = QuantSteps{0.0f, 0.0f};
+    const int act = q.qact >= 0 ? q.qact : n.a.activation;
+    base.floor = act == ZANT_QACT_NONE ? INT_MIN : 0;
+    std::vector<uint8_t> table;                              // behind the ReLU: the bound of a ReLU6, the activation's table
+    const int six = lean_six(n.a.y_scale);
+    if (act == ZANT_QACT_RELU6 || q.lut_node >= 0) {
+        table.resize(256);
+        uint8_t lut[256];
+        if (q.lut_node >= 0) activation_lut(pl->nodes[q.lut_node], ZANT_I8, lut);
+        for (int v = 0; v < 256; ++v) {
+            const uint8_t code = (uint8_t)(act == ZANT_QACT_RELU6 ? std::min(v, six & 255) : v);
+            table[v] = q.lut_node >= 0 ? lut[code] : code;
+        }
+    }
+    const int alut = table.empty() ? -1 : pl->add_aux(table.data(), table.size());
+    std::vector<uint32_t> wfrag;
+    first_q8_weights(g, (const int8_t*)pl->t[n.in[1]].host.data(), wfrag);
+    const int aw = pl->add_aux(wfrag.data(), wfrag.size() * 4);
+    int am, ab;
+    nh_int8_constants(pl, q, g, (size_t)g.M, am, ab);
+    pl->steps.push_back([=]() {
+        FirstQ8Args a = base;
+        const NhView v = nh_view(pl, y);
+        a.x = pl->p<float>(x); a.wfrag = (const uint32_t*)pl->aux(aw); a.mult = (const float*)pl->aux(am); a.bias = (const int32_t*)pl->aux(ab);
+        a.lut = alut >= 0 ? (const uint8_t*)pl->aux(alut) : nullptr;
+        a.y = (uint8_t*)v.ptr; a.y_pix = v.pix; a.y_row = v.pix * v.W; a.y_img = a.y_row * v.H;
+        return first_q8_run(ctx, g, u8, a);
+    });
+    pl->step_names.push_back(std::string("Fused[QuantizeLinear+QLinearConv") + (q.qact >= 0 ? "+Relu" : "") + (q.lut_node >= 0 ? "+ActivationLut" : "") + "+MaxPool]");
+    record_step_cost(pl, first_step, (size_t)q.quant, q.count + 1);
+    consumed = q.count + 1;
+    return ZANT_OK;
 }
 
 static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
@@ -2191,11 +2269,14 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
         consumed = 1;
         return ZANT_OK;
     }
-    if (n.op == ZANT_OP_QUANTIZE_LINEAR && n.out.size() == 1 && T(n.out[0]).nh) {
+    const NhGroup* found = nullptr;
+    for (const NhGroup& q : pl->nh_groups) if (q.on && (q.quant >= 0 ? (size_t)q.quant : q.first) == i) found = &q;
+    if (n.op == ZANT_OP_QUANTIZE_LINEAR && n.out.size() == 1 && (T(n.out[0]).nh || found)) {
         ZB_TRY(need_inputs(n, 1, 1, "QuantizeLinear"));
         const int x = n.in[0], y = n.out[0];
         ZB_TRY(want_dtype(pl, x, ZANT_F32, "QuantizeLinear"));
         if (T(x).bytes != T(y).bytes * 4) return fail(ZANT_E_OUTPUT_TENSOR_DIFFERENT_SIZE, "QuantizeLinear sizes differ");
+        if (found) return build_first_layer(pl, *found, consumed);
         const int N = (int)T(y).shape[0], C = (int)T(y).shape[1];
         const long long hw = (long long)(T(y).shape[2] * T(y).shape[3]);
         const float sc = n.a.y_scale; const int zp = n.a.y_zp; const bool u8 = T(y).dtype == ZANT_U8;
@@ -2220,8 +2301,6 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
         consumed = 1;
         return ZANT_OK;
     }
-    const NhGroup* found = nullptr;
-    for (const NhGroup& q : pl->nh_groups) if (q.on && q.first == i) found = &q;
     if (!found) return ZANT_OK;
     const NhGroup q = *found;
     ConvGeom g;
@@ -2242,18 +2321,7 @@ static int32_t build_nh(zant_plan* pl, size_t i, size_t& consumed) {
     int am = -1, ab = -1, alut = -1;
     std::string name;
     if (i8) {
-        std::vector<float> mp; std::vector<int32_t> bp((size_t)base.const_n, 0);
-        const PlanTensor& ws = T(n.in[2]);
-        const int b = opt_in(n, 4);
-        requant_multipliers(n.a.x_scale, (const float*)ws.host.data(), ws.bytes / 4, n.a.y_scale, (size_t)g.M, mp);
-        mp.resize((size_t)base.const_n, 1.0f);
-        const int K = g.Cg * g.KH * g.KW;
-        for (int m = 0; m < g.M; ++m) {
-            int sum = 0;
-            if (n.a.x_zp != 0) for (int k = 0; k < K; ++k) sum += ((const int8_t*)T(n.in[1]).host.data())[(size_t)m * K + k];
-            bp[m] = (b >= 0 ? ((const int32_t*)T(b).host.data())[m] : 0) - n.a.x_zp * sum;
-        }
-        am = pl->add_aux(mp.data(), mp.size() * 4); ab = pl->add_aux(bp.data(), bp.size() * 4);
+        nh_int8_constants(pl, q, g, (size_t)base.const_n, am, ab);
         base.act = q.qact >= 0 ? q.qact : n.a.activation;
         base.six = lean_six(n.a.y_scale);
         name = "QLinearConv(tc-implicit)";
