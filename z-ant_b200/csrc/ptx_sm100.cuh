@@ -24,6 +24,15 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// 32 bytes to an address that is a multiple of 32.  Lanes that write to lines of their own cost the load-store unit a clock each per instruction,
+// whatever its width.
+__device__ __forceinline__ void st_global_v8(void* p, const float* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
 // ---------------------------------------------------------------------------- programmatic dependent launch
 // A kernel launched behind another one on its stream may start while that one drains.  grid_trigger: the next kernel may be
 // scheduled as soon as every CTA of this one has come here; grid_wait: returns when the kernels before this one are complete

@@ -82,6 +82,7 @@ struct NhConvArgs {
     int nchw;                     // 1: y is [N][M][GH][GW] codes or floats, 2: dequantised floats
     int up2;                      // channels-last: every pixel goes to a 2x2 block
     int act, six;                 // int8: zant_qact; TF32: FAct
+    int wide;                     // the epilogue stores 32 channels of a pixel at a time (int8, channels-last, no pool)
     float slope, dq_scale; int dq_zp;
     int lo_out;                   // split form: channel offset of the lo half in the output
     int round_out;                // TF32: the output feeds convolutions: rounded, split form: hi and lo
@@ -369,7 +370,11 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
         const int oh_l = row_i / a.PW, ow_l = row_i - oh_l * a.PW;
         const bool row_live = oh_l < a.BH && ow_l < a.BW && img_l < a.IB;
         const uint32_t hi4 = a.act == ZANT_QACT_RELU6 ? 0x01010101u * (uint32_t)(a.six & 255) : 0x7f7f7f7fu;
-        const int per_blk = NT / CH, chunks = a.RB * per_blk;
+        // int8 without a pool: two chunks of 16 filters at a time, one store of 32 bytes a pixel, where the four warps of a quarter still have as much to do
+        // each and the stores are aligned.  A lane's pixel is a line of its own, so a store takes the load-store unit 32 clocks at either width: for the
+        // chunks of sixteen warps 1545 clocks with two stores and 1233 with one
+        const int halves = I8 && !POOLED && a.wide ? 2 : 1;
+        const int per_blk = NT / CH / halves, chunks = a.RB * per_blk;
         int tile_it = 0;
         NhTile T = nh_first(a);
         const int rb0 = part / per_blk, hc0 = part - rb0 * per_blk;
@@ -387,33 +392,42 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                 const int g0 = h0 + rb * a.BH, gh = g0 + oh_l;
                 const int img = POOLED ? T.img : T.img * a.IB + img_l;
                 const bool live = row_live && gh < a.GH && gw < a.GW && (POOLED || img < a.imgs);
-                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((b * a.RB + rb) * SETS * NT + h * CH);
-                const int c0 = T.nt * NT + h * CH;
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((b * a.RB + rb) * SETS * NT + h * halves * CH);
+                const int c0 = T.nt * NT + h * halves * CH;
                 h += 4;
                 while (h >= per_blk) { h -= per_blk; ++rb; }
                 if (c0 < a.M && g0 < a.GH) {              // (filter padding, row blocks below the image)
                     __syncwarp();                                          // (the lanes without a pixel skip the stores below)
                     uint32_t v[SETS][CH];
+                    if (!I8) {
 #pragma unroll
-                    for (int m = 0; m < SETS; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * NT), v[m]);
-                    ptx::tmem_wait_ld();
+                        for (int m = 0; m < SETS; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * NT), v[m]);
+                        ptx::tmem_wait_ld();
+                    }
                     uint8_t* yp = a.nchw ? a.y : a.y + (long long)img * a.y_img + (long long)gh * (a.up2 ? 2 : 1) * a.y_row + (long long)gw * (a.up2 ? 2 : 1) * a.y_pix;
                     if constexpr (I8) {
-                        uint32_t wd[CH / 4];
+                        uint32_t wd[2 * CH / 4];
 #pragma unroll
-                        for (int j4 = 0; j4 < CH / 4; ++j4) {
-                            const float4 m4 = *reinterpret_cast<const float4*>(sMult + c0 + j4 * 4);
-                            const int4 b4 = *reinterpret_cast<const int4*>(sBias + c0 + j4 * 4);
-                            int s[4];
+                        for (int hf = 0; hf < (POOLED ? 1 : 2); ++hf) {
+                            if (hf == halves) break;
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                s[j] = (int)v[0][j4 * 4 + j];
-                                if (POOLED) s[j] = max(__vimax3_s32(s[j], (int)v[SETS > 1 ? 1 : 0][j4 * 4 + j], (int)v[SETS > 2 ? 2 : 0][j4 * 4 + j]), (int)v[SETS > 3 ? 3 : 0][j4 * 4 + j]);
+                            for (int m = 0; m < SETS; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * NT + hf * CH), v[m]);
+                            ptx::tmem_wait_ld();
+#pragma unroll
+                            for (int j4 = 0; j4 < CH / 4; ++j4) {
+                                const float4 m4 = *reinterpret_cast<const float4*>(sMult + c0 + hf * CH + j4 * 4);
+                                const int4 b4 = *reinterpret_cast<const int4*>(sBias + c0 + hf * CH + j4 * 4);
+                                int s[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    s[j] = (int)v[0][j4 * 4 + j];
+                                    if (POOLED) s[j] = max(__vimax3_s32(s[j], (int)v[SETS > 1 ? 1 : 0][j4 * 4 + j], (int)v[SETS > 2 ? 2 : 0][j4 * 4 + j]), (int)v[SETS > 3 ? 3 : 0][j4 * 4 + j]);
+                                }
+                                uint32_t pk = pack_act_s8x4(rq_round(s[0] + b4.x, m4.x), rq_round(s[1] + b4.y, m4.y), rq_round(s[2] + b4.z, m4.z), rq_round(s[3] + b4.w, m4.w),
+                                                            a.act != ZANT_QACT_NONE, hi4);
+                                if (a.lut) pk = lut4_smem(sLut, pk);
+                                wd[hf * (CH / 4) + j4] = pk;
                             }
-                            uint32_t pk = pack_act_s8x4(rq_round(s[0] + b4.x, m4.x), rq_round(s[1] + b4.y, m4.y), rq_round(s[2] + b4.z, m4.z), rq_round(s[3] + b4.w, m4.w),
-                                                        a.act != ZANT_QACT_NONE, hi4);
-                            if (a.lut) pk = lut4_smem(sLut, pk);
-                            wd[j4] = pk;
                         }
                         if (!live) continue;
                         if (a.nchw) {
@@ -430,7 +444,8 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                             for (int u = 0; u < 4; ++u) {
                                 if (u && !a.up2) break;
                                 uint8_t* yc = yp + (u >> 1) * a.y_row + (u & 1) * a.y_pix + c0;
-                                *reinterpret_cast<uint4*>(yc) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+                                if (halves == 2) ptx::st_global_v8(yc, wd);
+                                else *reinterpret_cast<uint4*>(yc) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
                             }
                         }
                     } else {
@@ -471,9 +486,9 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                                 if (u && !a.up2) break;
                                 uint8_t* yc = yp + (u >> 1) * a.y_row + (u & 1) * a.y_pix + (long long)c0 * 4;
 #pragma unroll
-                                for (int j = 0; j < CH; j += 4) {
-                                    *reinterpret_cast<float4*>(yc + j * 4) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-                                    if (KIND == NH_TF32X3 && a.round_out) *reinterpret_cast<float4*>(yc + (long long)a.lo_out * 4 + j * 4) = make_float4(lo[j], lo[j + 1], lo[j + 2], lo[j + 3]);
+                                for (int j = 0; j < CH; j += 8) {
+                                    ptx::st_global_v8(yc + j * 4, r + j);
+                                    if (KIND == NH_TF32X3 && a.round_out) ptx::st_global_v8(yc + (long long)a.lo_out * 4 + j * 4, lo + j);
                                 }
                             }
                         }
@@ -793,6 +808,7 @@ inline int32_t nh_conv_run(zant_ctx* ctx, const NhConvPlan& p, NhConvArgs a, con
         const int pr = p.pool == NH_STRIDE2 || p.half ? 1 - (pp >> 1) : pp >> 1, pc = p.pool == NH_STRIDE2 || p.half ? 1 - (pp & 1) : pp & 1;
         ZB_TRY(nh_encode_map(a.imgs, a.IB, x, a.parts > 1 ? x.lo + p.cin : p.cin, esz, a.KC, a.PW, a.PH, p.pool != 0 || p.half, pr, pc, &maps.m[pp]));
     }
+    a.wide = !a.nchw && a.M % 32 == 0 && a.NT % 32 == 0 && a.RB * a.NT % 128 == 0 && ((uintptr_t)a.y & 31) == 0 && a.y_pix % 32 == 0 && a.y_row % 32 == 0 && a.y_img % 32 == 0 ? 1 : 0;
     switch (p.kind) {
         case NH_I8: return nh_launch_k<NH_I8>(ctx, p, a, maps);
         case NH_U8: return nh_launch_k<NH_U8>(ctx, p, a, maps);
