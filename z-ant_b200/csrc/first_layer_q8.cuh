@@ -218,8 +218,10 @@ inline void first_q8_weights(const ConvGeom& g, const int8_t* w, std::vector<uin
 inline int32_t first_q8_run(zant_ctx* ctx, const ConvGeom& g, bool u8, FirstQ8Args a) {
     a.M = g.M; a.H = g.H; a.W = g.W; a.GH = g.OH / 2; a.GW = g.OW / 2;
     a.pitch = first_q8_pitch(g); a.units = (a.GW + 15) / 16;
+    // rows of a band: as many as leave two CTAs an SM (of the three that fit).  3 x 416 x 416, 16 filters, 2 / 4 / 8 / 16 images, bands of 1, 2, 4, 8 rows, us:
+    // 10.2 12.2 14.3 18.4 / 15.3 12.3 14.4 18.4 / 24.5 19.5 18.4 22.4 / 40.9 32.7 28.6 26.6
     a.PR = 8;
-    while (a.PR > 1 && (first_q8_smem_bytes(g, a.PR) > 48 * 1024 || (long long)g.N * ((a.GH + a.PR - 1) / a.PR) < 3LL * ctx->sm_count)) a.PR /= 2;
+    while (a.PR > 1 && (first_q8_smem_bytes(g, a.PR) > 48 * 1024 || (long long)g.N * ((a.GH + a.PR - 1) / a.PR) < 2LL * ctx->sm_count)) a.PR /= 2;
     a.rows = 2 * a.PR + 2; a.bands = (a.GH + a.PR - 1) / a.PR;
     a.vec = g.W % 4 == 0 && ((uintptr_t)a.x & 15) == 0;
     const size_t smem = first_q8_smem_bytes(g, a.PR);
