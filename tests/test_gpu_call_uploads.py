@@ -79,3 +79,24 @@ def test_small_arrays_of_one_call(ctx, oracle):
         args = (0.02, 0, w, ws, None, float(0.02 * 0.007 * 74 * 74 * np.sqrt(C * 9) / 45), 0)
         kw = dict(bias=bias, y_dtype=1, stride=(1, 1), pads=(1,) * 4, dilations=(1, 1), group=1, activation=None)
         assert np.array_equal(ctx.qlinearconv(x, *args, **kw), oracle.qlinearconv(x, *args, **kw))
+
+
+def test_stream_changed_between_calls(zb, oracle):
+    """Calls return with copies under way; the context's own stream goes away, and the next call, whose arrays share the ring, runs on another."""
+    import torch
+    ctx = zb.Context(0)
+    rng = np.random.default_rng(3)
+    cases = [call(ctx, oracle, rng, *s) for s in ((2, 16, 30, 30, 24, 3, 1, 0), (4, 256, 14, 14, 512, 3, 2, 0), (2, 170, 27, 27, 180, 3, 1, 0))]
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    for turn in range(5):
+        if turn:                                         # the first of these destroys the context's own stream
+            ctx.set_stream(streams[turn - 1].cuda_stream)
+        for i in (turn % 3, (turn + 1) % 3, 0):
+            want, y, go, _ = cases[i]
+            y.zero_()
+            torch.cuda.synchronize()
+            go()
+    ctx.synchronize()
+    for want, y, _, _ in cases:
+        assert np.array_equal(y.cpu().numpy(), want)
+    ctx.close()

@@ -105,8 +105,7 @@ int32_t zant_b200_ctx_destroy(zant_ctx* ctx) {
 
 int32_t zant_b200_ctx_set_stream(zant_ctx* ctx, void* cuda_stream) {
     ZB_NEED_CTX(ctx);
-    ZB_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (ctx->own_stream && ctx->stream) ZB_CUDA(cudaStreamDestroy(ctx->stream));
+    ZB_CUDA(leave_stream(ctx->stage, ctx->stream, ctx->own_stream && ctx->stream));
     ctx->stream = static_cast<cudaStream_t>(cuda_stream);
     ctx->own_stream = false;
     return ZANT_OK;

@@ -124,8 +124,8 @@ class HostStage {
         return cudaMemcpyAsync(dst, p, span, cudaMemcpyHostToDevice, stream);
     }
 
-    // The stream has been drained: every slot is free.
-    void drained() { idle_ = true; used_ = 0; dirty_ = false; }
+    // The stream has been drained: every slot is free, and no stream is remembered.
+    void drained() { idle_ = true; used_ = 0; dirty_ = false; stream_ = nullptr; }
 
     // Page-locked room for a result of at most a slot; valid until the next transfer of this context.
     void* result_slot(size_t bytes, cudaStream_t stream) {
@@ -239,5 +239,13 @@ class HostStage {
     std::unique_ptr<std::atomic<uint8_t>[]> done_;
     size_t done_cap_ = 0;
 };
+
+// A context leaves its stream, which goes away with `destroy` or with whoever owns it: nothing of the ring may refer to it any more.
+inline cudaError_t leave_stream(HostStage* stage, cudaStream_t stream, bool destroy) {
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return e;
+    if (stage) stage->drained();
+    return destroy ? cudaStreamDestroy(stream) : cudaSuccess;
+}
 
 }  // namespace zb
