@@ -183,6 +183,7 @@ inline int first_q8_pitch(const ConvGeom& g) {
     const int units = (g.OW / 2 + 15) / 16, need = std::max(units * 8 + 2, (g.W + 3) / 4 + 1);
     return (need + 7) / 16 * 16 + 8;
 }
+constexpr size_t kFirstQ8Smem = 48 * 1024 - 256;               // what a launch has beside the activation's table
 inline size_t first_q8_smem_bytes(const ConvGeom& g, int pr) { return (size_t)g.C * (2 * pr + 2) * first_q8_pitch(g) * 4; }
 
 // `g`: a layer that the channels-last kernel takes with its pool (3x3, stride 1, a border of one pixel, an even image).
@@ -193,7 +194,7 @@ inline size_t first_q8_smem_bytes(const ConvGeom& g, int pr) { return (size_t)g.
 // 300 x 3 x 130 x 130, 16 filters 101.9 and 105.2 (128 x 128 97.9 and 73.2).
 inline bool first_q8_takes(const ConvGeom& g, int sm_count) {
     if (g.OW / 2 < (g.W % 4 == 0 ? 64 : 128) && (long long)g.N * (g.OH / 2) > 3LL * sm_count) return false;
-    return g.C >= 1 && g.C <= 4 && g.M % 16 == 0 && g.M <= 64 && first_q8_smem_bytes(g, 1) <= 48 * 1024 && (long long)g.N * (g.OH / 2) < 0x7fffffffLL;
+    return g.C >= 1 && g.C <= 4 && g.M % 16 == 0 && g.M <= 64 && first_q8_smem_bytes(g, 1) <= kFirstQ8Smem && (long long)g.N * (g.OH / 2) < 0x7fffffffLL;
 }
 
 // Weights [M][C][3][3] in fragment order.
@@ -221,7 +222,7 @@ inline int32_t first_q8_run(zant_ctx* ctx, const ConvGeom& g, bool u8, FirstQ8Ar
     // rows of a band: as many as leave two CTAs an SM (of the three that fit).  3 x 416 x 416, 16 filters, 2 / 4 / 8 / 16 images, bands of 1, 2, 4, 8 rows, us:
     // 10.2 12.2 14.3 18.4 / 15.3 12.3 14.4 18.4 / 24.5 19.5 18.4 22.4 / 40.9 32.7 28.6 26.6
     a.PR = 8;
-    while (a.PR > 1 && (first_q8_smem_bytes(g, a.PR) > 48 * 1024 || (long long)g.N * ((a.GH + a.PR - 1) / a.PR) < 2LL * ctx->sm_count)) a.PR /= 2;
+    while (a.PR > 1 && (first_q8_smem_bytes(g, a.PR) > kFirstQ8Smem || (long long)g.N * ((a.GH + a.PR - 1) / a.PR) < 2LL * ctx->sm_count)) a.PR /= 2;
     a.rows = 2 * a.PR + 2; a.bands = (a.GH + a.PR - 1) / a.PR;
     a.vec = g.W % 4 == 0 && ((uintptr_t)a.x & 15) == 0;
     const size_t smem = first_q8_smem_bytes(g, a.PR);
