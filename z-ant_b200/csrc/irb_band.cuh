@@ -397,8 +397,8 @@ inline int irb_band_resident(int per_sm, int n, int sm_count) {
     return std::max(1, (int)((long long)clusters[per_sm - 1][n] * sm_count / 148));
 }
 
-// One split of a block: rb output rows a band, cs CTAs a cluster, ct tiles a chunk.  False when it does not fit.
-inline bool irb_band_split(const ConvGeom& d, int C, int M, int rb, int cs, int ct, int threads, int sm_count, IrbBandPlan& q) {
+// One split of a block: rb output rows a band, cs CTAs a cluster, ct tiles a chunk.  False when it does not fit, or takes `limit` us at least.
+inline bool irb_band_split(const ConvGeom& d, int C, int M, int rb, int cs, int ct, int threads, int sm_count, double limit, IrbBandPlan& q) {
     IrbBandArgs& a = q.a;
     a = IrbBandArgs{};
     const int S = d.sh, E = d.C, warps = threads / 32;
@@ -412,18 +412,9 @@ inline bool irb_band_split(const ConvGeom& d, int C, int M, int rb, int cs, int 
     auto pitch = [&](int px) { return 16 * (up(px, 16) | 1); };
     a.xp = a.ep = pitch(32 * g1); a.dp = pitch(32 * g2); a.dpx = 32 * g2;
     a.ks1 = up(C, 32); a.ks2 = up(ct, 2); a.mt2 = up(M, 16);
-    // the rows of a band in as many parts as give the threads the fewest rows
-    long long fewest = 1LL << 60;
-    for (int s = 1; s <= rb; ++s) {
-        const int rows = up(rb, s), segs = up(rb, rows);
-        const long long cost = (long long)up(a.OP / 4 * ct * 16 * segs, threads) * (S * rows + 2);
-        if (cost < fewest) { fewest = cost; a.segs = segs; a.seg_rows = rows; }
-    }
     // two tiles an item where that takes the warps less time (a second tile shares the columns' fragments: 1.6 times the time of one)
     auto tiles_of_item = [&](int groups, int tiles) { return up(groups * up(tiles, 2), warps) * 16 <= up(groups * tiles, warps) * 10 ? 2 : 1; };
     a.nm1 = tiles_of_item(g1, ct); a.nm2 = tiles_of_item(g2, a.mt2);
-    a.per_magic = magic_of(a.in_rows * a.P / 4); a.pw_magic = magic_of(a.P / 4); a.op_magic = magic_of(a.OP); a.opw_magic = magic_of(a.OP / 4);
-    a.ch_magic = magic_of(16 * ct); a.cs_magic = magic_of(cs);
     a.chunk_bytes = ct * a.ks1 * 512 + a.mt2 * a.ks2 * 512 + ct * 16 * (int)sizeof(IrbConst) + a.mt2 * 128;
     a.w_stages = a.chunks > 1 ? 2 : 1;
     const int items2 = g2 * up(a.mt2, a.nm2), blocks = a.mt2 * (a.dpx / 8);
@@ -444,11 +435,24 @@ inline bool irb_band_split(const ConvGeom& d, int C, int M, int rb, int cs, int 
     const int per_sm = std::max(1, std::min({(int)(227 * 1024 / (q.smem_bytes + 1024)), 65536 / (80 * threads), 3})), resident = irb_band_resident(per_sm, cs, sm_count);
     const long long tiles = (long long)a.N * a.bands, rounds = (tiles + resident - 1) / resident, rest = tiles - (rounds - 1) * resident;
     const double on_sm = (double)((rounds - 1) * per_sm + (rest * per_sm + resident - 1) / resident);
-    const int words = C * a.in_rows * a.P / 4, it1 = g1 * up(ct, a.nm1), dw = a.OP / 4 * ct * 16 * a.segs, rows = S * a.seg_rows + 2;
-    const double alone = 1.41 + 0.088 * up(words, 4 * threads) + a.chunks * (0.0145 * up(it1, warps) * a.nm1 * a.ks1 + 0.1445 * up(dw, threads) * rows + up(items2, warps) * a.nm2 * (0.048 * a.ks2 + 0.15)) +
-                         0.54 * (a.chunks - 1) + (cs > 1 ? 0.53 : 0.0);
-    const double issue = 0.242e-3 * words + a.chunks * (0.0055 * it1 * a.nm1 * a.ks1 + 0.3636e-3 * dw * rows + items2 * a.nm2 * (0.0031 * a.ks2 + 0.012)) + blocks * (cs > 1 ? 0.0099 : 0.005);
-    q.us = 0.93 + rounds * alone + on_sm * issue;
+    const int words = C * a.in_rows * a.P / 4, it1 = g1 * up(ct, a.nm1);
+    auto time = [&](int dw, int rows) {
+        const double alone = 1.41 + 0.088 * up(words, 4 * threads) + a.chunks * (0.0145 * up(it1, warps) * a.nm1 * a.ks1 + 0.1445 * up(dw, threads) * rows + up(items2, warps) * a.nm2 * (0.048 * a.ks2 + 0.15)) +
+                             0.54 * (a.chunks - 1) + (cs > 1 ? 0.53 : 0.0);
+        const double issue = 0.242e-3 * words + a.chunks * (0.0055 * it1 * a.nm1 * a.ks1 + 0.3636e-3 * dw * rows + items2 * a.nm2 * (0.0031 * a.ks2 + 0.012)) + blocks * (cs > 1 ? 0.0099 : 0.005);
+        return 0.93 + rounds * alone + on_sm * issue;
+    };
+    if (time(0, 0) >= limit) return false;
+    // the rows of a band in as many parts as give the threads the fewest rows
+    long long fewest = 1LL << 60;
+    for (int s = 1; s <= rb; ++s) {
+        const int rows = up(rb, s), segs = up(rb, rows);
+        const long long cost = (long long)up(a.OP / 4 * ct * 16 * segs, threads) * (S * rows + 2);
+        if (cost < fewest) { fewest = cost; a.segs = segs; a.seg_rows = rows; }
+    }
+    a.per_magic = magic_of(a.in_rows * a.P / 4); a.pw_magic = magic_of(a.P / 4); a.op_magic = magic_of(a.OP); a.opw_magic = magic_of(a.OP / 4);
+    a.ch_magic = magic_of(16 * ct); a.cs_magic = magic_of(cs);
+    q.us = time(a.OP / 4 * ct * 16 * a.segs, S * a.seg_rows + 2);
     return true;
 }
 
@@ -477,7 +481,7 @@ inline bool irb_band_plan(const ConvGeom& e, const ConvGeom& d, const ConvGeom& 
                 if (ct == last_ct) continue;
                 last_ct = ct;
                 for (int threads : {256, 384})
-                    if (irb_band_split(d, C, M, rb, cs, ct, threads, sm_count, q) && q.us < best.us) best = q;
+                    if (irb_band_split(d, C, M, rb, cs, ct, threads, sm_count, best.us, q) && q.us < best.us) best = q;
             }
         }
     }
@@ -491,25 +495,39 @@ inline bool irb_band_prepare(const IrbBandPlan& q, const int8_t* we, const float
     const IrbBandArgs& a = q.a;
     const int stages = a.cs * a.chunks, CH = a.ct * 16;
     out.assign((size_t)stages * a.chunk_bytes, 0);
-    auto put = [](uint8_t* block, int r, int k, int8_t v) { block[((r & 7) * 4 + ((k & 15) >> 2)) * 16 + ((r >> 3) + 2 * (k >> 4)) * 4 + (k & 3)] = (uint8_t)v; };
+    // Row r of a product: a K step is eight words, which with those of row r ^ 8 are 64 bytes of the block.  (A byte at a time the sixteen blocks of
+    // a MobileNetV2-style plan took 3.3 ms of host time instead of 0.4; finalizing it for one image: 6.1 -> 3.6 ms.)
+    auto row = [](uint8_t* blocks, int r, int ksteps, const int8_t* v, int n) {
+        uint8_t* to = blocks + (size_t)(r >> 4) * ksteps * 512 + (r & 7) * 64 + ((r >> 3) & 1) * 4;
+        for (; n > 0; n -= 32, v += 32, to += 512) {
+            uint32_t w[8] = {};
+            if (n >= 32) std::memcpy(w, v, 32); else std::memcpy(w, v, (size_t)n);
+            for (int i = 0; i < 4; ++i) { std::memcpy(to + 16 * i, w + i, 4); std::memcpy(to + 16 * i + 8, w + 4 + i, 4); }
+        }
+    };
+    const size_t w1_bytes = (size_t)a.ct * a.ks1 * 512, w12_bytes = w1_bytes + (size_t)a.mt2 * a.ks2 * 512;
     for (int e = 0; e < q.E; ++e) {
         uint8_t* stage = out.data() + (size_t)(e / CH) * a.chunk_bytes;
-        uint8_t* w2 = stage + (size_t)a.ct * a.ks1 * 512;
+        const int8_t* w = we + (size_t)e * a.C;
         const int r = e % CH;
         IrbConst k{};
         int s1 = 0, s2 = 0;
-        for (int c = 0; c < a.C; ++c) { put(stage + ((size_t)(r / 16) * a.ks1 + c / 32) * 512, r % 16, c % 32, we[(size_t)e * a.C + c]); s1 += std::abs((int)we[(size_t)e * a.C + c]); }
-        for (int m = 0; m < a.M; ++m) put(w2 + ((size_t)(m / 16) * a.ks2 + r / 32) * 512, m % 16, r % 32, wp[(size_t)m * q.E + e]);
+        for (int c = 0; c < a.C; ++c) s1 += std::abs((int)w[c]);
+        row(stage, r, a.ks1, w, a.C);
         for (int i = 0; i < 9; ++i) { k.k[i / 3] |= (uint32_t)(uint8_t)wd[e * 9 + i] << (8 * (i % 3)); s2 += std::abs((int)wd[e * 9 + i]); }
         if (!acc_base_ok(eb[e]) || !acc_base_ok(db[e]) || s1 * 128 + std::abs(eb[e]) >= (1 << 22) || s2 * 128 + std::abs(db[e]) >= (1 << 22)) return false;
         k.e_floor = kAccBase - (float)eb[e]; k.e_mult = em[e]; k.d_mult = dm[e]; k.d_base = kAccBaseBits + db[e];
-        std::memcpy(w2 + (size_t)a.mt2 * a.ks2 * 512 + (size_t)r * sizeof(IrbConst), &k, sizeof k);
+        std::memcpy(stage + w12_bytes + (size_t)r * sizeof(IrbConst), &k, sizeof k);
     }
-    for (int j = 0; j < stages; ++j)
+    for (int j = 0; j < stages; ++j) {
+        uint8_t* stage = out.data() + (size_t)j * a.chunk_bytes;
+        const int e0 = j * CH, live = std::min(CH, q.E - e0);
         for (int m = 0; m < a.M; ++m) {
-            uint8_t* at = out.data() + (size_t)(j + 1) * a.chunk_bytes - (size_t)a.mt2 * 128 + (size_t)m * 8;
-            std::memcpy(at, pm + m, 4); std::memcpy(at + 4, pb + m, 4);
+            row(stage + w1_bytes, m, a.ks2, wp + (size_t)m * q.E + e0, live);
+            uint8_t* tail = stage + a.chunk_bytes - (size_t)a.mt2 * 128 + (size_t)m * 8;
+            std::memcpy(tail, pm + m, 4); std::memcpy(tail + 4, pb + m, 4);
         }
+    }
     return true;
 }
 
