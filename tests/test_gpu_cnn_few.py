@@ -42,3 +42,31 @@ def test_four_kernels_above(zb, ctx, oracle, models, scales, batch):
     x = models.small_cnn_input(batch, batch)
     x.reshape(-1)[::97] = np.resize(np.array([np.nan, np.inf, -np.inf, -0.0, 1.0e-30], np.float32), x.reshape(-1)[::97].size)
     _check(zb, ctx, oracle, g, x, 4)
+
+
+@pytest.mark.parametrize("batch,steps", [(4, 1), (500, 4)])
+def test_device_input_of_any_address(zb, ctx, oracle, models, scales, batch, steps):
+    """Images are read 16 bytes at a time: a caller's device buffer at another address is refused, in a replayed graph, which copies it, it is not."""
+    import torch
+    g = models.small_cnn_int8(batch, act_scales=scales)
+    x = models.small_cnn_input(batch, batch)
+    want = graph_oracle.run(oracle, g, x)[g.output]
+    plan = zb.Plan(ctx, g, fuse=True)
+    assert len(plan.step_names()) == steps
+    buf = torch.zeros(x.size + 8, device="cuda")
+    y = torch.empty(want.shape, device="cuda")
+    for graph in (False, True):
+        plan.use_graph(graph)
+        for offset in (0, 1, 2, 4):
+            xd = buf[offset:offset + x.size].view(x.shape)
+            xd.copy_(torch.from_numpy(x))
+            y.fill_(99.0)
+            torch.cuda.synchronize()
+            if offset % 4 and not graph:
+                with pytest.raises(zb.ZantError, match="InvalidInput"):
+                    plan.run(xd, y)
+                continue
+            plan.run(xd, y)
+            ctx.synchronize()
+            assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    plan.close()

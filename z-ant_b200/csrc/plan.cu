@@ -1851,6 +1851,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
             using Cfg = CnnFewCfg;
             CnnFewArgs a = k;
             a.x = pl->p<float>(x); a.y = pl->p<float>(y); a.status = ctx->status_word;
+            if (!aligned16(a.x)) return fail(ZANT_E_INVALID_INPUT, "QuantizeLinear input buffer must be 16-byte aligned");
             a.wfrag = (const uint32_t*)pl->aux(a_wf); a.floor1 = (const float*)pl->aux(a_bf); a.mult1 = (const float*)pl->aux(a_mf);
             a.w = (const uint8_t*)pl->aux(a_blob); a.floor2 = (const float*)pl->aux(a_f2); a.mult2 = (const float*)pl->aux(a_m2);
             a.mult3 = (const float*)pl->aux(a_m3); a.bias3 = (const int32_t*)pl->aux(a_b3); a.mult4 = (const float*)pl->aux(a_m4); a.bias4 = (const int32_t*)pl->aux(a_b4);
@@ -1875,6 +1876,7 @@ static int32_t try_fuse_small_cnn(zant_plan* pl, size_t i0, size_t& consumed, bo
     push("Fused[QuantizeLinear+QLinearConv+Relu+MaxPool] mma", [=]() {
         Conv1MmaArgs k{};
         k.x = pl->p<float>(x); k.y = (int8_t*)pl->scratch(s_pool1); k.n_images = (int)B; k.ib = ib;
+        if (!aligned16(k.x)) return fail(ZANT_E_INVALID_INPUT, "QuantizeLinear input buffer must be 16-byte aligned");
         k.x_scale = a1.x_scale; k.x_zp = a1.x_zp; k.q_rh = steps.rh; k.q_rl = steps.rl;
         k.wfrag = (const uint32_t*)pl->aux(a_wf); k.floorfrag = (const float*)pl->aux(a_bf); k.multfrag = (const float*)pl->aux(a_mf); k.status = ctx->status_word;
         const int blocks = std::min<int>((int)((B + C1M_G - 1) / C1M_G), ctx->sm_count * 2);
