@@ -181,9 +181,9 @@ int32_t zant_b200_measure_int8_peak_sustained(zant_ctx* ctx, double seconds, dou
  * ZANT_E_DEVICE_TIMEOUT once and clears the word, after which the context works as before. */
 int32_t zant_b200_selftest_bounded_wait(zant_ctx* ctx, uint32_t budget_us);
 
-/* Failure-path self test (no reference counterpart).  In the next launch of a kernel that adds partial sums of
- * several CTAs in memory kept between runs (inverted residual blocks of a plan whose chunks are dealt to several
- * CTAs), half of the epilogue warps of CTA `cta` act as if a bounded wait had run out: that run reports
+/* Failure-path self test (no reference counterpart).  In the next launch of the kernel that runs an inverted residual
+ * block of a plan on bands of rows (few images), CTA `cta`, modulo the launch's CTAs, acts as if its first bounded wait
+ * had run out: it fetches no further weights and gives up later waits soon.  That run reports
  * ZANT_E_DEVICE_TIMEOUT as zant_b200_selftest_bounded_wait describes, and the runs after it are right again.
  * A negative `cta` disarms it. */
 int32_t zant_b200_selftest_give_up(zant_ctx* ctx, int32_t cta);

@@ -325,7 +325,7 @@ class Context:
         check(lib().zant_b200_selftest_bounded_wait(self._h, C.c_uint32(int(budget_us))))
 
     def selftest_give_up(self, cta):
-        """CTA `cta` of the next kernel that adds up partial sums gives up; that run raises DeviceTimeout."""
+        """CTA `cta` of the next inverted residual block that runs on clusters gives up a wait; that run raises DeviceTimeout."""
         check(lib().zant_b200_selftest_give_up(self._h, C.c_int32(int(cta))))
 
     def measure_int8_peak(self, iters=20000):

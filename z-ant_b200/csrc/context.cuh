@@ -26,7 +26,7 @@ struct zant_ctx {
     int* status_word = nullptr;   // device int: kernels with bounded waits report here
     zb::HostStage* stage = nullptr;   // page-locked ring for pageable host buffers, created on first use
     zb::UploadLane* lane = nullptr;   // uploads of a call's large weights beside the kernels of the call before, created on first use
-    int give_up_cta = -1;         // self test: this CTA of the next kernel that adds up partial sums gives up (-1: none)
+    int give_up_cta = -1;         // self test: this CTA of the next irb_band_kernel gives up its first wait (-1: none)
     bool in_plan = false;         // the launches are a plan's: weights and constants were written before the run
     int tf32 = 0;                 // float contractions: 0 = the exact FP32 kernels, 1 = tensor cores (kind::tf32, single pass), 2 = tensor cores, split operands (3 x TF32)
 };
