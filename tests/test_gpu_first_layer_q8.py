@@ -27,6 +27,11 @@ CASES = [
     (1, 1, 4736, 2628, 16, "U8", 0, 1 / 255, None),        # eight
     (1, 1, 2368, 4804, 16, "I8", 0, 1 / 127, "relu"),      # four
     (1, 1, 1184, 8068, 16, "U8", 0, 1 / 255, "leaky"),     # two
+    (1, 1, 2368, 4738, 16, "U8", 0, 1 / 255, "leaky"),     # four
+    (4, 4, 1184, 640, 16, "U8", 0, 1 / 255, None),         # eight
+    (2, 4, 600, 1924, 32, "U8", 0, 1 / 255, "leaky"),      # two
+    (1, 2, 4, 6080, 16, "U8", 0, 1 / 255, "leaky"),        # one
+    (1, 1, 4, 12160, 16, "U8", 0, 1 / 255, "leaky"),       # one
     (1, 1, 4, 12164, 16, "U8", 0, 1 / 255, "leaky"),       # one row is too wide: a conversion and the tcgen05 form
 ]
 

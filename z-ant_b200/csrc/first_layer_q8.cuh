@@ -112,10 +112,10 @@ __device__ __forceinline__ void first_q8_rows(const FirstQ8Args& a, uint32_t* s_
 
 template <int C, bool XU8>
 __global__ void __launch_bounds__(kFirstQ8Threads, 3) first_layer_q8_kernel(const __grid_constant__ FirstQ8Args a) {
-    extern __shared__ __align__(16) uint32_t first_q8_smem[];           // [C][rows][pitch]
-    __shared__ uint8_t s_lut[256];
+    extern __shared__ __align__(16) uint32_t first_q8_smem[];           // the activation's table, [C][rows][pitch]
     ptx::grid_start();
-    uint32_t* const s_in = first_q8_smem;
+    uint8_t* const s_lut = reinterpret_cast<uint8_t*>(first_q8_smem);
+    uint32_t* const s_in = first_q8_smem + 64;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int n = (int)blockIdx.x / a.bands, py0 = ((int)blockIdx.x - n * a.bands) * a.PR;
     if (a.lut) s_lut[threadIdx.x] = a.lut[threadIdx.x];
@@ -183,8 +183,8 @@ inline int first_q8_pitch(const ConvGeom& g) {
     const int units = (g.OW / 2 + 15) / 16, need = std::max(units * 8 + 2, (g.W + 3) / 4 + 1);
     return (need + 7) / 16 * 16 + 8;
 }
-constexpr size_t kFirstQ8Smem = 48 * 1024 - 256;               // what a launch has beside the activation's table
-inline size_t first_q8_smem_bytes(const ConvGeom& g, int pr) { return (size_t)g.C * (2 * pr + 2) * first_q8_pitch(g) * 4; }
+constexpr size_t kFirstQ8Smem = 48 * 1024;                     // of a launch; the table is part of it (as static memory it was rounded up to 1024 bytes)
+inline size_t first_q8_smem_bytes(const ConvGeom& g, int pr) { return 256 + (size_t)g.C * (2 * pr + 2) * first_q8_pitch(g) * 4; }
 
 // `g`: a layer that the channels-last kernel takes with its pool (3x3, stride 1, a border of one pixel, an even image).
 // Rows of at least four units, or so few rows that all CTAs are resident at once and the launch that is saved counts.  Two launches (conversion, tcgen05
