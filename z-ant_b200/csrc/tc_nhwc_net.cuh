@@ -141,12 +141,14 @@ __device__ __forceinline__ void nh_next(const NhConvArgs& a, NhTile& c) {
     c.img += c.d_img + k;
 }
 
-template <int KIND, int POOL>
+// WIDE: the epilogue can store 32 channels of a pixel at a time (nh_launch_k).
+template <int KIND, int POOL, bool WIDE>
 __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid_constant__ NhConvArgs a, const __grid_constant__ NhMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr bool I8 = KIND <= NH_U8;
     constexpr bool POOLED = POOL == NH_POOL_VIEWS || POOL == NH_POOL_PAIRS;
     constexpr int PLANES = POOL ? 4 : 1, SETS = POOLED ? 4 : 1;    // parity planes per stage, accumulators per row block
+    static_assert(!WIDE || (I8 && !POOLED), "");
     float* sMult = reinterpret_cast<float*>(smem + a.off_const);
     int* sBias = reinterpret_cast<int*>(sMult + a.const_n);         // TF32: the float bias' bits
     uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + a.const_n);
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
         // int8 without a pool: two chunks of 16 filters at a time, one store of 32 bytes a pixel, where the four warps of a quarter still have as much to do
         // each and the stores are aligned.  A lane's pixel is a line of its own, so a store takes the load-store unit 32 clocks at either width: for the
         // chunks of sixteen warps 1545 clocks with two stores and 1233 with one
-        const int halves = I8 && !POOLED && a.wide ? 2 : 1;
+        const int halves = WIDE && a.wide ? 2 : 1;
         const int per_blk = NT / CH / halves, chunks = a.RB * per_blk;
         int tile_it = 0;
         NhTile T = nh_first(a);
@@ -406,9 +408,9 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                     }
                     uint8_t* yp = a.nchw ? a.y : a.y + (long long)img * a.y_img + (long long)gh * (a.up2 ? 2 : 1) * a.y_row + (long long)gw * (a.up2 ? 2 : 1) * a.y_pix;
                     if constexpr (I8) {
-                        uint32_t wd[2 * CH / 4];
+                        uint32_t wd[(WIDE ? 2 : 1) * CH / 4];
 #pragma unroll
-                        for (int hf = 0; hf < (POOLED ? 1 : 2); ++hf) {
+                        for (int hf = 0; hf < (WIDE ? 2 : 1); ++hf) {
                             if (hf == halves) break;
 #pragma unroll
                             for (int m = 0; m < SETS; ++m) ptx::tmem_ld16(taddr + (uint32_t)(m * NT + hf * CH), v[m]);
@@ -444,8 +446,8 @@ __global__ void __launch_bounds__(kNhThreads, 1) tc_nhwc_net_kernel(const __grid
                             for (int u = 0; u < 4; ++u) {
                                 if (u && !a.up2) break;
                                 uint8_t* yc = yp + (u >> 1) * a.y_row + (u & 1) * a.y_pix + c0;
-                                if (halves == 2) ptx::st_global_v8(yc, wd);
-                                else *reinterpret_cast<uint4*>(yc) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+                                if constexpr (WIDE) if (halves == 2) { ptx::st_global_v8(yc, wd); continue; }
+                                *reinterpret_cast<uint4*>(yc) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
                             }
                         }
                     } else {
@@ -782,18 +784,26 @@ inline int32_t nh_encode_map(int N, int box_n, const NhView& x, int chan_elems, 
     return ZANT_OK;
 }
 
-template <int KIND, int POOL>
+template <int KIND, int POOL, bool WIDE = false>
 inline int32_t nh_launch_t(zant_ctx* ctx, const NhConvPlan& p, const NhConvArgs& a, const NhMaps& maps) {
-    ZB_SMEM_ATTR(ctx, (tc_nhwc_net_kernel<KIND, POOL>), 232448);
+    ZB_SMEM_ATTR(ctx, (tc_nhwc_net_kernel<KIND, POOL, WIDE>), 232448);
     const long long tiles = (long long)a.N * a.hseg * a.wseg * a.n_tiles;
-    launch_const(ctx, tc_nhwc_net_kernel<KIND, POOL>, (unsigned)std::min<long long>(tiles, ctx->sm_count), kNhThreads, p.smem_bytes, a, maps);
+    launch_const(ctx, tc_nhwc_net_kernel<KIND, POOL, WIDE>, (unsigned)std::min<long long>(tiles, ctx->sm_count), kNhThreads, p.smem_bytes, a, maps);
     return check_launch(ctx, "tc_nhwc_net_kernel");
 }
+// int8 without a pool: the kernel that can store 32 channels at a time takes 96 registers a thread, the other 78, beside which the CTAs of a next kernel
+// of another kind start early (28 x 32 x 5 x 5 -> 192 filters, depthwise, 64 filters 25.0 us, 31.8 when all took the larger one; 43 x 160 x 6 x 6 -> 960,
+// depthwise with stride 2, 160 39.4 and 45.7; with 80 registers for both 384 -> 256 filters on 32 x 26 x 26 went from 31.2 to 32.4).  So the larger
+// one runs where it does store 32 channels, and for dequantised values of layers like the ones whose results it stores (256 -> 255 18.1 -> 17.6); not
+// wherever it could: a chain that alternates between the two loads either's instructions each time, 2 us.
 template <int KIND>
 inline int32_t nh_launch_k(zant_ctx* ctx, const NhConvPlan& p, const NhConvArgs& a, const NhMaps& maps) {
     if (p.pool == NH_POOL_VIEWS) return nh_launch_t<KIND, NH_POOL_VIEWS>(ctx, p, a, maps);
     if (p.pool == NH_POOL_PAIRS) return nh_launch_t<KIND, NH_POOL_PAIRS>(ctx, p, a, maps);
-    if constexpr (KIND <= NH_U8) { if (p.pool == NH_STRIDE2) return nh_launch_t<KIND, NH_STRIDE2>(ctx, p, a, maps); }
+    if constexpr (KIND <= NH_U8) {
+        if (p.pool == NH_STRIDE2) return a.wide ? nh_launch_t<KIND, NH_STRIDE2, true>(ctx, p, a, maps) : nh_launch_t<KIND, NH_STRIDE2>(ctx, p, a, maps);
+        if (a.wide || (a.nchw == 2 && p.cin % 32 == 0 && a.RB * a.NT % 128 == 0)) return nh_launch_t<KIND, NH_POOL_NONE, true>(ctx, p, a, maps);
+    }
     return nh_launch_t<KIND, NH_POOL_NONE>(ctx, p, a, maps);
 }
 
