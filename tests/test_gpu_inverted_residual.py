@@ -1,4 +1,5 @@
-"""Expand 1x1 -> depthwise 3x3 -> project 1x1 [-> residual addition] as one kernel (irb_q8.cuh) against the oracle, bit for bit."""
+"""Expand 1x1 -> depthwise 3x3 -> project 1x1 [-> residual addition] as one step against the oracle, bit for bit: whichever kernel the plan takes, and, with
+as many images as it takes, the kernel for many images (irb_q8.cuh)."""
 import numpy as np
 import pytest
 
@@ -35,6 +36,43 @@ CASES = [
     (90, 64, 1100, 64, 4, 6, 0, True, 2, 1),        # nine chunks on three CTAs
     (160, 64, 384, 64, 14, 14, 0, True, 1, 1, "relu"),
     (31, 48, 700, 48, 5, 5, 0, True, 2, 1, "relu6"),
+]
+
+# Blocks that the kernel for many images takes (on 148 SMs): every width that it is instantiated for, images a tile, chunks, filter tiles.
+ONE = [
+    (53, 64, 384, 64, 14, 14, 0, True, 1, 1),       # whole chunks, one image a tile, both halves in one accumulator
+    (160, 96, 576, 96, 14, 14, 0, False, 2, 1),     # half a chunk at the end, CTAs with two tiles
+    (485, 32, 128, 32, 7, 7, 0, True, 1, 1),        # two images a tile, an odd image, CTAs with two tiles, one chunk
+    (101, 160, 960, 160, 7, 7, 0, True, 1, 1),      # two filter tiles, an odd image
+    (49, 160, 960, 320, 7, 7, -3, True, 0, 1),      # three filter tiles, input zero point
+    (33, 40, 200, 48, 14, 16, 2, True, 0, 1),
+    (33, 40, 240, 112, 5, 16, -1, False, 0, 1),     # odd rows, halves apart
+    (177, 64, 136, 16, 2, 5, 9, True, 0, 1),        # eight channels in the last chunk
+    (179, 64, 384, 64, 6, 8, 0, True, 1, 1),
+    (43, 96, 576, 160, 14, 14, 2, True, 0, 2),      # stride 2, two filter tiles
+    (77, 24, 144, 80, 12, 12, 3, False, 0, 2),      # the second half reads more rows than the first
+    (9, 8, 128, 16, 8, 10, 0, True, 0, 2),          # both halves in one accumulator
+    (185, 48, 700, 48, 5, 5, 0, True, 1, 1),        # 60 channels in the last chunk, an odd image
+    (221, 64, 1100, 64, 4, 6, 0, True, 2, 1),       # nine chunks
+    (185, 48, 700, 48, 5, 5, 0, True, 2, 1, "relu6"),
+    (19, 40, 128, 8, 2, 4, 4, True, 0, 1),          # widths in the kernel's steps, without and with an addition
+    (275, 8, 128, 8, 2, 3, 0, True, 1, 1),
+    (21, 24, 128, 96, 3, 6, 0, True, 0, 1),
+    (59, 80, 128, 80, 2, 5, 0, True, 2, 1),
+    (17, 40, 128, 48, 2, 7, 0, True, 0, 1),
+    (189, 12, 128, 12, 4, 7, 1, True, 1, 1),
+    (31, 40, 128, 8, 3, 8, 0, False, 0, 1),
+    (125, 8, 128, 8, 2, 8, 0, True, 1, 1),
+    (11, 40, 128, 96, 2, 10, 0, True, 0, 1),
+    (99, 80, 200, 80, 13, 9, 0, True, 1, 1),
+    (125, 24, 384, 24, 13, 10, 0, True, 2, 1),
+    (17, 24, 128, 16, 2, 12, 0, True, 0, 1),        # one output row a half
+    (105, 32, 384, 32, 11, 12, 5, True, 1, 1),
+    (9, 72, 128, 96, 4, 13, 0, True, 0, 1),
+    (129, 80, 136, 80, 9, 14, 0, True, 1, 1),
+    (11, 12, 128, 160, 2, 15, 0, True, 0, 1),
+    (101, 80, 256, 80, 6, 15, 0, True, 1, 1),
+    (127, 12, 256, 12, 11, 16, 0, True, 1, 1),      # an odd plane
 ]
 
 
@@ -84,6 +122,23 @@ def test_block(zb, ctx, oracle, case):
     for _ in range(2):
         assert np.array_equal(plan.run(xv), want[g.output])
     assert len(np.unique(want[t1])) > 30 and len(np.unique(want[t2])) > 20 and len(np.unique(want[cur])) > 30
+    plan.close()
+
+
+@pytest.mark.parametrize("case", ONE, ids=["x".join(map(str, c[:6] + c[9:])) for c in ONE])
+def test_block_of_many_images(zb, ctx, oracle, case):
+    g, t1, t2, cur, xv = block(zb, case)
+    out = g.tensor("out", zb.F32, g.tensors[cur]["shape"])
+    g.node("DequantizeLinear", [cur], [out], x_scale=0.2, x_zp=0)
+    g.output = out
+    want = graph_oracle.run(oracle, g, xv)
+    plan = zb.Plan(ctx, g, fuse=True)
+    assert any("expand+depthwise+project" in n for n in plan.step_names())
+    ctx.selftest_give_up(0)                                  # (only the kernel on bands of rows would)
+    for _ in range(2):
+        assert np.array_equal(plan.run(xv), want[g.output])
+    ctx.selftest_give_up(-1)
+    assert len(np.unique(want[t1])) > 20 and len(np.unique(want[t2])) > 15 and len(np.unique(want[cur])) > 30
     plan.close()
 
 

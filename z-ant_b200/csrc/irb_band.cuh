@@ -539,9 +539,13 @@ inline bool irb_band_prepare(const IrbBandPlan& q, const int8_t* we, const float
 //     32 -> 192 at 28 x 28: 16 images 9 / 17, 148 43 / 41; 16 -> 96 at 112 x 112, stride 2: 8 images 16 / 20, 24 38 / 34, 200 289 / 181)
 //   irb_q8.cuh: rounds of the SMs of a tile's time, which grows with its chunks (64 -> 384 at 14 x 14: 24 images 9 / 22 / 15, 64 17 / 26 / 17, 148 29 / 33 / 15;
 //     96 -> 576 at 10 x 10: 37 images 13 / 26 / 20, 100 30 / 36 / 21; stride 2: 37 images 10 / 30 / 9; 160 -> 960 at 7 x 7: 8 images 7 / 23 / 19, 37 13 / 31 / 21, 64
-//     22 / 37 / 28, 100 30 / 44 / 24; -> 320: 24 images 12 / 24 / 31, 64 31 / 32 / 25)
+//     22 / 37 / 28, 100 30 / 44 / 24; -> 320: 24 images 12 / 24 / 31, 64 31 / 32 / 25).  Without an addition this kernel has to be faster by 1.3: such blocks
+//     often have a last chunk with few channels, which costs irb_q8.cuh less than a whole one, or planes that the times here were not fitted to (1773 x 40 x
+//     7 x 7, 160 -> 96 filters 62 / - / 40, 3646 x 40 x 6 x 6, 160 -> 16 86 / 153 / 67, 238 x 40 x 9 x 9, 160 -> 96 19 / 39 / 15).  Of 231 random blocks that
+//     irb_q8.cuh takes, seven were slower by 8 to 29 % than in it without the factor, one by 9 % with it, and the others gain as much.  Of 1552 blocks, most of
+//     them random, seven are slower by 4 to 9 % than without this kernel
 enum class IrbForm { kSeparate, kOne, kBand };
-inline IrbForm irb_form(const IrbPlan* one, const IrbBandPlan* band, const ConvGeom& d, bool long_add, int sm_count) {
+inline IrbForm irb_form(const IrbPlan* one, const IrbBandPlan* band, const ConvGeom& d, bool add, bool long_add, int sm_count) {
     const bool one_pays = one && irb_pays(*one, long_add, sm_count);
     if (band) {
         const double values = 1e-6 * d.N * d.C * d.H * d.W;
@@ -552,7 +556,7 @@ inline IrbForm irb_form(const IrbPlan* one, const IrbBandPlan* band, const ConvG
             if (a.IB == 1) tile = d.sh == 2 ? 1.0 + 3.2 * a.chunks : (long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : 2.0 + 4.1 * a.chunks) * (0.7 + 0.3 * a.H / 14.0);
             other = ((a.tiles + sm_count - 1) / sm_count) * tile;
         }
-        if (band->us < other) return IrbForm::kBand;
+        if (band->us * (one_pays && !add ? 1.3 : 1.0) < other) return IrbForm::kBand;
     }
     return one_pays ? IrbForm::kOne : IrbForm::kSeparate;
 }

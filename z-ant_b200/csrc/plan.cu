@@ -1432,7 +1432,7 @@ static int32_t try_fuse_irb(zant_plan* pl, size_t i0, size_t& consumed) {
     IrbPlan q;
     IrbBandPlan qb;
     const bool can_one = irb_plan(g[0], g[1], g[2], with_add, q), can_band = irb_band_plan(g[0], g[1], g[2], with_add, ctx->sm_count, qb);
-    const IrbForm form = irb_form(can_one ? &q : nullptr, can_band ? &qb : nullptr, g[1], with_add && !add.proved, ctx->sm_count);
+    const IrbForm form = irb_form(can_one ? &q : nullptr, can_band ? &qb : nullptr, g[1], with_add, with_add && !add.proved, ctx->sm_count);
     std::vector<uint8_t> stages;
     if (form == IrbForm::kSeparate ||
         !(form == IrbForm::kBand ? irb_band_prepare(qb, host(e->in[1]), mult[0].data(), bias[0].data(), host(d->in[1]), mult[1].data(), bias[1].data(), host(p->in[1]), mult[2].data(), bias[2].data(), stages)
