@@ -32,7 +32,6 @@ CASES = [
     (2, 4, 600, 1924, 32, "U8", 0, 1 / 255, "leaky"),      # two
     (1, 2, 4, 6080, 16, "U8", 0, 1 / 255, "leaky"),        # one
     (1, 1, 4, 12160, 16, "U8", 0, 1 / 255, "leaky"),       # one
-    (1, 1, 4, 12164, 16, "U8", 0, 1 / 255, "leaky"),       # one row is too wide: a conversion and the tcgen05 form
 ]
 
 
@@ -83,9 +82,58 @@ def test_quantising_first_layer(zb, ctx, oracle, case):
     xin.reshape(-1)[:3] = [np.nan, np.inf, -np.inf]
     want = graph_oracle.run(oracle, g, xin)
     plan = zb.Plan(ctx, g)
-    assert plan.step_names()[0].startswith("Fused[QuantizeLinear+QLinearConv") == (W <= 12160), plan.step_names()
+    assert plan.step_names()[0].startswith("Fused[QuantizeLinear+QLinearConv"), plan.step_names()
     got = plan.run(xin)
     assert np.array_equal(plan.read_tensor(p), want[p])
     assert np.array_equal(got, want[out])
     assert len(np.unique(want[p])) > (16 if H > 2 else 4)
+    plan.close()
+
+
+@pytest.mark.parametrize("N,C,H,W,M,order,one", [
+    (2, 3, 64, 64, 16, (0, 1), True),           # the result is the first part of a Concat's pixels, a convolution of it the other
+    (2, 1, 34, 66, 48, (1, 0), True),           # it starts behind 16 channels
+    (1, 4, 36, 70, 64, (1, 0), True),
+    (230, 1, 28, 128, 32, (1, 0), True),
+    (1, 1, 4, 12164, 16, (1, 0), False),        # a row is too wide: a conversion and the tcgen05 form
+])
+def test_result_inside_a_concat(zb, ctx, oracle, N, C, H, W, M, order, one):
+    rng = np.random.default_rng(N + W)
+    conv = dict(strides=(1, 1), dilations=(1, 1), group=1, auto_pad="NOTSET")
+    g = zb.Graph("first")
+    PH, PW = H // 2, W // 2
+    x = g.tensor("x", zb.F32, (N, C, H, W))
+    q = g.tensor("xq", zb.U8, (N, C, H, W))
+    c = g.tensor("c", zb.I8, (N, M, H, W))
+    a = g.tensor("a", zb.I8, (N, M, H, W))
+    p = g.tensor("p", zb.I8, (N, M, PH, PW))
+    c1 = g.tensor("c1", zb.I8, (N, 16, PH, PW))
+    cat = g.tensor("cat", zb.I8, (N, M + 16, PH, PW))
+    c2 = g.tensor("c2", zb.I8, (N, 16, PH, PW))
+    out = g.tensor("y", zb.F32, (N, 16, PH, PW))
+    sx = float(np.float32(1 / 255))
+    sy, s1, s2 = (float(np.float32(v)) for v in (sx * 0.007 * 74 * 90 * np.sqrt(C * 9) / 40, 0.02 * np.sqrt(M), 0.05 * np.sqrt(M + 16)))
+
+    def weights(name, m, k, r):
+        return (g.tensor("w" + name, zb.I8, (m, k, r, r), rng.integers(-127, 128, (m, k, r, r), dtype=np.int8)),
+                g.tensor("s" + name, zb.F32, (m,), (rng.random(m, dtype=np.float32) * 0.01 + 0.002).astype(np.float32)))
+
+    g.node("QuantizeLinear", [x], [q], y_scale=sx, y_zp=0)
+    g.node("QLinearConv", [q, *weights("0", M, C, 3)], [c], x_scale=sx, x_zp=0, y_scale=sy, y_zp=0, pads=(1, 1, 1, 1), **conv)
+    g.node("LeakyRelu", [c], [a], alpha=0.1, x_scale=sy, x_zp=0, y_scale=sy, y_zp=0)
+    g.node("MaxPool", [a], [p], **POOL)
+    g.node("QLinearConv", [p, *weights("1", 16, M, 1)], [c1], x_scale=0.02, x_zp=0, y_scale=s1, y_zp=0, pads=(0, 0, 0, 0), **conv)
+    g.node("Concat", [(p, c1)[i] for i in order], [cat], axis=1)
+    g.node("QLinearConv", [cat, *weights("2", 16, M + 16, 1)], [c2], x_scale=0.02, x_zp=0, y_scale=s2, y_zp=0, pads=(0, 0, 0, 0), **conv)
+    g.node("DequantizeLinear", [c2], [out], x_scale=s2, x_zp=0)
+    g.input, g.output = x, out
+    xin = (rng.random((N, C, H, W), dtype=np.float32) * 1.2 - 0.1).astype(np.float32)
+    want = graph_oracle.run(oracle, g, xin)
+    plan = zb.Plan(ctx, g)
+    names = plan.step_names()
+    assert names[0].startswith("Fused[QuantizeLinear+QLinearConv") == one and "Concat" not in names, names
+    got = plan.run(xin)
+    for t in (p, c1, cat):
+        assert np.array_equal(plan.read_tensor(t), want[t]) and len(np.unique(want[t])) > 16
+    assert np.array_equal(got, want[out])
     plan.close()

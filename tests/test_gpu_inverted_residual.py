@@ -1,5 +1,4 @@
-"""Expand 1x1 -> depthwise 3x3 -> project 1x1 [-> residual addition] as one step against the oracle, bit for bit: whichever kernel the plan takes, and, with
-as many images as it takes, the kernel for many images (irb_q8.cuh)."""
+"""Expand 1x1 -> depthwise 3x3 -> project 1x1 [-> residual addition] as one kernel (irb_q8.cuh) against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -169,12 +168,10 @@ def test_result_behind_a_reshape_is_the_output(zb, ctx, oracle, res):
     plan.close()
 
 
-@pytest.mark.parametrize("case,ctas", [((31, 48, 700, 48, 5, 5, 0, True, 1, 1), 96), ((16, 160, 960, 320, 7, 7, -3, True, 0, 1), 64),
-                                       ((64, 160, 960, 160, 7, 7, 0, True, 1, 1), 128),          # four chunks a CTA: weights that it stops fetching; pairs of CTAs
-                                       ((148, 160, 960, 160, 4, 4, 0, True, 1, 1), 148)])        # four chunks, no cluster
+@pytest.mark.parametrize("case,ctas", [((31, 48, 700, 48, 5, 5, 0, True, 1, 1), 96), ((16, 160, 960, 320, 7, 7, -3, True, 0, 1), 64)])
 @pytest.mark.parametrize("graph", [False, True])
-def test_runs_behind_a_time_out(zb, oracle, case, ctas, graph):
-    """A CTA of the kernel on bands of rows that gives up a wait reports a time-out in its run, once; the runs behind it are right."""
+def test_sums_are_clean_after_a_time_out(zb, oracle, case, ctas, graph):
+    """A CTA that gives up half way through its additions reports a time-out in its run; the runs behind it are right."""
     ctx = zb.Context(0)
     g, t1, t2, cur, xv = block(zb, case)
     out = g.tensor("out", zb.F32, g.tensors[cur]["shape"])
@@ -196,3 +193,11 @@ def test_runs_behind_a_time_out(zb, oracle, case, ctas, graph):
             assert np.array_equal(plan.run(xv), want)
     plan.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("case,ctas", [((64, 160, 960, 160, 7, 7, 0, True, 1, 1), 128),          # four chunks a CTA: weights that it stops fetching; pairs of CTAs
+                                       ((148, 160, 960, 160, 4, 4, 0, True, 1, 1), 148)])        # four chunks, no cluster
+@pytest.mark.parametrize("graph", [False, True])
+def test_several_chunks_a_cta_and_a_time_out(zb, oracle, case, ctas, graph):
+    """A CTA of the kernel on bands of rows gives up its first wait: a time-out in that run, once; the runs behind it are right."""
+    test_sums_are_clean_after_a_time_out(zb, oracle, case, ctas, graph)
