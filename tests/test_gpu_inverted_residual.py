@@ -43,33 +43,33 @@ ONE = [
     (160, 96, 576, 96, 14, 14, 0, False, 2, 1),     # half a chunk at the end, CTAs with two tiles
     (485, 32, 128, 32, 7, 7, 0, True, 1, 1),        # two images a tile, an odd image, CTAs with two tiles, one chunk
     (101, 160, 960, 160, 7, 7, 0, True, 1, 1),      # two filter tiles, an odd image
-    (49, 160, 960, 320, 7, 7, -3, True, 0, 1),      # three filter tiles, input zero point
-    (33, 40, 200, 48, 14, 16, 2, True, 0, 1),
-    (33, 40, 240, 112, 5, 16, -1, False, 0, 1),     # odd rows, halves apart
-    (177, 64, 136, 16, 2, 5, 9, True, 0, 1),        # eight channels in the last chunk
+    (53, 160, 960, 320, 7, 7, -3, True, 0, 1),      # three filter tiles, input zero point
+    (65, 40, 200, 48, 14, 16, 2, True, 0, 1),
+    (61, 40, 240, 112, 5, 16, -1, False, 0, 1),     # odd rows, halves apart
+    (1037, 64, 136, 16, 2, 5, 9, True, 0, 1),       # eight channels in the last chunk
     (179, 64, 384, 64, 6, 8, 0, True, 1, 1),
-    (43, 96, 576, 160, 14, 14, 2, True, 0, 2),      # stride 2, two filter tiles
-    (77, 24, 144, 80, 12, 12, 3, False, 0, 2),      # the second half reads more rows than the first
-    (9, 8, 128, 16, 8, 10, 0, True, 0, 2),          # both halves in one accumulator
+    (47, 96, 576, 160, 14, 14, 2, True, 0, 2),      # stride 2, two filter tiles
+    (297, 24, 144, 160, 12, 12, 3, False, 0, 2),    # the second half reads more rows than the first
+    (99, 24, 128, 16, 10, 10, 0, True, 0, 2),        # both halves in one accumulator
     (185, 48, 700, 48, 5, 5, 0, True, 1, 1),        # 60 channels in the last chunk, an odd image
     (221, 64, 1100, 64, 4, 6, 0, True, 2, 1),       # nine chunks
     (185, 48, 700, 48, 5, 5, 0, True, 2, 1, "relu6"),
-    (19, 40, 128, 8, 2, 4, 4, True, 0, 1),          # widths in the kernel's steps, without and with an addition
+    (1333, 40, 128, 8, 2, 4, 4, True, 0, 1),        # widths in the kernel's steps, without and with an addition
     (275, 8, 128, 8, 2, 3, 0, True, 1, 1),
-    (21, 24, 128, 96, 3, 6, 0, True, 0, 1),
+    (221, 24, 128, 96, 3, 6, 0, True, 0, 1),
     (59, 80, 128, 80, 2, 5, 0, True, 2, 1),
-    (17, 40, 128, 48, 2, 7, 0, True, 0, 1),
+    (445, 40, 128, 48, 2, 7, 0, True, 0, 1),
     (189, 12, 128, 12, 4, 7, 1, True, 1, 1),
-    (31, 40, 128, 8, 3, 8, 0, False, 0, 1),
+    (445, 40, 128, 8, 3, 8, 0, False, 0, 1),
     (125, 8, 128, 8, 2, 8, 0, True, 1, 1),
-    (11, 40, 128, 96, 2, 10, 0, True, 0, 1),
+    (115, 72, 128, 112, 6, 10, 0, True, 0, 1),
     (99, 80, 200, 80, 13, 9, 0, True, 1, 1),
     (125, 24, 384, 24, 13, 10, 0, True, 2, 1),
-    (17, 24, 128, 16, 2, 12, 0, True, 0, 1),        # one output row a half
+    (91, 24, 640, 256, 2, 12, 0, True, 0, 1),       # one output row a half
     (105, 32, 384, 32, 11, 12, 5, True, 1, 1),
-    (9, 72, 128, 96, 4, 13, 0, True, 0, 1),
+    (75, 72, 128, 96, 4, 13, 0, True, 0, 1),
     (129, 80, 136, 80, 9, 14, 0, True, 1, 1),
-    (11, 12, 128, 160, 2, 15, 0, True, 0, 1),
+    (125, 12, 128, 160, 2, 15, 0, True, 0, 1),
     (101, 80, 256, 80, 6, 15, 0, True, 1, 1),
     (127, 12, 256, 12, 11, 16, 0, True, 1, 1),      # an odd plane
 ]

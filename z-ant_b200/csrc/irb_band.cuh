@@ -391,7 +391,8 @@ struct IrbBandPlan {
 };
 
 // Clusters of n CTAs that an SM's share of shared memory and registers lets run at once, one to three CTAs an SM (the occupancy calculator's
-// answers on a device of 148 SMs: clusters do not straddle its groups of SMs).
+// answers on a device of 148 SMs: clusters do not straddle its groups of SMs; scaled for another count).  Expected
+// times are all that they decide.
 inline int irb_band_resident(int per_sm, int n, int sm_count) {
     static const int clusters[3][9] = {{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 296, 148, 93, 71, 56, 45, 37, 33}, {0, 444, 222, 142, 104, 82, 71, 56, 48}};
     return std::max(1, (int)((long long)clusters[per_sm - 1][n] * sm_count / 148));
@@ -539,24 +540,33 @@ inline bool irb_band_prepare(const IrbBandPlan& q, const int8_t* we, const float
 //     32 -> 192 at 28 x 28: 16 images 9 / 17, 148 43 / 41; 16 -> 96 at 112 x 112, stride 2: 8 images 16 / 20, 24 38 / 34, 200 289 / 181)
 //   irb_q8.cuh: rounds of the SMs of a tile's time, which grows with its chunks (64 -> 384 at 14 x 14: 24 images 9 / 22 / 15, 64 17 / 26 / 17, 148 29 / 33 / 15;
 //     96 -> 576 at 10 x 10: 37 images 13 / 26 / 20, 100 30 / 36 / 21; stride 2: 37 images 10 / 30 / 9; 160 -> 960 at 7 x 7: 8 images 7 / 23 / 19, 37 13 / 31 / 21, 64
-//     22 / 37 / 28, 100 30 / 44 / 24; -> 320: 24 images 12 / 24 / 31, 64 31 / 32 / 25).  Without an addition this kernel has to be faster by 1.3: such blocks
-//     often have a last chunk with few channels, which costs irb_q8.cuh less than a whole one, or planes that the times here were not fitted to (1773 x 40 x
-//     7 x 7, 160 -> 96 filters 62 / - / 40, 3646 x 40 x 6 x 6, 160 -> 16 86 / 153 / 67, 238 x 40 x 9 x 9, 160 -> 96 19 / 39 / 15).  Of 231 random blocks that
-//     irb_q8.cuh takes, seven were slower by 8 to 29 % than in it without the factor, one by 9 % with it, and the others gain as much.  Of 1552 blocks, most of
-//     them random, seven are slower by 4 to 9 % than without this kernel
+//     22 / 37 / 28, 100 30 / 44 / 24; -> 320: 24 images 12 / 24 / 31, 64 31 / 32 / 25)
+//   irb_q8.cuh without an addition: blocks of any widths, fitted to 1413 of them in both kernels (rms 6 %).  A launch of irb_q8.cuh takes 2.7 us more
+//     than one of this kernel beside the rounds, a chunk K steps of the input and filters besides its rows; this kernel's results go out a word, two or one
+//     bytes at a time, which counts where filters are many beside the expanded channels and rows are not whole words (2169 x 12 x 13 x 13, 144 -> 64 filters
+//     199 / - / 112, 281 x 8 x 11 x 11, 160 -> 96 35 / - / 23).  Of 756 blocks of MobileNetV2 widths, 298 of them not among the fitted, six are slower than in
+//     irb_q8.cuh by 4 to 16 % of a plan that holds little else, and all lose 0.1 % against the better kernel of each; of 1278 random ones 25 and 0.5 %
+//     (by rounds of whole tiles as above: 17 and 0.3 %, 166 and 2.1 %)
 enum class IrbForm { kSeparate, kOne, kBand };
 inline IrbForm irb_form(const IrbPlan* one, const IrbBandPlan* band, const ConvGeom& d, bool add, bool long_add, int sm_count) {
     const bool one_pays = one && irb_pays(*one, long_add, sm_count);
     if (band) {
         const double values = 1e-6 * d.N * d.C * d.H * d.W;
-        double other = d.sh == 2 ? 9.0 + 0.87 * values : 12.0 + 1.2 * values;
+        double mine = band->us, other = d.sh == 2 ? 9.0 + 0.87 * values : 12.0 + 1.2 * values;
         if (one_pays) {
             const IrbArgs& a = one->a;
-            double tile = 2.0 + a.chunks * (1.2 + 0.25 * a.H);
-            if (a.IB == 1) tile = d.sh == 2 ? 1.0 + 3.2 * a.chunks : (long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : 2.0 + 4.1 * a.chunks) * (0.7 + 0.3 * a.H / 14.0);
-            other = ((a.tiles + sm_count - 1) / sm_count) * tile;
+            const double rounds = (a.tiles + sm_count - 1) / sm_count;
+            if (add) {
+                other = rounds * (a.IB > 1 ? 2.0 + a.chunks * (1.2 + 0.25 * a.H) : (long_add ? std::max(13.5, 2.0 + 5.0 * a.chunks) : 2.0 + 4.1 * a.chunks) * (0.7 + 0.3 * a.H / 14.0));
+            } else {
+                const IrbBandArgs& b = band->a;
+                const double h = a.H / 14.0, k = (b.C + 31) / 32, m = (b.M + 63) / 64;
+                const double tile = a.IB > 1 ? 1.3 + a.chunks * (3.2 * h + 0.1 * k + 0.12 * m) : (d.sh == 2 ? 1.75 + a.chunks * (0.9 * h + 0.25 * k + 0.16 * m) : 1.85 + a.chunks * (2.2 * h + 0.23 * k + 0.24 * m));
+                other = 2.7 + rounds * tile;
+                mine = 0.93 * mine + 1e-3 * d.N * b.M * d.OH * d.OW / sm_count * (d.OW % 4 == 0 ? 0.026 : (d.OW % 2 == 0 ? 0.1 : 0.245));
+            }
         }
-        if (band->us * (one_pays && !add ? 1.3 : 1.0) < other) return IrbForm::kBand;
+        if (mine < other) return IrbForm::kBand;
     }
     return one_pays ? IrbForm::kOne : IrbForm::kSeparate;
 }
