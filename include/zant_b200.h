@@ -151,7 +151,10 @@ int32_t zant_b200_ctx_get_tf32(zant_ctx* ctx);
 /* Caps the staging arena that host-pointer calls grow on demand (0 = no cap, the default).  A call
  * whose host buffers and workspace need more returns ZANT_E_ARENA_EXHAUSTED and changes nothing
  * (QLinearConv and QLinearMatMul run on a slower kernel without workspace where only that does not fit);
- * device-pointer calls and plans (which own their arena) are not affected.  No reference
+ * device-pointer calls and plans (which own their arena) are not affected.  Without a cap, a context whose
+ * QLinearConv calls bring weights of 256 KB to 8 MB from pageable host memory keeps, beside the arena, a copy
+ * stream and two device buffers of the largest of them (at most 16 MB) until zant_b200_ctx_destroy; while a cap
+ * is set they are neither made nor used.  No reference
  * counterpart: the reference allocates temporaries from the process heap. */
 int32_t zant_b200_ctx_set_arena_limit(zant_ctx* ctx, size_t max_bytes);
 /* The stream kernels are launched on (a cudaStream_t as void*). */
@@ -677,9 +680,9 @@ int32_t zant_b200_plan_profile(zant_plan* plan, int32_t enable);
 int32_t zant_b200_plan_profile_read(zant_plan* plan, float* sum_ms, int32_t* runs);
 /* Device pointer of a tensor's buffer (for tests that inspect intermediates).  A fused plan (`fuse` != 0) does not store every tensor:
  * for one interior to a fused step the result is NULL (here) or ZANT_E_UNSUPPORTED (zant_b200_plan_read_tensor): between a convolution and
- * the activation or pool behind it, inside the small CNN's stages, and the expanded tensors (with an addition also the projection's
- * result) of an inverted residual block that runs as one step.  Tensors that it keeps
- * channels-last between convolutions get a buffer in the graph's order at the first call that asks for theirs; every later run brings
+ * the activation or pool behind it, the quantised input of an int8 first layer that takes its QuantizeLinear along, inside the small CNN's
+ * stages, and the expanded tensors (with an addition also the projection's result) of an inverted residual block that runs as one step, which
+ * blocks on planes of any size may.  Tensors that it keeps channels-last between convolutions get a buffer in the graph's order at the first call that asks for theirs; every later run brings
  * that buffer up to date.  In TF32 mode such a tensor holds what the convolutions behind it read: values rounded to TF32 (mode 1), or the
  * sum of two TF32 parts (mode 2).  `fuse` = 0 stores every tensor in full. */
 void* zant_b200_plan_tensor_ptr(zant_plan* plan, int32_t id);

@@ -7,7 +7,8 @@
 // output: the pool is three maxima, before the requantisation as elsewhere (it does not decrease).  Filters are permuted (column n of group j is filter
 // 4 (n / 2) + 2 j + n % 2 of its 16), so that a lane's four outputs of a pixel are one word.
 // The tcgen05 form reads 16-byte pixels, twelve of them zeros, which a conversion writes first: four bytes stored and four loaded for one that counts,
-// and K rows of zeros.  32 x 3 x 416 x 416 -> 16 filters: 30 us of conversion and 48 of convolution there, 46 here (88 MB, 14 us at the rate of a copy).  What
+// and K rows of zeros.  32 x 3 x 416 x 416 -> 16 filters: 30 us of conversion and 48 of convolution there, 46 here (each kernel's own time; as steps of a plan, between
+// events, 88.0 and 51.5; 88 MB are 14 us at the rate of a copy).  What
 // bounds it is the chain of a unit - loads, sixteen MMAs of eight clocks each, maxima, conversions, table - at 24 warps an SM: 57 % of the issue slots, no
 // pipe above 40 %.  Four CTAs of 64 registers an SM 48 us, five of 48 (spills) 59; rounding by an addition of 1.5 * 2^23 instead of the conversion
 // instruction 51.
@@ -188,7 +189,7 @@ inline size_t first_q8_smem_bytes(const ConvGeom& g, int pr) { return 256 + (siz
 
 // `g`: a layer that the channels-last kernel takes with its pool (3x3, stride 1, a border of one pixel, an even image).
 // Rows of at least four units, or so few rows that all CTAs are resident at once and the launch that is saved counts.  Two launches (conversion, tcgen05
-// form) and one, us: 32 x 3 x 416 x 416, 16 filters, 88.0 and 51.5; 224 x 224, 16 / 64 filters 39.3 / 66.7 and 30.4 / 57.2; 1 x 3 x 224 x 224, 64 filters
+// form) and one, us between events: 32 x 3 x 416 x 416, 16 filters, 88.0 and 51.5; 224 x 224, 16 / 64 filters 39.3 / 66.7 and 30.4 / 57.2; 1 x 3 x 224 x 224, 64 filters
 // 23.5 and 13.5.  Narrow rows leave a warp one unit or none a band, against the filters' fragments that it loads: 500 x 3 x 64 x 64, 16 / 64 filters
 // 46.4 / 91.9 and 49.7 / 84.2, 2000 x 3 x 32 x 32, 16 filters 49.2 and 79.5.  Rows that are not whole float4s are read float by float:
 // 300 x 3 x 130 x 130, 16 filters 101.9 and 105.2 (128 x 128 97.9 and 73.2).

@@ -152,7 +152,8 @@ def fusion_groups(graph, tf32=False):
     the graph output; in TF32 mode also Conv -> Relu | LeakyRelu.  Whether the pool really joins the group is decided at
     finalize time by the kernel that takes the convolution (it needs the implicit-GEMM tiling), so groups that end in
     MaxPool are an upper bound: the plan may leave the pool as a step of its own.  The whole example CNN in QLinear form
-    (12 nodes) is recognised by the plan as four fused steps and is reported here as one group."""
+    (12 nodes) is recognised by the plan as four fused steps, up to 480 images as one, and is reported here as one group
+    whose label names the larger form."""
     readers = {}
     for n in graph.nodes:
         for t in n["inputs"]:
